@@ -7,9 +7,9 @@
 // set, which is why the reference's Dense and CellList variants share a test
 // suite).  Pipeline, all stream-ordered:
 //   count atoms per system -> per-system setup (inverse cell, widths, image
-//   counts, cell grid) -> bin atoms -> scan -> scatter -> sort each cell by
-//   particle index (deterministic order) -> count edges per lh particle ->
-//   scan -> write edges (never past capacity) -> pad the tail.
+//   counts, cell grid) -> bin atoms -> scan -> scatter -> order each cell by
+//   particle index (deterministic) -> find and write the edges of every lh
+//   particle in one pass (never past capacity) -> pad the tail.
 #include <algorithm>
 
 #include "common.cuh"
@@ -22,6 +22,8 @@ struct SysNL {
   Tril64 L;
   Tril64 inv;
   double rc2;
+  float Lf[6];
+  float lo2, hi2;  // float32 squared distance below lo2: surely inside the cutoff, at or above hi2: outside
   int nc[3];
   int nimg[3];
   int image_mode;  // prod(nimg) > 1: explicit image offsets, all system pairs are candidates
@@ -35,28 +37,32 @@ struct SysNL {
 // reference's own image replication would materialise that many copies of every pair).
 constexpr double kMaxNLImages = 1331.0;
 
+// Neighbour cells per particle.
+constexpr int kNLCells = 27;
+// Pair search: warps (particles) per block and hits a warp keeps in shared memory.
+constexpr int kPairWarps = 8, kPairStage = 512;
+
 struct NLWork {
-  SysNL *sys;
+  char *zero;           // start of the words a call zeroes first (through zero_bytes)
+  size_t zero_bytes;
+  SysNL *sys;           // [S], zeroed (n_atoms counts up)
+  unsigned *tickets;    // [4]: block counters of the setup, cell scan and pair search
+  unsigned long long *scan_state;  // [chained_scan_blocks(n_cells_cap + 1)]
+  unsigned long long *pair_state;  // [pair blocks]
+  int *cell_start;      // [n_cells_cap + 1], zeroed (counts, then starts)
   double *frac;         // [N, 3] unwrapped fractional coordinates
+  float4 *wrapped;      // [N] f - rint(f) in float32, packed rint(f) (pack_image)
   int *cell_of;         // [N] global cell id or -1
-  int *cell_start;      // [n_cells_cap + 1]
-  int *cell_fill;       // [n_cells_cap]
-  int *cell_items;      // [N]
-  int64_t *edge_off;    // [N + 1], or [27 N + 1] for the split pair search
-  bool split;           // one thread per (particle, neighbour cell): N <= kNLSplitMax
-  int64_t *scan_tmp;    // scan block sums (int64)
-  int *scan_tmp32;      // scan block sums (int32)
-  int64_t *n_cells;     // [1]
+  int *slot_of;         // [N] arrival order inside the cell
+  int *cell_any;        // [N] particles by cell, in arrival order
+  int *cell_items;      // [N] particles by cell, in index order
+  float4 *cand;         // [N] the same order: f - rint(f), particle index
+  int4 *cand_label;     // [N] the same order: inclusion, exclusion, packed rint(f)
   int64_t n_cells_cap;
+  int64_t scan_blocks, pair_blocks;
 };
 
 inline size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
-
-// Neighbour cells per particle, and the batch size up to which the pair search runs one
-// thread per (particle, neighbour cell) instead of one per particle (a single system of a
-// few thousand particles otherwise occupies a few SMs).
-constexpr int kNLCells = 27;
-constexpr int64_t kNLSplitMax = 32768;
 
 // Cells allotted: never more than max(1, 2 * atoms) per system, so the total
 // is bounded by n_systems + 2 * n_particles.
@@ -71,93 +77,139 @@ size_t layout(NLWork *w, char *base, int64_t n, int32_t s) {
   };
   const int64_t cc = cells_capacity(n, s);
   NLWork t;
+  t.scan_blocks = chained_scan_blocks(cc + 1);
+  t.pair_blocks = (n + kPairWarps - 1) / kPairWarps;
+  t.zero = base;
   t.sys = (SysNL *)take(sizeof(SysNL) * (size_t)s);
-  t.frac = (double *)take(sizeof(double) * 3 * (size_t)n);
-  t.cell_of = (int *)take(sizeof(int) * (size_t)n);
+  t.tickets = (unsigned *)take(sizeof(unsigned) * 4);
+  t.scan_state = (unsigned long long *)take(sizeof(unsigned long long) * (size_t)t.scan_blocks);
+  t.pair_state = (unsigned long long *)take(sizeof(unsigned long long) * (size_t)t.pair_blocks);
   t.cell_start = (int *)take(sizeof(int) * (size_t)(cc + 1));
-  t.cell_fill = (int *)take(sizeof(int) * (size_t)cc);
+  t.zero_bytes = off;
+  t.frac = (double *)take(sizeof(double) * 3 * (size_t)n);
+  t.wrapped = (float4 *)take(sizeof(float4) * (size_t)n);
+  t.cand = (float4 *)take(sizeof(float4) * (size_t)n);
+  t.cand_label = (int4 *)take(sizeof(int4) * (size_t)n);
+  t.cell_of = (int *)take(sizeof(int) * (size_t)n);
+  t.slot_of = (int *)take(sizeof(int) * (size_t)n);
+  t.cell_any = (int *)take(sizeof(int) * (size_t)n);
   t.cell_items = (int *)take(sizeof(int) * (size_t)n);
-  t.split = n <= kNLSplitMax;
-  const int64_t n_off = t.split ? kNLCells * n : n;
-  t.edge_off = (int64_t *)take(sizeof(int64_t) * (size_t)(n_off + 1));
-  const int64_t nb = scan_blocks_needed(std::max<int64_t>(n_off + 1, cc + 1));
-  t.scan_tmp = (int64_t *)take(sizeof(int64_t) * (size_t)nb);
-  t.scan_tmp32 = (int *)take(sizeof(int) * (size_t)nb);
-  t.n_cells = (int64_t *)take(sizeof(int64_t));
   t.n_cells_cap = cc;
   if (w) *w = t;
   return off;
 }
 
+// Atoms per system: one atomic per warp while its particles share a system (the usual grouped table).
 __global__ void count_atoms_kernel(const int32_t *system, int64_t n, int32_t s, SysNL *sys) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int32_t si = system[i];
-  if (si >= 0 && si < s) atomicAdd(&sys[si].n_atoms, 1);
+  const int32_t si = i < n ? system[i] : -1;
+  const unsigned same = __match_any_sync(0xffffffffu, si);
+  if (si >= 0 && si < s && (int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&sys[si].n_atoms, __popc(same));
 }
 
-// One block: per-system parameters and the exclusive scan of cells per system.
-__global__ void __launch_bounds__(1024) setup_systems_kernel(const double *tril, const double *cutoffs, int32_t s,
-                                     SysNL *sys, int64_t *n_cells, kups_status *status) {
+// Per-system parameters and the exclusive scan of cells per system.  Each block takes 32 systems
+// (one per lane): warps 0..2 form the width, image count and cell count of one axis each, warp 3 the
+// inverse, so the float64 divisions (a latency chain of several microseconds when one thread does
+// all of them: 11 us for one system, 19 us for 256) run side by side; the block that finishes last
+// scans the cell counts.  Measured: 5 us for one system, 7 us for 256.
+constexpr int kSetupSystems = 32;
+__global__ void __launch_bounds__(4 * kSetupSystems) setup_systems_kernel(const double *tril, const double *cutoffs,
+                                                                         int32_t s, SysNL *sys, unsigned *ticket,
+                                                                         kups_status *status) {
+  __shared__ int nimg[3][kSetupSystems], ncell[3][kSetupSystems];
   __shared__ int64_t scratch[32];
+  __shared__ unsigned done;
+  const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
+  const int k = blockIdx.x * kSetupSystems + lane;
+  const double rc = k < s ? cutoffs[k] : 0.0;
+  const bool finite = isfinite(rc);
+  if (k < s) {
+    const Tril64 L = load_tril64(tril + 6 * (int64_t)k);
+    if (role < 3) {
+      double w3[3];
+      perpendicular_widths64(L, w3);
+      const double w = role == 0 ? w3[0] : role == 1 ? w3[1] : w3[2];
+      int n = 1, c = 1;
+      if (finite) {
+        const double x = ceil(2.0 * rc / w);
+        n = x > 1e6 ? 1000001 : (int)x;
+        if (n < 1) n = 1;
+        if (n % 2 == 0) n += 1;
+        const double y = floor(w / rc);
+        c = y < 1.0 ? 1 : (y > 1024.0 ? 1024 : (int)y);
+      }
+      nimg[role][lane] = n;
+      ncell[role][lane] = c;
+    } else {
+      const Tril64 inv = inverse_tril64(L);
+      SysNL &p = sys[k];
+      p.L = L;
+      p.inv = inv;
+    }
+  }
+  __syncthreads();
+  if (role == 0 && k < s) {
+    SysNL &p = sys[k];
+    int n[3] = {nimg[0][lane], nimg[1][lane], nimg[2][lane]};
+    double prod = 1.0;
+    for (int a = 0; a < 3; ++a) prod *= (double)n[a];
+    const bool refused = prod > kMaxNLImages;
+    if (refused) {
+      status_error(status, KUPS_ERR_UNSUPPORTED, k);
+      n[0] = n[1] = n[2] = 1;
+      prod = 1.0;
+    }
+    const bool image_mode = prod > 1.0;
+    int64_t budget = 2 * (int64_t)p.n_atoms;
+    if (budget < 1) budget = 1;
+    int nc[3];
+    for (int a = 0; a < 3; ++a) nc[a] = image_mode ? 1 : ncell[a][lane];
+    while ((int64_t)nc[0] * nc[1] * nc[2] > budget) {
+      int am = 0;
+      for (int a = 1; a < 3; ++a)
+        if (nc[a] > nc[am]) am = a;
+      nc[am] = (nc[am] + 1) / 2;
+    }
+    // float32 prefilter: a fractional difference of two stored float32 coordinates is off by at most
+    // 2^-24 (plus its own rounding), the products with L and their sum by a few 2^-24 of the terms;
+    // 2^-19 sum|L| bounds the error of the distance with a factor of several to spare, and 2^-16 of
+    // the squared cutoff the rounding of its square.  Between lo2 and hi2 the float64 test decides.
+    const double rc2 = rc * rc;
+    double sum = 0.0;
+    for (int a = 0; a < 6; ++a) {
+      const double v = tril[6 * (int64_t)k + a];
+      p.Lf[a] = (float)v;
+      sum += fabs(v);
+    }
+    const double err = sum * (1.0 / 524288.0);
+    const double margin = rc2 * (1.0 / 65536.0) + 2.0 * fabs(rc) * err + err * err;
+    p.rc2 = rc2;
+    p.hi2 = finite ? (float)(rc2 + margin) : (float)rc2;
+    p.lo2 = finite ? (float)(rc2 - margin) : -1.0f;
+    for (int a = 0; a < 3; ++a) {
+      p.nimg[a] = n[a];
+      p.nc[a] = nc[a];
+    }
+    p.image_mode = image_mode;
+    p.refused = refused;
+    p.cell_base = (int64_t)nc[0] * nc[1] * nc[2];  // the count until the scan below
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) done = atomicAdd(ticket, 1u);
+  __syncthreads();
+  if (done != gridDim.x - 1) return;
+  __threadfence();
   int64_t carry = 0;
   for (int base = 0; base < s; base += blockDim.x) {
-    const int k = base + threadIdx.x;
-    int64_t cells = 0;
-    if (k < s) {
-      SysNL p = sys[k];
-      p.L = load_tril64(tril + 6 * (int64_t)k);
-      p.inv = inverse_tril64(p.L);
-      const double rc = cutoffs[k];
-      p.rc2 = rc * rc;
-      double w[3];
-      perpendicular_widths64(p.L, w);
-      const bool finite = isfinite(rc);
-      double prod = 1.0;
-      for (int a = 0; a < 3; ++a) {
-        int n = 1;
-        if (finite) {
-          const double x = ceil(2.0 * rc / w[a]);
-          n = x > 1e6 ? 1000001 : (int)x;
-          if (n < 1) n = 1;
-          if (n % 2 == 0) n += 1;
-        }
-        p.nimg[a] = n;
-        prod *= (double)n;
-      }
-      p.refused = prod > kMaxNLImages;
-      if (p.refused) {
-        status_error(status, KUPS_ERR_UNSUPPORTED, k);
-        p.nimg[0] = p.nimg[1] = p.nimg[2] = 1;
-        prod = 1.0;
-      }
-      p.image_mode = prod > 1.0;
-      int64_t budget = 2 * (int64_t)p.n_atoms;
-      if (budget < 1) budget = 1;
-      for (int a = 0; a < 3; ++a) {
-        int c = 1;
-        if (finite && !p.image_mode) {
-          const double x = floor(w[a] / rc);
-          c = x < 1.0 ? 1 : (x > 1024.0 ? 1024 : (int)x);
-        }
-        p.nc[a] = c;
-      }
-      while ((int64_t)p.nc[0] * p.nc[1] * p.nc[2] > budget) {
-        int am = 0;
-        for (int a = 1; a < 3; ++a)
-          if (p.nc[a] > p.nc[am]) am = a;
-        p.nc[am] = (p.nc[am] + 1) / 2;
-      }
-      cells = (int64_t)p.nc[0] * p.nc[1] * p.nc[2];
-      sys[k] = p;
-    }
+    const int q = base + threadIdx.x;
+    const int64_t cells = q < s ? __ldcg(reinterpret_cast<const long long *>(&sys[q].cell_base)) : 0;
     int64_t chunk;
     const int64_t ex = block_exclusive_scan<int64_t>(cells, scratch, &chunk);
-    if (k < s) sys[k].cell_base = carry + ex;
+    if (q < s) sys[q].cell_base = carry + ex;
     carry += chunk;
     __syncthreads();
   }
-  if (threadIdx.x == 0) *n_cells = carry;
 }
 
 __device__ inline int wrap_cell(double f, int nc) {
@@ -166,8 +218,21 @@ __device__ inline int wrap_cell(double f, int nc) {
   return c >= nc ? nc - 1 : (c < 0 ? 0 : c);
 }
 
-__global__ void bin_kernel(const double *positions, const int32_t *system, int64_t n, int32_t s,
-                           const SysNL *sys, double *frac, int *cell_of, int *cell_count) {
+// rint(f) of the three axes in 10 bits each (offset 512); kWideImage marks one outside [-512, 511].
+constexpr int kWideImage = 1 << 30;
+__device__ inline int pack_image(const double n[3]) {
+  int v = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if (!(n[a] >= -512.0 && n[a] <= 511.0)) return kWideImage;
+    v |= ((int)n[a] + 512) << (10 * a);
+  }
+  return v;
+}
+__device__ inline int image_axis(int packed, int a) { return ((packed >> (10 * a)) & 1023) - 512; }
+
+__global__ void bin_kernel(const double *positions, const int32_t *system, int64_t n, int32_t s, const SysNL *sys,
+                           double *frac, float4 *wrapped, int *cell_of, int *slot_of, int *cell_count) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int32_t si = system[i];
@@ -177,41 +242,50 @@ __global__ void bin_kernel(const double *positions, const int32_t *system, int64
   }
   const SysNL &p = sys[si];
   const double r[3] = {positions[3 * i], positions[3 * i + 1], positions[3 * i + 2]};
-  double f[3];
+  double f[3], img[3];
   row_times_tril64(r, p.inv, f);
-  frac[3 * i] = f[0];
-  frac[3 * i + 1] = f[1];
-  frac[3 * i + 2] = f[2];
+  float w[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    frac[3 * i + a] = f[a];
+    img[a] = rint(f[a]);
+    w[a] = (float)(f[a] - img[a]);
+  }
+  wrapped[i] = make_float4(w[0], w[1], w[2], __int_as_float(pack_image(img)));
   const int cx = wrap_cell(f[0], p.nc[0]), cy = wrap_cell(f[1], p.nc[1]),
             cz = wrap_cell(f[2], p.nc[2]);
   const int c = (int)p.cell_base + (cz * p.nc[1] + cy) * p.nc[0] + cx;
   cell_of[i] = c;
-  atomicAdd(&cell_count[c], 1);
+  slot_of[i] = atomicAdd(&cell_count[c], 1);
 }
 
-__global__ void scatter_kernel(const int *cell_of, int64_t n, const int *cell_start,
-                               int *cell_fill, int *cell_items) {
+__global__ void scatter_kernel(const int *cell_of, const int *slot_of, int64_t n, const int *cell_start,
+                               int *cell_any) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int c = cell_of[i];
+  if (c >= 0) cell_any[cell_start[c] + slot_of[i]] = (int)i;
+}
+
+// A particle's place in its cell is the number of smaller indices in it: each cell ends up in index
+// order whatever the arrival order, with one thread per particle (an insertion sort by one thread
+// per cell took 945 us for 4000 particles in 27 cells, this 9 us).  Writes the candidate records of
+// the pair search in that order.
+__global__ void order_cells_kernel(const int *cell_of, int64_t n, const int *cell_start, const int *cell_any,
+                                   const float4 *wrapped, const int32_t *inclusion, const int32_t *exclusion,
+                                   int *cell_items, float4 *cand, int4 *cand_label) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int c = cell_of[i];
   if (c < 0) return;
-  const int slot = atomicAdd(&cell_fill[c], 1);
-  cell_items[cell_start[c] + slot] = (int)i;
-}
-
-__global__ void sort_cells_kernel(const int *cell_start, const int64_t *n_cells, int *items) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= *n_cells) return;
   const int b = cell_start[c], e = cell_start[c + 1];
-  for (int k = b + 1; k < e; ++k) {
-    const int v = items[k];
-    int m = k - 1;
-    while (m >= b && items[m] > v) {
-      items[m + 1] = items[m];
-      --m;
-    }
-    items[m + 1] = v;
-  }
+  int r = b;
+#pragma unroll 8
+  for (int k = b; k < e; ++k) r += cell_any[k] < (int)i;
+  cell_items[r] = (int)i;
+  const float4 w = wrapped[i];
+  cand[r] = make_float4(w.x, w.y, w.z, __int_as_float((int)i));
+  cand_label[r] = make_int4(inclusion[i], exclusion[i], __float_as_int(w.w), 0);
 }
 
 // Candidate test of the reference for the pair (i, j) and offset o.
@@ -244,114 +318,289 @@ __device__ inline bool edge_test(const SysNL &p, const double fi[3], const doubl
   return true;
 }
 
-// One thread per particle, or with SPLIT one thread per (particle, neighbour cell): thread
-// a n + i scans cell a = (az * 3 + ay) * 3 + ax of particle i's (up to) 3 x 3 x 3 cells, so
-// that a batch of few particles still fills the GPU, and the lanes of a warp (consecutive,
-// cell-sorted particles) scan the same relative cell in step.  Offsets are kept at 27 i + a,
-// the (particle, az, ay, ax) order of the per-particle form's loops, so both forms write the
-// same edges in the same order.
-template <bool WRITE, bool SPLIT>
-__global__ void pairs_kernel(const int32_t *system, const int32_t *inclusion,
-                             const int32_t *exclusion, int64_t n, int32_t n_incl, int32_t s,
-                             const SysNL *sys, const double *frac, const int *cell_of,
-                             const int *cell_start, const int *cell_items, int64_t *edge_off,
-                             int32_t *edges, int32_t *shifts, int64_t cap) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (SPLIT ? kNLCells * n : n)) return;
-  const int a_only = SPLIT ? (int)(t / n) : -1;
-  const int64_t i = SPLIT ? t - (int64_t)a_only * n : t;
-  const int64_t slot = SPLIT ? i * kNLCells + a_only : i;  // this thread's offset entry
-  const int32_t si = system[i];
-  const int32_t inc = inclusion[i];
-  int64_t count = 0;
-  int64_t out = WRITE ? edge_off[slot] : 0;
-  if (si >= 0 && si < s && inc >= 0 && inc < n_incl && !sys[si].refused) {
-    const SysNL p = sys[si];
-    const double fi[3] = {frac[3 * i], frac[3 * i + 1], frac[3 * i + 2]};
-    const int32_t exi = exclusion[i];
-    const int ci = cell_of[i] - (int)p.cell_base;
-    const int cx = ci % p.nc[0], cy = (ci / p.nc[0]) % p.nc[1], cz = ci / (p.nc[0] * p.nc[1]);
-    // Distinct neighbour cells per axis (1, 2 or 3 of them).
-    int lx[3], ly[3], lz[3], nx, ny, nz;
-    auto axis = [](int c, int nc, int *l, int &m) {
-      if (nc == 1) {
-        l[0] = 0;
-        m = 1;
-      } else if (nc == 2) {
-        l[0] = 0;
-        l[1] = 1;
-        m = 2;
-      } else {
-        l[0] = (c + nc - 1) % nc;
-        l[1] = c;
-        l[2] = (c + 1) % nc;
-        m = 3;
+// The candidates of one particle: up to 27 cells, each a contiguous run of the cell-ordered records,
+// read as one flat range of `total` candidates in (cell, index) order.
+struct CandRange {
+  int pre[kNLCells + 1];  // exclusive prefix of the run lengths
+  int start[kNLCells];    // first record of the run minus its prefix
+};
+
+// Scans the candidates (times the image offsets) of particle i, a lane per candidate, in the order
+// of the reference: cells, then particle index, then offsets.  The float32 distance settles nearly
+// every candidate; within the margin of the cutoff, within 2^-18 of half a cell (the rounding of the
+// image shift), for image counts beyond 10 bits and for excluded pairs among image offsets the exact
+// float64 test decides, so the edge set is that of the float64 test alone.  Returns the number of
+// edges; with DIRECT they are written from row `out` on, else the first kPairStage are kept in `stage`
+// (wide: some shift does not fit its 10 bits).
+template <bool DIRECT>
+__device__ int scan_particle(const SysNL &p, int i, const float4 &wi, int inc, int exi, const CandRange &rg, int total,
+                             const float4 *cand, const int4 *label, const double *frac, uint2 *stage, bool &wide,
+                             int64_t out, int32_t *edges, int32_t *shifts, int64_t cap) {
+  const int lane = threadIdx.x & 31;
+  const float L0 = p.Lf[0], L1 = p.Lf[1], L2 = p.Lf[2], L3 = p.Lf[3], L4 = p.Lf[4], L5 = p.Lf[5];
+  const float hi2 = p.hi2, lo2 = p.lo2;
+  const int wn = __float_as_int(wi.w);
+  int cnt = 0;
+  bool too_wide = false;
+  // appends the hits of the 32 lanes in lane order
+  auto append = [&](bool hit, int j, int sx, int sy, int sz) {
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (hit) {
+      const int at = cnt + __popc(m & ((1u << lane) - 1u));
+      if (DIRECT) {
+        const int64_t o = out + at;
+        if (o < cap) {
+          edges[2 * o] = i;
+          edges[2 * o + 1] = j;
+          shifts[3 * o] = sx;
+          shifts[3 * o + 1] = sy;
+          shifts[3 * o + 2] = sz;
+        }
+      } else if (at < kPairStage) {
+        too_wide |= sx < -512 || sx > 511 || sy < -512 || sy > 511 || sz < -512 || sz > 511;
+        stage[at] = make_uint2((unsigned)j, (unsigned)((sx + 512) | ((sy + 512) << 10) | ((sz + 512) << 20)));
       }
-    };
-    axis(cx, p.nc[0], lx, nx);
-    axis(cy, p.nc[1], ly, ny);
-    axis(cz, p.nc[2], lz, nz);
-    const int hx = (p.nimg[0] - 1) / 2, hy = (p.nimg[1] - 1) / 2, hz = (p.nimg[2] - 1) / 2;
-    for (int az = 0; az < nz; ++az)
-      for (int ay = 0; ay < ny; ++ay)
-        for (int ax = 0; ax < nx; ++ax) {
-          if (SPLIT && (az * 3 + ay) * 3 + ax != a_only) continue;
-          const int c = (int)p.cell_base + (lz[az] * p.nc[1] + ly[ay]) * p.nc[0] + lx[ax];
-          const int b = cell_start[c], e = cell_start[c + 1];
-          for (int k = b; k < e; ++k) {
-            const int j = cell_items[k];
-            if (inclusion[j] != inc) continue;
-            const double fj[3] = {frac[3 * j], frac[3 * j + 1], frac[3 * j + 2]};
-            const bool same_ex = exclusion[j] == exi;
-            int sh[3];
-            if (!p.image_mode) {
+    }
+    cnt += __popc(m);
+  };
+  auto exact = [&](int j, const int o[3], bool image, bool same_ex, int sh[3]) {
+    const double fi[3] = {frac[3 * (int64_t)i], frac[3 * (int64_t)i + 1], frac[3 * (int64_t)i + 2]};
+    const double fj[3] = {frac[3 * (int64_t)j], frac[3 * (int64_t)j + 1], frac[3 * (int64_t)j + 2]};
+    return edge_test(p, fi, fj, o, image, sh, same_ex);
+  };
+  if (!p.image_mode) {
+    constexpr float kHalf = 0.5f - 1.0f / 262144.0f;
+    int a = 0;
+    for (int base = 0; base < total; base += 32) {
+      const int idx = base + lane;
+      bool hit = false;
+      int j = 0, sh[3] = {0, 0, 0};
+      if (idx < total) {
+        while (idx >= rg.pre[a + 1]) ++a;
+        const int k = rg.start[a] + idx;
+        const float4 c = cand[k];
+        float dx = wi.x - c.x, dy = wi.y - c.y, dz = wi.z - c.z;
+        const float rx = rintf(dx), ry = rintf(dy), rz = rintf(dz);
+        dx -= rx;
+        dy -= ry;
+        dz -= rz;
+        const float X = fmaf(dz, L3, fmaf(dy, L1, dx * L0)), Y = fmaf(dz, L4, dy * L2), Z = dz * L5;
+        const float d2 = fmaf(Z, Z, fmaf(Y, Y, X * X));
+        if (d2 < hi2) {
+          const int4 lb = label[k];
+          j = __float_as_int(c.w);
+          if (lb.x == inc) {
+            const bool same_ex = lb.y == exi;
+            if (!(d2 < lo2) || fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) > kHalf || ((wn | lb.z) & kWideImage)) {
               const int o[3] = {0, 0, 0};
-              if (edge_test(p, fi, fj, o, false, sh, same_ex)) {
-                if (WRITE && out < cap) {
-                  edges[2 * out] = (int32_t)i;
-                  edges[2 * out + 1] = j;
-                  shifts[3 * out] = sh[0];
-                  shifts[3 * out + 1] = sh[1];
-                  shifts[3 * out + 2] = sh[2];
-                }
-                ++out;
-                ++count;
-              }
+              hit = exact(j, o, false, same_ex, sh);
             } else {
-              for (int ox = -hx; ox <= hx; ++ox)
-                for (int oy = -hy; oy <= hy; ++oy)
-                  for (int oz = -hz; oz <= hz; ++oz) {
-                    const int o[3] = {ox, oy, oz};
-                    if (edge_test(p, fi, fj, o, true, sh, same_ex)) {
-                      if (WRITE && out < cap) {
-                        edges[2 * out] = (int32_t)i;
-                        edges[2 * out + 1] = j;
-                        shifts[3 * out] = sh[0];
-                        shifts[3 * out + 1] = sh[1];
-                        shifts[3 * out + 2] = sh[2];
-                      }
-                      ++out;
-                      ++count;
-                    }
-                  }
+              hit = !same_ex;  // the shift is the minimum image
+              sh[0] = image_axis(wn, 0) - image_axis(lb.z, 0) + (int)rx;
+              sh[1] = image_axis(wn, 1) - image_axis(lb.z, 1) + (int)ry;
+              sh[2] = image_axis(wn, 2) - image_axis(lb.z, 2) + (int)rz;
             }
           }
         }
+      }
+      append(hit, j, sh[0], sh[1], sh[2]);
+    }
+  } else {
+    // one cell; (candidate, x, y, z offset) as a mixed-radix counter that every lane steps by 32
+    const int n1 = p.nimg[1], n2 = p.nimg[2], n0 = p.nimg[0];
+    const int step_z = 32 % n2, step_y = (32 / n2) % n1, step_x = (32 / n2 / n1) % n0, step_c = 32 / n2 / n1 / n0;
+    int oz = lane % n2, oy = (lane / n2) % n1, ox = (lane / n2 / n1) % n0;
+    int64_t c = lane / n2 / n1 / n0;
+    while (__any_sync(0xffffffffu, c < total)) {
+      bool hit = false;
+      int j = 0, sh[3] = {0, 0, 0};
+      if (c < total) {
+        const int k = rg.start[0] + (int)c;
+        const float4 q = cand[k];
+        const int4 lb = label[k];
+        j = __float_as_int(q.w);
+        if (lb.x == inc) {
+          const int o[3] = {ox - (n0 - 1) / 2, oy - (n1 - 1) / 2, oz - (n2 - 1) / 2};
+          const bool same_ex = lb.y == exi;
+          bool sure = !((wn | lb.z) & kWideImage);
+          if (sure) {
+            const float dx = (wi.x - q.x) + (float)(image_axis(wn, 0) - image_axis(lb.z, 0) - o[0]);
+            const float dy = (wi.y - q.y) + (float)(image_axis(wn, 1) - image_axis(lb.z, 1) - o[1]);
+            const float dz = (wi.z - q.z) + (float)(image_axis(wn, 2) - image_axis(lb.z, 2) - o[2]);
+            const float X = fmaf(dz, L3, fmaf(dy, L1, dx * L0)), Y = fmaf(dz, L4, dy * L2), Z = dz * L5;
+            const float d2 = fmaf(Z, Z, fmaf(Y, Y, X * X));
+            if (d2 < hi2) {
+              sure = d2 < lo2 && !same_ex;
+              hit = sure;
+              sh[0] = o[0];
+              sh[1] = o[1];
+              sh[2] = o[2];
+            }
+          }
+          if (!sure) hit = exact(j, o, true, same_ex, sh);
+        }
+      }
+      append(hit, j, sh[0], sh[1], sh[2]);
+      c += step_c;
+      oz += step_z;
+      oy += step_y;
+      ox += step_x;
+      if (oz >= n2) {
+        oz -= n2;
+        ++oy;
+      }
+      if (oy >= n1) {
+        oy -= n1;
+        ++ox;
+      }
+      if (ox >= n0) {
+        ox -= n0;
+        ++c;
+      }
+    }
   }
-  if (!WRITE) edge_off[slot] = count;
+  wide = __any_sync(0xffffffffu, too_wide);
+  return cnt;
+}
+
+// The edge list in one pass: a warp per particle (index order) finds its edges into shared memory,
+// the block's count joins the chained prefix over blocks, and the rows are written at their final
+// place with coalesced stores.  A particle with more than kPairStage edges is scanned again to write
+// them.  Bounded by issue: about 45 instructions per 32 candidates.  With the float64 test per
+// candidate (30 operations at 2 per clock per SM, one thread per particle, a counting and a writing
+// pass) 264 k particles in 256 systems took 19.3 ms; see the figures at the launch.
+__global__ void __launch_bounds__(32 * kPairWarps) pairs_kernel(
+    const int32_t *system, const int32_t *inclusion, const int32_t *exclusion, int64_t n, int32_t n_incl, int32_t s,
+    const SysNL *sys, const double *frac, const float4 *wrapped, const int *cell_of, const int *cell_start,
+    const float4 *cand, const int4 *label, unsigned *ticket, unsigned long long *state, int64_t *n_edges,
+    int32_t *edges, int32_t *shifts, int64_t cap, kups_status *status) {
+  __shared__ uint2 stage_all[kPairWarps][kPairStage];
+  __shared__ CandRange ranges[kPairWarps];
+  __shared__ int counts[kPairWarps];
+  __shared__ int64_t base;
+  __shared__ unsigned bid;
+  __shared__ bool chained;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) bid = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const int64_t i = (int64_t)bid * kPairWarps + warp;
+  uint2 *stage = stage_all[warp];
+  CandRange &rg = ranges[warp];
+  const int32_t si = i < n ? system[i] : -1, inc = i < n ? inclusion[i] : -1;
+  const bool on = si >= 0 && si < s && inc >= 0 && inc < n_incl && !sys[si].refused;
+  int cnt = 0, total = 0, exi = 0;
+  bool wide = false;
+  float4 wi = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (on) {  // the same for the whole warp
+    const SysNL &p = sys[si];
+    wi = wrapped[i];
+    exi = exclusion[i];
+    int first = 0, len = 0;
+    if (lane < kNLCells) {
+      const int nx = p.nc[0], ny = p.nc[1], nz = p.nc[2];
+      const int ci = cell_of[i] - (int)p.cell_base;
+      const int cx = ci % nx, cy = (ci / nx) % ny, cz = ci / (nx * ny);
+      // the distinct neighbour cells of an axis (1, 2 or 3 of them), in this order
+      auto axis = [](int c, int nc, int t, int &out) {
+        if (t >= min(nc, 3)) return false;
+        out = nc <= 2 ? t : (c + nc - 1 + t) % nc;
+        return true;
+      };
+      int x, y, z;
+      if (axis(cx, nx, lane % 3, x) && axis(cy, ny, (lane / 3) % 3, y) && axis(cz, nz, lane / 9, z)) {
+        const int c = (int)p.cell_base + (z * ny + y) * nx + x;
+        first = cell_start[c];
+        len = cell_start[c + 1] - first;
+      }
+    }
+    int sum = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    total = __shfl_sync(0xffffffffu, sum, 31);
+    if (lane < kNLCells) {
+      rg.pre[lane] = sum - len;
+      rg.start[lane] = first - (sum - len);
+    }
+    if (lane == kNLCells) rg.pre[kNLCells] = total;
+    __syncwarp();
+    cnt = scan_particle<false>(p, (int)i, wi, inc, exi, rg, total, cand, label, frac, stage, wide, 0, edges, shifts,
+                               cap);
+  }
+  if (lane == 0) counts[warp] = cnt;
+  __syncthreads();
+  if (warp == 0) {
+    int own = 0;
+#pragma unroll
+    for (int k = 0; k < kPairWarps; ++k) own += counts[k];
+    bool ok;
+    const int64_t before = chained_prefix(state, bid, own, ok);
+    if (lane == 0) {
+      base = before;
+      chained = ok;
+      if (!ok) status_error(status, KUPS_ERR_UNSUPPORTED, bid);
+      if (bid == gridDim.x - 1) {
+        const int64_t all = ok ? before + own : 0;
+        *n_edges = all;
+        if (all > cap) status_capacity(status, KUPS_CAP_EDGES, all, -1);
+      }
+    }
+  }
+  __syncthreads();
+  if (!chained || cnt == 0) return;
+  int64_t out = base;
+  for (int k = 0; k < warp; ++k) out += counts[k];
+  if (cnt > kPairStage || wide) {
+    scan_particle<true>(sys[si], (int)i, wi, inc, exi, rg, total, cand, label, frac, stage, wide, out, edges, shifts,
+                        cap);
+    return;
+  }
+  const int rows = (int)max((int64_t)0, min((int64_t)cnt, cap - out));
+  for (int t = lane; t < 2 * rows; t += 32) edges[2 * out + t] = (t & 1) ? (int)stage[t >> 1].x : (int)i;
+  for (int t = lane; t < 3 * rows; t += 32) {
+    const int e = t / 3;
+    shifts[3 * out + t] = image_axis((int)stage[e].y, t - 3 * e);
+  }
 }
 
 __global__ void check_capacity_kernel(const int64_t *n_edges, int64_t cap, kups_status *st) {
   if (*n_edges > cap) status_capacity(st, KUPS_CAP_EDGES, *n_edges, -1);
 }
 
+// Rows [n_edges, cap) hold index n and a zero shift; a fixed grid walks from the first of them, so a
+// nearly full list costs nothing.
 __global__ void pad_kernel(const int64_t *n_edges, int64_t cap, int64_t n, int32_t *edges,
                            int32_t *shifts) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= cap || e < *n_edges) return;
-  edges[2 * e] = (int32_t)n;
-  edges[2 * e + 1] = (int32_t)n;
-  shifts[3 * e] = shifts[3 * e + 1] = shifts[3 * e + 2] = 0;
+  const int64_t first = *n_edges, step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t t = 2 * first + t0; t < 2 * cap; t += step) edges[t] = (int32_t)n;
+  for (int64_t t = 3 * first + t0; t < 3 * cap; t += step) shifts[t] = 0;
+}
+
+inline unsigned pad_blocks(int64_t cap) {
+  return (unsigned)std::min<int64_t>((cap + 255) / 256, 8 * (int64_t)device_sm_count());
+}
+
+// Cells, candidate records and per-system parameters of a particle table (both searches start here).
+cudaError_t bin_particles(const NLWork &w, const double *positions, const int32_t *system, const int32_t *inclusion,
+                          const int32_t *exclusion, int64_t n, const double *tril, const double *cutoffs, int32_t s,
+                          kups_status *status, cudaStream_t stream) {
+  const unsigned gb = (unsigned)((n + 255) / 256);
+  cudaError_t e = cudaMemsetAsync(w.zero, 0, w.zero_bytes, stream);
+  if (e != cudaSuccess) return e;
+  count_atoms_kernel<<<gb, 256, 0, stream>>>(system, n, s, w.sys);
+  setup_systems_kernel<<<(unsigned)((s + kSetupSystems - 1) / kSetupSystems), 4 * kSetupSystems, 0, stream>>>(
+      tril, cutoffs, s, w.sys, w.tickets, status);
+  bin_kernel<<<gb, 256, 0, stream>>>(positions, system, n, s, w.sys, w.frac, w.wrapped, w.cell_of, w.slot_of,
+                                     w.cell_start);
+  chained_scan_kernel<<<(unsigned)w.scan_blocks, kChainedThreads, 0, stream>>>(w.cell_start, w.n_cells_cap + 1,
+                                                                               w.scan_state, w.tickets + 1, status);
+  scatter_kernel<<<gb, 256, 0, stream>>>(w.cell_of, w.slot_of, n, w.cell_start, w.cell_any);
+  order_cells_kernel<<<gb, 256, 0, stream>>>(w.cell_of, n, w.cell_start, w.cell_any, w.wrapped, inclusion, exclusion,
+                                             w.cell_items, w.cand, w.cand_label);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -376,46 +625,16 @@ extern "C" int32_t kups_neighborlist_build(const double *positions, const int32_
   char *base = (char *)(((uintptr_t)workspace + 255) & ~uintptr_t(255));
   NLWork w;
   layout(&w, base, n, s);
-  KUPS_CUDA_TRY(cudaMemsetAsync(n_edges, 0, sizeof(int64_t), stream));
   if (s == 0 || n == 0) {
-    if (cap > 0)
-      pad_kernel<<<(unsigned)((cap + 255) / 256), 256, 0, stream>>>(n_edges, cap, n, edges, shifts);
+    KUPS_CUDA_TRY(cudaMemsetAsync(n_edges, 0, sizeof(int64_t), stream));
+    if (cap > 0) pad_kernel<<<pad_blocks(cap), 256, 0, stream>>>(n_edges, cap, n, edges, shifts);
     return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
   }
-  const unsigned gb = (unsigned)((n + 255) / 256);
-  KUPS_CUDA_TRY(cudaMemsetAsync(w.sys, 0, sizeof(SysNL) * s, stream));
-  KUPS_CUDA_TRY(cudaMemsetAsync(w.cell_start, 0, sizeof(int) * (w.n_cells_cap + 1), stream));
-  KUPS_CUDA_TRY(cudaMemsetAsync(w.cell_fill, 0, sizeof(int) * w.n_cells_cap, stream));
-  count_atoms_kernel<<<gb, 256, 0, stream>>>(system, n, s, w.sys);
-  setup_systems_kernel<<<1, 1024, 0, stream>>>(tril, cutoffs, s, w.sys, w.n_cells, status);
-  bin_kernel<<<gb, 256, 0, stream>>>(positions, system, n, s, w.sys, w.frac, w.cell_of,
-                                     w.cell_start);
-  KUPS_CUDA_TRY(exclusive_scan<int>(w.cell_start, w.n_cells_cap + 1, w.scan_tmp32, nullptr, stream));
-  scatter_kernel<<<gb, 256, 0, stream>>>(w.cell_of, n, w.cell_start, w.cell_fill, w.cell_items);
-  sort_cells_kernel<<<(unsigned)((w.n_cells_cap + 255) / 256), 256, 0, stream>>>(
-      w.cell_start, w.n_cells, w.cell_items);
-  const int64_t n_thr = w.split ? kNLCells * n : n;
-  const unsigned gp = (unsigned)((n_thr + 127) / 128);
-  if (w.split)
-    pairs_kernel<false, true><<<gp, 128, 0, stream>>>(system, inclusion, exclusion, n, n_incl, s, w.sys, w.frac,
-                                                      w.cell_of, w.cell_start, w.cell_items, w.edge_off, edges,
-                                                      shifts, cap);
-  else
-    pairs_kernel<false, false><<<gp, 128, 0, stream>>>(system, inclusion, exclusion, n, n_incl, s, w.sys, w.frac,
-                                                       w.cell_of, w.cell_start, w.cell_items, w.edge_off, edges,
-                                                       shifts, cap);
-  KUPS_CUDA_TRY(exclusive_scan<int64_t>(w.edge_off, n_thr, w.scan_tmp, n_edges, stream));
-  if (w.split)
-    pairs_kernel<true, true><<<gp, 128, 0, stream>>>(system, inclusion, exclusion, n, n_incl, s, w.sys, w.frac,
-                                                     w.cell_of, w.cell_start, w.cell_items, w.edge_off, edges,
-                                                     shifts, cap);
-  else
-    pairs_kernel<true, false><<<gp, 128, 0, stream>>>(system, inclusion, exclusion, n, n_incl, s, w.sys, w.frac,
-                                                      w.cell_of, w.cell_start, w.cell_items, w.edge_off, edges,
-                                                      shifts, cap);
-  check_capacity_kernel<<<1, 1, 0, stream>>>(n_edges, cap, status);
-  if (cap > 0)
-    pad_kernel<<<(unsigned)((cap + 255) / 256), 256, 0, stream>>>(n_edges, cap, n, edges, shifts);
+  KUPS_CUDA_TRY(bin_particles(w, positions, system, inclusion, exclusion, n, tril, cutoffs, s, status, stream));
+  pairs_kernel<<<(unsigned)w.pair_blocks, 32 * kPairWarps, 0, stream>>>(
+      system, inclusion, exclusion, n, n_incl, s, w.sys, w.frac, w.wrapped, w.cell_of, w.cell_start, w.cand,
+      w.cand_label, w.tickets + 2, w.pair_state, n_edges, edges, shifts, cap, status);
+  if (cap > 0) pad_kernel<<<pad_blocks(cap), 256, 0, stream>>>(n_edges, cap, n, edges, shifts);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 
@@ -645,23 +864,14 @@ extern "C" int32_t kups_neighborlist_build_rh(
   rh_layout(&w, base, n_lh, n_rh, s);
   KUPS_CUDA_TRY(cudaMemsetAsync(n_edges, 0, sizeof(int64_t), stream));
   if (s == 0 || n_lh == 0 || n_rh == 0) {
-    if (cap > 0) pad_kernel<<<(unsigned)((cap + 255) / 256), 256, 0, stream>>>(n_edges, cap, oob, edges, shifts);
+    if (cap > 0) pad_kernel<<<pad_blocks(cap), 256, 0, stream>>>(n_edges, cap, oob, edges, shifts);
     return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
   }
   const int64_t n = n_lh;
-  const unsigned gb = (unsigned)((n + 255) / 256);
   NLWork &l = w.lh;
-  KUPS_CUDA_TRY(cudaMemsetAsync(l.sys, 0, sizeof(SysNL) * s, stream));
-  KUPS_CUDA_TRY(cudaMemsetAsync(l.cell_start, 0, sizeof(int) * (l.n_cells_cap + 1), stream));
-  KUPS_CUDA_TRY(cudaMemsetAsync(l.cell_fill, 0, sizeof(int) * l.n_cells_cap, stream));
   KUPS_CUDA_TRY(cudaMemsetAsync(w.in_remap, 0, (size_t)std::max<int64_t>(n, 1), stream));
-  count_atoms_kernel<<<gb, 256, 0, stream>>>(lh_system, n, s, l.sys);
-  setup_systems_kernel<<<1, 1024, 0, stream>>>(tril, cutoffs, s, l.sys, l.n_cells, status);
-  bin_kernel<<<gb, 256, 0, stream>>>(lh_positions, lh_system, n, s, l.sys, l.frac, l.cell_of, l.cell_start);
-  KUPS_CUDA_TRY(exclusive_scan<int>(l.cell_start, l.n_cells_cap + 1, l.scan_tmp32, nullptr, stream));
-  scatter_kernel<<<gb, 256, 0, stream>>>(l.cell_of, n, l.cell_start, l.cell_fill, l.cell_items);
-  sort_cells_kernel<<<(unsigned)((l.n_cells_cap + 255) / 256), 256, 0, stream>>>(l.cell_start, l.n_cells,
-                                                                                 l.cell_items);
+  KUPS_CUDA_TRY(bin_particles(l, lh_positions, lh_system, lh_inclusion, lh_exclusion, n, tril, cutoffs, s, status,
+                              stream));
   if (rh_index_remap != nullptr)
     mark_remap_kernel<<<(unsigned)((n_rh + 255) / 256), 256, 0, stream>>>(rh_index_remap, n_rh, n, w.in_remap);
   const unsigned gr = (unsigned)((n_rh + 127) / 128);
@@ -675,7 +885,7 @@ extern "C" int32_t kups_neighborlist_build_rh(
                                                 s, l.sys, l.frac, l.cell_start, l.cell_items, w.rh_off, oob, edges,
                                                 shifts, cap);
   check_capacity_kernel<<<1, 1, 0, stream>>>(n_edges, cap, status);
-  if (cap > 0) pad_kernel<<<(unsigned)((cap + 255) / 256), 256, 0, stream>>>(n_edges, cap, oob, edges, shifts);
+  if (cap > 0) pad_kernel<<<pad_blocks(cap), 256, 0, stream>>>(n_edges, cap, oob, edges, shifts);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 

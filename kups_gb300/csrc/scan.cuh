@@ -55,4 +55,106 @@ inline cudaError_t exclusive_scan(T *data, int64_t n, T *block_sums, T *total, c
   return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------- single-pass prefix
+// Chained prefix over blocks that take their numbers from a ticket (a block's predecessors have
+// therefore started before it): state[b] holds a 2-bit flag above a 62-bit value, 0 = nothing yet,
+// 1 = the block's own sum, 2 = the sum of blocks 0..b, 3 = a predecessor's wait ran out.  The words
+// must be zero before the launch.  One full warp per block calls this; every lane returns the sum of
+// blocks 0..b-1.  The wait for a predecessor is bounded: when it runs out the block publishes flag 3,
+// so no later block waits on it, and ok comes back false.
+constexpr int kPrefixPolls = 1 << 22;
+
+__device__ inline unsigned long long prefix_load(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ inline void prefix_store(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__device__ inline int64_t chained_prefix(unsigned long long *state, int64_t b, int64_t own, bool &ok) {
+  const int lane = threadIdx.x & 31;
+  constexpr unsigned long long kValue = (1ull << 62) - 1;
+  ok = true;
+  if (b == 0) {
+    if (lane == 0) prefix_store(state, (2ull << 62) | (unsigned long long)own);
+    return 0;
+  }
+  if (lane == 0) prefix_store(state + b, (1ull << 62) | (unsigned long long)own);
+  int64_t sum = 0;
+  for (int64_t top = b - 1;; top -= 32) {
+    const int64_t at = top - lane;
+    unsigned long long v = at >= 0 ? prefix_load(state + at) : (2ull << 62);
+    for (int polls = 0; __any_sync(0xffffffffu, (v >> 62) == 0); ++polls) {
+      if (polls == kPrefixPolls) {
+        if (lane == 0) prefix_store(state + b, 3ull << 62);
+        ok = false;
+        return 0;
+      }
+      __nanosleep(20);
+      if ((v >> 62) == 0) v = prefix_load(state + at);
+    }
+    const unsigned last = __ballot_sync(0xffffffffu, (v >> 62) >= 2);
+    const int stop = last ? __ffs(last) - 1 : 31;
+    if (__shfl_sync(0xffffffffu, (unsigned)(v >> 62), stop) == 3u) {
+      if (lane == 0) prefix_store(state + b, 3ull << 62);
+      ok = false;
+      return 0;
+    }
+    int64_t part = lane <= stop ? (int64_t)(v & kValue) : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    sum += part;
+    if (last) break;
+  }
+  if (lane == 0) prefix_store(state + b, (2ull << 62) | (unsigned long long)(sum + own));
+  return sum;
+}
+
+// In-place exclusive scan of data[0..n) in one launch (kScanItems entries per thread): 2 launches
+// and one read of the data fewer than exclusive_scan.  state: chained_scan_blocks(n) zeroed words,
+// ticket: a zeroed word.
+constexpr int kScanItems = 4, kChainedThreads = 512;
+
+inline int64_t chained_scan_blocks(int64_t n) {
+  return (n + kScanItems * kChainedThreads - 1) / (kScanItems * kChainedThreads);
+}
+
+__global__ void __launch_bounds__(kChainedThreads) chained_scan_kernel(int *data, int64_t n,
+                                                                       unsigned long long *state, unsigned *ticket,
+                                                                       kups_status *status) {
+  __shared__ int scratch[32];
+  __shared__ int64_t base;
+  __shared__ unsigned bid;
+  if (threadIdx.x == 0) bid = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const int64_t b = bid;
+  const int64_t i0 = (b * kChainedThreads + threadIdx.x) * kScanItems;
+  int v[kScanItems], own = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    v[k] = i0 + k < n ? data[i0 + k] : 0;
+    own += v[k];
+  }
+  int total;
+  int ex = block_exclusive_scan<int>(own, scratch, &total);
+  if (threadIdx.x < 32) {
+    bool ok;
+    const int64_t before = chained_prefix(state, b, total, ok);
+    if (threadIdx.x == 0) {
+      base = before;
+      if (!ok) status_error(status, KUPS_ERR_UNSUPPORTED, b);
+    }
+  }
+  __syncthreads();
+  ex += (int)base;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    if (i0 + k < n) data[i0 + k] = ex;
+    ex += v[k];
+  }
+}
+
 }  // namespace kups
