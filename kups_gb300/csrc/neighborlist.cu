@@ -111,7 +111,7 @@ __global__ void count_atoms_kernel(const int32_t *system, int64_t n, int32_t s, 
 // (one per lane): warps 0..2 form the width, image count and cell count of one axis each, warp 3 the
 // inverse, so the float64 divisions (a latency chain of several microseconds when one thread does
 // all of them: 11 us for one system, 19 us for 256) run side by side; the block that finishes last
-// scans the cell counts.  Measured: 5 us for one system, 7 us for 256.
+// scans the cell counts: 8 us for one system, 10 us for 256.
 constexpr int kSetupSystems = 32;
 __global__ void __launch_bounds__(4 * kSetupSystems) setup_systems_kernel(const double *tril, const double *cutoffs,
                                                                          int32_t s, SysNL *sys, unsigned *ticket,
@@ -269,7 +269,7 @@ __global__ void scatter_kernel(const int *cell_of, const int *slot_of, int64_t n
 
 // A particle's place in its cell is the number of smaller indices in it: each cell ends up in index
 // order whatever the arrival order, with one thread per particle (an insertion sort by one thread
-// per cell took 945 us for 4000 particles in 27 cells, this 9 us).  Writes the candidate records of
+// per cell took 945 us for 4000 particles in 27 cells, this 14 us).  Writes the candidate records of
 // the pair search in that order.
 __global__ void order_cells_kernel(const int *cell_of, int64_t n, const int *cell_start, const int *cell_any,
                                    const float4 *wrapped, const int32_t *inclusion, const int32_t *exclusion,
@@ -319,163 +319,212 @@ __device__ inline bool edge_test(const SysNL &p, const double fi[3], const doubl
 }
 
 // The candidates of one particle: up to 27 cells, each a contiguous run of the cell-ordered records,
-// read as one flat range of `total` candidates in (cell, index) order.
-struct CandRange {
-  int pre[kNLCells + 1];  // exclusive prefix of the run lengths
-  int start[kNLCells];    // first record of the run minus its prefix
+// read as one flat range of `total` candidates in (cell, index) order.  Lane c holds run c (the
+// non-empty ones, in order): the flat index it begins at and its first record minus that index.
+struct CandRuns {
+  int begin, shift, total;
 };
 
-// Scans the candidates (times the image offsets) of particle i, a lane per candidate, in the order
-// of the reference: cells, then particle index, then offsets.  The float32 distance settles nearly
-// every candidate; within the margin of the cutoff, within 2^-18 of half a cell (the rounding of the
-// image shift), for image counts beyond 10 bits and for excluded pairs among image offsets the exact
-// float64 test decides, so the edge set is that of the float64 test alone.  Returns the number of
-// edges; with DIRECT they are written from row `out` on, else the first kPairStage are kept in `stage`
-// (wide: some shift does not fit its 10 bits).
-template <bool DIRECT>
-__device__ int scan_particle(const SysNL &p, int i, const float4 &wi, int inc, int exi, const CandRange &rg, int total,
-                             const float4 *cand, const int4 *label, const double *frac, uint2 *stage, bool &wide,
-                             int64_t out, int32_t *edges, int32_t *shifts, int64_t cap) {
+// Record of flat candidate base + lane; `a` is the number of runs that begin before `base`, minus
+// one, and is moved on to the next 32.  One reduction marks where runs begin among these 32.
+__device__ inline int cand_record(const CandRuns &rg, int base, int &a) {
   const int lane = threadIdx.x & 31;
-  const float L0 = p.Lf[0], L1 = p.Lf[1], L2 = p.Lf[2], L3 = p.Lf[3], L4 = p.Lf[4], L5 = p.Lf[5];
-  const float hi2 = p.hi2, lo2 = p.lo2;
-  const int wn = __float_as_int(wi.w);
+  const unsigned at = (unsigned)(rg.begin - base);
+  const unsigned begins = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
+  const int run = a + __popc(begins & (0xffffffffu >> (31 - lane)));
+  a += __popc(begins);
+  return __shfl_sync(0xffffffffu, rg.shift, run & 31) + base + lane;
+}
+
+// rint(x) for |x| < 2^22 by two additions (the rounding instruction runs at a quarter of their rate).
+__device__ inline float rint_small(float x) { return __fadd_rn(__fadd_rn(x, 12582912.0f), -12582912.0f); }
+
+// Minimum-image float32 difference of two wrapped coordinates: d (fractional) in [-0.5, 0.5], the
+// image r, and the squared length.
+__device__ inline float image_distance(const float4 &wi, const float4 &c, const float L[6], float d[3], float r[3]) {
+  d[0] = wi.x - c.x;
+  d[1] = wi.y - c.y;
+  d[2] = wi.z - c.z;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    r[a] = rint_small(d[a]);
+    d[a] -= r[a];
+  }
+  const float X = fmaf(d[2], L[3], fmaf(d[1], L[1], d[0] * L[0])), Y = fmaf(d[2], L[4], d[1] * L[2]), Z = d[2] * L[5];
+  return fmaf(Z, Z, fmaf(Y, Y, X * X));
+}
+
+// What a search makes of particle i (the same in every lane of its warp).
+struct PairQuery {
+  int i, inc, exi;
+  float4 wi;
+  float L[6], lo2, hi2;
+};
+
+__device__ __noinline__ bool exact_pair(const SysNL &p, const double *frac, int i, int j, const int o[3], bool image,
+                                  bool same_ex, int sh[3]) {
+  const double fi[3] = {frac[3 * (int64_t)i], frac[3 * (int64_t)i + 1], frac[3 * (int64_t)i + 2]};
+  const double fj[3] = {frac[3 * (int64_t)j], frac[3 * (int64_t)j + 1], frac[3 * (int64_t)j + 2]};
+  return edge_test(p, fi, fj, o, image, sh, same_ex);
+}
+
+// Whether record k is an edge of the particle at its minimum image, with its shift.  The float32
+// distance settles nearly every candidate; within the margin of the cutoff, within 2^-18 of half a
+// cell (the rounding of the image) and for images beyond 10 bits the float64 test decides, so the
+// edge set is that of the float64 test alone.
+__device__ inline bool settle_pair(const SysNL &p, const PairQuery &q, const float4 *cand, const int4 *label,
+                                   const double *frac, int k, int &j, int sh[3]) {
+  constexpr float kHalf = 0.5f - 1.0f / 262144.0f;
+  const float4 c = cand[k];
+  float d[3], r[3];
+  const float d2 = image_distance(q.wi, c, q.L, d, r);
+  if (!(d2 < q.hi2)) return false;
+  const int4 lb = label[k];
+  if (lb.x != q.inc) return false;
+  j = __float_as_int(c.w);
+  const int wn = __float_as_int(q.wi.w);
+  const bool same_ex = lb.y == q.exi;
+  if (!(d2 < q.lo2) || fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fabsf(d[2])) > kHalf || ((wn | lb.z) & kWideImage)) {
+    const int o[3] = {0, 0, 0};
+    return exact_pair(p, frac, q.i, j, o, false, same_ex, sh);
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) sh[a] = image_axis(wn, a) - image_axis(lb.z, a) + (int)r[a];
+  return !same_ex;  // the shift is the minimum image, where equal exclusion labels drop the pair
+}
+
+__device__ inline bool fits_packed(const int sh[3]) {
+  return (unsigned)(sh[0] + 512) < 1024u && (unsigned)(sh[1] + 512) < 1024u && (unsigned)(sh[2] + 512) < 1024u;
+}
+__device__ inline unsigned pack_shift(const int sh[3]) {
+  return (unsigned)((sh[0] + 512) | ((sh[1] + 512) << 10) | ((sh[2] + 512) << 20));
+}
+
+// One image per axis: every candidate's distance first, keeping the records inside hi2 (a tenth of
+// them), then the labels, shifts and close calls of those with every lane at work.  Returns the
+// number of edges, the edges (j, packed shift) in `stage`; -1 if they do not fit there.
+__device__ int search_staged(const SysNL &p, const PairQuery &q, const CandRuns &rg, const float4 *cand,
+                             const int4 *label, const double *frac, uint2 *stage) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  int near = 0, a = -1;
+#pragma unroll 2
+  for (int base = 0; base < rg.total; base += 32) {
+    const int k = cand_record(rg, base, a);
+    float d2 = INFINITY;
+    if (base + lane < rg.total) {
+      float d[3], r[3];
+      d2 = image_distance(q.wi, cand[k], q.L, d, r);
+    }
+    const bool in = d2 < q.hi2;
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    const int at = near + __popc(m & below);
+    if (in && at < kPairStage) stage[at].x = (unsigned)k;
+    near += __popc(m);
+  }
+  if (near > kPairStage) return -1;
+  __syncwarp();
   int cnt = 0;
-  bool too_wide = false;
-  // appends the hits of the 32 lanes in lane order
-  auto append = [&](bool hit, int j, int sx, int sy, int sz) {
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
+  bool wide = false;
+  for (int base = 0; base < near; base += 32) {
+    int j = 0, sh[3] = {0, 0, 0};
+    const bool hit = base + lane < near && settle_pair(p, q, cand, label, frac, (int)stage[base + lane].x, j, sh);
+    const unsigned m = __ballot_sync(0xffffffffu, hit);  // every lane has read its record
     if (hit) {
-      const int at = cnt + __popc(m & ((1u << lane) - 1u));
-      if (DIRECT) {
-        const int64_t o = out + at;
-        if (o < cap) {
-          edges[2 * o] = i;
-          edges[2 * o + 1] = j;
-          shifts[3 * o] = sx;
-          shifts[3 * o + 1] = sy;
-          shifts[3 * o + 2] = sz;
-        }
-      } else if (at < kPairStage) {
-        too_wide |= sx < -512 || sx > 511 || sy < -512 || sy > 511 || sz < -512 || sz > 511;
-        stage[at] = make_uint2((unsigned)j, (unsigned)((sx + 512) | ((sy + 512) << 10) | ((sz + 512) << 20)));
-      }
+      wide |= !fits_packed(sh);
+      stage[cnt + __popc(m & below)] = make_uint2((unsigned)j, pack_shift(sh));
     }
     cnt += __popc(m);
-  };
-  auto exact = [&](int j, const int o[3], bool image, bool same_ex, int sh[3]) {
-    const double fi[3] = {frac[3 * (int64_t)i], frac[3 * (int64_t)i + 1], frac[3 * (int64_t)i + 2]};
-    const double fj[3] = {frac[3 * (int64_t)j], frac[3 * (int64_t)j + 1], frac[3 * (int64_t)j + 2]};
-    return edge_test(p, fi, fj, o, image, sh, same_ex);
-  };
+    __syncwarp();
+  }
+  return __any_sync(0xffffffffu, wide) ? -1 : cnt;
+}
+
+// The general search, edges handed to emit(hit, j, shift) 32 candidates at a time in the order of the
+// reference: cells, then particle index, then image offsets.
+template <typename Emit>
+__device__ void search_each(const SysNL &p, const PairQuery &q, const CandRuns &rg, const float4 *cand,
+                            const int4 *label, const double *frac, Emit emit) {
+  const int lane = threadIdx.x & 31;
   if (!p.image_mode) {
-    constexpr float kHalf = 0.5f - 1.0f / 262144.0f;
-    int a = 0;
-    for (int base = 0; base < total; base += 32) {
-      const int idx = base + lane;
-      bool hit = false;
+    int a = -1;
+    for (int base = 0; base < rg.total; base += 32) {
+      const int k = cand_record(rg, base, a);
       int j = 0, sh[3] = {0, 0, 0};
-      if (idx < total) {
-        while (idx >= rg.pre[a + 1]) ++a;
-        const int k = rg.start[a] + idx;
-        const float4 c = cand[k];
-        float dx = wi.x - c.x, dy = wi.y - c.y, dz = wi.z - c.z;
-        const float rx = rintf(dx), ry = rintf(dy), rz = rintf(dz);
-        dx -= rx;
-        dy -= ry;
-        dz -= rz;
-        const float X = fmaf(dz, L3, fmaf(dy, L1, dx * L0)), Y = fmaf(dz, L4, dy * L2), Z = dz * L5;
-        const float d2 = fmaf(Z, Z, fmaf(Y, Y, X * X));
-        if (d2 < hi2) {
-          const int4 lb = label[k];
-          j = __float_as_int(c.w);
-          if (lb.x == inc) {
-            const bool same_ex = lb.y == exi;
-            if (!(d2 < lo2) || fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) > kHalf || ((wn | lb.z) & kWideImage)) {
-              const int o[3] = {0, 0, 0};
-              hit = exact(j, o, false, same_ex, sh);
-            } else {
-              hit = !same_ex;  // the shift is the minimum image
-              sh[0] = image_axis(wn, 0) - image_axis(lb.z, 0) + (int)rx;
-              sh[1] = image_axis(wn, 1) - image_axis(lb.z, 1) + (int)ry;
-              sh[2] = image_axis(wn, 2) - image_axis(lb.z, 2) + (int)rz;
-            }
-          }
-        }
-      }
-      append(hit, j, sh[0], sh[1], sh[2]);
+      const bool hit = base + lane < rg.total && settle_pair(p, q, cand, label, frac, k, j, sh);
+      emit(hit, j, sh);
     }
-  } else {
-    // one cell; (candidate, x, y, z offset) as a mixed-radix counter that every lane steps by 32
-    const int n1 = p.nimg[1], n2 = p.nimg[2], n0 = p.nimg[0];
-    const int step_z = 32 % n2, step_y = (32 / n2) % n1, step_x = (32 / n2 / n1) % n0, step_c = 32 / n2 / n1 / n0;
-    int oz = lane % n2, oy = (lane / n2) % n1, ox = (lane / n2 / n1) % n0;
-    int64_t c = lane / n2 / n1 / n0;
-    while (__any_sync(0xffffffffu, c < total)) {
-      bool hit = false;
-      int j = 0, sh[3] = {0, 0, 0};
-      if (c < total) {
-        const int k = rg.start[0] + (int)c;
-        const float4 q = cand[k];
-        const int4 lb = label[k];
-        j = __float_as_int(q.w);
-        if (lb.x == inc) {
-          const int o[3] = {ox - (n0 - 1) / 2, oy - (n1 - 1) / 2, oz - (n2 - 1) / 2};
-          const bool same_ex = lb.y == exi;
-          bool sure = !((wn | lb.z) & kWideImage);
-          if (sure) {
-            const float dx = (wi.x - q.x) + (float)(image_axis(wn, 0) - image_axis(lb.z, 0) - o[0]);
-            const float dy = (wi.y - q.y) + (float)(image_axis(wn, 1) - image_axis(lb.z, 1) - o[1]);
-            const float dz = (wi.z - q.z) + (float)(image_axis(wn, 2) - image_axis(lb.z, 2) - o[2]);
-            const float X = fmaf(dz, L3, fmaf(dy, L1, dx * L0)), Y = fmaf(dz, L4, dy * L2), Z = dz * L5;
-            const float d2 = fmaf(Z, Z, fmaf(Y, Y, X * X));
-            if (d2 < hi2) {
-              sure = d2 < lo2 && !same_ex;
-              hit = sure;
-              sh[0] = o[0];
-              sh[1] = o[1];
-              sh[2] = o[2];
-            }
+    return;
+  }
+  // one cell; (candidate, x, y, z offset) as a mixed-radix counter that every lane steps by 32.  An
+  // excluded pair needs its minimum image, a matter of the float64 test.
+  const int n0 = p.nimg[0], n1 = p.nimg[1], n2 = p.nimg[2];
+  const int wn = __float_as_int(q.wi.w);
+  const int step_z = 32 % n2, step_y = (32 / n2) % n1, step_x = (32 / n2 / n1) % n0, step_c = 32 / n2 / n1 / n0;
+  int oz = lane % n2, oy = (lane / n2) % n1, ox = (lane / n2 / n1) % n0, c = lane / n2 / n1 / n0;
+  const int first = __shfl_sync(0xffffffffu, rg.shift, 0);
+  while (__any_sync(0xffffffffu, c < rg.total)) {
+    bool hit = false;
+    int j = 0, sh[3] = {0, 0, 0};
+    if (c < rg.total) {
+      const float4 w = cand[first + c];
+      const int4 lb = label[first + c];
+      j = __float_as_int(w.w);
+      if (lb.x == q.inc) {
+        const int o[3] = {ox - (n0 - 1) / 2, oy - (n1 - 1) / 2, oz - (n2 - 1) / 2};
+        const bool same_ex = lb.y == q.exi;
+        bool sure = !((wn | lb.z) & kWideImage);
+        if (sure) {
+          const float dx = (q.wi.x - w.x) + (float)(image_axis(wn, 0) - image_axis(lb.z, 0) - o[0]);
+          const float dy = (q.wi.y - w.y) + (float)(image_axis(wn, 1) - image_axis(lb.z, 1) - o[1]);
+          const float dz = (q.wi.z - w.z) + (float)(image_axis(wn, 2) - image_axis(lb.z, 2) - o[2]);
+          const float X = fmaf(dz, q.L[3], fmaf(dy, q.L[1], dx * q.L[0])), Y = fmaf(dz, q.L[4], dy * q.L[2]),
+                      Z = dz * q.L[5];
+          const float d2 = fmaf(Z, Z, fmaf(Y, Y, X * X));
+          if (d2 < q.hi2) {
+            sure = d2 < q.lo2 && !same_ex;
+            hit = sure;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) sh[a] = o[a];
           }
-          if (!sure) hit = exact(j, o, true, same_ex, sh);
         }
+        if (!sure) hit = exact_pair(p, frac, q.i, j, o, true, same_ex, sh);
       }
-      append(hit, j, sh[0], sh[1], sh[2]);
-      c += step_c;
-      oz += step_z;
-      oy += step_y;
-      ox += step_x;
-      if (oz >= n2) {
-        oz -= n2;
-        ++oy;
-      }
-      if (oy >= n1) {
-        oy -= n1;
-        ++ox;
-      }
-      if (ox >= n0) {
-        ox -= n0;
-        ++c;
-      }
+    }
+    emit(hit, j, sh);
+    c += step_c;
+    oz += step_z;
+    oy += step_y;
+    ox += step_x;
+    if (oz >= n2) {
+      oz -= n2;
+      ++oy;
+    }
+    if (oy >= n1) {
+      oy -= n1;
+      ++ox;
+    }
+    if (ox >= n0) {
+      ox -= n0;
+      ++c;
     }
   }
-  wide = __any_sync(0xffffffffu, too_wide);
-  return cnt;
 }
 
 // The edge list in one pass: a warp per particle (index order) finds its edges into shared memory,
 // the block's count joins the chained prefix over blocks, and the rows are written at their final
-// place with coalesced stores.  A particle with more than kPairStage edges is scanned again to write
-// them.  Bounded by issue: about 45 instructions per 32 candidates.  With the float64 test per
-// candidate (30 operations at 2 per clock per SM, one thread per particle, a counting and a writing
-// pass) 264 k particles in 256 systems took 19.3 ms; see the figures at the launch.
-__global__ void __launch_bounds__(32 * kPairWarps) pairs_kernel(
+// place with coalesced stores.  A particle whose edges do not fit there (more than kPairStage, or
+// shifts beyond 10 bits) is searched again to write them.  Bounded by issue: about 40 instructions
+// per 32 candidates, and 80 per 32 edges.  264 k particles in 256 systems (about 500 candidates
+// each): 0.89 ms (1.29 ms with labels and shifts taken up
+// candidate by candidate); the float64 test per candidate (30 operations at 2 per clock per SM, one thread per
+// particle, a counting and a writing pass) took 19.3 ms.
+__global__ void __launch_bounds__(32 * kPairWarps, 4) pairs_kernel(
     const int32_t *system, const int32_t *inclusion, const int32_t *exclusion, int64_t n, int32_t n_incl, int32_t s,
     const SysNL *sys, const double *frac, const float4 *wrapped, const int *cell_of, const int *cell_start,
     const float4 *cand, const int4 *label, unsigned *ticket, unsigned long long *state, int64_t *n_edges,
     int32_t *edges, int32_t *shifts, int64_t cap, kups_status *status) {
   __shared__ uint2 stage_all[kPairWarps][kPairStage];
-  __shared__ CandRange ranges[kPairWarps];
   __shared__ int counts[kPairWarps];
   __shared__ int64_t base;
   __shared__ unsigned bid;
@@ -485,16 +534,23 @@ __global__ void __launch_bounds__(32 * kPairWarps) pairs_kernel(
   __syncthreads();
   const int64_t i = (int64_t)bid * kPairWarps + warp;
   uint2 *stage = stage_all[warp];
-  CandRange &rg = ranges[warp];
   const int32_t si = i < n ? system[i] : -1, inc = i < n ? inclusion[i] : -1;
   const bool on = si >= 0 && si < s && inc >= 0 && inc < n_incl && !sys[si].refused;
-  int cnt = 0, total = 0, exi = 0;
-  bool wide = false;
-  float4 wi = make_float4(0.f, 0.f, 0.f, 0.f);
+  int cnt = 0;
+  bool again = false;
+  PairQuery q;
+  CandRuns rg;
+  rg.total = 0;
   if (on) {  // the same for the whole warp
     const SysNL &p = sys[si];
-    wi = wrapped[i];
-    exi = exclusion[i];
+    q.i = (int)i;
+    q.inc = inc;
+    q.exi = exclusion[i];
+    q.wi = wrapped[i];
+    q.lo2 = p.lo2;
+    q.hi2 = p.hi2;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) q.L[a] = p.Lf[a];
     int first = 0, len = 0;
     if (lane < kNLCells) {
       const int nx = p.nc[0], ny = p.nc[1], nz = p.nc[2];
@@ -502,12 +558,14 @@ __global__ void __launch_bounds__(32 * kPairWarps) pairs_kernel(
       const int cx = ci % nx, cy = (ci / nx) % ny, cz = ci / (nx * ny);
       // the distinct neighbour cells of an axis (1, 2 or 3 of them), in this order
       auto axis = [](int c, int nc, int t, int &out) {
-        if (t >= min(nc, 3)) return false;
-        out = nc <= 2 ? t : (c + nc - 1 + t) % nc;
-        return true;
+        out = c + t - 1;
+        if (nc <= 2) out = t;
+        else if (out < 0) out += nc;
+        else if (out >= nc) out -= nc;
+        return t < min(nc, 3);
       };
       int x, y, z;
-      if (axis(cx, nx, lane % 3, x) && axis(cy, ny, (lane / 3) % 3, y) && axis(cz, nz, lane / 9, z)) {
+      if (axis(cx, nx, lane % 3, x) & axis(cy, ny, (lane / 3) % 3, y) & axis(cz, nz, lane / 9, z)) {
         const int c = (int)p.cell_base + (z * ny + y) * nx + x;
         first = cell_start[c];
         len = cell_start[c + 1] - first;
@@ -519,15 +577,30 @@ __global__ void __launch_bounds__(32 * kPairWarps) pairs_kernel(
       const int v = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += v;
     }
-    total = __shfl_sync(0xffffffffu, sum, 31);
-    if (lane < kNLCells) {
-      rg.pre[lane] = sum - len;
-      rg.start[lane] = first - (sum - len);
-    }
-    if (lane == kNLCells) rg.pre[kNLCells] = total;
+    rg.total = __shfl_sync(0xffffffffu, sum, 31);
+    // the non-empty runs to the leading lanes, in order
+    const unsigned full = __ballot_sync(0xffffffffu, len > 0);
+    if (len > 0) stage[__popc(full & ((1u << lane) - 1u))] = make_uint2((unsigned)(sum - len), (unsigned)first);
     __syncwarp();
-    cnt = scan_particle<false>(p, (int)i, wi, inc, exi, rg, total, cand, label, frac, stage, wide, 0, edges, shifts,
-                               cap);
+    const uint2 run = lane < __popc(full) ? stage[lane] : make_uint2(0x7fffffffu, 0u);
+    rg.begin = (int)run.x;
+    rg.shift = (int)(run.y - run.x);
+    __syncwarp();
+    cnt = p.image_mode ? -1 : search_staged(p, q, rg, cand, label, frac, stage);
+    if (cnt < 0) {
+      cnt = 0;
+      search_each(p, q, rg, cand, label, frac, [&](bool hit, int j, const int *sh) {
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        const int at = cnt + __popc(m & ((1u << lane) - 1u));
+        if (hit) {
+          again |= !fits_packed(sh) || at >= kPairStage;
+          if (at < kPairStage) stage[at] = make_uint2((unsigned)j, pack_shift(sh));
+        }
+        cnt += __popc(m);
+      });
+      again = __any_sync(0xffffffffu, again);
+      __syncwarp();
+    }
   }
   if (lane == 0) counts[warp] = cnt;
   __syncthreads();
@@ -552,9 +625,17 @@ __global__ void __launch_bounds__(32 * kPairWarps) pairs_kernel(
   if (!chained || cnt == 0) return;
   int64_t out = base;
   for (int k = 0; k < warp; ++k) out += counts[k];
-  if (cnt > kPairStage || wide) {
-    scan_particle<true>(sys[si], (int)i, wi, inc, exi, rg, total, cand, label, frac, stage, wide, out, edges, shifts,
-                        cap);
+  if (again) {
+    search_each(sys[si], q, rg, cand, label, frac, [&](bool hit, int j, const int *sh) {
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      const int64_t o = out + __popc(m & ((1u << lane) - 1u));
+      if (hit && o < cap) {
+        edges[2 * o] = (int32_t)i;
+        edges[2 * o + 1] = j;
+        for (int a = 0; a < 3; ++a) shifts[3 * o + a] = sh[a];
+      }
+      out += __popc(m);
+    });
     return;
   }
   const int rows = (int)max((int64_t)0, min((int64_t)cnt, cap - out));
