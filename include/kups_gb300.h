@@ -182,6 +182,16 @@ int32_t kups_lj_edges(const double *positions, const int32_t *system,
                       const int32_t *edges, const int32_t *shifts, int64_t n_edges,
                       double *energy, double *grad, double *grad_tril,
                       int32_t pair_fp32, kups_status *status, void *stream);
+/* kups_lj_edges_paired: the same sums for a list that holds every edge (i, j, s) together with its
+ * reverse (j, i, -s), as kups_neighborlist_build writes it: one of the two is evaluated for both.
+ * Results differ from kups_lj_edges by the rounding of the float64 sums.  Padding rows as there. */
+int32_t kups_lj_edges_paired(const double *positions, const int32_t *system,
+                             const int32_t *species, int64_t n_particles,
+                             const double *tril, const double *cutoffs, int32_t n_systems,
+                             const double *sigma, const double *epsilon, int32_t n_species,
+                             const int32_t *edges, const int32_t *shifts, int64_t n_edges,
+                             double *energy, double *grad, double *grad_tril,
+                             int32_t pair_fp32, kups_status *status, void *stream);
 
 /* ------------------------------------------------------------------------
  * Fused Lennard-Jones MD — replaces one or more calls of the propagator built
@@ -441,6 +451,17 @@ int32_t kups_pair_edges(const double *positions, const int32_t *system, const in
                         const int32_t *edges, const int32_t *shifts, int64_t n_edges,
                         double *energy, double *grad, double *grad_tril, kups_status *status,
                         void *stream);
+
+/* kups_pair_edges_paired: kups_pair_edges for a list that holds every edge together with its
+ * reverse (see kups_lj_edges_paired). */
+int32_t kups_pair_edges_paired(const double *positions, const int32_t *system, const int32_t *species,
+                               const double *charges, int64_t n_particles, const double *tril,
+                               int32_t n_systems, const double *lj_sigma, const double *lj_epsilon,
+                               int32_t n_species, const double *lj_cutoff, const double *alpha,
+                               const double *ewald_cutoff, double coulomb_k, int32_t terms,
+                               const int32_t *edges, const int32_t *shifts, int64_t n_edges,
+                               double *energy, double *grad, double *grad_tril, kups_status *status,
+                               void *stream);
 
 /* ------------------------------------------------------------------------
  * Bonded edge-set potentials — replace the energies of

@@ -106,6 +106,7 @@ SIGNATURES = {
     "kups_edge_segment_sum": (_I32, [_P, _I32, _P, _I64, _I64, _P, _P]),
     "kups_edge_gradients": (_I32, [_P, _P, _I64, _I32, _P, _P, _I64, _P, _P, _P]),
     "kups_lj_edges": (_I32, [_P, _P, _P, _I64, _P, _P, _I32, _P, _P, _I32, _P, _P, _I64, _P, _P, _P, _I32, _P, _P]),
+    "kups_lj_edges_paired": (_I32, [_P, _P, _P, _I64, _P, _P, _I32, _P, _P, _I32, _P, _P, _I64, _P, _P, _P, _I32, _P, _P]),
     "kups_lj_md_workspace_bytes": (_SZ, [C.POINTER(MdArgs)]),
     "kups_lj_md_run": (_I32, [C.POINTER(MdArgs), _P, _SZ, _P, _P]),
     "kups_lj_md_max_atoms": (_I32, []),
@@ -147,6 +148,7 @@ SIGNATURES = {
                                  _P, _I32, _P, _SZ, _P, _P]),
     "kups_erfc_eval": (_I32, [_P, _I64, _P, _P]),
     "kups_pair_edges": (_I32, [_P, _P, _P, _P, _I64, _P, _I32, _P, _P, _I32, _P, _P, _P, C.c_double, _I32, _P, _P, _I64, _P, _P, _P, _P, _P]),
+    "kups_pair_edges_paired": (_I32, [_P, _P, _P, _P, _I64, _P, _I32, _P, _P, _I32, _P, _P, _P, C.c_double, _I32, _P, _P, _I64, _P, _P, _P, _P, _P]),
 }
 
 _lib = None

@@ -24,7 +24,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from .neighborlist import CellListNeighborList, NeighborListPoints, _f64, _i32, _stream, new_status, read_status
+from .neighborlist import (CellListNeighborList, NeighborListPoints, _f64, _i32, _stream, lists_pairs, new_status,
+                           read_status)
 from .potential import PositionAndUnitCell, PotentialOut
 from .units import BOLTZMANN_CONSTANT, TO_STANDARD_UNITS
 
@@ -208,7 +209,8 @@ def ewald_self(charges, sys_offset, alpha, n_systems):
 
 
 def pair_edges(positions, system, species, charges, tril, edges, shifts, n_edges, terms, lj_sigma=None,
-               lj_epsilon=None, lj_cutoff=None, alpha=None, ewald_cutoff=None, grad_tril=True, out=None, status=None):
+               lj_epsilon=None, lj_cutoff=None, alpha=None, ewald_cutoff=None, grad_tril=True, out=None, status=None,
+               paired=False):
     lib = _lib.load()
     pos, tril = _f64(positions), _f64(tril)
     n, s = pos.shape[0], tril.shape[0]
@@ -223,10 +225,11 @@ def pair_edges(positions, system, species, charges, tril, edges, shifts, n_edges
         torch.empty((s, 6), dtype=torch.float64, device="cuda"))
     nsp = int(keep["sig"].shape[0]) if keep["sig"] is not None else 0
     status = status if status is not None else new_status()
-    rc = lib.kups_pair_edges(pos.data_ptr(), ptr("system"), ptr("species"), ptr("charges"), n, tril.data_ptr(), s,
-                             ptr("sig"), ptr("eps"), nsp, ptr("rc_lj"), ptr("alpha"), ptr("rc_ew"), TO_STANDARD_UNITS,
-                             int(terms), ptr("edges"), ptr("shifts"), int(n_edges), energy.data_ptr(), grad.data_ptr(),
-                             gtril.data_ptr() if grad_tril else None, status.data_ptr(), _stream())
+    fn = lib.kups_pair_edges_paired if paired else lib.kups_pair_edges
+    rc = fn(pos.data_ptr(), ptr("system"), ptr("species"), ptr("charges"), n, tril.data_ptr(), s, ptr("sig"),
+            ptr("eps"), nsp, ptr("rc_lj"), ptr("alpha"), ptr("rc_ew"), TO_STANDARD_UNITS, int(terms), ptr("edges"),
+            ptr("shifts"), int(n_edges), energy.data_ptr(), grad.data_ptr(), gtril.data_ptr() if grad_tril else None,
+            status.data_ptr(), _stream())
     _lib.check(rc, "kups_pair_edges")
     return energy, grad, gtril
 
@@ -288,7 +291,8 @@ class LJEwaldPotential:
         pts = NeighborListPoints(particles.positions, particles.system, None, particles.exclusion)
         e, self.neighborlist = self.neighborlist.call_and_fix(pts, None, tril, rc_nl)
         en, g, gt = pair_edges(particles.positions, particles.system, particles.species, particles.charges, tril,
-                               e.indices, e.shifts.view(-1, 3), e.n_edges, terms, sig, eps, rc_lj, alpha, rc_ew)
+                               e.indices, e.shifts.view(-1, 3), e.n_edges, terms, sig, eps, rc_lj, alpha, rc_ew,
+                               paired=lists_pairs(self.neighborlist))
         off, mx = _offsets(_i32(particles.system), s)
         self._last_recip = ewald_recip(particles.positions, particles.charges, off, mx, tril,
                                        self.ewald.reciprocal_lattice_shifts, alpha, ws=self.ws)
@@ -469,7 +473,7 @@ class LJEwaldMD:
         terms = TERM_EWALD_REAL | (TERM_LJ if self.lj else 0)
         pair_edges(pos, self.system, self.species, self.q, self.tril, self.edges, self.shifts, self.cap, terms,
                    self.sig, self.eps, self.rc_lj, self.alpha, self.rc_ew, grad_tril=False,
-                   out=(self.e_pair, self.g_pair, self.t_pair), status=self.status)
+                   out=(self.e_pair, self.g_pair, self.t_pair), status=self.status, paired=True)
         ewald_recip(pos, self.q, self.off, self.max_atoms, self.tril, self.kn, self.alpha, grad_tril=False,
                     ws=self.rws, out=(self.e_rec, self.g_rec, self.t_rec, self.sk), status=self.status)
         torch.add(self.g_pair, self.g_rec, out=self.grad)

@@ -645,12 +645,12 @@ class LennardJonesMD64:
                                          self.status.data_ptr(), st)
         _lib.check(rc, "kups_neighborlist_build")
         # edges past n_edges are padded with the out-of-bounds index and skipped by the kernel
-        rc = lib.kups_lj_edges(self.pos.data_ptr(), self.system.data_ptr(), self.species.data_ptr(), self.n,
-                               self.tril.data_ptr(), self.cut.data_ptr(), self.s, self.sig.data_ptr(),
-                               self.eps.data_ptr(), self.nsp, self.edges.data_ptr(), self.shifts.data_ptr(), self.cap,
-                               self.energy.data_ptr(), self.grad.data_ptr(), self.gtril.data_ptr(), 0,
-                               self.status.data_ptr(), st)
-        _lib.check(rc, "kups_lj_edges")
+        rc = lib.kups_lj_edges_paired(self.pos.data_ptr(), self.system.data_ptr(), self.species.data_ptr(), self.n,
+                                      self.tril.data_ptr(), self.cut.data_ptr(), self.s, self.sig.data_ptr(),
+                                      self.eps.data_ptr(), self.nsp, self.edges.data_ptr(), self.shifts.data_ptr(),
+                                      self.cap, self.energy.data_ptr(), self.grad.data_ptr(), self.gtril.data_ptr(), 0,
+                                      self.status.data_ptr(), st)
+        _lib.check(rc, "kups_lj_edges_paired")
 
     def _step(self, step: int):
         lib = _lib.load()

@@ -175,6 +175,12 @@ class DenseNearestNeighborList(CellListNeighborList):
     """Same edge set as the cell list (neighborlist.py:902-982)."""
 
 
+def lists_pairs(neighborlist) -> bool:
+    """Whether a full call of ``neighborlist`` is known to hold every edge together with its reverse:
+    this module's own classes (the membership test is symmetric bit for bit), not a user's."""
+    return type(neighborlist) in (CellListNeighborList, DenseNearestNeighborList)
+
+
 class NeighborListChangesResult(NamedTuple):
     added: Edges
     removed: Edges

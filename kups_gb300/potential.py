@@ -16,7 +16,8 @@ from typing import Any, NamedTuple
 import torch
 
 from . import _lib
-from .neighborlist import CellListNeighborList, NeighborListPoints, _f64, _i32, _stream, new_status, read_status
+from .neighborlist import (CellListNeighborList, NeighborListPoints, _f64, _i32, _stream, lists_pairs, new_status,
+                           read_status)
 from .unitcell import as_tril
 
 
@@ -136,13 +137,15 @@ class LennardJonesPotential:
         pts = NeighborListPoints(p.positions, p.system, p.inclusion, p.exclusion)
         edges, self.neighborlist = self.neighborlist.call_and_fix(pts, None, tril, cut)
         out = lj_from_edges(p.positions, p.system, p.species, tril, prm.sigma, prm.epsilon, cut, edges.indices,
-                            edges.shifts, edges.n_edges, self.pair_fp32)
+                            edges.shifts, edges.n_edges, self.pair_fp32, lists_pairs(self.neighborlist))
         out.cache = out.total_energies
         return out
 
 
 def lj_from_edges(positions, system, species, tril, sigma, epsilon, cutoffs, edges, shifts, n_edges,
-                  pair_fp32: bool = True) -> PotentialOut:
+                  pair_fp32: bool = True, paired: bool = False) -> PotentialOut:
+    """LJ energies and gradients over an edge list (``kups_lj_edges``); ``paired``: the list holds
+    every edge together with its reverse, as this package's neighbour lists do."""
     lib = _lib.load()
     pos = _f64(positions)
     n = pos.shape[0]
@@ -160,10 +163,10 @@ def lj_from_edges(positions, system, species, tril, sigma, epsilon, cutoffs, edg
     grad = torch.empty((n, 3), device="cuda", dtype=torch.float64)
     gtril = torch.empty((s, 6), device="cuda", dtype=torch.float64)
     status = new_status()
-    rc = lib.kups_lj_edges(pos.data_ptr(), sysi.data_ptr(), sp.data_ptr(), n, tril.data_ptr(), cut.data_ptr(), s,
-                           sig.data_ptr(), eps.data_ptr(), t, e_idx.data_ptr(), e_sh.data_ptr(), int(n_edges),
-                           energy.data_ptr(), grad.data_ptr(), gtril.data_ptr(), int(bool(pair_fp32)),
-                           status.data_ptr(), _stream())
+    fn = lib.kups_lj_edges_paired if paired else lib.kups_lj_edges
+    rc = fn(pos.data_ptr(), sysi.data_ptr(), sp.data_ptr(), n, tril.data_ptr(), cut.data_ptr(), s, sig.data_ptr(),
+            eps.data_ptr(), t, e_idx.data_ptr(), e_sh.data_ptr(), int(n_edges), energy.data_ptr(), grad.data_ptr(),
+            gtril.data_ptr(), int(bool(pair_fp32)), status.data_ptr(), _stream())
     _lib.check(rc, "kups_lj_edges")
     _lib.raise_status(read_status(status))
     return PotentialOut(energy, PositionAndUnitCell(grad, gtril))
