@@ -39,8 +39,8 @@ constexpr double kMaxNLImages = 1331.0;
 
 // Neighbour cells per particle.
 constexpr int kNLCells = 27;
-// Pair search: warps (particles) per block and hits a warp keeps in shared memory.
-constexpr int kPairWarps = 8, kPairStage = 512;
+// Pair search: warps (particles) per block.
+constexpr int kPairWarps = 8;
 
 struct NLWork {
   char *zero;           // start of the words a call zeroes first (through zero_bytes)
@@ -402,9 +402,9 @@ __device__ inline unsigned pack_shift(const int sh[3]) {
 
 // One image per axis: every candidate's distance first, keeping the records inside hi2 (a tenth of
 // them), then the labels, shifts and close calls of those with every lane at work.  Returns the
-// number of edges, the edges (j, packed shift) in `stage`; -1 if they do not fit there.
+// number of edges, the edges (j, packed shift) in `stage`; -1 if they do not fit its `room` rows.
 __device__ int search_staged(const SysNL &p, const PairQuery &q, const CandRuns &rg, const float4 *cand,
-                             const int4 *label, const double *frac, uint2 *stage) {
+                             const int4 *label, const double *frac, uint2 *stage, int room) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   int near = 0, a = -1;
@@ -419,10 +419,10 @@ __device__ int search_staged(const SysNL &p, const PairQuery &q, const CandRuns 
     const bool in = d2 < q.hi2;
     const unsigned m = __ballot_sync(0xffffffffu, in);
     const int at = near + __popc(m & below);
-    if (in && at < kPairStage) stage[at].x = (unsigned)k;
+    if (in && at < room) stage[at].x = (unsigned)k;
     near += __popc(m);
   }
-  if (near > kPairStage) return -1;
+  if (near > room) return -1;
   __syncwarp();
   int cnt = 0;
   bool wide = false;
@@ -511,139 +511,198 @@ __device__ void search_each(const SysNL &p, const PairQuery &q, const CandRuns &
   }
 }
 
+struct PairSearch {
+  const int32_t *system, *inclusion, *exclusion;
+  int64_t n;
+  int32_t n_incl, s;
+  const SysNL *sys;
+  const double *frac;
+  const float4 *wrapped;
+  const int *cell_of, *cell_start;
+  const float4 *cand;
+  const int4 *label;
+};
+
+// The query of particle i and its candidate runs, by a whole warp; null if it has no edges.  `tmp`:
+// 32 rows of shared memory of the warp's own.
+__device__ const SysNL *pair_query(const PairSearch &a, int64_t i, PairQuery &q, CandRuns &rg, uint2 *tmp) {
+  const int lane = threadIdx.x & 31;
+  if (i >= a.n) return nullptr;
+  const int32_t si = a.system[i], inc = a.inclusion[i];
+  if (si < 0 || si >= a.s || inc < 0 || inc >= a.n_incl) return nullptr;
+  const SysNL &p = a.sys[si];
+  if (p.refused) return nullptr;
+  q.i = (int)i;
+  q.inc = inc;
+  q.exi = a.exclusion[i];
+  q.wi = a.wrapped[i];
+  q.lo2 = p.lo2;
+  q.hi2 = p.hi2;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) q.L[k] = p.Lf[k];
+  int first = 0, len = 0;
+  if (lane < kNLCells) {
+    const int nx = p.nc[0], ny = p.nc[1], nz = p.nc[2];
+    const int ci = a.cell_of[i] - (int)p.cell_base;
+    const int cx = ci % nx, cy = (ci / nx) % ny, cz = ci / (nx * ny);
+    // the distinct neighbour cells of an axis (1, 2 or 3 of them), in this order
+    auto axis = [](int c, int nc, int t, int &out) {
+      out = c + t - 1;
+      if (nc <= 2) out = t;
+      else if (out < 0) out += nc;
+      else if (out >= nc) out -= nc;
+      return t < min(nc, 3);
+    };
+    int x, y, z;
+    if (axis(cx, nx, lane % 3, x) & axis(cy, ny, (lane / 3) % 3, y) & axis(cz, nz, lane / 9, z)) {
+      const int c = (int)p.cell_base + (z * ny + y) * nx + x;
+      first = a.cell_start[c];
+      len = a.cell_start[c + 1] - first;
+    }
+  }
+  int sum = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += v;
+  }
+  rg.total = __shfl_sync(0xffffffffu, sum, 31);
+  // the non-empty runs to the leading lanes, in order
+  const unsigned full = __ballot_sync(0xffffffffu, len > 0);
+  if (len > 0) tmp[__popc(full & ((1u << lane) - 1u))] = make_uint2((unsigned)(sum - len), (unsigned)first);
+  __syncwarp();
+  const uint2 run = lane < __popc(full) ? tmp[lane] : make_uint2(0x7fffffffu, 0u);
+  rg.begin = (int)run.x;
+  rg.shift = (int)(run.y - run.x);
+  __syncwarp();
+  return &p;
+}
+
 // The edge list in one pass: a warp per particle (index order) finds its edges into shared memory,
 // the block's count joins the chained prefix over blocks, and the rows are written at their final
-// place with coalesced stores.  A particle whose edges do not fit there (more than kPairStage, or
-// shifts beyond 10 bits) is searched again to write them.  Bounded by issue: about 40 instructions
-// per 32 candidates, and 80 per 32 edges.  264 k particles in 256 systems (about 500 candidates
-// each): 0.89 ms (1.29 ms with labels and shifts taken up
-// candidate by candidate); the float64 test per candidate (30 operations at 2 per clock per SM, one thread per
-// particle, a counting and a writing pass) took 19.3 ms.
-__global__ void __launch_bounds__(32 * kPairWarps, 4) pairs_kernel(
-    const int32_t *system, const int32_t *inclusion, const int32_t *exclusion, int64_t n, int32_t n_incl, int32_t s,
-    const SysNL *sys, const double *frac, const float4 *wrapped, const int *cell_of, const int *cell_start,
-    const float4 *cand, const int4 *label, unsigned *ticket, unsigned long long *state, int64_t *n_edges,
-    int32_t *edges, int32_t *shifts, int64_t cap, kups_status *status) {
-  __shared__ uint2 stage_all[kPairWarps][kPairStage];
-  __shared__ int counts[kPairWarps];
+// place with coalesced stores.  With `defer`, blocks take the next eight particles before they resolve
+// the prefix of the last eight, so no warp waits for a slower predecessor (with a wait after every
+// search a third of the warps' time went into it); a list of few groups takes one buffer instead, so
+// that more blocks fit an SM (4000 ions with 450 edges each: 85 against 124 us).  A particle whose edges do not fit its
+// `room` rows, or with shifts beyond 10 bits, is searched again to write them.  Bounded by issue:
+// about 40 instructions per 32 candidates, and 80 per 32 edges.  264 k particles in 256 systems
+// (about 500 candidates each): 0.73 ms (0.89 ms with the wait, 1.29 ms also with labels and shifts
+// taken up candidate by candidate); the float64 test per candidate (30 operations at 2 per clock per
+// SM, one thread per particle, a counting and a writing pass) took 19.3 ms.
+__global__ void __launch_bounds__(32 * kPairWarps, 4) pairs_kernel(PairSearch a, int room, bool defer, int64_t n_groups,
+                                                                   unsigned *ticket, unsigned long long *state,
+                                                                   int64_t *n_edges, int32_t *edges, int32_t *shifts,
+                                                                   int64_t cap, kups_status *status) {
+  extern __shared__ uint2 stage_all[];  // [1 + defer][kPairWarps][room]
+  __shared__ int counts[2][kPairWarps];
   __shared__ int64_t base;
-  __shared__ unsigned bid;
+  __shared__ unsigned next;
   __shared__ bool chained;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) bid = atomicAdd(ticket, 1u);
-  __syncthreads();
-  const int64_t i = (int64_t)bid * kPairWarps + warp;
-  uint2 *stage = stage_all[warp];
-  const int32_t si = i < n ? system[i] : -1, inc = i < n ? inclusion[i] : -1;
-  const bool on = si >= 0 && si < s && inc >= 0 && inc < n_incl && !sys[si].refused;
-  int cnt = 0;
-  bool again = false;
-  PairQuery q;
-  CandRuns rg;
-  rg.total = 0;
-  if (on) {  // the same for the whole warp
-    const SysNL &p = sys[si];
-    q.i = (int)i;
-    q.inc = inc;
-    q.exi = exclusion[i];
-    q.wi = wrapped[i];
-    q.lo2 = p.lo2;
-    q.hi2 = p.hi2;
-#pragma unroll
-    for (int a = 0; a < 6; ++a) q.L[a] = p.Lf[a];
-    int first = 0, len = 0;
-    if (lane < kNLCells) {
-      const int nx = p.nc[0], ny = p.nc[1], nz = p.nc[2];
-      const int ci = cell_of[i] - (int)p.cell_base;
-      const int cx = ci % nx, cy = (ci / nx) % ny, cz = ci / (nx * ny);
-      // the distinct neighbour cells of an axis (1, 2 or 3 of them), in this order
-      auto axis = [](int c, int nc, int t, int &out) {
-        out = c + t - 1;
-        if (nc <= 2) out = t;
-        else if (out < 0) out += nc;
-        else if (out >= nc) out -= nc;
-        return t < min(nc, 3);
-      };
-      int x, y, z;
-      if (axis(cx, nx, lane % 3, x) & axis(cy, ny, (lane / 3) % 3, y) & axis(cz, nz, lane / 9, z)) {
-        const int c = (int)p.cell_base + (z * ny + y) * nx + x;
-        first = cell_start[c];
-        len = cell_start[c + 1] - first;
-      }
-    }
-    int sum = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += v;
-    }
-    rg.total = __shfl_sync(0xffffffffu, sum, 31);
-    // the non-empty runs to the leading lanes, in order
-    const unsigned full = __ballot_sync(0xffffffffu, len > 0);
-    if (len > 0) stage[__popc(full & ((1u << lane) - 1u))] = make_uint2((unsigned)(sum - len), (unsigned)first);
-    __syncwarp();
-    const uint2 run = lane < __popc(full) ? stage[lane] : make_uint2(0x7fffffffu, 0u);
-    rg.begin = (int)run.x;
-    rg.shift = (int)(run.y - run.x);
-    __syncwarp();
-    cnt = p.image_mode ? -1 : search_staged(p, q, rg, cand, label, frac, stage);
-    if (cnt < 0) {
-      cnt = 0;
-      search_each(p, q, rg, cand, label, frac, [&](bool hit, int j, const int *sh) {
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        const int at = cnt + __popc(m & ((1u << lane) - 1u));
-        if (hit) {
-          again |= !fits_packed(sh) || at >= kPairStage;
-          if (at < kPairStage) stage[at] = make_uint2((unsigned)j, pack_shift(sh));
+  const unsigned below = (1u << lane) - 1u;
+  int64_t last = -1;  // the group found but not yet written
+  int last_cnt = 0;
+  bool last_again = false;
+  for (int buf = 0;; buf ^= defer) {
+    if (threadIdx.x == 0) next = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const int64_t group = next < n_groups ? (int64_t)next : -1;
+    if (group < 0 && last < 0) return;
+    uint2 *stage = stage_all + (size_t)(buf * kPairWarps + warp) * room;
+    PairQuery q;
+    CandRuns rg;
+    int cnt = 0;
+    bool again = false;
+    if (group >= 0) {
+      const SysNL *p = pair_query(a, group * kPairWarps + warp, q, rg, stage);
+      if (p != nullptr) {  // the same for the whole warp
+        cnt = p->image_mode ? -1 : search_staged(*p, q, rg, a.cand, a.label, a.frac, stage, room);
+        if (cnt < 0) {
+          cnt = 0;
+          search_each(*p, q, rg, a.cand, a.label, a.frac, [&](bool hit, int j, const int *sh) {
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            const int at = cnt + __popc(m & below);
+            if (hit) {
+              again |= !fits_packed(sh) || at >= room;
+              if (at < room) stage[at] = make_uint2((unsigned)j, pack_shift(sh));
+            }
+            cnt += __popc(m);
+          });
+          again = __any_sync(0xffffffffu, again);
         }
-        cnt += __popc(m);
-      });
-      again = __any_sync(0xffffffffu, again);
-      __syncwarp();
+      }
     }
-  }
-  if (lane == 0) counts[warp] = cnt;
-  __syncthreads();
-  if (warp == 0) {
-    int own = 0;
+    if (lane == 0) counts[buf][warp] = cnt;
+    __syncthreads();
+    const int done_buf = defer ? buf ^ 1 : buf;
+    if (!defer) {
+      last = group;
+      last_cnt = cnt;
+      last_again = again;
+    }
+    if (warp == 0) {  // this group's count for the blocks behind, then the place of the last group
+      int own = 0, before_own = 0;
 #pragma unroll
-    for (int k = 0; k < kPairWarps; ++k) own += counts[k];
-    bool ok;
-    const int64_t before = chained_prefix(state, bid, own, ok);
-    if (lane == 0) {
-      base = before;
-      chained = ok;
-      if (!ok) status_error(status, KUPS_ERR_UNSUPPORTED, bid);
-      if (bid == gridDim.x - 1) {
-        const int64_t all = ok ? before + own : 0;
-        *n_edges = all;
-        if (all > cap) status_capacity(status, KUPS_CAP_EDGES, all, -1);
+      for (int k = 0; k < kPairWarps; ++k) {
+        own += counts[buf][k];
+        before_own += counts[done_buf][k];
+      }
+      if (group >= 0) chained_publish(state, group, own);
+      if (last >= 0) {
+        bool ok;
+        const int64_t before = chained_prefix(state, last, before_own, ok);
+        if (lane == 0) {
+          base = before;
+          chained = ok;
+          if (!ok) status_error(status, KUPS_ERR_UNSUPPORTED, last);
+          if (last == n_groups - 1) {
+            const int64_t all = ok ? before + before_own : 0;
+            *n_edges = all;
+            if (all > cap) status_capacity(status, KUPS_CAP_EDGES, all, -1);
+          }
+        }
       }
     }
-  }
-  __syncthreads();
-  if (!chained || cnt == 0) return;
-  int64_t out = base;
-  for (int k = 0; k < warp; ++k) out += counts[k];
-  if (again) {
-    search_each(sys[si], q, rg, cand, label, frac, [&](bool hit, int j, const int *sh) {
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      const int64_t o = out + __popc(m & ((1u << lane) - 1u));
-      if (hit && o < cap) {
-        edges[2 * o] = (int32_t)i;
-        edges[2 * o + 1] = j;
-        for (int a = 0; a < 3; ++a) shifts[3 * o + a] = sh[a];
+    __syncthreads();
+    if (last >= 0 && chained && last_cnt > 0) {
+      const int64_t i = last * kPairWarps + warp;
+      uint2 *done = stage_all + (size_t)(done_buf * kPairWarps + warp) * room;
+      int64_t out = base;
+      for (int k = 0; k < warp; ++k) out += counts[done_buf][k];
+      if (last_again) {
+        PairQuery ql;
+        CandRuns rl;
+        const SysNL *p = pair_query(a, i, ql, rl, done);
+        search_each(*p, ql, rl, a.cand, a.label, a.frac, [&](bool hit, int j, const int *sh) {
+          const unsigned m = __ballot_sync(0xffffffffu, hit);
+          const int64_t o = out + __popc(m & below);
+          if (hit && o < cap) {
+            edges[2 * o] = (int32_t)i;
+            edges[2 * o + 1] = j;
+            for (int k = 0; k < 3; ++k) shifts[3 * o + k] = sh[k];
+          }
+          out += __popc(m);
+        });
+      } else {
+        const int rows = (int)max((int64_t)0, min((int64_t)last_cnt, cap - out));
+        for (int t = lane; t < 2 * rows; t += 32) edges[2 * out + t] = (t & 1) ? (int)done[t >> 1].x : (int)i;
+        for (int t = lane; t < 3 * rows; t += 32) {
+          const int e = t / 3;
+          shifts[3 * out + t] = image_axis((int)done[e].y, t - 3 * e);
+        }
       }
-      out += __popc(m);
-    });
-    return;
+    }
+    last = defer ? group : -1;
+    last_cnt = cnt;
+    last_again = again;
   }
-  const int rows = (int)max((int64_t)0, min((int64_t)cnt, cap - out));
-  for (int t = lane; t < 2 * rows; t += 32) edges[2 * out + t] = (t & 1) ? (int)stage[t >> 1].x : (int)i;
-  for (int t = lane; t < 3 * rows; t += 32) {
-    const int e = t / 3;
-    shifts[3 * out + t] = image_axis((int)stage[e].y, t - 3 * e);
-  }
+}
+
+// Rows a warp stages: twice the edge rows per particle that the caller allots (a guess at the longest
+// list), 64 to 512; more only costs resident blocks, fewer a second search.
+inline int pair_room(int64_t cap, int64_t n) {
+  const int64_t want = 2 * (cap / std::max<int64_t>(n, 1));
+  return (int)std::min<int64_t>(512, std::max<int64_t>(64, (want + 31) / 32 * 32));
 }
 
 __global__ void check_capacity_kernel(const int64_t *n_edges, int64_t cap, kups_status *st) {
@@ -712,9 +771,17 @@ extern "C" int32_t kups_neighborlist_build(const double *positions, const int32_
     return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
   }
   KUPS_CUDA_TRY(bin_particles(w, positions, system, inclusion, exclusion, n, tril, cutoffs, s, status, stream));
-  pairs_kernel<<<(unsigned)w.pair_blocks, 32 * kPairWarps, 0, stream>>>(
-      system, inclusion, exclusion, n, n_incl, s, w.sys, w.frac, w.wrapped, w.cell_of, w.cell_start, w.cand,
-      w.cand_label, w.tickets + 2, w.pair_state, n_edges, edges, shifts, cap, status);
+  const PairSearch a{system,    inclusion,    exclusion, n,      n_incl,      s,      w.sys,
+                     w.frac, w.wrapped, w.cell_of, w.cell_start, w.cand, w.cand_label};
+  const int room = pair_room(cap, n);
+  // at most two groups for each block that can be resident: one wave, nothing to defer behind
+  const bool defer = w.pair_blocks > 8 * (int64_t)device_sm_count();
+  const size_t smem = sizeof(uint2) * (defer ? 2 : 1) * kPairWarps * (size_t)room;
+  KUPS_CUDA_TRY(cudaFuncSetAttribute(pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(sizeof(uint2) * 2 * kPairWarps * 512)));
+  const unsigned blocks = (unsigned)std::min<int64_t>(w.pair_blocks, 4 * (int64_t)device_sm_count());
+  pairs_kernel<<<blocks, 32 * kPairWarps, smem, stream>>>(a, room, defer, w.pair_blocks, w.tickets + 2, w.pair_state,
+                                                          n_edges, edges, shifts, cap, status);
   if (cap > 0) pad_kernel<<<pad_blocks(cap), 256, 0, stream>>>(n_edges, cap, n, edges, shifts);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }

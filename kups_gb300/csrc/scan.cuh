@@ -59,8 +59,8 @@ inline cudaError_t exclusive_scan(T *data, int64_t n, T *block_sums, T *total, c
 // Chained prefix over blocks that take their numbers from a ticket (a block's predecessors have
 // therefore started before it): state[b] holds a 2-bit flag above a 62-bit value, 0 = nothing yet,
 // 1 = the block's own sum, 2 = the sum of blocks 0..b, 3 = a predecessor's wait ran out.  The words
-// must be zero before the launch.  One full warp per block calls this; every lane returns the sum of
-// blocks 0..b-1.  The wait for a predecessor is bounded: when it runs out the block publishes flag 3,
+// must be zero before the launch.  A block first publishes its own sum, then (at once or after other
+// work) one full warp of it asks for the sum of blocks 0..b-1, which every lane returns.  The wait for a predecessor is bounded: when it runs out the block publishes flag 3,
 // so no later block waits on it, and ok comes back false.
 constexpr int kPrefixPolls = 1 << 22;
 
@@ -74,15 +74,16 @@ __device__ inline void prefix_store(unsigned long long *p, unsigned long long v)
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// Block b's own sum, before it goes on to other work; a full warp calls it.
+__device__ inline void chained_publish(unsigned long long *state, int64_t b, int64_t own) {
+  if ((threadIdx.x & 31) == 0) prefix_store(state + b, ((b == 0 ? 2ull : 1ull) << 62) | (unsigned long long)own);
+}
+
 __device__ inline int64_t chained_prefix(unsigned long long *state, int64_t b, int64_t own, bool &ok) {
   const int lane = threadIdx.x & 31;
   constexpr unsigned long long kValue = (1ull << 62) - 1;
   ok = true;
-  if (b == 0) {
-    if (lane == 0) prefix_store(state, (2ull << 62) | (unsigned long long)own);
-    return 0;
-  }
-  if (lane == 0) prefix_store(state + b, (1ull << 62) | (unsigned long long)own);
+  if (b == 0) return 0;
   int64_t sum = 0;
   for (int64_t top = b - 1;; top -= 32) {
     const int64_t at = top - lane;
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(kChainedThreads) chained_scan_kernel(int *data
   int ex = block_exclusive_scan<int>(own, scratch, &total);
   if (threadIdx.x < 32) {
     bool ok;
+    chained_publish(state, b, total);
     const int64_t before = chained_prefix(state, b, total, ok);
     if (threadIdx.x == 0) {
       base = before;
