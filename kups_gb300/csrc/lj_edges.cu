@@ -53,8 +53,8 @@ struct LjEval {
   }
 };
 
-// 264 k particles in 256 systems, 14 M directed edges, float32 pairs: 0.61 ms with PAIRED, 1.0 ms
-// without; one thread per edge with six atomics and seven float64 warp sums took 2.47 ms.
+// 264 k particles in 256 systems, 14 M directed edges, float32 pairs: 0.52 ms with PAIRED, 0.9 ms
+// without (0.61 and 1.0 ms with shifted and other edges mixed); one thread per edge with six atomics and seven float64 warp sums took 2.47 ms.
 template <typename R, bool PAIRED>
 __global__ void __launch_bounds__(32 * kRunWarps) lj_edges_kernel(PairList p, LjEval<R> ev) {
   ev.key = -1;

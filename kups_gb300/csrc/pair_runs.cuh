@@ -10,8 +10,11 @@
 //    component, an atomic per edge as much traffic again as the second particle's);
 //  * with PAIRED the list is known to hold every edge together with its reverse (what the neighbour
 //    list writes): only one of the two is evaluated, with twice its weight;
-//  * an image shift of 0 or +-1 times a cell vector is a selection and a sign, cells without
-//    off-diagonal entries add one term per axis, and dE/dtril is touched by shifted edges only.
+//  * edges with and without an image shift are collected apart, so that the shift's three float64
+//    additions and the six of dE/dtril are spent on shifted edges only, with every lane at work
+//    (mixed, 40 float64 instructions were issued per 32 pairs of which 17 lanes' worth did work);
+//    a shift of 0 or +-1 times a cell vector is a selection and a sign, and cells without
+//    off-diagonal entries add one term per axis.
 // Per-system sums leave as one atomic per warp while it stays in one system.
 #pragma once
 
@@ -42,15 +45,28 @@ __device__ inline double shift_times(int s, double v) {
   return __dmul_rn((double)s, v);
 }
 
+// (double)s, without a conversion (which takes the float64 pipe's time) for s in {-1, 0, 1}.
+__device__ inline double shift_double(int s) {
+  if (s >= -1 && s <= 1) return __hiloint2double(s == 0 ? 0 : 0x3ff00000 | (s & (int)0x80000000), 0);
+  return (double)s;
+}
+
 __device__ inline bool finite64(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+
+template <bool B>
+struct Const {
+  static constexpr bool value = B;
+};
 
 // Eval: load_system(s), load_first(i), and eval(e, j, r2, en, dedr2): energy and dE/d(r^2) of edge e.
 template <bool PAIRED, typename Eval>
 __device__ void run_pairs(const PairList &p, Eval &ev) {
-  __shared__ int q_i[kRunWarps][kRunQueue], q_j[kRunWarps][kRunQueue], q_s[kRunWarps][3][kRunQueue];
-  __shared__ int q_e[kRunWarps][kRunQueue];  // edge number from the warp's first (a report names it)
+  // edges to evaluate: [0] without a shift, [1] shifted; qe: the edge's number from the warp's first
+  // (a report names it)
+  __shared__ int q_i[kRunWarps][2][kRunQueue], q_j[kRunWarps][2][kRunQueue], q_e[kRunWarps][2][kRunQueue];
+  __shared__ int q_s[kRunWarps][3][kRunQueue];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int *qi = q_i[warp], *qj = q_j[warp], *q0 = q_s[warp][0], *q1 = q_s[warp][1], *q2 = q_s[warp][2], *qe = q_e[warp];
+  int *q0 = q_s[warp][0], *q1 = q_s[warp][1], *q2 = q_s[warp][2];
   const int64_t w = (int64_t)blockIdx.x * kRunWarps + warp;
   const int64_t e0 = w * p.edges_per_warp, e1 = min(p.n_edges, e0 + p.edges_per_warp);
   if (e0 >= e1) return;  // the same for the whole warp; no block barrier below
@@ -74,11 +90,19 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
     for (int a = 0; a < 6; ++a) dl[a] = 0.0;
     any_dl = false;
   };
-  // evaluates the first `count` queued edges, `per` consecutive ones per lane
-  auto evaluate = [&](int count, int per) {
+  // evaluates the first `count` edges of a queue, `per` consecutive ones per lane
+  auto evaluate = [&](auto shifted, int count, int per) {
+    constexpr bool kShifted = decltype(shifted)::value;
+    const int *qi = q_i[warp][kShifted], *qj = q_j[warp][kShifted], *qe = q_e[warp][kShifted];
     const int k1 = min(count, (lane + 1) * per);
     for (int k = lane * per; k < k1; ++k) {
-      const int i = qi[k], j = qj[k], s0 = q0[k], s1 = q1[k], s2 = q2[k];
+      const int i = qi[k], j = qj[k];
+      int s0 = 0, s1 = 0, s2 = 0;
+      if (kShifted) {
+        s0 = q0[k];
+        s1 = q1[k];
+        s2 = q2[k];
+      }
       if (i != fi) {
         flush_first();
         fi = i;
@@ -95,7 +119,7 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
       }
       const double *xj = p.pos + 3 * (int64_t)j;
       double d[3] = {xj[0] - xi[0], xj[1] - xi[1], xj[2] - xi[2]};
-      if (s0 | s1 | s2) {
+      if (kShifted) {
         double y0 = shift_times(s0, L.t[0]), y1 = shift_times(s1, L.t[2]), y2 = shift_times(s2, L.t[5]);
         if (skew) {
           y0 = __dadd_rn(__dadd_rn(y0, shift_times(s1, L.t[1])), shift_times(s2, L.t[3]));
@@ -116,9 +140,9 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
         atomicAdd(&p.grad[3 * (int64_t)j + a], h[a]);
         gi[a] -= h[a];
       }
-      if ((s0 | s1 | s2) || !(finite64(h[0]) && finite64(h[1]) && finite64(h[2]))) {
+      if (kShifted || !(finite64(h[0]) && finite64(h[1]) && finite64(h[2]))) {
         any_dl = true;
-        const double t0 = s0, t1 = s1, t2 = s2;
+        const double t0 = shift_double(s0), t1 = shift_double(s1), t2 = shift_double(s2);
         dl[0] += t0 * h[0];
         dl[1] += t1 * h[0];
         dl[2] += t1 * h[1];
@@ -128,7 +152,29 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
       }
     }
   };
-  int queued = 0;
+  int queued[2] = {0, 0};
+  // the first 128 of a queue, then the rest moves to the front (at most 127 entries)
+  auto drain = [&](auto shifted) {
+    constexpr bool kShifted = decltype(shifted)::value;
+    evaluate(shifted, 128, 4);
+    __syncwarp();
+    const int rest = queued[kShifted] - 128;
+    int *qi = q_i[warp][kShifted], *qj = q_j[warp][kShifted], *qe = q_e[warp][kShifted];
+    for (int k = lane; k < rest; k += 32) {
+      qi[k] = qi[128 + k];
+      qj[k] = qj[128 + k];
+      qe[k] = qe[128 + k];
+      if (kShifted) {
+        q0[k] = q0[128 + k];
+        q1[k] = q1[128 + k];
+        q2[k] = q2[128 + k];
+      }
+    }
+    queued[kShifted] = rest;
+    __syncwarp();
+  };
+  const Const<false> plain;
+  const Const<true> shifted;
   for (int64_t base = e0; base < e1; base += 128) {
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
@@ -150,37 +196,29 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
         // a particle and its own images: the shift that is lexicographically positive
         if (PAIRED && i == j) take = take && (s0 > 0 || (s0 == 0 && (s1 > 0 || (s1 == 0 && s2 > 0))));
       }
-      const unsigned m = __ballot_sync(0xffffffffu, take);
+      const int kind = (s0 | s1 | s2) != 0;
+      const unsigned m1 = __ballot_sync(0xffffffffu, take && kind == 1);
+      const unsigned m0 = __ballot_sync(0xffffffffu, take && kind == 0);
       if (take) {
-        const int at = queued + __popc(m & ((1u << lane) - 1u));
-        qi[at] = i;
-        qj[at] = j;
-        q0[at] = s0;
-        q1[at] = s1;
-        q2[at] = s2;
-        qe[at] = (int)(e - e0);
+        const int at = (kind ? queued[1] : queued[0]) + __popc((kind ? m1 : m0) & ((1u << lane) - 1u));
+        q_i[warp][kind][at] = i;
+        q_j[warp][kind][at] = j;
+        q_e[warp][kind][at] = (int)(e - e0);
+        if (kind) {
+          q0[at] = s0;
+          q1[at] = s1;
+          q2[at] = s2;
+        }
       }
-      queued += __popc(m);
+      queued[0] += __popc(m0);
+      queued[1] += __popc(m1);
     }
     __syncwarp();
-    if (queued >= 128) {
-      evaluate(128, 4);
-      __syncwarp();
-      // the rest moves to the front (at most 127 entries, each lane its own positions)
-      const int rest = queued - 128;
-      for (int k = lane; k < rest; k += 32) {
-        qi[k] = qi[128 + k];
-        qj[k] = qj[128 + k];
-        q0[k] = q0[128 + k];
-        q1[k] = q1[128 + k];
-        q2[k] = q2[128 + k];
-        qe[k] = qe[128 + k];
-      }
-      queued = rest;
-      __syncwarp();
-    }
+    if (queued[0] >= 128) drain(plain);
+    if (queued[1] >= 128) drain(shifted);
   }
-  evaluate(queued, (queued + 31) / 32);
+  evaluate(plain, queued[0], (queued[0] + 31) / 32);
+  evaluate(shifted, queued[1], (queued[1] + 31) / 32);
   flush_first();
   // one system in the whole warp (lanes without an edge have none): summed over the warp first
   const int top = __reduce_max_sync(0xffffffffu, sys);
