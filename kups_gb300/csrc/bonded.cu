@@ -32,9 +32,11 @@
 // p = b1.b2 / |b2|^2, q = b3.b2 / |b2|^2.  Inversion: derivatives of
 // sin w = (v1 . n / (|n| + eps)) / (|v1| + eps), n = v2 x v3, with the
 // reference's 1e-10 regularisers kept.
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
+#include "pair_runs.cuh"
 
 namespace kups {
 namespace {
@@ -67,11 +69,98 @@ struct Kind<4> { static constexpr int order = 4, params = 3; };  // dihedral: V,
 template <>
 struct Kind<5> { static constexpr int order = 4, params = 2; };  // inversion: omega0, k
 
-// Energy of one edge and g[m] = dE/dv_{m+1}.
+// What an edge's parameter row contributes, formed once per row (block) instead of once per edge:
+// the trigonometry of equilibrium angles and the force constants' factors.
+//   0: x0, k   1: r0, D, alpha   2: theta0, k
+//   3: linear (0 / 1), k, then (float64) k c0, k c1, k c2 of k (c0 + c1 c + c2 (2 c^2 - 1)),
+//      (float32) cos theta0, 2 k c2, 4 k c2 of 2 k c2 (c - cos theta0)^2
+//   4: V / 2, n, cos(n phi0), V / 2 cos(n phi0) n, n as a small integer (0: none)
+//   5: (float64) ks c0, ks c1, ks c2; (float32) planar (0 / 1), k, omega0, 8 ks c2
+constexpr int kRowConsts = 5;
+
+template <int KIND, typename R>
+__device__ inline void row_constants(const double *raw, R c[kRowConsts]) {
+  R p[Kind<KIND>::params];
+  for (int k = 0; k < Kind<KIND>::params; ++k) p[k] = (R)raw[k];
+  for (int k = 0; k < kRowConsts; ++k) c[k] = k < Kind<KIND>::params ? p[k] : R(0.0);
+  if (KIND == 3) {
+    const R th0 = p[0], k = p[1];
+    c[0] = fabs(th0 - R(M_PI)) < p[2] ? R(1.0) : R(0.0);
+    const R s2 = sin(th0) * sin(th0), ct0 = cos(th0);
+    const R c2 = R(1.0) / (R(4.0) * fmax(s2, R(1e-10)));
+    if (sizeof(R) == 4) {
+      c[2] = ct0;
+      c[3] = R(2.0) * k * c2;
+      c[4] = R(4.0) * k * c2;
+    } else {
+      c[2] = k * (c2 * (R(2.0) * ct0 * ct0 + R(1.0)));
+      c[3] = k * (-R(4.0) * c2 * ct0);
+      c[4] = k * c2;
+    }
+  } else if (KIND == 4) {
+    const R V = p[0], per = p[1], cp = cos(per * p[2]);
+    c[0] = R(0.5) * V;
+    c[2] = cp;
+    c[3] = R(0.5) * V * cp * per;
+    c[4] = per == R(1.0) || per == R(2.0) || per == R(3.0) || per == R(4.0) || per == R(6.0) ? per : R(0.0);
+  } else if (KIND == 5) {
+    const R om0 = p[0], k = p[1];
+    const bool planar = fabs(om0) < R(1e-6);
+    const R s2 = sin(om0) * sin(om0);
+    if (sizeof(R) == 4) {
+      const R h0 = sin(R(0.5) * om0);
+      const R c2 = R(1.0) / (R(4.0) * (s2 > R(1e-10) ? s2 : R(1.0)));
+      const R ks = k / fmax(R(8.0) * c2 * h0 * h0 * h0 * h0, R(1e-10));
+      c[0] = planar ? R(1.0) : R(0.0);
+      c[1] = k;
+      c[2] = om0;
+      c[3] = R(8.0) * ks * c2;
+    } else {
+      const R cw0 = cos(om0);
+      const R c2 = planar ? R(0.0) : R(1.0) / (R(4.0) * (s2 > R(1e-10) ? s2 : R(1.0)));
+      const R c1 = planar ? -R(1.0) : -R(4.0) * c2 * cw0;
+      const R c0 = planar ? R(1.0) : c2 * (R(2.0) * cw0 * cw0 + R(1.0));
+      const R ks = planar ? k : k / fmax(c0 + c1 + c2, R(1e-10));
+      c[0] = ks * c0;
+      c[1] = ks * c1;
+      c[2] = ks * c2;
+    }
+  }
+}
+
+// sqrt(x) and 1 / sqrt(x) of x > 0 from one reciprocal root (the root corrected to its last bit), a
+// third of the float64 instructions of a root and a division.
+__device__ inline double root64(double x, double &inv) {
+  inv = rsqrt(x);
+  const double r = x * inv;
+  return fma(0.5 * inv, fma(-r, r, x), r);
+}
+
+// Tests of float64 values by their bits: a float64 comparison, minimum or conversion takes the
+// float64 pipe like an addition.
+__device__ inline bool positive64(double x) { return __double_as_longlong(x) > 0; }
+__device__ inline int exponent64(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }  // biased by 1023
+__device__ inline double clamp_unit(double c) {  // c to [-1, 1] (a NaN to an end)
+  const int hi = __double2hiint(c);
+  return (hi & 0x7fffffff) >= 0x3ff00000 ? __hiloint2double(0x3ff00000 | (hi & (int)0x80000000), 0) : c;
+}
+
+// x / (sqrt(x) + eps) and 1 / (sqrt(x) + eps) from inv = 1 / sqrt(x), eps = 1e-10: eps / sqrt(x) = u
+// is below 1e-7 from x = 2^-19 on, where 1 / (1 + u) = 1 - u + u^2 to 1e-21; a division below that.
+__device__ inline double inverse_regularised(double root, double inv) {
+  if (exponent64(root) < 1023 - 10) return 1.0 / (root + kEps);
+  const double u = kEps * inv;
+  return fma(inv, fma(u, u, -u), inv);
+}
+
+// Energy of one edge and g[m] = dE/dv_{m+1}; p the row's constants.
 template <int KIND, typename R>
 __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
   if (KIND == 0 || KIND == 1) {
-    const R r = sqrt(dot3(v[0], v[0]));
+    const R rr = dot3(v[0], v[0]);
+    R r, inv = R(0.0);
+    if (sizeof(R) == 8) r = rr > R(0.0) ? (R)root64((double)rr, (double &)inv) : R(0.0);
+    else r = sqrt(rr);
     R e, dedr;
     if (KIND == 0) {
       e = (r - p[0]) * (r - p[0]) * p[1];
@@ -81,7 +170,7 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
       e = p[1] * (R(1.0) - x) * (R(1.0) - x);
       dedr = R(2.0) * p[1] * (R(1.0) - x) * p[2] * x;
     }
-    const R f = r > R(0.0) ? dedr / r : R(0.0);
+    const R f = sizeof(R) == 8 ? dedr * inv : (r > R(0.0) ? dedr / r : R(0.0));
     for (int a = 0; a < 3; ++a) g[0][a] = f * v[0][a];
     return e;
   } else if ((KIND == 2 || KIND == 3) && sizeof(R) == 4) {
@@ -105,15 +194,14 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
       // k (c0 + c1 c + c2 (2c^2 - 1)) = 2 k c2 (c - cos theta0)^2
       const R r12 = sqrt(r1s * r2s), c = cs / r12;
       const R cc = fmin(fmax(c, -R(1.0)), R(1.0));
-      const R th0 = p[0], k = p[1];
       R dedc;
-      if (fabs(th0 - R(M_PI)) < p[2]) {
-        e = k * (R(1.0) + cc);
-        dedc = k;
+      if (p[0] != R(0.0)) {
+        e = p[1] * (R(1.0) + cc);
+        dedc = p[1];
       } else {
-        const R c2 = R(1.0) / (R(4.0) * fmax(sin(th0) * sin(th0), R(1e-10))), d = cc - cos(th0);
-        e = R(2.0) * k * c2 * d * d;
-        dedc = R(4.0) * k * c2 * d;
+        const R d = cc - p[2];
+        e = p[3] * d * d;
+        dedc = p[4] * d;
       }
       if (fabs(c) > R(1.0)) dedc = R(0.0);
       f1 = -dedc / (r1s * r12);
@@ -125,35 +213,101 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
     }
     return e;
   } else if (KIND == 2 || KIND == 3) {
-    const R r1 = sqrt(dot3(v[0], v[0])), r2 = sqrt(dot3(v[1], v[1]));
-    const R c = dot3(v[0], v[1]) / (r1 * r2);
+    // one reciprocal root per length and one of 1 - cos^2, which serves the gradient and, as
+    // theta = pi / 2 - atan(cot theta), the angle (arccos takes two branches, both by most warps)
+    const R i1 = rsqrt(dot3(v[0], v[0])), i2 = rsqrt(dot3(v[1], v[1])), i12 = i1 * i2;
+    const R c = dot3(v[0], v[1]) * i12;
     R e, dedc;
     if (KIND == 2) {
       // the reference takes arccos of the unclipped cosine; clamping keeps
       // round-off above 1 from turning a straight angle into NaN
-      const R cc = fmin(fmax(c, -R(1.0)), R(1.0));
-      const R th = acos(cc) * (R(180.0) / R(M_PI));
-      e = (th - p[0]) * (th - p[0]) * p[1];
-      dedc = -R(2.0) * p[1] * (th - p[0]) * (R(180.0) / R(M_PI)) / sqrt(fmax(R(1.0) - cc * cc, R(1e-30)));
+      const double cc = clamp_unit((double)c);
+      double w = fma(-cc, cc, 1.0);
+      if (exponent64(w) < 1023 - 100) w = 1e-30;
+      const double is = rsqrt(w);
+      const double th = (M_PI / 2 - atan(cc * is)) * (180.0 / M_PI), d = th - (double)p[0];
+      e = (R)(d * d * (double)p[1]);
+      dedc = (R)((-2.0 * 180.0 / M_PI) * (double)p[1] * d * is);
     } else {
-      const R cc = fmin(fmax(c, -R(1.0)), R(1.0));
-      const R th0 = p[0], k = p[1];
-      if (fabs(th0 - R(M_PI)) < p[2]) {
-        e = k * (R(1.0) + cc);
-        dedc = k;
+      const double cc = clamp_unit((double)c);
+      if (__double2hiint((double)p[0]) != 0) {
+        e = (R)((double)p[1] * (1.0 + cc));
+        dedc = p[1];
       } else {
-        const R s2 = sin(th0) * sin(th0), ct0 = cos(th0);
-        const R c2 = R(1.0) / (R(4.0) * fmax(s2, R(1e-10)));
-        const R c1 = -R(4.0) * c2 * ct0, c0 = c2 * (R(2.0) * ct0 * ct0 + R(1.0));
-        e = k * (c0 + c1 * cc + c2 * (R(2.0) * cc * cc - R(1.0)));
-        dedc = k * (c1 + R(4.0) * c2 * cc);
+        e = (R)((double)p[2] + (double)p[3] * cc + (double)p[4] * (2.0 * cc * cc - 1.0));
+        dedc = (R)((double)p[3] + 4.0 * (double)p[4] * cc);
       }
       if (fabs(c) > R(1.0)) dedc = R(0.0);  // clipped: no gradient
     }
-    const R i12 = R(1.0) / (r1 * r2);
+    const R f12 = dedc * i12, fc = -dedc * c, f1 = fc * i1 * i1, f2 = fc * i2 * i2;
     for (int a = 0; a < 3; ++a) {
-      g[0][a] = dedc * (v[1][a] * i12 - c * v[0][a] / (r1 * r1));
-      g[1][a] = dedc * (v[0][a] * i12 - c * v[1][a] / (r2 * r2));
+      g[0][a] = f12 * v[1][a] + f1 * v[0][a];
+      g[1][a] = f12 * v[0][a] + f2 * v[1][a];
+    }
+    return e;
+  } else if (KIND == 4 && sizeof(R) == 8) {
+    // tan phi = |b2|^2 (b1 . n) / (|b2| + eps) : m . n, since m x n = b2 (b1 . n) and the regularised
+    // lengths of m and n are common positive factors
+    R b2[3], b3[3], m[3], n[3];
+    const R *b1 = v[0];
+    for (int a = 0; a < 3; ++a) {
+      b2[a] = v[1][a] - v[0][a];
+      b3[a] = v[2][a] - v[1][a];
+    }
+    cross3(b1, b2, m);
+    cross3(b2, b3, n);
+    const R mm = dot3(m, m), nn = dot3(n, n), l2 = dot3(b2, b2);
+    const bool bent = positive64((double)mm) && positive64((double)nn) && positive64((double)l2);
+    double ilb = 0.0;
+    const R lb = bent ? (R)root64((double)l2, ilb) : R(0.0);
+    R y = R(0.0), x = R(0.0);
+    if (bent) {
+      y = l2 * dot3(b1, n) * (R)inverse_regularised((double)lb, ilb);
+      x = dot3(m, n);
+    }
+    R cn, sn;  // cos and sin of n phi
+    const R h2 = x * x + y * y;
+    const int small_n = __double2hiint((double)p[4]), eh = exponent64((double)h2);
+    if (small_n != 0 && eh > 100 && eh < 1946) {
+      // integer n: the n-th power of (cos phi, sin phi), no inverse tangent and no sine
+      const R ih = rsqrt(h2), c = x * ih, s = y * ih;
+      const int per = small_n == 0x3ff00000   ? 1
+                      : small_n == 0x40000000 ? 2
+                      : small_n == 0x40080000 ? 3
+                      : small_n == 0x40100000 ? 4
+                                              : 6;
+      cn = c;
+      sn = s;
+      if (per == 2 || per == 4 || per == 6) {
+        cn = c * c - s * s;
+        sn = R(2.0) * c * s;
+      }
+      const R c1 = cn, s1 = sn;
+      if (per == 4) {
+        cn = c1 * c1 - s1 * s1;
+        sn = R(2.0) * c1 * s1;
+      } else if (per == 3 || per == 6) {
+        const R c2 = c1 * c1 - s1 * s1, s2 = R(2.0) * c1 * s1;
+        cn = c2 * c1 - s2 * s1;
+        sn = s2 * c1 + c2 * s1;
+      }
+    } else {
+      sincos((double)(p[1] * atan2(y, x)), (double *)&sn, (double *)&cn);
+    }
+    const R e = p[0] * (R(1.0) - p[2] * cn);
+    if (bent) {
+      const R dedphi = p[3] * sn, il2 = (R)(ilb * ilb);
+      const R pp = dot3(b1, b2) * il2, qq = dot3(b3, b2) * il2;
+      const R f = dedphi * lb, fi = -f * (R)__drcp_rn((double)mm), fl = f * (R)__drcp_rn((double)nn);
+      for (int a = 0; a < 3; ++a) {
+        const R di = fi * m[a], dl = fl * n[a];
+        g[0][a] = -(R(1.0) + pp) * di + qq * dl;
+        g[1][a] = pp * di - (R(1.0) + qq) * dl;
+        g[2][a] = dl;
+      }
+    } else {
+      for (int k = 0; k < 3; ++k)
+        for (int a = 0; a < 3; ++a) g[k][a] = R(0.0);
     }
     return e;
   } else if (KIND == 4) {
@@ -176,9 +330,9 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
     }
     cross3(n1, n2, x);
     const R phi = atan2(dot3(x, bn), dot3(n1, n2));
-    const R V = p[0], per = p[1], phi0 = p[2];
-    const R e = R(0.5) * V * (R(1.0) - cos(per * phi0) * cos(per * phi));
-    const R dedphi = R(0.5) * V * cos(per * phi0) * per * sin(per * phi);
+    const R per = p[1];
+    const R e = p[0] * (R(1.0) - p[2] * cos(per * phi));
+    const R dedphi = p[3] * sin(per * phi);
     if (mm > R(0.0) && nn > R(0.0) && lb > R(0.0)) {
       const R pp = dot3(b1, b2) / (lb * lb), qq = dot3(b3, b2) / (lb * lb);
       for (int a = 0; a < 3; ++a) {
@@ -206,21 +360,18 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
     cross3(v[0], u, vu);
     const R nn = dot3(n, n), la2 = dot3(v[0], v[0]), an = dot3(v[0], n), lu = sqrt(dot3(u, u));
     const R w = atan2(an, lu);
-    const R om0 = p[0], k = p[1];
+    const R om0 = p[2], k = p[1];
     const R den = nn * la2;
     const R sw = den > R(0.0) ? an * rsqrt(den) : R(0.0);
     R e, dedw;
-    if (fabs(om0) < R(1e-6)) {
+    if (p[0] != R(0.0)) {
       const R h = sin(R(0.5) * w);
       e = R(2.0) * k * h * h;  // k (1 - cos w)
       dedw = k * sw;
     } else {
-      const R s2 = sin(om0) * sin(om0), h0 = sin(R(0.5) * om0);
-      const R c2 = R(1.0) / (R(4.0) * (s2 > R(1e-10) ? s2 : R(1.0)));
-      const R ks = k / fmax(R(8.0) * c2 * h0 * h0 * h0 * h0, R(1e-10));
       const R X = sin(R(0.5) * (w + om0)) * sin(R(0.5) * (w - om0));
-      e = R(8.0) * ks * c2 * X * X;
-      dedw = R(8.0) * ks * c2 * X * sw;
+      e = p[3] * X * X;
+      dedw = p[3] * X * sw;
     }
     const R f = den > R(0.0) ? dedw / den : R(0.0);
     const R q = lu > R(0.0) ? an / lu : R(0.0);
@@ -235,122 +386,285 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
     for (int a = 0; a < 3; ++a) g[2][a] = t[a];
     return e;
   } else {
+    // w = asin s lies in [-pi/2, pi/2]: cos w = sqrt(1 - s^2), cos 2w = 1 - 2 s^2, sin 2w = 2 s cos w
     R n[3];
     cross3(v[1], v[2], n);
-    const R ln = sqrt(dot3(n, n)), la = sqrt(dot3(v[0], v[0]));
-    const R an = dot3(v[0], n);
-    const R s_raw = an / (ln + R(kEps)) / (la + R(kEps));
-    const R s = fmin(fmax(s_raw, -R(1.0)), R(1.0));
-    const R w = asin(s);
-    const R om0 = p[0], k = p[1];
-    const bool sp2 = fabs(om0) < R(1e-6);
-    const R s2 = sin(om0) * sin(om0), cw0 = cos(om0);
-    const R c2 = sp2 ? R(0.0) : R(1.0) / (R(4.0) * (s2 > R(1e-10) ? s2 : R(1.0)));
-    const R c1 = sp2 ? -R(1.0) : -R(4.0) * c2 * cw0;
-    const R c0 = sp2 ? R(1.0) : c2 * (R(2.0) * cw0 * cw0 + R(1.0));
-    const R ks = sp2 ? k : k / fmax(c0 + c1 + c2, R(1e-10));
-    const R e = ks * (c0 + c1 * cos(w) + c2 * cos(R(2.0) * w));
-    const R dedw = ks * (-c1 * sin(w) - R(2.0) * c2 * sin(R(2.0) * w));
-    const R deds = fabs(s_raw) <= R(1.0) ? dedw / sqrt(fmax(R(1.0) - s * s, R(1e-30))) : R(0.0);
+    const R nn = dot3(n, n), aa = dot3(v[0], v[0]), an = dot3(v[0], n);
+    double iln = 1.0, ila = 1.0;
+    const R ln = positive64((double)nn) ? (R)root64((double)nn, iln) : R(0.0);
+    const R la = positive64((double)aa) ? (R)root64((double)aa, ila) : R(0.0);
+    const R inv_la = (R)inverse_regularised((double)la, ila), inv_ln = (R)inverse_regularised((double)ln, iln);
+    const double s_raw = (double)(an * inv_ln * inv_la), s = clamp_unit(s_raw);
+    const double w2 = fma(-s, s, 1.0), icw = rsqrt(exponent64(w2) < 1023 - 100 ? 1e-30 : w2), cw = w2 * icw;
+    const R e = (R)((double)p[0] + (double)p[1] * cw + (double)p[2] * (w2 - s * s));
+    const R deds = fabs(s_raw) <= 1.0 ? (R)(-s * ((double)p[1] + 4.0 * (double)p[2] * cw) * icw) : R(0.0);
     // ds/dv1 and ds/dn; dn/dv2 (x) and dn/dv3 (x) through the cross product
+    const R f = deds * inv_la * inv_ln, f0 = -f * an * inv_la * (R)ila, f1 = -f * an * inv_ln * (R)iln;
     R wv[3], t[3];
-    const R inv_la = R(1.0) / (la + R(kEps)), inv_ln = R(1.0) / (ln + R(kEps));
     for (int a = 0; a < 3; ++a) {
-      const R nu = n[a] * inv_ln;
-      g[0][a] = deds * (nu * inv_la - (an * inv_ln) * inv_la * inv_la / (la > R(0.0) ? la : R(1.0)) * v[0][a]);
-      wv[a] = (v[0][a] * inv_ln - an * inv_ln * inv_ln / (ln > R(0.0) ? ln : R(1.0)) * n[a]) * inv_la;
+      g[0][a] = f * n[a] + f0 * v[0][a];
+      wv[a] = f * v[0][a] + f1 * n[a];
     }
     cross3(v[2], wv, t);
-    for (int a = 0; a < 3; ++a) g[1][a] = deds * t[a];
+    for (int a = 0; a < 3; ++a) g[1][a] = t[a];
     cross3(wv, v[1], t);
-    for (int a = 0; a < 3; ++a) g[2][a] = deds * t[a];
+    for (int a = 0; a < 3; ++a) g[2][a] = t[a];
     return e;
   }
 }
 
-// add_system for a float or double value: the warp's sum in R, added to the float64 array.
-template <typename R>
-__device__ inline void add_system_r(double *arr, int stride, int comp, int sys, R v) {
-  const unsigned full = 0xffffffffu;
-  const int s0 = __shfl_sync(full, sys, 0);
-  if (__all_sync(full, sys == s0)) {
-    v = warp_sum(v);
-    if ((threadIdx.x & 31) == 0 && sys >= 0) atomicAdd(&arr[(int64_t)sys * stride + comp], (double)v);
-  } else if (sys >= 0) {
-    atomicAdd(&arr[(int64_t)sys * stride + comp], (double)v);
+// Running per-system sums of one lane (float64 mode) or one warp (float32 mode: lane 0 holds the
+// float64 total of the warps' float sums of 32 edges), added to the caller's arrays when the system
+// changes and at the end.
+struct SystemSums {
+  int sys;
+  double en, dl[6];
+
+  __device__ void flush(double *energy, double *grad_tril) {
+    if (sys >= 0) {
+      atomicAdd(&energy[sys], en);
+      if (grad_tril != nullptr)
+        for (int k = 0; k < 6; ++k)
+          if (dl[k] != 0.0) atomicAdd(&grad_tril[6 * (int64_t)sys + k], dl[k]);
+    }
+    clear(-1);
   }
+  __device__ void clear(int s) {
+    sys = s;
+    en = 0.0;
+    for (int k = 0; k < 6; ++k) dl[k] = 0.0;
+  }
+};
+
+__device__ inline bool is_finite(double v) { return finite64(v); }
+__device__ inline bool is_finite(float v) { return (__float_as_int(v) & 0x7f800000) != 0x7f800000; }
+
+template <typename R>
+__device__ inline R shift_real(int s);
+template <>
+__device__ inline double shift_real<double>(int s) { return shift_double(s); }
+template <>
+__device__ inline float shift_real<float>(int s) { return (float)s; }
+
+constexpr int kBondedThreads = 128, kRowTable = 256;  // parameter rows kept in shared memory
+
+struct BondedArgs {
+  const double *pos;
+  const int32_t *system, *species;
+  int64_t n;
+  const double *tril;
+  int32_t n_sys;
+  const int32_t *edges, *shifts;
+  int64_t n_edges;
+  const double *params;
+  int32_t nsp;
+  int n_rows, per;
+  double *energy, *grad, *grad_tril;
+  kups_status *status;
+};
+
+// Atoms, parameter row and system of edge e; false (status recorded) for an index, species or system
+// out of range.
+template <int D>
+__device__ inline bool bonded_atoms(const BondedArgs &a, int64_t e, int idx[D], int64_t &row, int &sys) {
+  bool ok = true;
+  for (int d = 0; d < D; ++d) {
+    idx[d] = a.edges[(int64_t)D * e + d];
+    ok &= idx[d] >= 0 && idx[d] < a.n;
+  }
+  row = 0;
+  if (ok)
+    for (int d = 0; d < D; ++d) {
+      const int k = a.species[idx[d]];
+      ok &= k >= 0 && k < a.nsp;
+      row = row * a.nsp + k;
+    }
+  sys = ok ? a.system[idx[0]] : -1;
+  if (sys < 0 || sys >= a.n_sys) {
+    status_error(a.status, KUPS_ERR_INVALID, e);
+    sys = -1;
+    return false;
+  }
+  return true;
 }
 
+template <int D>
+__device__ inline bool bonded_shifts(const BondedArgs &a, int64_t e, int sh[D - 1][3]) {
+  int any = 0;
+  for (int m = 0; m < D - 1; ++m)
+    for (int k = 0; k < 3; ++k) {
+      sh[m][k] = a.shifts[((int64_t)(D - 1) * e + m) * 3 + k];
+      any |= sh[m][k];
+    }
+  return any != 0;
+}
+
+// Energy of edge e with its gradient added to the atoms; `shifted`: some sh is not zero, and dl
+// receives sum_m s_ma g_mb (also for a non-finite gradient, which reaches dE/dtril through a zero
+// shift).  Returns whether dl was set.
 template <int KIND, typename R>
-__global__ void bonded_kernel(const double *pos, const int32_t *system, const int32_t *species, int64_t n,
-                              const double *tril, int32_t n_sys, const int32_t *edges, const int32_t *shifts,
-                              int64_t n_edges, const double *params, int32_t nsp, double *energy, double *grad,
-                              double *grad_tril, kups_status *status) {
+__device__ inline bool bonded_edge(const BondedArgs &a, const R (*table)[kRowConsts], int64_t e, const int *idx,
+                                   int64_t row, int sys, const int (*sh)[3], bool shifted, R &en, R dl[6]) {
   constexpr int D = Kind<KIND>::order, P = Kind<KIND>::params;
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int sys = -1;
-  R en = R(0.0), dl[6] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)};
-  if (e < n_edges) {
-    int idx[D];
-    bool ok = true;
-    int64_t row = 0;
-    for (int d = 0; d < D; ++d) {
-      idx[d] = edges[(int64_t)D * e + d];
-      ok &= idx[d] >= 0 && idx[d] < n;
+  // difference vectors in float64 (positions are float64), then the edge's arithmetic in R
+  R v[D - 1][3], g[D - 1][3], own[kRowConsts];
+  const double *x0 = a.pos + 3 * (int64_t)idx[0];
+  const double o[3] = {x0[0], x0[1], x0[2]};
+  Tril64 L;
+  if (shifted) L = load_tril64(a.tril + 6 * (int64_t)sys);
+  for (int m = 0; m < D - 1; ++m) {
+    const double *xm = a.pos + 3 * (int64_t)idx[m + 1];
+    double d[3] = {xm[0] - o[0], xm[1] - o[1], xm[2] - o[2]};
+    if (shifted && (sh[m][0] | sh[m][1] | sh[m][2])) {
+      double sL[3];
+      shift_vector(sh[m], L, sL);
+      for (int k = 0; k < 3; ++k) d[k] += sL[k];
     }
-    if (ok) {
-      for (int d = 0; d < D; ++d) {
-        const int t = species[idx[d]];
-        ok &= t >= 0 && t < nsp;
-        row = row * nsp + t;
-      }
-    }
-    const int s0 = ok ? system[idx[0]] : -1;
-    if (!ok || s0 < 0 || s0 >= n_sys) {
-      status_error(status, KUPS_ERR_INVALID, e);
-    } else {
-      sys = s0;
-      const Tril64 L = load_tril64(tril + 6 * (int64_t)s0);
-      // difference vectors in float64 (positions are float64), then the edge's arithmetic in R
-      R v[D - 1][3], g[D - 1][3], pr[P];
-      int sh[D - 1][3];
-      const double *x0 = pos + 3 * (int64_t)idx[0];
-      for (int m = 0; m < D - 1; ++m) {
-        for (int a = 0; a < 3; ++a) sh[m][a] = shifts[((int64_t)(D - 1) * e + m) * 3 + a];
-        // s @ L only for a non-zero shift (zero adds nothing: same result)
-        double sL[3] = {0.0, 0.0, 0.0};
-        if (sh[m][0] | sh[m][1] | sh[m][2]) {
-          const double shd[3] = {(double)sh[m][0], (double)sh[m][1], (double)sh[m][2]};
-          row_times_tril64(shd, L, sL);
-        }
-        for (int a = 0; a < 3; ++a) v[m][a] = (R)(pos[3 * (int64_t)idx[m + 1] + a] - x0[a] + sL[a]);
-      }
-      for (int k = 0; k < P; ++k) pr[k] = (R)params[row * P + k];
-      en = edge_energy_grad<KIND, R>(v, pr, g);
-      bool finite = isfinite(en);
-      for (int m = 0; m < D - 1; ++m)
-        for (int a = 0; a < 3; ++a) finite &= isfinite(g[m][a]);
-      if (!finite) status_error(status, KUPS_ERR_NONFINITE, e);
-      R g0[3] = {R(0.0), R(0.0), R(0.0)};  // atom 0 takes -sum_m g_m in one atomic per axis
-      for (int m = 0; m < D - 1; ++m) {
-        for (int a = 0; a < 3; ++a) {
-          atomicAdd(&grad[3 * (int64_t)idx[m + 1] + a], (double)g[m][a]);
-          g0[a] -= g[m][a];
-        }
-        dl[0] += R(sh[m][0]) * g[m][0];
-        dl[1] += R(sh[m][1]) * g[m][0];
-        dl[2] += R(sh[m][1]) * g[m][1];
-        dl[3] += R(sh[m][2]) * g[m][0];
-        dl[4] += R(sh[m][2]) * g[m][1];
-        dl[5] += R(sh[m][2]) * g[m][2];
-      }
-      for (int a = 0; a < 3; ++a) atomicAdd(&grad[3 * (int64_t)idx[0] + a], (double)g0[a]);
-    }
+    for (int k = 0; k < 3; ++k) v[m][k] = (R)d[k];
   }
-  // warp sums in R (float32 mode: float, the warp total added in float64), one atomic per warp
-  add_system_r<R>(energy, 1, 0, sys, en);
-  if (grad_tril != nullptr)
-    for (int k = 0; k < 6; ++k) add_system_r<R>(grad_tril, 6, k, sys, dl[k]);
+  const R *c = table[a.n_rows > 0 ? row : 0];
+  if (a.n_rows == 0) {  // more rows than the table holds
+    row_constants<KIND, R>(a.params + row * P, own);
+    c = own;
+  }
+  en = edge_energy_grad<KIND, R>(v, c, g);
+  bool finite = is_finite(en);
+  for (int m = 0; m < D - 1; ++m)
+    for (int k = 0; k < 3; ++k) finite &= is_finite(g[m][k]);
+  if (!finite) status_error(a.status, KUPS_ERR_NONFINITE, e);
+  R g0[3] = {R(0.0), R(0.0), R(0.0)};  // atom 0 takes -sum_m g_m in one atomic per axis
+  for (int m = 0; m < D - 1; ++m)
+    for (int k = 0; k < 3; ++k) {
+      atomicAdd(&a.grad[3 * (int64_t)idx[m + 1] + k], (double)g[m][k]);
+      g0[k] -= g[m][k];
+    }
+  for (int k = 0; k < 3; ++k) atomicAdd(&a.grad[3 * (int64_t)idx[0] + k], (double)g0[k]);
+  if (!shifted && finite) return false;
+  for (int m = 0; m < D - 1; ++m) {
+    const R t[3] = {shift_real<R>(sh[m][0]), shift_real<R>(sh[m][1]), shift_real<R>(sh[m][2])};
+    dl[0] += t[0] * g[m][0];
+    dl[1] += t[1] * g[m][0];
+    dl[2] += t[1] * g[m][1];
+    dl[3] += t[2] * g[m][0];
+    dl[4] += t[2] * g[m][1];
+    dl[5] += t[2] * g[m][2];
+  }
+  return true;
+}
+
+// A warp takes `per` groups of 32 consecutive edges.  Float64 mode is bound by the float64 pipe (2
+// operations per clock per SM): edges with an image shift are put aside and evaluated 32 at a time,
+// so that the shift vectors and dE/dtril (27 operations per difference vector) cost nothing for the
+// others, and the per-system sums leave as one warp sum at the end (one for every 32 edges was 35 of a
+// bond's 111 float64 instructions).  Float32 mode sums each 32 edges in float, as its callers' results
+// have always been rounded, and adds those totals in float64.
+// 5.2e5 edges of each kind, float64: 66 us (bonds), 187 (angles), 228 (dihedrals), 208 (inversions);
+// with a division or root for every quotient, trigonometry of the row's constants per edge and the
+// angle taken through acos / atan2 / asin and back: 99, 281, 443 and 438 us.
+template <int KIND, typename R>
+__global__ void __launch_bounds__(kBondedThreads) bonded_kernel(BondedArgs a) {
+  constexpr int D = Kind<KIND>::order, P = Kind<KIND>::params, kWarps = kBondedThreads / 32;
+  __shared__ R table[kRowTable][kRowConsts];
+  __shared__ int aside[kWarps][64];  // shifted edges of a warp, from its first
+  for (int r = threadIdx.x; r < a.n_rows; r += kBondedThreads) row_constants<KIND, R>(a.params + (int64_t)r * P, table[r]);
+  __syncthreads();
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * kBondedThreads + threadIdx.x) >> 5;
+  const int64_t first = warp * a.per * 32;
+  SystemSums sum;
+  sum.clear(-1);
+  if constexpr (sizeof(R) == 8) {
+    int *queue = aside[threadIdx.x >> 5];
+    int queued = 0;
+    auto add = [&](int sys, R en, bool has_dl, const R *dl) {
+      if (sys != sum.sys) {
+        sum.flush(a.energy, a.grad_tril);
+        sum.sys = sys;
+      }
+      sum.en += (double)en;
+      if (has_dl)
+        for (int k = 0; k < 6; ++k) sum.dl[k] += (double)dl[k];
+    };
+    auto shifted_edges = [&](int count) {  // the first `count` put aside, a lane each
+      if (lane < count) {
+        const int64_t e = first + queue[lane];
+        int idx[D], sh[D - 1][3], sys;
+        int64_t row;
+        bonded_atoms<D>(a, e, idx, row, sys);
+        bonded_shifts<D>(a, e, sh);
+        R en, dl[6] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)};
+        bonded_edge<KIND, R>(a, table, e, idx, row, sys, sh, true, en, dl);
+        add(sys, en, true, dl);
+      }
+    };
+    for (int t = 0; t < a.per; ++t) {
+      const int64_t e = first + 32 * t + lane;
+      int idx[D], sh[D - 1][3], sys = -1;
+      int64_t row;
+      const bool ok = e < a.n_edges && bonded_atoms<D>(a, e, idx, row, sys);
+      const bool shifted = ok && bonded_shifts<D>(a, e, sh);
+      const unsigned m = __ballot_sync(full, shifted);
+      if (shifted) queue[queued + __popc(m & ((1u << lane) - 1u))] = 32 * t + lane;
+      queued += __popc(m);
+      if (ok && !shifted) {
+        R en, dl[6] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)};
+        const bool has_dl = bonded_edge<KIND, R>(a, table, e, idx, row, sys, sh, false, en, dl);
+        add(sys, en, has_dl, dl);
+      }
+      __syncwarp();
+      if (queued >= 32) {
+        shifted_edges(32);
+        queued -= 32;
+        const int keep = lane < queued ? queue[32 + lane] : 0;
+        __syncwarp();
+        if (lane < queued) queue[lane] = keep;
+        __syncwarp();
+      }
+    }
+    shifted_edges(queued);
+    __syncwarp();
+    const int s0 = __reduce_max_sync(full, sum.sys);
+    if (__all_sync(full, sum.sys == s0 || sum.sys < 0)) {
+      sum.en = warp_sum(sum.en);
+      bool some = false;
+      for (int k = 0; k < 6; ++k) some |= sum.dl[k] != 0.0;
+      if (__any_sync(full, some))
+        for (int k = 0; k < 6; ++k) sum.dl[k] = warp_sum(sum.dl[k]);
+      sum.sys = lane == 0 ? s0 : -1;
+    }
+    sum.flush(a.energy, a.grad_tril);
+  } else {
+    for (int t = 0; t < a.per; ++t) {
+      const int64_t e = first + 32 * t + lane;
+      if (e - lane >= a.n_edges) break;  // the same for the whole warp
+      int idx[D], sh[D - 1][3], sys = -1;
+      int64_t row;
+      bool has_dl = false;
+      R en = R(0.0), dl[6] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)};
+      if (e < a.n_edges && bonded_atoms<D>(a, e, idx, row, sys)) {
+        const bool shifted = bonded_shifts<D>(a, e, sh);
+        has_dl = bonded_edge<KIND, R>(a, table, e, idx, row, sys, sh, shifted, en, dl);
+      }
+      // 32 edges of one system: summed in float over the warp, else edge by edge
+      const int s0 = __shfl_sync(full, sys, 0);
+      const bool any_dl = __any_sync(full, has_dl);
+      if (__all_sync(full, sys == s0)) {
+        if (s0 != sum.sys) {
+          if (lane == 0) sum.flush(a.energy, a.grad_tril);
+          sum.clear(s0);
+        }
+        sum.en += (double)warp_sum(en);
+        if (any_dl)
+          for (int k = 0; k < 6; ++k) sum.dl[k] += (double)warp_sum(dl[k]);
+      } else if (sys >= 0) {
+        atomicAdd(&a.energy[sys], (double)en);
+        if (a.grad_tril != nullptr && has_dl)
+          for (int k = 0; k < 6; ++k) atomicAdd(&a.grad_tril[6 * (int64_t)sys + k], (double)dl[k]);
+      }
+    }
+    if (lane == 0) sum.flush(a.energy, a.grad_tril);
+  }
 }
 
 // slot[i] = k for the k-th changed particle, -1 for every other particle (slot preset to -1).
@@ -401,7 +715,7 @@ __device__ int edge_delta(int64_t e, const int *idx, const int *sl, const double
       x_new[d][a] = sl[d] >= 0 ? new_pos[3 * (int64_t)sl[d] + a] : x_old[d][a];
       img[d][a] = (sl[d] >= 0 && new_image) ? (double)new_image[3 * (int64_t)sl[d] + a] : 0.0;
     }
-  R v_old[D - 1][3], v_new[D - 1][3], g[D - 1][3], pr[P];
+  R v_old[D - 1][3], v_new[D - 1][3], g[D - 1][3], pr[kRowConsts];
   for (int m = 0; m < D - 1; ++m) {
     double sh[3], sh_new[3], sL[3], sL_new[3];
     for (int a = 0; a < 3; ++a) {
@@ -415,7 +729,7 @@ __device__ int edge_delta(int64_t e, const int *idx, const int *sl, const double
       v_new[m][a] = (R)(x_new[m + 1][a] - x_new[0][a] + sL_new[a]);
     }
   }
-  for (int k = 0; k < P; ++k) pr[k] = (R)params[row * P + k];
+  row_constants<KIND, R>(params + row * P, pr);
   const double e_new = (double)edge_energy_grad<KIND, R>(v_new, pr, g);
   const double e_old = (double)edge_energy_grad<KIND, R>(v_old, pr, g);
   de = e_new - e_old;
@@ -513,9 +827,15 @@ cudaError_t launch_bonded(const double *pos, const int32_t *system, const int32_
                           const double *tril, int32_t s, const int32_t *edges, const int32_t *shifts,
                           int64_t n_edges, const double *params, int32_t nsp, double *energy, double *grad,
                           double *grad_tril, kups_status *status, cudaStream_t stream) {
-  const unsigned grid = (unsigned)((n_edges + 127) / 128);
-  bonded_kernel<KIND, R><<<grid, 128, 0, stream>>>(pos, system, species, n, tril, s, edges, shifts, n_edges, params,
-                                                nsp, energy, grad, grad_tril, status);
+  int64_t rows = 1;
+  for (int d = 0; d < Kind<KIND>::order && rows <= kRowTable; ++d) rows *= nsp;
+  // up to eight edges per thread while every SM still gets four blocks
+  const int64_t wave = 4 * (int64_t)device_sm_count() * kBondedThreads;
+  const int per = (int)std::min<int64_t>(8, std::max<int64_t>(1, n_edges / wave));
+  const int64_t block = (int64_t)kBondedThreads * per;
+  const BondedArgs args{pos,    system, species, n,   tril,   s,    edges,     shifts, n_edges,
+                        params, nsp,    rows <= kRowTable ? (int)rows : 0, per, energy, grad, grad_tril, status};
+  bonded_kernel<KIND, R><<<(unsigned)((n_edges + block - 1) / block), kBondedThreads, 0, stream>>>(args);
   return cudaGetLastError();
 }
 

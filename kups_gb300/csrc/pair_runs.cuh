@@ -51,6 +51,19 @@ __device__ inline double shift_double(int s) {
   return (double)s;
 }
 
+// s @ L for small integers s (the sums in the order of row_times_tril64).
+__device__ inline void shift_vector(const int s[3], const Tril64 &L, double y[3]) {
+  y[0] = shift_times(s[0], L.t[0]);
+  y[1] = shift_times(s[1], L.t[2]);
+  y[2] = shift_times(s[2], L.t[5]);
+  // (a test of the bits: float64 comparisons take the float64 pipe)
+  const long long skew = __double_as_longlong(L.t[1]) | __double_as_longlong(L.t[3]) | __double_as_longlong(L.t[4]);
+  if ((skew << 1) != 0) {
+    y[0] = __dadd_rn(__dadd_rn(y[0], shift_times(s[1], L.t[1])), shift_times(s[2], L.t[3]));
+    y[1] = __dadd_rn(y[1], shift_times(s[2], L.t[4]));
+  }
+}
+
 __device__ inline bool finite64(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
 template <bool B>
@@ -73,7 +86,7 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
   int sys = -1, fi = -1;
   double en_sum = 0.0, dl[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, gi[3] = {0.0, 0.0, 0.0}, xi[3] = {0.0, 0.0, 0.0};
   Tril64 L;
-  bool skew = false, any_dl = false;
+  bool any_dl = false;
   constexpr double kShare = PAIRED ? 1.0 : 0.5;  // of an edge's energy
   auto flush_first = [&]() {
     if (fi >= 0)
@@ -111,7 +124,6 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
           flush_system();
           sys = si;
           L = load_tril64(p.tril + 6 * (int64_t)si);
-          skew = L.t[1] != 0.0 || L.t[3] != 0.0 || L.t[4] != 0.0;
           ev.load_system(si);
         }
         for (int a = 0; a < 3; ++a) xi[a] = p.pos[3 * (int64_t)i + a];
@@ -120,14 +132,10 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
       const double *xj = p.pos + 3 * (int64_t)j;
       double d[3] = {xj[0] - xi[0], xj[1] - xi[1], xj[2] - xi[2]};
       if (kShifted) {
-        double y0 = shift_times(s0, L.t[0]), y1 = shift_times(s1, L.t[2]), y2 = shift_times(s2, L.t[5]);
-        if (skew) {
-          y0 = __dadd_rn(__dadd_rn(y0, shift_times(s1, L.t[1])), shift_times(s2, L.t[3]));
-          y1 = __dadd_rn(y1, shift_times(s2, L.t[4]));
-        }
-        d[0] += y0;
-        d[1] += y1;
-        d[2] += y2;
+        const int sh[3] = {s0, s1, s2};
+        double y[3];
+        shift_vector(sh, L, y);
+        for (int a = 0; a < 3; ++a) d[a] += y[a];
       }
       const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
       double en, dedr2;
