@@ -74,9 +74,26 @@ __device__ inline bool mbar_wait(uint32_t addr, uint32_t phase) {
   return false;
 }
 
+__device__ inline float exp2_sfu(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ inline float log2_sfu(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // softplus(x) = max(x, 0) + ln(1 + exp(-|x|)) with SFU exp / log (no overflow; the absolute
-// error, a few 1e-8, is far below the bfloat16 rounding that follows)
-__device__ inline float softplus_fast(float x) { return fmaxf(x, 0.f) + __logf(1.0f + __expf(-fabsf(x))); }
+// error, a few 1e-8, is far below the bfloat16 rounding that follows), as 2^(-|x| log2 e) and
+// ln 2 log2(1 + t): two SFU operations and six others per element.  The flush-to-zero forms skip the
+// scaling of subnormal arguments (2^-126 and below vanish beside the 1; the logarithm's argument is at
+// least 1), half of the instructions of __expf and __logf, with the same bits for every finite x.
+__device__ inline float softplus_fast(float x) {
+  const float t = exp2_sfu(__fmul_rn(-1.44269504088896341f, fabsf(x)));
+  return fmaf(log2_sfu(1.0f + t), 0.69314718055994531f, fmaxf(x, 0.f));
+}
 
 // One 32-byte store (a whole L2 sector) of eight 32-bit values.
 __device__ inline void st_v8(void *p, const uint32_t (&w)[8]) {
@@ -1260,80 +1277,104 @@ __global__ void proposal_density_kernel(const float *node, const double *cdf, in
 }
 
 // ============================================================================
-// Fused forward pass (inference: kups_mlp_fwd and the grid refresh).  A persistent
-// CTA (16 warps, one per SM) takes tiles of 256 points, two 128-row halves that share
-// every weight chunk:
-//   * features: each point's fractional coordinates reduced to [-0.5, 0.5) once in
-//     float64 and split into float pairs, the 32 phases m_j . f as float pairs
-//     (phase_sincos), written
-//     straight into shared memory as the first layer's A operand (bfloat16,
-//     no-swizzle K-major core matrices);
-//   * weights: K-chunks of 64 columns of W [256, K] (32 KB) stream through a two-stage
-//     ring of 16-byte cp.async copies; the chunk after the current one is in flight
-//     while the tensor cores work on the current one (the copies run ahead across
-//     layer and tile boundaries: they never depend on the activations);
-//   * one thread issues tcgen05.mma (128 x 256 x 16, BF16 in, FP32 accumulate) for both
-//     halves per K step into two accumulators of 256 tensor-memory columns each (all
-//     512 columns) and commits each chunk to its stage's mbarrier;
-//   * the epilogue (all warps: warp w reads TMEM lanes 32 (w % 4) .. + 31 of both halves,
-//     64 columns w / 4 ..) adds the bias and applies softplus through the SFU
-//     (exp2 / log2: the result is rounded to bfloat16), writes the next layer's A operand
-//     into shared memory, and after the last layer folds in the head (w4 . h3 + b4).
-// Every mbarrier wait is bounded; on time-out the kernel records KUPS_ERR_UNSUPPORTED,
-// waits (bounded) for its own copies, frees its tensor memory and returns.
-constexpr int kFwdThreads = 512, kFwdRows = 256, kFwdHalf = 128, kFwdKc = 64;
-
-constexpr size_t kFwdA = (size_t)kFwdRows * kHid * 2;           // 128 KB: A operand, K up to 256
-constexpr size_t kFwdStage = (size_t)kHid * kFwdKc * 2;          // 32 KB: one weight chunk
-// shared memory: A operand | two weight stages | head partials [4][256] | coordinates [6][256] |
-// biases b1 b2 b3 and head weights w4 [4][256] | frequencies [32][3] | b4 | mbarriers, TMEM slot
-constexpr size_t kFwdOffPart = kFwdA + 2 * kFwdStage;
-constexpr size_t kFwdOffFr = kFwdOffPart + 4 * kFwdRows * 4;
-constexpr size_t kFwdOffPar = kFwdOffFr + 6 * kFwdRows * 4;
+// Fused forward pass (inference: kups_mlp_fwd and the grid refresh).  A persistent CTA works on two
+// tiles of 128 points at a time, each with its own A operand in shared memory and its own 256-column
+// accumulator in tensor memory, by three kinds of warps that meet only at mbarriers:
+//   * eight epilogue warps per tile: features of the tile's points (coordinates reduced to
+//     [-0.5, 0.5) once in float64 and split into float pairs, the 32 phases as float pairs,
+//     phase_sincos) written as the first layer's A operand (bfloat16, no-swizzle K-major core
+//     matrices); after each layer tcgen05.ld, bias, softplus, and the next layer's A operand, or
+//     after the last the head (w4 . h3 + b4);
+//   * one warp loading the weights by TMA, 64 columns of W (256 rows, 128-byte swizzle, 32 KB) at a
+//     time, through a ring of two stages, in the order the MMAs take them;
+//   * one warp issuing tcgen05.mma (128 x 256 x 16, BF16 in, FP32 accumulate): the layers of the two
+//     tiles in turn, so that one tile's MMAs run under the other tile's epilogue.
+// What bounds it is the epilogue's SFU work (two operations per activation, 16 per clock per SM: 6.4 us
+// per tile) and its issue slots; the MMAs of a tile take 2.6 us.  With one tile of 256 points whose
+// MMAs and epilogue took turns, block barriers at every weight chunk and 16-byte copies by all
+// threads, 3e5 points took 292 us; now FIGURE.
+// Every mbarrier wait is bounded; the one that runs out raises a flag that ends the others, the
+// kernel records KUPS_ERR_UNSUPPORTED, waits (bounded) for its copies and MMAs, frees its tensor
+// memory and returns.
+constexpr int kFwdTile = 128, kFwdEpiWarps = 16, kFwdThreads = 32 * (kFwdEpiWarps + 2), kFwdKc = 64;
+constexpr uint32_t kFwdStage = kHid * kFwdKc * 2;  // 32 KB: one weight chunk
+constexpr size_t kFwdA = (size_t)kFwdTile * kHid * 2;  // 64 KB: a tile's A operand, K up to 256
+// shared memory: weight stages | A operands | head partials [2][4][128] | coordinates [2][6][128] |
+// biases b1 b2 b3 and head weights w4 [4][256] | frequencies [32][3] | b4 | mbarriers, TMEM slot, flag
+constexpr size_t kFwdOffA = 2 * (size_t)kFwdStage;
+constexpr size_t kFwdOffPart = kFwdOffA + 2 * kFwdA;
+constexpr size_t kFwdOffFr = kFwdOffPart + 2 * 4 * kFwdTile * 4;
+constexpr size_t kFwdOffPar = kFwdOffFr + 2 * 6 * kFwdTile * 4;
 constexpr size_t kFwdOffFreq = kFwdOffPar + 4 * kHid * 4;
 constexpr size_t kFwdOffB4 = kFwdOffFreq + 3 * kFreq * 4;
 constexpr size_t kFwdOffBar = kFwdOffB4 + 16;
-constexpr size_t kFwdSmem = kFwdOffBar + 64;
+constexpr size_t kFwdSmem = kFwdOffBar + 128 + 1024;  // the stages start on 1024 bytes
 static_assert(kFwdOffBar % 8 == 0, "mbarriers are 8-byte aligned");
+static_assert(kFwdSmem <= 227 * 1024, "forward pass shared memory above the per-CTA limit");
 
 __device__ inline int fwd_core(int r, int kk, int K) {
   return ((r >> 3) * (K / 8) + (kk >> 3)) * 64 + (r & 7) * 8 + (kk & 7);
 }
 
-// Chunk q of the per-tile sequence W1 (1 chunk of 64 columns), W2 (4), W3 (4).
-constexpr int kFwdChunks = 1 + 4 + 4;
-__device__ inline void fwd_chunk_of(int q, int &layer, int &kc) {
-  layer = q == 0 ? 0 : (q <= 4 ? 1 : 2);
-  kc = q == 0 ? 0 : (q <= 4 ? q - 1 : q - 5);
+// mbar_wait that also ends when another wait of the CTA has run out (*stop), and raises it itself.
+__device__ inline bool mbar_wait_or_stop(uint32_t addr, uint32_t phase, volatile int *stop) {
+  for (long long i = 0; i < kWaitLimit; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(addr), "r"(phase)
+        : "memory");
+    if (done) return true;
+    if (*stop) return false;
+  }
+  *stop = 1;
+  return false;
 }
 
-// columns [64 kc, 64 kc + 64) of W [256, K] -> core-matrix layout of 256 rows x 64; copy e
-// takes row (e / 64) * 8 + e % 8, column group (e / 8) % 8 and lands at element 8 e
-__device__ inline void fwd_stage_chunk(__nv_bfloat16 *sB, const __nv_bfloat16 *pb, int q, int tid) {
-  int layer, kc;
-  fwd_chunk_of(q, layer, kc);
-  const __nv_bfloat16 *W = pb + (layer == 0 ? kOffW1 : layer == 1 ? kOffW2 : kOffW3);
-  const int K = layer == 0 ? kIn : kHid;
-  const uint32_t s0 = smem_u32(sB);
-  for (int e = tid; e < kHid * (kFwdKc / 8); e += kFwdThreads) {
-    const int lo = e & 7, kg = (e >> 3) & 7, rb = e >> 6;
-    cp_async16(s0 + (uint32_t)e * 16u, W + (size_t)(rb * 8 + lo) * K + kc * kFwdKc + kg * 8, 16u);
-  }
+__device__ inline void mbar_arrive(uint32_t addr) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+
+__device__ inline void mma_commit(uint32_t mbar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+
+__device__ inline void mma_f16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate ? 1u : 0u));
+}
+
+__device__ inline void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+      "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
 }
 
 __global__ void __launch_bounds__(kFwdThreads, 1)
-mlp_forward_kernel(const __nv_bfloat16 *pb, const float *p, const int32_t *freq, const double *x, int64_t n,
-                   int grid, float *g_out, kups_status *status) {
-  extern __shared__ __align__(1024) unsigned char smem[];
-  __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smem);
-  auto sB = [&](int st) { return reinterpret_cast<__nv_bfloat16 *>(smem + kFwdA + st * kFwdStage); };
-  float *part = reinterpret_cast<float *>(smem + kFwdOffPart);  // [4][256] head partials
-  float *fr = reinterpret_cast<float *>(smem + kFwdOffFr);       // [6][256] coordinates hi, lo
-  float *spar = reinterpret_cast<float *>(smem + kFwdOffPar);    // [4][256] b1, b2, b3, w4
+mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant__ CUtensorMap w2,
+                   const __grid_constant__ CUtensorMap w3, const float *p, const int32_t *freq, const double *x,
+                   int64_t n, int grid, float *g_out, kups_status *status) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                                          ~uintptr_t(1023));
+  float *spar = reinterpret_cast<float *>(smem + kFwdOffPar);  // [4][256] b1, b2, b3, w4
   int32_t *sfreq = reinterpret_cast<int32_t *>(smem + kFwdOffFreq);
   float *sb4 = reinterpret_cast<float *>(smem + kFwdOffB4);
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kFwdOffBar);  // [2]
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 2);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kFwdOffBar);
+  uint64_t *full = bars, *freed = bars + 2;        // [2] weight stage landed / its MMAs done
+  uint64_t *ready = bars + 4, *acc = bars + 6;     // [2] tile's A operand written / accumulator complete
+  uint64_t *meet = bars + 8;                       // [2] the epilogue threads of a tile meet
+  uint64_t *drained = bars + 10;                   // every MMA done (after a stop)
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 11);
+  volatile int *stop = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int e = tid; e < 4 * kHid; e += kFwdThreads) {
     const int which = e / kHid;
@@ -1342,195 +1383,221 @@ mlp_forward_kernel(const __nv_bfloat16 *pb, const float *p, const int32_t *freq,
   }
   for (int e = tid; e < 3 * kFreq; e += kFwdThreads) sfreq[e] = freq[e];
   if (tid == 0) sb4[0] = p[kOffB4];
-  const int quarter = warp & 3, cq = warp >> 2;  // TMEM lanes 32 quarter .., columns 64 cq .. of each half
-  if (warp == 0) {
+  if (warp == kFwdEpiWarps) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(2 * kHid));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    mbar_init(smem_u32(&mbar[0]), 1);
-    mbar_init(smem_u32(&mbar[1]), 1);
+    for (int k = 0; k < 2; ++k) {
+      mbar_init(smem_u32(&full[k]), 1);
+      mbar_init(smem_u32(&freed[k]), 1);
+      mbar_init(smem_u32(&ready[k]), 32 * kFwdEpiWarps / 2);
+      mbar_init(smem_u32(&acc[k]), 1);
+      mbar_init(smem_u32(&meet[k]), 32 * kFwdEpiWarps / 2);
+    }
+    mbar_init(smem_u32(drained), 1);
+    *stop = 0;
   }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = make_idesc(kFwdHalf, kHid);
-  // per stage (bit st): parity of the next completion to wait for, and whether MMAs reading it are
-  // in flight (bit fields, not arrays: the stage index is dynamic)
-  uint32_t phase = 0u, pending = 0u;
-  bool ok = true;
-  const int64_t n_tiles = (n + kFwdRows - 1) / kFwdRows;
-  const int64_t my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const int64_t total_chunks = my_tiles * kFwdChunks;
-  int64_t qg = 0;  // this CTA's chunk counter; stage qg & 1
-  if (total_chunks > 0) {
-    fwd_stage_chunk(sB(0), pb, 0, tid);
-    cp_async_commit();
-  }
-  for (int64_t t = 0; t < my_tiles && ok; ++t) {
-    const int64_t tile = blockIdx.x + t * gridDim.x;
-    // coordinates of the tile's points reduced to [-0.5, 0.5) in float64, kept in float32
-    if (tid < kFwdRows) {
-      const int64_t pt = tile * kFwdRows + tid;
-      double f[3] = {0.0, 0.0, 0.0};
-      if (pt < n) {
-        if (x != nullptr) {
-          for (int a = 0; a < 3; ++a) f[a] = x[3 * pt + a];
-        } else {
-          const int64_t g2 = (int64_t)grid * grid;
-          f[0] = (double)(pt / g2) / grid;
-          f[1] = (double)((pt / grid) % grid) / grid;
-          f[2] = (double)(pt % grid) / grid;
-        }
-      }
-      for (int a = 0; a < 3; ++a) {
-        const double red = f[a] - rint(f[a]);
-        const float hi = (float)red;
-        fr[a * kFwdRows + tid] = hi;
-        fr[(3 + a) * kFwdRows + tid] = (float)(red - (double)hi);
-      }
-    }
-    __syncthreads();
-    for (int e = tid; e < kFwdRows * kFreq; e += kFwdThreads) {
-      const int r = e % kFwdRows, j = e / kFwdRows;
-      const int64_t pt = tile * kFwdRows + r;
-      float sn = 0.f, cs = 0.f;
-      if (pt < n) {
-        const float fh[3] = {fr[r], fr[kFwdRows + r], fr[2 * kFwdRows + r]};
-        const float fl[3] = {fr[3 * kFwdRows + r], fr[4 * kFwdRows + r], fr[5 * kFwdRows + r]};
-        phase_sincos(sfreq + 3 * j, fh, fl, sn, cs);
-      }
-      *reinterpret_cast<__nv_bfloat162 *>(sA + fwd_core(r, 2 * j, kIn)) = __floats2bfloat162_rn(sn, cs);
-    }
-    for (int layer = 0; layer < 3 && ok; ++layer) {
-      const int K = layer == 0 ? kIn : kHid;
-      const int nch = K / kFwdKc;
-      for (int c = 0; c < nch && ok; ++c, ++qg) {
-        const int st = (int)(qg & 1), nx = st ^ 1;
-        if (qg + 1 < total_chunks) {
-          if ((pending >> nx) & 1u) {  // the MMAs of chunk qg - 1 read stage nx
-            ok = mbar_wait(smem_u32(&mbar[nx]), (phase >> nx) & 1u);
-            if (ok) {  // after a time-out the clean-up waits for these MMAs again
-              phase ^= 1u << nx;
-              pending &= ~(1u << nx);
-            }
-          }
-          if (!__syncthreads_and(ok)) {
-            ok = false;
-            break;
-          }
-          fwd_stage_chunk(sB(nx), pb, (int)((qg + 1) % kFwdChunks), tid);
-          cp_async_commit();
-          cp_async_wait<1>();  // chunk qg has landed (this thread's copies)
-        } else {
-          cp_async_wait<0>();
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // A written by the generic proxy
-        __syncthreads();
-        if (tid == 0) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          for (int ks = 0; ks < kFwdKc / 16; ++ks) {
-            const uint64_t bd = make_sdesc(smem_u32(sB(st)) + ks * 256, 128, (kFwdKc / 8) * 128);
-            const uint32_t accumulate = (c > 0 || ks > 0) ? 1u : 0u;
-            for (int h = 0; h < 2; ++h) {
-              const uint64_t ad = make_sdesc(smem_u32(sA) + (uint32_t)(h * kFwdHalf * K * 2) + (c * 4 + ks) * 256,
-                                             128, (K / 8) * 128);
-              asm volatile(
-                  "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem + (uint32_t)(h * kHid)),
-                  "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
-            }
-          }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_u32(&mbar[st]))
-                       : "memory");
-        }
-        pending |= 1u << st;
-        if (c == nch - 1) {  // the layer's accumulators are complete once its last chunk is
-          ok = mbar_wait(smem_u32(&mbar[st]), (phase >> st) & 1u);
-          if (ok) {
-            phase ^= 1u << st;
-            pending &= ~(1u << st);
+  // tiles u = blockIdx + gridDim (2 t + h) go to slot h of this CTA: the first gridDim tiles to every
+  // CTA's slot 0, so that few points still spread over the chip
+  const int64_t n_tiles = (n + kFwdTile - 1) / kFwdTile;
+  auto tiles_of = [&](int h) {
+    const int64_t first = blockIdx.x + (int64_t)gridDim.x * h;
+    return first < n_tiles ? (n_tiles - 1 - first) / (2 * (int64_t)gridDim.x) + 1 : (int64_t)0;
+  };
+  const int64_t count[2] = {tiles_of(0), tiles_of(1)};  // count[0] >= count[1]
+  if (warp < kFwdEpiWarps) {
+    const int h = warp >> 3, ht = tid & 255;                     // tile slot, thread inside it
+    const int quarter = warp & 3, colh = (warp >> 2) & 1;        // TMEM lanes 32 quarter .., columns 128 colh ..
+    const int row = quarter * 32 + lane;
+    __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smem + kFwdOffA + h * kFwdA);
+    float *part = reinterpret_cast<float *>(smem + kFwdOffPart) + h * 4 * kFwdTile;
+    float *fr = reinterpret_cast<float *>(smem + kFwdOffFr) + h * 6 * kFwdTile;
+    const float *w4 = spar + 3 * kHid;
+    bool ok = true;
+    uint32_t parity = 0u, met = 0u;  // of the slot's next accumulator and next meeting
+    // waits end alike for a whole warp (tcgen05.ld is a warp's operation)
+    auto wait = [&](uint64_t *bar, uint32_t &phase) {
+      const bool done = __all_sync(0xffffffffu, mbar_wait_or_stop(smem_u32(bar), phase, stop));
+      phase ^= 1u;
+      return done;
+    };
+    auto meeting = [&]() {
+      mbar_arrive(smem_u32(&meet[h]));
+      return wait(&meet[h], met);
+    };
+    for (int64_t t = 0; t < count[h] && ok; ++t) {
+      const int64_t row0 = (blockIdx.x + (int64_t)gridDim.x * (2 * t + h)) * kFwdTile;
+      if (ht < kFwdTile) {  // coordinates reduced to [-0.5, 0.5) in float64, kept as float pairs
+        const int64_t pt = row0 + ht;
+        double f[3] = {0.0, 0.0, 0.0};
+        if (pt < n) {
+          if (x != nullptr) {
+            for (int a = 0; a < 3; ++a) f[a] = x[3 * pt + a];
+          } else {
+            const int64_t g2 = (int64_t)grid * grid;
+            f[0] = (double)(pt / g2) / grid;
+            f[1] = (double)((pt / grid) % grid) / grid;
+            f[2] = (double)(pt % grid) / grid;
           }
         }
+        for (int a = 0; a < 3; ++a) {
+          const double red = f[a] - rint(f[a]);
+          const float hi = (float)red;
+          fr[a * kFwdTile + ht] = hi;
+          fr[(3 + a) * kFwdTile + ht] = (float)(red - (double)hi);
+        }
       }
-      if (!__syncthreads_and(ok)) {
-        ok = false;
-        break;
+      ok = meeting();
+      if (!ok) break;
+      {
+        const int r = ht & (kFwdTile - 1);
+        const bool in = row0 + r < n;
+        const float fh[3] = {fr[r], fr[kFwdTile + r], fr[2 * kFwdTile + r]};
+        const float fl[3] = {fr[3 * kFwdTile + r], fr[4 * kFwdTile + r], fr[5 * kFwdTile + r]};
+        for (int j = ht / kFwdTile; j < kFreq; j += 2) {
+          float sn = 0.f, cs = 0.f;
+          if (in) phase_sincos(sfreq + 3 * j, fh, fl, sn, cs);
+          *reinterpret_cast<__nv_bfloat162 *>(sA + fwd_core(r, 2 * j, kIn)) = __floats2bfloat162_rn(sn, cs);
+        }
       }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const float *bias = spar + layer * kHid;
-      const float *w4 = spar + 3 * kHid;
-      for (int h = 0; h < 2; ++h) {
-        const int row = h * kFwdHalf + quarter * 32 + lane;
+      for (int layer = 0; layer < 3; ++layer) {
+        // the A operand is visible to the tensor cores and the accumulator read: the layer may start
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        mbar_arrive(smem_u32(&ready[h]));
+        ok = wait(&acc[h], parity);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const float *bias = spar + layer * kHid;
         float head = 0.f;
-        for (int c0 = cq * (kHid / 4); c0 < (cq + 1) * (kHid / 4); c0 += 32) {
+        for (int c0 = colh * 128; c0 < colh * 128 + 128; c0 += 32) {
           uint32_t r[32];
-          const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * kHid + c0);
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-              "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-              : "r"(taddr));
+          tmem_load32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * kHid + c0), r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          const float4 *b4 = reinterpret_cast<const float4 *>(bias + c0);
+          float v[32];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const float4 b = b4[q];
+            v[4 * q] = softplus_fast(__uint_as_float(r[4 * q]) + b.x);
+            v[4 * q + 1] = softplus_fast(__uint_as_float(r[4 * q + 1]) + b.y);
+            v[4 * q + 2] = softplus_fast(__uint_as_float(r[4 * q + 2]) + b.z);
+            v[4 * q + 3] = softplus_fast(__uint_as_float(r[4 * q + 3]) + b.w);
+          }
           if (layer < 2) {
             // next layer's A operand: 4 core-matrix rows of 8 bfloat16 (16 bytes each)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               __nv_bfloat162 hv[4];
 #pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const int i = q * 8 + 2 * u;
-                hv[u] = __floats2bfloat162_rn(softplus_fast(__uint_as_float(r[i]) + bias[c0 + i]),
-                                              softplus_fast(__uint_as_float(r[i + 1]) + bias[c0 + i + 1]));
-              }
+              for (int u = 0; u < 4; ++u) hv[u] = __floats2bfloat162_rn(v[q * 8 + 2 * u], v[q * 8 + 2 * u + 1]);
               *reinterpret_cast<uint4 *>(sA + fwd_core(row, c0 + q * 8, kHid)) = *reinterpret_cast<uint4 *>(hv);
             }
           } else {
+            const float4 *h4 = reinterpret_cast<const float4 *>(w4 + c0);
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              head = fmaf(softplus_fast(__uint_as_float(r[i]) + bias[c0 + i]), w4[c0 + i], head);
+            for (int q = 0; q < 8; ++q) {
+              const float4 w = h4[q];
+              head = fmaf(v[4 * q], w.x, head);
+              head = fmaf(v[4 * q + 1], w.y, head);
+              head = fmaf(v[4 * q + 2], w.z, head);
+              head = fmaf(v[4 * q + 3], w.w, head);
+            }
+            if ((c0 & 63) == 32) {  // sums of 64 columns
+              part[(c0 >> 6) * kFwdTile + row] = head;
+              head = 0.f;
+            }
           }
         }
-        if (layer == 2) part[cq * kFwdRows + row] = head;
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncthreads();
-      if (layer == 2 && tid < kFwdRows) {
-        const int64_t pt = tile * kFwdRows + tid;
-        if (pt < n)
-          g_out[pt] = ((part[tid] + part[kFwdRows + tid]) + (part[2 * kFwdRows + tid] + part[3 * kFwdRows + tid])) +
-                      sb4[0];
-      }
+      if (!ok) break;
+      ok = meeting();
+      if (ok && ht < kFwdTile && row0 + ht < n)
+        g_out[row0 + ht] = ((part[ht] + part[kFwdTile + ht]) + (part[2 * kFwdTile + ht] + part[3 * kFwdTile + ht])) +
+                           sb4[0];
+    }
+  } else if (warp == kFwdEpiWarps) {
+    if (lane == 0) {  // weights, in the order of the MMAs
+      int64_t q = 0;
+      bool ok = true;
+      for (int64_t t = 0; t < count[0] && ok; ++t)
+        for (int layer = 0; layer < 3 && ok; ++layer)
+          for (int h = 0; h < 2 && ok; ++h) {
+            if (t >= count[h]) continue;
+            const CUtensorMap *map = layer == 0 ? &w1 : layer == 1 ? &w2 : &w3;
+            for (int c = 0; c < (layer == 0 ? kIn : kHid) / kFwdKc; ++c, ++q) {
+              const int st = (int)(q & 1);
+              if (q >= 2) ok = mbar_wait_or_stop(smem_u32(&freed[st]), (uint32_t)((q >> 1) - 1) & 1u, stop);
+              if (!ok) break;
+              mbar_expect_tx(smem_u32(&full[st]), kFwdStage);
+              tma_load_2d(smem_u32(smem + st * kFwdStage), map, c * kFwdKc, 0, smem_u32(&full[st]));
+            }
+          }
+      if (*stop)  // copies in flight land before the CTA ends
+        for (int64_t k = q > 2 ? q - 2 : 0; k < q; ++k) mbar_wait(smem_u32(&full[k & 1]), (uint32_t)(k >> 1) & 1u);
+    }
+  } else if (lane == 0) {
+    const uint32_t idesc = make_idesc(kFwdTile, kHid);
+    int64_t q = 0;
+    uint32_t parity[2] = {0u, 0u};
+    bool ok = true;
+    for (int64_t t = 0; t < count[0] && ok; ++t)
+      for (int layer = 0; layer < 3 && ok; ++layer)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (!ok || t >= count[h]) continue;
+          ok = mbar_wait_or_stop(smem_u32(&ready[h]), parity[h], stop);
+          if (!ok) continue;
+          parity[h] ^= 1u;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const int K = layer == 0 ? kIn : kHid;
+          const uint32_t a0 = smem_u32(smem + kFwdOffA + h * kFwdA);
+          for (int c = 0; c < K / kFwdKc; ++c, ++q) {
+            const int st = (int)(q & 1);
+            ok = mbar_wait_or_stop(smem_u32(&full[st]), (uint32_t)(q >> 1) & 1u, stop);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t b0 = smem_u32(smem + st * kFwdStage);
+            for (int ks = 0; ks < kFwdKc / 16; ++ks)
+              mma_f16(tmem + (uint32_t)(h * kHid), make_sdesc(a0 + (c * 4 + ks) * 256, 128, (K / 8) * 128),
+                      make_sdesc_sw128(b0 + ks * 32), idesc, c > 0 || ks > 0);
+            mma_commit(smem_u32(&freed[st]));
+          }
+          if (ok) mma_commit(smem_u32(&acc[h]));
+        }
+    if (*stop) {  // MMAs in flight end before the tensor memory is freed
+      mma_commit(smem_u32(drained));
+      mbar_wait(smem_u32(drained), 0u);
     }
   }
-  cp_async_wait<0>();
-  // a time-out leaves MMAs possibly in flight: wait for them (bounded) before freeing TMEM
-  for (int st = 0; st < 2; ++st)
-    if ((pending >> st) & 1u) {
-      (void)mbar_wait(smem_u32(&mbar[st]), (phase >> st) & 1u);
-      pending &= ~(1u << st);
-    }
-  if (!ok && tid == 0) status_error(status, KUPS_ERR_UNSUPPORTED, blockIdx.x);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kHid));
+  if (tid == 0 && *stop) status_error(status, KUPS_ERR_UNSUPPORTED, blockIdx.x);
+  if (warp == kFwdEpiWarps) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kHid));
+  }
 }
 
 int32_t fused_forward(const kups_mlp *net, const double *x, int64_t n, int grid, float *g, kups_status *status,
                       cudaStream_t st) {
   if (n <= 0) return KUPS_OK;
+  const __nv_bfloat16 *pb = (const __nv_bfloat16 *)net->param_bf16;
+  CUtensorMap w1, w2, w3;
+  if (!operand_map(&w1, pb + kOffW1, kHid, kIn, kIn, kHid) || !operand_map(&w2, pb + kOffW2, kHid, kHid, kHid, kHid) ||
+      !operand_map(&w3, pb + kOffW3, kHid, kHid, kHid, kHid))
+    return KUPS_ERR_CUDA;
   KUPS_CUDA_TRY(cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem));
-  const int sms = device_sm_count();
-  const int64_t tiles = (n + kFwdRows - 1) / kFwdRows;
-  const unsigned ctas = (unsigned)std::min<int64_t>(tiles, sms);
-  mlp_forward_kernel<<<ctas, kFwdThreads, kFwdSmem, st>>>((const __nv_bfloat16 *)net->param_bf16, net->param,
-                                                          net->freq, x, n, grid, g, status);
+  const int64_t tiles = (n + kFwdTile - 1) / kFwdTile;
+  const unsigned ctas = (unsigned)std::min<int64_t>(tiles, device_sm_count());
+  mlp_forward_kernel<<<ctas, kFwdThreads, kFwdSmem, st>>>(w1, w2, w3, net->param, net->freq, x, n, grid, g, status);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 
