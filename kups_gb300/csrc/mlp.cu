@@ -1289,10 +1289,11 @@ __global__ void proposal_density_kernel(const float *node, const double *cdf, in
 //     time, through a ring of two stages, in the order the MMAs take them;
 //   * one warp issuing tcgen05.mma (128 x 256 x 16, BF16 in, FP32 accumulate): the layers of the two
 //     tiles in turn, so that one tile's MMAs run under the other tile's epilogue.
-// What bounds it is the epilogue's SFU work (two operations per activation, 16 per clock per SM: 6.4 us
-// per tile) and its issue slots; the MMAs of a tile take 2.6 us.  With one tile of 256 points whose
-// MMAs and epilogue took turns, block barriers at every weight chunk and 16-byte copies by all
-// threads, 3e5 points took 292 us; now FIGURE.
+// What bounds it is the epilogue's issue slots (about ten instructions per activation, two of them on
+// the SFU, which is a third busy) with the hand-overs between layers: 52 % issue, tensor pipe 24 %.
+// 3e5 points: 158 us (162 without the next 16 columns on their way during the epilogue's work); 292 us
+// with one tile of 256 points whose MMAs and epilogue took turns, block barriers at every weight
+// chunk and 16-byte copies by all threads.
 // Every mbarrier wait is bounded; the one that runs out raises a flag that ends the others, the
 // kernel records KUPS_ERR_UNSUPPORTED, waits (bounded) for its copies and MMAs, frees its tensor
 // memory and returns.
@@ -1347,14 +1348,12 @@ __device__ inline void mma_f16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t
       "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate ? 1u : 0u));
 }
 
-__device__ inline void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ inline void tmem_load16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-      "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+      "%13, %14, %15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
 
@@ -1477,14 +1476,22 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const float *bias = spar + layer * kHid;
         float head = 0.f;
-        for (int c0 = colh * 128; c0 < colh * 128 + 128; c0 += 32) {
-          uint32_t r[32];
-          tmem_load32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * kHid + c0), r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          const float4 *b4 = reinterpret_cast<const float4 *>(bias + c0);
-          float v[32];
+        // 16 columns at a time, the next 16 on their way from tensor memory meanwhile
+        uint32_t next[16];
+        const uint32_t t0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * kHid + colh * 128);
+        tmem_load16(t0, next);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
+        for (int s = 0; s < 8; ++s) {
+          const int c0 = colh * 128 + 16 * s;
+          uint32_t r[16];
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = next[i];
+          if (s < 7) tmem_load16(t0 + 16 * (s + 1), next);
+          const float4 *b4 = reinterpret_cast<const float4 *>(bias + c0);
+          float v[16];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
             const float4 b = b4[q];
             v[4 * q] = softplus_fast(__uint_as_float(r[4 * q]) + b.x);
             v[4 * q + 1] = softplus_fast(__uint_as_float(r[4 * q + 1]) + b.y);
@@ -1492,9 +1499,9 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
             v[4 * q + 3] = softplus_fast(__uint_as_float(r[4 * q + 3]) + b.w);
           }
           if (layer < 2) {
-            // next layer's A operand: 4 core-matrix rows of 8 bfloat16 (16 bytes each)
+            // next layer's A operand: 2 core-matrix rows of 8 bfloat16 (16 bytes each)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < 2; ++q) {
               __nv_bfloat162 hv[4];
 #pragma unroll
               for (int u = 0; u < 4; ++u) hv[u] = __floats2bfloat162_rn(v[q * 8 + 2 * u], v[q * 8 + 2 * u + 1]);
@@ -1503,14 +1510,14 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
           } else {
             const float4 *h4 = reinterpret_cast<const float4 *>(w4 + c0);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < 4; ++q) {
               const float4 w = h4[q];
               head = fmaf(v[4 * q], w.x, head);
               head = fmaf(v[4 * q + 1], w.y, head);
               head = fmaf(v[4 * q + 2], w.z, head);
               head = fmaf(v[4 * q + 3], w.w, head);
             }
-            if ((c0 & 63) == 32) {  // sums of 64 columns
+            if ((s & 3) == 3) {  // sums of 64 columns
               part[(c0 >> 6) * kFwdTile + row] = head;
               head = 0.f;
             }
