@@ -6,7 +6,7 @@
 //
 // GEMM: C[M, N] = act(alpha * A[M, K] . B[N, K]^T + bias[N]) with arbitrary
 // element strides for A, B and C (so transposed operands need no copies);
-// split-K (grid z) for the weight gradients, whose K is the batch.
+// split-K (grid z) for products with a long K.
 // One CTA computes a 128 x BN tile.  Bfloat16 operands with K contiguous are
 // loaded by TMA (cp.async.bulk.tensor, 128-byte swizzle) into a ring of
 // stages (gemm_tma_kernel); other layouts are staged by the threads with
@@ -138,11 +138,8 @@ struct GemmArgs {
   int gate_kind;      // 0 none, 1: multiply by relu'(gate) (gate > 0), 2: by softplus'(gate) = sigmoid,
                       // 3: by softplus' expressed through its output h = softplus(z): 1 - exp(-h)
   int split_k;        // > 1: blockIdx.z takes a slice of K and atomically adds alpha * partial to C
-  void *c3;           // optional third output, bfloat16, its own strides (a transposed copy)
-  int64_t sc3r, sc3c;
   int row_epi;        // set by dispatch_gemm: the register (lane = row) epilogue applies
   int row_v8;         // ... and C (and c2) rows are 32-byte aligned: whole-sector 32-byte stores
-  int fast_math;      // softplus and the gates through SFU exp / log (the network's own calls)
 };
 
 __device__ inline void cp_async16(uint32_t dst, const void *src, uint32_t src_bytes) {
@@ -197,9 +194,7 @@ __device__ inline bool fast_operand(const void *p, int is_bf16, int64_t sr, int6
 // 16-byte aligned rows, N a multiple of 32, beta = 0 or split K): warp w reads TMEM lanes
 // 32 (w % 4) .. + 31, so lane l holds row m0 + 32 (w % 4) + l, 32 columns at a time of the
 // column half w / 4, and applies every term in registers: 16-byte loads of bias and gate,
-// 16-byte stores of C and of the bfloat16 copy (c2), vector reductions for split K, and the
-// transposed bfloat16 copy (c3, element (row, col) at col * sc3c + row) written with
-// lane = row (64 contiguous bytes per warp instruction).
+// 16-byte stores of C and of the bfloat16 copy (c2), vector reductions for split K.
 template <int BN>
 __device__ inline void register_epilogue(const GemmArgs &g, uint32_t tmem, int m0, int n0, int warp, int lane) {
   const int quarter = warp & 3, half = warp >> 2;
@@ -243,7 +238,7 @@ __device__ inline void register_epilogue(const GemmArgs &g, uint32_t tmem, int m
     }
     if (g.gate_kind != 0 && rin) {
       const float4 *g4 = reinterpret_cast<const float4 *>(g.gate + (int64_t)row * g.sgr + col0);
-      const int kind = g.gate_kind + (g.fast_math ? 3 : 0);
+      const int kind = g.gate_kind;
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const float4 t = g4[q];
@@ -252,11 +247,9 @@ __device__ inline void register_epilogue(const GemmArgs &g, uint32_t tmem, int m
         for (int e = 0; e < 4; ++e) {
           const float x = pre[e];
           float f;
-          if (kind == 1 || kind == 4) f = x > 0.f ? 1.f : 0.f;
+          if (kind == 1) f = x > 0.f ? 1.f : 0.f;
           else if (kind == 2) f = 1.f / (1.f + expf(-x));
-          else if (kind == 5) f = __frcp_rn(1.f + __expf(-x));
-          else if (kind == 3) f = -expm1f(-x);
-          else f = 1.f - __expf(-x);
+          else f = -expm1f(-x);
           v[4 * q + e] *= f;
         }
       }
@@ -265,13 +258,8 @@ __device__ inline void register_epilogue(const GemmArgs &g, uint32_t tmem, int m
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.f);
     } else if (g.act == 2) {
-      if (g.fast_math) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = softplus_fast(v[i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = act_fn(v[i], 2);
-      }
+      for (int i = 0; i < 32; ++i) v[i] = act_fn(v[i], 2);
     }
     if (rin) {
       float *cr = (float *)g.c + (int64_t)row * g.scr + col0;
@@ -303,14 +291,6 @@ __device__ inline void register_epilogue(const GemmArgs &g, uint32_t tmem, int m
           uint4 *c2p = reinterpret_cast<uint4 *>(c2r);
 #pragma unroll
           for (int q = 0; q < 4; ++q) c2p[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-        }
-      }
-      if (g.c3 != nullptr) {
-        __nv_bfloat16 *c3p = (__nv_bfloat16 *)g.c3 + (int64_t)col0 * g.sc3c + row;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          *c3p = __float2bfloat16(v[i]);
-          c3p += g.sc3c;
         }
       }
     }
@@ -415,8 +395,7 @@ __global__ void __launch_bounds__(kGemmThreads, 4) gemm_tcgen05_kernel(GemmArgs 
     // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows) and the column half
     // w / 4, 32 columns at a time, into a padded 32 x 33 shared-memory block.  The
     // elementwise terms run with lane = column (coalesced bias / gate / C loads and
-    // row-major stores, 128 contiguous bytes of one row per instruction); the transposed
-    // bfloat16 copy (c3) is written back with lane = row (coalesced as well).
+    // row-major stores, 128 contiguous bytes of one row per instruction).
     const int quarter = warp & 3, half = warp >> 2;
     const int rbase = m0 + quarter * 32;
     float *blk = reinterpret_cast<float *>(smem) + warp * 32 * 33;  // pipeline stages are free now
@@ -464,20 +443,6 @@ __global__ void __launch_bounds__(kGemmThreads, 4) gemm_tcgen05_kernel(GemmArgs 
             const int64_t o2 = (int64_t)row * g.sc2r + (int64_t)col * g.sc2c;
             if (g.c2_bf16) ((__nv_bfloat16 *)g.c2)[o2] = __float2bfloat16(v);
             else ((float *)g.c2)[o2] = v;
-          }
-          blk[rr * 33 + lane] = v;
-        }
-      }
-      __syncwarp();
-      if (g.c3 != nullptr && g.split_k == 1) {
-        const int row = rbase + lane;
-        if (row < g.m) {
-#pragma unroll 8
-          for (int i = 0; i < 32; ++i) {
-            const int cc = n0 + c0 + i;
-            if (cc >= g.n) continue;
-            ((__nv_bfloat16 *)g.c3)[(int64_t)row * g.sc3r + (int64_t)cc * g.sc3c] =
-                __float2bfloat16(blk[lane * 33 + i]);
           }
         }
       }
@@ -724,7 +689,7 @@ int32_t launch_gemm_tma(const GemmArgs &g, kups_status *status, cudaStream_t str
 // CTAs per SM) beat 256-wide ones (two CTAs per SM) on the network's K <= 256 GEMMs.
 // Whether the register epilogue of gemm_tcgen05_kernel applies: float32 C (and the optional
 // bias, gate and bfloat16 copy) row-major with unit column stride and 16-byte aligned rows,
-// N a multiple of 32, no beta term; the transposed copy (c3) with unit row stride.
+// N a multiple of 32, no beta term.
 bool row_epilogue(const GemmArgs &g) {
   auto al16 = [](const void *q) { return (((uintptr_t)q) & 15) == 0; };
   if (g.c_bf16 || g.scc != 1 || g.scr % 4 != 0 || !al16(g.c) || g.n % 32 != 0) return false;
@@ -733,7 +698,6 @@ bool row_epilogue(const GemmArgs &g) {
   if (g.bias != nullptr && !al16(g.bias)) return false;
   if (g.gate_kind != 0 && (g.sgc != 1 || g.sgr % 4 != 0 || !al16(g.gate))) return false;
   if (g.c2 != nullptr && (!g.c2_bf16 || g.sc2c != 1 || g.sc2r % 8 != 0 || !al16(g.c2))) return false;
-  if (g.c3 != nullptr && g.sc3r != 1) return false;
   return true;
 }
 
@@ -761,30 +725,6 @@ int32_t dispatch_gemm(const GemmArgs &g0, kups_status *status, cudaStream_t st) 
   return launch_gemm<256>(g, status, st);
 }
 
-// Row-major operand helper for the network's own GEMM calls.
-struct Op {
-  const void *p;
-  int bf16;
-  int64_t sr, sc;
-};
-
-// c: float32 with strides (scr, scc); c2: bfloat16 copy, same strides; c3: bfloat16
-// transposed copy (element (r, col) at col * m + r).
-int32_t gemm_call(Op a, Op b, void *c, int64_t scr, int64_t scc, void *c2, const float *bias, const float *gate,
-                  int gate_kind, int m, int n, int k, float beta, int act, int split, kups_status *status,
-                  cudaStream_t st, void *c3 = nullptr) {
-  GemmArgs g;
-  g.a = a.p; g.b = b.p; g.c = c; g.c2 = c2; g.bias = bias; g.gate = gate;
-  g.c3 = c3; g.sc3r = 1; g.sc3c = m;
-  g.sar = a.sr; g.sac = a.sc; g.sbr = b.sr; g.sbc = b.sc; g.scr = scr; g.scc = scc;
-  g.sc2r = scr; g.sc2c = scc; g.sgr = scr; g.sgc = scc;
-  g.m = m; g.n = n; g.k = k; g.alpha = 1.f; g.beta = beta; g.act = act;
-  g.a_bf16 = a.bf16; g.b_bf16 = b.bf16; g.c_bf16 = 0; g.c2_bf16 = 1; g.gate_kind = gate_kind;
-  g.split_k = split;
-  g.fast_math = 1;
-  return dispatch_gemm(g, status, st);
-}
-
 // ============================================================================
 // Learned insertion proposal: network, training and grid density.
 //
@@ -792,9 +732,7 @@ int32_t gemm_call(Op a, Op b, void *c, int64_t scr, int64_t scc, void *c2, const
 // (sin, cos)(2 pi m_j . f) for 32 integer vectors m_j, three softplus layers of
 // width 256 (tensor-core GEMMs, bfloat16 operands, float32 accumulation) and
 // a linear output g(f).  Parameters are one flat float32 array at the kOff*
-// offsets plus a bfloat16 copy read by the GEMMs.  Each layer's output h is
-// stored in float32 (the head and the gates read it) and, where it is the
-// next GEMM's operand, in bfloat16.  Training minimises the noise-contrastive
+// offsets plus a bfloat16 copy that the matrix products read.  Training minimises the noise-contrastive
 // loss with equal halves of data and uniform points,
 //   L = (1/n) [sum_data softplus(-g) + sum_uniform softplus(g)],
 // whose minimiser is g(f) = ln p_data(f) for f uniform on the unit cube.
@@ -807,13 +745,18 @@ constexpr int64_t kChunk = 65536;  // points per forward pass over the workspace
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Activations of c points: float32 (the head and the gates read them), bfloat16
-// row-major (the next layer's A operand) and bfloat16 transposed [width, c]
-// (the weight-gradient GEMMs' operands, K = points contiguous).
+// Rows of c points that the weight gradients read, bfloat16: features, h1, h2 and dL/dz of the three
+// layers; h1 in float32 (its gate in the backward pass); scratch of the grid normaliser.
 struct MlpWork {
-  __nv_bfloat16 *feat, *featT, *h1b, *h1T, *h2b, *h2T, *dzab, *dzaT, *dzbb, *dzbT;
-  float *h1, *h2, *h3, *dza, *dzb, *g;
+  __nv_bfloat16 *feat, *h1b, *h2b, *dz1, *dz2, *dz3;
+  float *h1;
+  double *partial;
+  __nv_bfloat16 *weights;  // aligned copy of the weights, if the network's own are not
 };
+
+constexpr int64_t kWeightCopy = (kParams + 7) / 8 * 8 + 2 * kHid * kHid;
+
+constexpr int kNormBlocks = 152, kNormThreads = 1024;
 
 MlpWork carve(void *ws, int64_t c) {
   char *p = (char *)(((uintptr_t)ws + 255) & ~uintptr_t(255));
@@ -824,27 +767,20 @@ MlpWork carve(void *ws, int64_t c) {
     return (void *)q;
   };
   w.feat = (__nv_bfloat16 *)take(2 * (size_t)c * kIn);
-  w.featT = (__nv_bfloat16 *)take(2 * (size_t)c * kIn);
   w.h1b = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
-  w.h1T = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
   w.h2b = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
-  w.h2T = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
-  w.dzab = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
-  w.dzaT = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
-  w.dzbb = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
-  w.dzbT = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
+  w.dz1 = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
+  w.dz2 = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
+  w.dz3 = (__nv_bfloat16 *)take(2 * (size_t)c * kHid);
   w.h1 = (float *)take(4 * (size_t)c * kHid);
-  w.h2 = (float *)take(4 * (size_t)c * kHid);
-  w.h3 = (float *)take(4 * (size_t)c * kHid);
-  w.dza = (float *)take(4 * (size_t)c * kHid);
-  w.dzb = (float *)take(4 * (size_t)c * kHid);
-  w.g = (float *)take(4 * (size_t)c);
+  w.partial = (double *)take(8 * (size_t)3 * kNormBlocks);
+  w.weights = (__nv_bfloat16 *)take(2 * (size_t)kWeightCopy);
   return w;
 }
 
 size_t work_bytes(int64_t c) {
-  return 2 * align256(2 * (size_t)c * kIn) + 8 * align256(2 * (size_t)c * kHid) + 5 * align256(4 * (size_t)c * kHid) +
-         align256(4 * (size_t)c) + 256;
+  return align256(2 * (size_t)c * kIn) + 5 * align256(2 * (size_t)c * kHid) + align256(4 * (size_t)c * kHid) +
+         align256(8 * (size_t)3 * kNormBlocks) + align256(2 * (size_t)kWeightCopy) + 256;
 }
 
 __device__ inline float warp_sum(float v) {
@@ -875,41 +811,6 @@ __device__ inline void phase_sincos(const int32_t *m, const float fh[3], const f
   sincospif(2.0f * t, &sn, &cs);
 }
 
-// Features of point row0 + r: from x (fractional, f64 [., 3]) or, with x null,
-// of grid node row0 + r of a grid^3 lattice.
-__global__ void features_kernel(const double *x, int64_t row0, int64_t n, int grid, const int32_t *freq,
-                                __nv_bfloat16 *feat, __nv_bfloat16 *featT) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  double f[3];
-  if (x != nullptr) {
-    for (int a = 0; a < 3; ++a) f[a] = x[3 * (row0 + r) + a];
-  } else {
-    const int64_t v = row0 + r, g2 = (int64_t)grid * grid;
-    f[0] = (double)(v / g2) / grid;
-    f[1] = (double)((v / grid) % grid) / grid;
-    f[2] = (double)(v % grid) / grid;
-  }
-  // coordinates reduced to [-0.5, 0.5) once in float64 and split into float pairs, phases
-  // as float pairs (phase_sincos), as the fused forward pass computes them
-  float fh[3], fl[3];
-  for (int a = 0; a < 3; ++a) {
-    const double red = f[a] - rint(f[a]);
-    fh[a] = (float)red;
-    fl[a] = (float)(red - (double)fh[a]);
-  }
-  __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(feat + r * kIn);
-  for (int j = 0; j < kFreq; ++j) {
-    float sn, cs;
-    phase_sincos(freq + 3 * j, fh, fl, sn, cs);
-    o[j] = __floats2bfloat162_rn(sn, cs);
-    if (featT != nullptr) {
-      featT[(int64_t)(2 * j) * n + r] = __float2bfloat16(sn);
-      featT[(int64_t)(2 * j + 1) * n + r] = __float2bfloat16(cs);
-    }
-  }
-}
-
 // Equal halves: rows [0, batch/2) are data points drawn with replacement,
 // rows [batch/2, batch) uniform points; Philox keyed by (seed, step, row).
 __global__ void nce_batch_kernel(const double *data, int64_t n_data, int64_t batch, uint64_t seed, uint64_t step,
@@ -928,125 +829,6 @@ __global__ void nce_batch_kernel(const double *data, int64_t n_data, int64_t bat
     x[3 * r + 2] = w.z * (1.0 / 4294967296.0);
     label[r] = 0.f;
   }
-}
-
-// g = h3 . w4 + b4, one warp per row.
-__global__ void head_kernel(const float *h, int64_t n, const float *w4, const float *b4, float *g) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (row >= n) return;
-  float acc = 0.f;
-  for (int j = lane; j < kHid; j += 32) acc = fmaf(h[row * kHid + j], w4[j], acc);
-  acc = warp_sum(acc);
-  if (lane == 0) g[row] = acc + b4[0];
-}
-
-// Head forward + loss + first backward step, 8 warps per block, a warp per row:
-//   dL/dg = (sigmoid(g) - y) / n,  dz3 = dL/dg * w4 * (1 - exp(-h3)),
-//   grad_w4 += sum_rows dL/dg h3,  grad_b4 += sum_rows dL/dg,  loss += L.
-__global__ void __launch_bounds__(256) head_nce_kernel(const float *h, int64_t n, const float *w4, const float *b4,
-                                                       const float *label, float *dz, __nv_bfloat16 *dzb,
-                                                       __nv_bfloat16 *dzT, float *grad_w4, float *grad_b4,
-                                                       float *loss) {
-  __shared__ float red_w[8][kHid];
-  __shared__ float red_b[8], red_l[8];
-  // a tile of 32 rows of dz in bfloat16, written out transposed (dzT[col, row]) with consecutive
-  // threads on consecutive rows, so the transposed copy's stores coalesce
-  __shared__ __nv_bfloat16 tile[32][kHid + 8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float wl[8], dw[8];
-  for (int j = 0; j < 8; ++j) {
-    wl[j] = w4[lane + 32 * j];
-    dw[j] = 0.f;
-  }
-  float db = 0.f, ls = 0.f;
-  const float inv_n = 1.f / (float)n;
-  for (int64_t r0 = (int64_t)blockIdx.x * 32; r0 < n; r0 += (int64_t)gridDim.x * 32) {
-    // warp w takes rows r0 + 4 w .. r0 + 4 w + 3, all four rows' loads issued first
-    float hk[4][8];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int64_t row = r0 + warp * 4 + k;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) hk[k][j] = row < n ? h[row * kHid + lane + 32 * j] : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int rl = warp * 4 + k;
-      const int64_t row = r0 + rl;
-      if (row >= n) break;
-      const float *hv = hk[k];
-      float acc = 0.f;
-      for (int j = 0; j < 8; ++j) acc = fmaf(hv[j], wl[j], acc);
-      const float gg = warp_sum(acc) + b4[0];
-      const float y = label[row];
-      const float dg = (1.f / (1.f + expf(-gg)) - y) * inv_n;
-      if (lane == 0) {
-        ls += y > 0.5f ? softplus(-gg) : softplus(gg);
-        db += dg;
-      }
-      for (int j = 0; j < 8; ++j) {
-        dw[j] = fmaf(dg, hv[j], dw[j]);
-        const float d = dg * wl[j] * (1.f - __expf(-hv[j]));  // softplus' through its output (SFU exp)
-        const int col = lane + 32 * j;
-        dz[row * kHid + col] = d;
-        const __nv_bfloat16 db16 = __float2bfloat16(d);
-        dzb[row * kHid + col] = db16;
-        tile[rl][col] = db16;
-      }
-    }
-    __syncthreads();
-    const int nr = n - r0 < 32 ? (int)(n - r0) : 32;
-    for (int e = threadIdx.x; e < 32 * kHid; e += blockDim.x) {
-      const int col = e >> 5, rl = e & 31;
-      if (rl < nr) dzT[(int64_t)col * n + r0 + rl] = tile[rl][col];
-    }
-    __syncthreads();
-  }
-  for (int j = 0; j < 8; ++j) red_w[warp][lane + 32 * j] = dw[j];
-  if (lane == 0) {
-    red_b[warp] = db;
-    red_l[warp] = ls;
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < kHid; c += blockDim.x) {
-    float s = 0.f;
-    for (int w = 0; w < 8; ++w) s += red_w[w][c];
-    atomicAdd(&grad_w4[c], s);
-  }
-  if (threadIdx.x == 0) {
-    float s = 0.f, l = 0.f;
-    for (int w = 0; w < 8; ++w) {
-      s += red_b[w];
-      l += red_l[w];
-    }
-    atomicAdd(grad_b4, s);
-    if (loss != nullptr) atomicAdd(loss, l * inv_n);
-  }
-}
-
-// Column sums of z [n, 256] (float32) added into out: thread t reads columns 4 (t % 64) .. + 3
-// (16-byte loads, a warp reads 512 contiguous bytes of a row) of every fourth row of the
-// block's slab, and the four row groups meet in shared memory.
-__global__ void __launch_bounds__(kHid) colsum_kernel(const float *z, int64_t n, float *out) {
-  __shared__ float4 part[4][kHid / 4];
-  const int t = threadIdx.x, q = t & (kHid / 4 - 1), grp = t / (kHid / 4);
-  const int64_t per = (n + gridDim.x - 1) / gridDim.x;
-  const int64_t r0 = (int64_t)blockIdx.x * per, r1 = min(n, r0 + per);
-  const float4 *z4 = reinterpret_cast<const float4 *>(z);
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int64_t r = r0 + grp; r < r1; r += 4) {
-    const float4 v = z4[r * (kHid / 4) + q];
-    s.x += v.x;
-    s.y += v.y;
-    s.z += v.z;
-    s.w += v.w;
-  }
-  part[grp][q] = s;
-  __syncthreads();
-  const float *pf = reinterpret_cast<const float *>(part);
-  if (r0 < r1) atomicAdd(&out[t], (pf[t] + pf[kHid + t]) + (pf[2 * kHid + t] + pf[3 * kHid + t]));
 }
 
 // Adam (Kingma & Ba 2015) with bias corrections c1 = 1 / (1 - beta1^t),
@@ -1138,8 +920,6 @@ __device__ inline double block_sum_d(double v, double *red) {
 // share of the nodes to (its max m_b, sum exp(temper (g - m_b)) in float64, a non-finite flag);
 // every block of grid_apply_kernel combines the partials (M = max m_b,
 // Z = sum_b s_b exp(temper (m_b - M))) and rewrites its share of the nodes.
-constexpr int kNormBlocks = 152, kNormThreads = 1024;
-
 __global__ void __launch_bounds__(kNormThreads) grid_partials_kernel(const float *node, int64_t n, float temper,
                                                                      double *partial, kups_status *status) {
   __shared__ float redf[32];
@@ -1610,30 +1390,516 @@ int32_t fused_forward(const kups_mlp *net, const double *x, int64_t n, int grid,
 
 inline unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// Forward pass of rows [row0, row0 + c) into w (activations) and g_out; ``train``
-// also writes the transposed copies the weight gradients need.
-int32_t forward_chunk(const kups_mlp *net, const double *x, int64_t row0, int64_t c, int grid, const MlpWork &w,
-                      float *g_out, kups_status *status, cudaStream_t st, bool train = false) {
-  const __nv_bfloat16 *pb = (const __nv_bfloat16 *)net->param_bf16;
-  const float *p = net->param;
-  features_kernel<<<blocks(c, 256), 256, 0, st>>>(x, row0, c, grid, net->freq, w.feat, train ? w.featT : nullptr);
-  int32_t rc;
-  rc = gemm_call(Op{w.feat, 1, kIn, 1}, Op{pb + kOffW1, 1, kIn, 1}, w.h1, kHid, 1, w.h1b, p + kOffB1, nullptr, 0,
-                 (int)c, kHid, kIn, 0.f, 2, 1, status, st, train ? w.h1T : nullptr);
-  if (rc) return rc;
-  rc = gemm_call(Op{w.h1b, 1, kHid, 1}, Op{pb + kOffW2, 1, kHid, 1}, w.h2, kHid, 1, w.h2b, p + kOffB2, nullptr, 0,
-                 (int)c, kHid, kHid, 0.f, 2, 1, status, st, train ? w.h2T : nullptr);
-  if (rc) return rc;
-  rc = gemm_call(Op{w.h2b, 1, kHid, 1}, Op{pb + kOffW3, 1, kHid, 1}, w.h3, kHid, 1, nullptr, p + kOffB3, nullptr, 0,
-                 (int)c, kHid, kHid, 0.f, 2, 1, status, st);
-  if (rc) return rc;
-  if (g_out != nullptr) head_kernel<<<blocks(c * 32, 256), 256, 0, st>>>(w.h3, c, p + kOffW4, p + kOffB4, g_out);
-  return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
+// ============================================================================
+// Training step.  One kernel runs forward, loss and backward of a tile of 128 points from its
+// coordinates to the three layers' dL/dz, everything between the layers on chip, by the same three
+// kinds of warps as the forward pass: sixteen epilogue warps (warp w: TMEM lanes 32 (w % 4) ..,
+// columns 64 (w / 4) ..), one loading weights, one issuing MMAs:
+//   h1 = softplus(F W1^T + b1), h2 = softplus(h1 W2^T + b2), h3 = softplus(h2 W3^T + b3),
+//   g = h3 . w4 + b4, dL/dg = (sigmoid(g) - y) / n,
+//   dz3 = dL/dg w4 (1 - e^-h3), dz2 = (dz3 W3) (1 - e^-h2), dz1 = (dz2 W2) (1 - e^-h1)
+// (softplus' through its output).  h3 and h2 stay in tensor memory in float32, h1 goes to the
+// workspace in float32 and comes back to the thread that wrote it; bias and head gradients are
+// float32 column sums.  What the weight gradients read (F, h1, h2 and the dz, bfloat16 row-major) is
+// the kernel's only other traffic, 2.7 KB per point.  A second kernel forms all three weight
+// gradients dz^T h from those rows (points along K, both operands MN-major), so no transposed copy is
+// written.  Sixteen launches with float32 activations, transposed copies and column sums in memory
+// took 172 us of device time for 16384 points and 199 us with their enqueueing; three with Adam now take 70 us, enqueueing included (46 + 18 + 4).
+constexpr int kTrainStages = 4, kTrainEpi = 512, kTrainThreads = kTrainEpi + 64;
+// shared memory: weight stages | A operand | head partials [4][128] | coordinates [6][128] | biases
+// b1 b2 b3 and head weights w4 [4][256] | column sums of dz1, dz2, dz3 and of dL/dg h3 [4][256] |
+// frequencies [32][3] | mbarriers, TMEM slot, flag
+constexpr size_t kTrainOffA = (size_t)kTrainStages * kFwdStage;
+constexpr size_t kTrainOffPart = kTrainOffA + kFwdA;
+constexpr size_t kTrainOffFr = kTrainOffPart + 4 * kFwdTile * 4;
+constexpr size_t kTrainOffPar = kTrainOffFr + 6 * kFwdTile * 4;
+constexpr size_t kTrainOffSum = kTrainOffPar + 4 * kHid * 4;
+constexpr size_t kTrainOffFreq = kTrainOffSum + 4 * kHid * 4;
+constexpr size_t kTrainOffBar = kTrainOffFreq + 3 * kFreq * 4;
+constexpr size_t kTrainSmem = kTrainOffBar + 128 + 1024;
+static_assert(kTrainOffBar % 8 == 0, "mbarriers are 8-byte aligned");
+static_assert(kTrainSmem <= 227 * 1024, "training shared memory above the per-CTA limit");
+
+struct TrainMaps {
+  CUtensorMap w[5];  // W1, W2, W3, W3^T, W2^T in the order a tile takes them
+};
+
+struct TrainRows {  // row-major outputs of n points
+  __nv_bfloat16 *feat, *h1b, *h2b, *dz1, *dz2, *dz3;
+  float *h1;
+};
+
+__device__ inline void tmem_store16(uint32_t taddr, const float (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15, %16};" ::"r"(taddr),
+      "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+      "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+      "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])),
+      "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])),
+      "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])));
 }
 
-int split_for(int64_t k) {
-  const int64_t chunks = (k + kBK - 1) / kBK;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(74, chunks / 4));
+__device__ inline void tmem_get16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  tmem_load16(taddr, r);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// softplus' through the output h = softplus(z): 1 - e^-h (the same bits as through __expf)
+__device__ inline float softplus_gate(float h) { return 1.f - exp2_sfu(__fmul_rn(-1.44269504088896341f, h)); }
+
+// Sum over the warp's 32 lanes (rows) of 16 columns: lane l returns the sum of column l / 2.  Each
+// step halves the columns a lane keeps: 16 shuffles instead of five per column.
+__device__ inline float column_sums16(const float (&v)[16], int lane) {
+  float a[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float keep = lane & 16 ? v[8 + i] : v[i], send = lane & 16 ? v[i] : v[8 + i];
+    a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int o = 8, w = 4; o >= 2; o >>= 1, w >>= 1)
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float keep = lane & o ? a[w + i] : a[i], send = lane & o ? a[i] : a[w + i];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
+}
+
+__device__ inline void add_columns16(float *sums, const float (&v)[16], int lane) {
+  const float t = column_sums16(v, lane);
+  if (!(lane & 1)) atomicAdd(&sums[lane >> 1], t);
+}
+
+// 16 columns of a row in bfloat16: two core-matrix rows of the next A operand and 32 bytes of global
+// memory (whole sectors).
+__device__ inline void store_row16(__nv_bfloat16 *sA, int row, int c0, int K, __nv_bfloat16 *out, bool in,
+                                   const float (&v)[16]) {
+  uint32_t w[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+    w[q] = *reinterpret_cast<const uint32_t *>(&h);
+  }
+  if (sA != nullptr) {
+    *reinterpret_cast<uint4 *>(sA + fwd_core(row, c0, K)) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4 *>(sA + fwd_core(row, c0 + 8, K)) = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+  if (in) st_v8(out, w);
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
+mlp_train_kernel(const __grid_constant__ TrainMaps maps, const float *p, const int32_t *freq, const double *x,
+                 const float *label, int64_t n, TrainRows out, float *grad, float *loss, kups_status *status) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                                          ~uintptr_t(1023));
+  __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smem + kTrainOffA);
+  float *part = reinterpret_cast<float *>(smem + kTrainOffPart);
+  float *fr = reinterpret_cast<float *>(smem + kTrainOffFr);
+  float *spar = reinterpret_cast<float *>(smem + kTrainOffPar);
+  float *sums = reinterpret_cast<float *>(smem + kTrainOffSum);
+  int32_t *sfreq = reinterpret_cast<int32_t *>(smem + kTrainOffFreq);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kTrainOffBar);
+  uint64_t *full = bars, *freed = bars + kTrainStages;
+  uint64_t *ready = bars + 2 * kTrainStages, *acc = ready + 1, *meet = ready + 2, *drained = ready + 3;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ready + 4);
+  volatile int *stop = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int e = tid; e < 4 * kHid; e += kTrainThreads) {
+    const int which = e / kHid;
+    const int64_t off = which == 0 ? kOffB1 : which == 1 ? kOffB2 : which == 2 ? kOffB3 : kOffW4;
+    spar[e] = p[off + e % kHid];
+    sums[e] = 0.f;
+  }
+  for (int e = tid; e < 3 * kFreq; e += kTrainThreads) sfreq[e] = freq[e];
+  if (warp == kTrainEpi / 32) {
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(2 * kHid));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int k = 0; k < kTrainStages; ++k) {
+      mbar_init(smem_u32(&full[k]), 1);
+      mbar_init(smem_u32(&freed[k]), 1);
+    }
+    mbar_init(smem_u32(ready), kTrainEpi);
+    mbar_init(smem_u32(acc), 1);
+    mbar_init(smem_u32(meet), kTrainEpi);
+    mbar_init(smem_u32(drained), 1);
+    *stop = 0;
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const int64_t n_tiles = (n + kFwdTile - 1) / kFwdTile;
+  if (warp < kTrainEpi / 32) {
+    const int quarter = warp & 3, cq = warp >> 2, row = quarter * 32 + lane, cb = cq * 64;
+    const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);  // accumulator columns; h2 at + 256
+    const float *w4 = spar + 3 * kHid;
+    const float b4 = p[kOffB4], inv_n = 1.f / (float)n;
+    float db4 = 0.f, ls = 0.f;
+    uint32_t parity = 0u, met = 0u;
+    auto wait = [&](uint64_t *bar, uint32_t &phase) {
+      const bool done = __all_sync(0xffffffffu, mbar_wait_or_stop(smem_u32(bar), phase, stop));
+      phase ^= 1u;
+      return done;
+    };
+    auto meeting = [&]() {
+      mbar_arrive(smem_u32(meet));
+      return wait(meet, met);
+    };
+    auto next_layer = [&]() {  // A operand written and accumulator read: run the MMAs, wait for them
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(smem_u32(ready));
+      const bool done = wait(acc, parity);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return done;
+    };
+    for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      const int64_t row0 = tile * kFwdTile, pt = row0 + row;
+      const bool in = pt < n;
+      const float y = in ? label[pt] : 0.f;
+      if (tid < kFwdTile) {  // coordinates reduced to [-0.5, 0.5) in float64, kept as float pairs
+        for (int a = 0; a < 3; ++a) {
+          const double f = row0 + tid < n ? x[3 * (row0 + tid) + a] : 0.0, red = f - rint(f);
+          const float hi = (float)red;
+          fr[a * kFwdTile + tid] = hi;
+          fr[(3 + a) * kFwdTile + tid] = (float)(red - (double)hi);
+        }
+      }
+      if (!meeting()) break;
+      {  // 8 of the 32 phases of a row: 16 columns of the first A operand
+        const float fh[3] = {fr[row], fr[kFwdTile + row], fr[2 * kFwdTile + row]};
+        const float fl[3] = {fr[3 * kFwdTile + row], fr[4 * kFwdTile + row], fr[5 * kFwdTile + row]};
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[2 * j] = v[2 * j + 1] = 0.f;
+          if (in) phase_sincos(sfreq + 3 * (8 * cq + j), fh, fl, v[2 * j], v[2 * j + 1]);
+        }
+        store_row16(sA, row, 16 * cq, kIn, out.feat + pt * kIn + 16 * cq, in, v);
+      }
+      if (!next_layer()) break;
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {  // h1: float32 to memory, bfloat16 to the A operand and to memory
+        const int c0 = cb + 16 * s;
+        float v[16];
+        tmem_get16(lanes + c0, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = softplus_fast(v[i] + spar[c0 + i]);
+        if (in) {
+          uint32_t w[8];
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(v[8 * q + e]);
+            st_v8(out.h1 + pt * kHid + c0 + 8 * q, w);
+          }
+        }
+        store_row16(sA, row, c0, kHid, out.h1b + pt * kHid + c0, in, v);
+      }
+      if (!next_layer()) break;
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {  // h2: float32 to the spare tensor memory
+        const int c0 = cb + 16 * s;
+        float v[16];
+        tmem_get16(lanes + c0, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = softplus_fast(v[i] + spar[kHid + c0 + i]);
+        tmem_store16(lanes + kHid + c0, v);
+        store_row16(sA, row, c0, kHid, out.h2b + pt * kHid + c0, in, v);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      if (!next_layer()) break;
+      // h3 in place of its accumulator, and g = h3 . w4 + b4: four interleaved sums per thread of 64
+      // columns, then a tree, the same whatever the timing
+      float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {
+        const int c0 = cb + 16 * s;
+        float v[16];
+        tmem_get16(lanes + c0, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          v[i] = softplus_fast(v[i] + spar[2 * kHid + c0 + i]);
+          dot[i & 3] = fmaf(v[i], w4[c0 + i], dot[i & 3]);
+        }
+        tmem_store16(lanes + c0, v);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      part[cq * kFwdTile + row] = (dot[0] + dot[1]) + (dot[2] + dot[3]);
+      if (!meeting()) break;
+      float dg = 0.f;
+      if (in) {
+        const float gg = ((part[row] + part[kFwdTile + row]) + (part[2 * kFwdTile + row] + part[3 * kFwdTile + row])) + b4;
+        dg = (1.f / (1.f + expf(-gg)) - y) * inv_n;
+        if (cq == 0) {
+          ls += y > 0.5f ? softplus(-gg) : softplus(gg);
+          db4 += dg;
+        }
+      }
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {  // dz3, and the head's gradient dL/dg h3
+        const int c0 = cb + 16 * s;
+        float h[16], v[16];
+        tmem_get16(lanes + c0, h);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = dg * w4[c0 + i] * softplus_gate(h[i]);
+        store_row16(sA, row, c0, kHid, out.dz3 + pt * kHid + c0, in, v);
+        add_columns16(sums + 2 * kHid + c0, v, lane);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = dg * h[i];
+        add_columns16(sums + 3 * kHid + c0, v, lane);
+      }
+      if (!next_layer()) break;
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {  // dz2
+        const int c0 = cb + 16 * s;
+        float h[16], v[16];
+        tmem_get16(lanes + kHid + c0, h);
+        tmem_get16(lanes + c0, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] *= softplus_gate(h[i]);
+        store_row16(sA, row, c0, kHid, out.dz2 + pt * kHid + c0, in, v);
+        add_columns16(sums + kHid + c0, v, lane);
+      }
+      float4 h1v[4];  // this thread's h1 of the first 16 columns, on its way during the MMAs
+      const float4 *h1p = reinterpret_cast<const float4 *>(out.h1 + (in ? pt : 0) * kHid + cb);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) h1v[q] = h1p[q];
+      if (!next_layer()) break;
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {  // dz1 (no gradient into the features)
+        const int c0 = cb + 16 * s;
+        float v[16];
+        const float h[16] = {h1v[0].x, h1v[0].y, h1v[0].z, h1v[0].w, h1v[1].x, h1v[1].y, h1v[1].z, h1v[1].w,
+                             h1v[2].x, h1v[2].y, h1v[2].z, h1v[2].w, h1v[3].x, h1v[3].y, h1v[3].z, h1v[3].w};
+        if (s < 3)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) h1v[q] = h1p[4 * (s + 1) + q];
+        tmem_get16(lanes + c0, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = in ? v[i] * softplus_gate(h[i]) : 0.f;
+        store_row16(nullptr, row, c0, kHid, out.dz1 + pt * kHid + c0, in, v);
+        add_columns16(sums + c0, v, lane);
+      }
+    }
+    if (cq == 0) {
+      db4 = warp_sum(db4);
+      ls = warp_sum(ls);
+      if (lane == 0) {
+        atomicAdd(&grad[kOffB4], db4);
+        if (loss != nullptr) atomicAdd(loss, ls * inv_n);
+      }
+    }
+  } else if (warp == kTrainEpi / 32) {
+    if (lane == 0) {  // weights, in the order of the MMAs
+      int64_t q = 0;
+      bool ok = true;
+      for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x)
+        for (int layer = 0; layer < 5 && ok; ++layer)
+          for (int c = 0; c < (layer == 0 ? kIn : kHid) / kFwdKc; ++c, ++q) {
+            const int st = (int)(q % kTrainStages);
+            if (q >= kTrainStages)
+              ok = mbar_wait_or_stop(smem_u32(&freed[st]), (uint32_t)(q / kTrainStages - 1) & 1u, stop);
+            if (!ok) break;
+            mbar_expect_tx(smem_u32(&full[st]), kFwdStage);
+            tma_load_2d(smem_u32(smem + st * kFwdStage), &maps.w[layer], c * kFwdKc, 0, smem_u32(&full[st]));
+          }
+      if (*stop)  // copies in flight land before the CTA ends
+        for (int64_t k = q > kTrainStages ? q - kTrainStages : 0; k < q; ++k)
+          mbar_wait(smem_u32(&full[k % kTrainStages]), (uint32_t)(k / kTrainStages) & 1u);
+    }
+  } else if (lane == 0) {
+    const uint32_t idesc = make_idesc(kFwdTile, kHid), a0 = smem_u32(sA);
+    int64_t q = 0;
+    uint32_t parity = 0u;
+    bool ok = true;
+    for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x)
+      for (int layer = 0; layer < 5 && ok; ++layer) {
+        ok = mbar_wait_or_stop(smem_u32(ready), parity, stop);
+        if (!ok) break;
+        parity ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int K = layer == 0 ? kIn : kHid;
+        for (int c = 0; c < K / kFwdKc; ++c, ++q) {
+          const int st = (int)(q % kTrainStages);
+          ok = mbar_wait_or_stop(smem_u32(&full[st]), (uint32_t)(q / kTrainStages) & 1u, stop);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t b0 = smem_u32(smem + st * kFwdStage);
+          for (int ks = 0; ks < kFwdKc / 16; ++ks)
+            mma_f16(tmem, make_sdesc(a0 + (c * 4 + ks) * 256, 128, (K / 8) * 128), make_sdesc_sw128(b0 + ks * 32),
+                    idesc, c > 0 || ks > 0);
+          mma_commit(smem_u32(&freed[st]));
+        }
+        if (ok) mma_commit(smem_u32(acc));
+      }
+    if (*stop) {  // MMAs in flight end before the tensor memory is freed
+      mma_commit(smem_u32(drained));
+      mbar_wait(smem_u32(drained), 0u);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (tid == 0 && *stop) status_error(status, KUPS_ERR_UNSUPPORTED, blockIdx.x);
+  for (int e = tid; e < 4 * kHid; e += kTrainThreads) {
+    const int which = e / kHid;
+    const int64_t off = which == 0 ? kOffB1 : which == 1 ? kOffB2 : which == 2 ? kOffB3 : kOffW4;
+    atomicAdd(&grad[off + e % kHid], sums[e]);
+  }
+  if (warp == kTrainEpi / 32) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kHid));
+  }
+}
+
+// Weight gradients dW[o, i] += sum over points of dz[p, o] h[p, i] of the three layers in one launch.
+// Both operands are row-major in points (K), so they are MN-major to the tensor cores: a TMA box of 64
+// columns x 64 points (128-byte rows, 128-byte swizzle) holds 64 of M or N for four K steps of 16, with
+// 8-point groups 1024 bytes apart (stride offset) and the next 64 columns one box further (leading
+// offset).  A CTA forms one 128 x 128 tile (128 x 64 for the first layer) over a share of the points
+// and adds it to the gradient with 16-byte reductions; sixteen shares per tile fill the chip while the
+// reductions stay at 8 MB (64 shares of 128 x 256 tiles moved 34 MB and took 39 us in three launches).
+constexpr int kWgStages = 6, kWgThreads = 256;
+constexpr uint32_t kWgBox = 64 * 64 * 2;  // 8 KB
+constexpr size_t kWgSmem = (size_t)kWgStages * 4 * kWgBox + 1024 + 256;
+
+struct GradMaps {
+  CUtensorMap dz[3], h[3];  // layers 3, 2, 1
+};
+
+__device__ inline uint64_t make_sdesc_sw128_mn(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)(kWgBox >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
+__global__ void __launch_bounds__(kWgThreads, 1)
+mlp_weight_grad_kernel(const __grid_constant__ GradMaps maps, int64_t n, int shares, int shares1, float *grad,
+                       int aligned, kups_status *status) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                                          ~uintptr_t(1023));
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)kWgStages * 4 * kWgBox);
+  uint64_t *freed = full + kWgStages, *done = freed + kWgStages;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
+  int *ok_flag = reinterpret_cast<int *>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // unit: layers 3 and 2: 2 x 2 tiles x shares, then layer 1: 2 tiles x shares1
+  int u = blockIdx.x, which, m0, n0, share, total;
+  if (u < 8 * shares) {
+    which = u / (4 * shares);
+    u -= which * 4 * shares;
+    share = u >> 2;
+    m0 = ((u >> 1) & 1) * 128;
+    n0 = (u & 1) * 128;
+    total = shares;
+  } else {
+    u -= 8 * shares;
+    which = 2;
+    share = u >> 1;
+    m0 = (u & 1) * 128;
+    n0 = 0;
+    total = shares1;
+  }
+  const int bn = which == 2 ? 64 : 128;
+  const int64_t chunks = (n + 63) / 64;
+  const int64_t c_begin = chunks * share / total, nc = chunks * (share + 1) / total - c_begin;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(128));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int k = 0; k < kWgStages; ++k) {
+      mbar_init(smem_u32(&full[k]), 1);
+      mbar_init(smem_u32(&freed[k]), 1);
+    }
+    mbar_init(smem_u32(done), 1);
+    *ok_flag = 1;
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  if (tid == 0) {
+    const uint32_t idesc = make_idesc(128, bn) | (1u << 15) | (1u << 16);  // A and B MN-major
+    const CUtensorMap *ma = &maps.dz[which], *mb = &maps.h[which];
+    const uint32_t bytes = (2 + bn / 64) * kWgBox;
+    auto box = [&](int st, int k) { return smem_u32(smem + ((size_t)st * 4 + k) * kWgBox); };
+    auto load = [&](int64_t j) {
+      const int st = (int)(j % kWgStages), p0 = (int)((c_begin + j) * 64);
+      const uint32_t bar = smem_u32(&full[st]);
+      mbar_expect_tx(bar, bytes);
+      tma_load_2d(box(st, 0), ma, m0, p0, bar);
+      tma_load_2d(box(st, 1), ma, m0 + 64, p0, bar);
+      tma_load_2d(box(st, 2), mb, n0, p0, bar);
+      if (bn == 128) tma_load_2d(box(st, 3), mb, n0 + 64, p0, bar);
+    };
+    bool ok = true;
+    int64_t issued = 0, consumed = 0;
+    for (; issued < kWgStages && issued < nc; ++issued) load(issued);
+    for (int64_t i = 0; i < nc && ok; ++i) {
+      const int st = (int)(i % kWgStages);
+      ok = mbar_wait(smem_u32(&full[st]), (uint32_t)(i / kWgStages) & 1u);
+      if (!ok) break;
+      consumed = i + 1;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int ks = 0; ks < 4; ++ks)
+        mma_f16(tmem, make_sdesc_sw128_mn(box(st, 0) + ks * 2048), make_sdesc_sw128_mn(box(st, 2) + ks * 2048), idesc,
+                i > 0 || ks > 0);
+      mma_commit(smem_u32(&freed[st]));
+      // refill the stage of the chunk before this one, whose MMAs end first
+      if (i > 0 && issued < nc) {
+        const int64_t k = i - 1;
+        ok = mbar_wait(smem_u32(&freed[k % kWgStages]), (uint32_t)(k / kWgStages) & 1u);
+        if (ok) load(issued++);
+      }
+    }
+    mma_commit(smem_u32(done));
+    const bool mma_done = mbar_wait(smem_u32(done), 0u);
+    if (!ok)  // loads still in flight land before the tile ends
+      for (int64_t j = consumed; j < issued; ++j)
+        mbar_wait(smem_u32(&full[j % kWgStages]), (uint32_t)(j / kWgStages) & 1u);
+    *ok_flag = ok && mma_done ? 1 : 0;
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (!*ok_flag) {
+    if (tid == 0) status_error(status, KUPS_ERR_UNSUPPORTED, blockIdx.x);
+  } else if (nc > 0) {
+    const int quarter = warp & 3, half = warp >> 2, row = m0 + quarter * 32 + lane;
+    const int width = which == 2 ? kIn : kHid;
+    float *c = grad + (which == 0 ? kOffW3 : which == 1 ? kOffW2 : kOffW1) + (int64_t)row * width + n0;
+    for (int c0 = half * (bn / 2); c0 < (half + 1) * (bn / 2); c0 += 16) {
+      float v[16];
+      tmem_get16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
+      if (aligned) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) red_add_v4(c + c0 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) atomicAdd(c + c0 + i, v[i]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128));
 }
 
 }  // namespace
@@ -1660,9 +1926,6 @@ extern "C" int32_t kups_gemm_bf16(const void *a, int32_t a_bf16, int64_t sa_row,
   g.m = m; g.n = n; g.k = k; g.alpha = alpha; g.beta = beta; g.act = act;
   g.a_bf16 = a_bf16; g.b_bf16 = b_bf16; g.c_bf16 = c_bf16; g.c2_bf16 = c2_bf16; g.gate_kind = gate_kind;
   g.split_k = split_k;
-  g.c3 = nullptr;
-  g.sc3r = g.sc3c = 0;
-  g.fast_math = 0;
   return dispatch_gemm(g, status, (cudaStream_t)stream);
 }
 
@@ -1699,39 +1962,40 @@ extern "C" int32_t kups_mlp_bwd(const kups_mlp *net, const double *x, const floa
   if (workspace_bytes < kups_mlp_workspace_bytes(n)) return KUPS_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
   const MlpWork w = carve(workspace, n);
-  int32_t rc = forward_chunk(net, x, 0, n, 0, w, nullptr, status, st, true);
-  if (rc) return rc;
-  const __nv_bfloat16 *pbt = (const __nv_bfloat16 *)net->param_bf16_t;  // W2^T, W3^T
-  const float *p = net->param;
-  float *gr = net->grad;
-  const int sms = 148;
-  head_nce_kernel<<<std::min<int64_t>(blocks(n, 32), 4 * sms), 256, 0, st>>>(
-      w.h3, n, p + kOffW4, p + kOffB4, label, w.dza, w.dzab, w.dzaT, gr + kOffW4, gr + kOffB4, loss);
-  const int split = split_for(n);
-  const unsigned cs_blocks = (unsigned)std::min<int64_t>(blocks(n, 32), 4 * sms);
-  // Every GEMM operand is bfloat16 with K contiguous: the weight gradients read the
-  // transposed copies ([width, n], K = points), the input gradients W^T.
-  // layer 3: dW3 += dz3^T h2, db3 += colsum dz3, dz2 = (dz3 W3) * (1 - exp(-h2))
-  rc = gemm_call(Op{w.dzaT, 1, n, 1}, Op{w.h2T, 1, n, 1}, gr + kOffW3, kHid, 1, nullptr, nullptr, nullptr, 0, kHid,
-                 kHid, n, 1.f, 0, split, status, st);
-  if (rc) return rc;
-  colsum_kernel<<<cs_blocks, kHid, 0, st>>>(w.dza, n, gr + kOffB3);
-  rc = gemm_call(Op{w.dzab, 1, kHid, 1}, Op{pbt + kHid * kHid, 1, kHid, 1}, w.dzb, kHid, 1, w.dzbb, nullptr, w.h2, 3,
-                 n, kHid, kHid, 0.f, 0, 1, status, st, w.dzbT);
-  if (rc) return rc;
-  // layer 2
-  rc = gemm_call(Op{w.dzbT, 1, n, 1}, Op{w.h1T, 1, n, 1}, gr + kOffW2, kHid, 1, nullptr, nullptr, nullptr, 0, kHid,
-                 kHid, n, 1.f, 0, split, status, st);
-  if (rc) return rc;
-  colsum_kernel<<<cs_blocks, kHid, 0, st>>>(w.dzb, n, gr + kOffB2);
-  rc = gemm_call(Op{w.dzbb, 1, kHid, 1}, Op{pbt, 1, kHid, 1}, w.dza, kHid, 1, nullptr, nullptr, w.h1, 3, n, kHid,
-                 kHid, 0.f, 0, 1, status, st, w.dzaT);
-  if (rc) return rc;
-  // layer 1 (no gradient into the features)
-  rc = gemm_call(Op{w.dzaT, 1, n, 1}, Op{w.featT, 1, n, 1}, gr + kOffW1, kIn, 1, nullptr, nullptr, nullptr, 0, kHid,
-                 kIn, n, 1.f, 0, split, status, st);
-  if (rc) return rc;
-  colsum_kernel<<<cs_blocks, kHid, 0, st>>>(w.dza, n, gr + kOffB1);
+  const __nv_bfloat16 *pb = (const __nv_bfloat16 *)net->param_bf16, *pbt = (const __nv_bfloat16 *)net->param_bf16_t;
+  if ((((uintptr_t)pb | (uintptr_t)pbt) & 15) != 0) {  // TMA reads from 16-byte boundaries
+    KUPS_CUDA_TRY(cudaMemcpyAsync(w.weights, pb, 2 * kParams, cudaMemcpyDeviceToDevice, st));
+    __nv_bfloat16 *t = w.weights + kWeightCopy - 2 * kHid * kHid;
+    KUPS_CUDA_TRY(cudaMemcpyAsync(t, pbt, 2 * 2 * kHid * kHid, cudaMemcpyDeviceToDevice, st));
+    pb = w.weights;
+    pbt = t;
+  }
+  TrainMaps tm;
+  GradMaps gm;
+  const __nv_bfloat16 *weights[5] = {pb + kOffW1, pb + kOffW2, pb + kOffW3, pbt + kHid * kHid, pbt};
+  for (int k = 0; k < 5; ++k) {
+    const int64_t cols = k == 0 ? kIn : kHid;
+    if (!operand_map(&tm.w[k], weights[k], kHid, cols, cols, kHid)) return KUPS_ERR_CUDA;
+  }
+  const __nv_bfloat16 *dz[3] = {w.dz3, w.dz2, w.dz1}, *h[3] = {w.h2b, w.h1b, w.feat};
+  for (int k = 0; k < 3; ++k) {
+    const int64_t cols = k == 2 ? kIn : kHid;
+    if (!operand_map(&gm.dz[k], dz[k], n, kHid, kHid, 64) || !operand_map(&gm.h[k], h[k], n, cols, cols, 64))
+      return KUPS_ERR_CUDA;
+  }
+  KUPS_CUDA_TRY(cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
+  KUPS_CUDA_TRY(cudaFuncSetAttribute(mlp_weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kWgSmem));
+  const int64_t tiles = (n + kFwdTile - 1) / kFwdTile, chunks = (n + 63) / 64;
+  const TrainRows rows{w.feat, w.h1b, w.h2b, w.dz1, w.dz2, w.dz3, w.h1};
+  mlp_train_kernel<<<(unsigned)std::min<int64_t>(tiles, device_sm_count()), kTrainThreads, kTrainSmem, st>>>(
+      tm, net->param, net->freq, x, label, n, rows, net->grad, loss, status);
+  // shares of the points: 8 x 16 + 2 x 10 CTAs for a batch that gives each at least two chunks of 64
+  const int shares = (int)std::min<int64_t>(16, std::max<int64_t>(1, chunks / 2));
+  const int shares1 = (int)std::min<int64_t>(10, std::max<int64_t>(1, chunks / 2));
+  const int aligned = ((uintptr_t)net->grad & 15) == 0;
+  mlp_weight_grad_kernel<<<8 * shares + 2 * shares1, kWgThreads, kWgSmem, st>>>(gm, n, shares, shares1, net->grad,
+                                                                                aligned, status);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 
@@ -1756,14 +2020,13 @@ extern "C" int32_t kups_mlp_grid_norm(const kups_mlp *net, int32_t grid, float t
   const MlpWork w = carve(workspace, std::min<int64_t>(n, kChunk));
   const int32_t rc = fused_forward(net, nullptr, n, grid, node, status, st);
   if (rc) return rc;
-  // the normaliser's partials and the scan's block totals live in the (unused) activation buffers
-  double *partial = reinterpret_cast<double *>(w.h2);
+  double *partial = w.partial;
   const int n_norm = (int)std::min<int64_t>(kNormBlocks, (n + kNormThreads - 1) / kNormThreads);
   grid_partials_kernel<<<n_norm, kNormThreads, 0, st>>>(node, n, temper, partial, status);
   grid_apply_kernel<<<4 * kNormBlocks, 256, 0, st>>>(node, n, temper, floor_frac, partial, n_norm);
   // three-pass scan
   const int n_blocks = (int)((n + kCdfPerBlock - 1) / kCdfPerBlock);
-  double *totals = reinterpret_cast<double *>(w.h1);
+  double *totals = reinterpret_cast<double *>(w.h1);  // unused here: at least a double per 2048 nodes
   grid_cdf_local_kernel<<<n_blocks, kCdfThreads, 0, st>>>(node, grid, cdf, totals);
   grid_cdf_totals_kernel<<<1, kCdfThreads, 0, st>>>(totals, n_blocks, cdf, n);
   grid_cdf_offset_kernel<<<blocks(n, 256), 256, 0, st>>>(cdf, n, totals);
