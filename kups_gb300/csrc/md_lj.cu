@@ -421,25 +421,32 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
   }
   __syncthreads();
   prof_add(prof, 7, tp);
-  // 3. Verlet list.  Work unit: a chunk of up to 32 consecutive (cell-sorted)
-  //    atoms of one x-row of cells, one lane per atom (a system's atoms fill
+  // 3. Verlet list.  Work unit: a chunk of up to 16 consecutive (cell-sorted)
+  //    atoms of one x-row of cells, two lanes per atom (a system's atoms fill
   //    only the central rows of the extended grid, so whole rows as units left
   //    warps idle); sm.bin_b[r] holds the exclusive prefix of the rows' chunk
   //    counts.  The candidates of a chunk are the contiguous atom and ghost
-  //    ranges of the 3 x 3 neighbour rows over the x-range of the chunk's cells
-  //    plus one cell either side, read once per warp (shared-memory broadcast).
-  //    Hits of 32 candidates are gathered in a per-lane bit mask, then appended
-  //    in candidate order (deterministic), four per 8-byte store.
+  //    ranges of the 3 x 3 neighbour rows over the x-range of its cells (those
+  //    of 32 atoms) plus one cell either side.  The warp first tests 32 of them
+  //    at a time, one per lane, against the chunk's bounding box: their squared
+  //    distance to it, rounded as the test's, is never above that to an atom in
+  //    it.  The third that is left is queued in order (sm.bin_a, 64 per warp)
+  //    and tested 32 at a time, lane h of an atom taking 16 of them (a
+  //    shared-memory broadcast); the hits are appended in candidate order
+  //    (deterministic), each lane its own, four entries per 8-byte unit.
+  //    864 atoms with 75 neighbours: one lane per atom on all candidates was
+  //    bound by issue, 190 us on its SM; now 117.
   const int lane = threadIdx.x & 31;
   const int ltpa = __ffs(tpa) - 1;
   const uint32_t sent = (uint32_t)n_items;
   const int n_rows = p.nc[1] * p.nc[2];
   uint16_t *rowp = sm.bin_b;
+  uint16_t *queue = sm.bin_a + 64 * (threadIdx.x >> 5);
   {
     int carry = 0;
     for (int r0 = 0; r0 < n_rows; r0 += nt) {
       const int r = r0 + tid;
-      const int v = r < n_rows ? (sm.cell_start[(r + 1) * p.nc[0]] - sm.cell_start[r * p.nc[0]] + 31) >> 5 : 0;
+      const int v = r < n_rows ? (sm.cell_start[(r + 1) * p.nc[0]] - sm.cell_start[r * p.nc[0]] + 15) >> 4 : 0;
       int tot;
       const int ex = block_exclusive_scan<int>(v, sm.iscan, &tot);
       __syncthreads();
@@ -467,67 +474,104 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
     const int z0 = max(cz - 1, 0), z1 = min(cz + 1, p.nc[2] - 1);
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, p.nc[1] - 1);
     const float rl2 = p.rl2;
-    {
-      const int a0 = ab + (unit - rowp[row]) * 32;
-      // x-range of the chunk's cells (cells of a row are consecutive)
-      const int last = min(a0 + 32, ae) - 1;
-      int cfirst = 0, clast = 0;
-      for (int c = 0; c < p.nc[0]; ++c) {
-        if (sm.cell_start[rowc + c] <= a0) cfirst = c;
-        if (sm.cell_start[rowc + c] <= last) clast = c;
-      }
-      const int x0 = max(cfirst - 1, 0), x1 = min(clast + 1, p.nc[0] - 1);
-      const bool mine = a0 + lane < ae;
-      const int i = mine ? a0 + lane : ab;
-      const float4 q = sm.pos[i];
-      int cnt = 0;
-      // entry e of atom i: row t = e / (4 tpa) of its list, lane g = e % tpa, slot k of
-      // the lane's 4-entry unit = (e / tpa) % 4, so at each slot the atom's tpa lanes read
-      // tpa consecutive entries (consecutive candidates in cell order: mostly distinct banks)
-      uint16_t *nl16 = reinterpret_cast<uint16_t *>(nl);
-      auto put = [&](int e, uint32_t j) {
-        const int t = e >> (ltpa + 2), g = e & (tpa - 1), k = (e >> ltpa) & 3;
-        nl16[((((size_t)t * n + i) << ltpa) + g) * 4 + k] = (uint16_t)j;
-      };
-      auto push = [&](uint32_t j) {
-        if (cnt < nb_cap) put(cnt, j);
-        ++cnt;
-      };
-      auto scan_range = [&](int kb, int ke) {
-        for (int k0 = kb; k0 < ke; k0 += 32) {
-          const int kn = min(32, ke - k0);
-          uint32_t hits = 0;
+    const int a0 = ab + (unit - rowp[row]) * 16;
+    // x-range of the cells of the chunk's 32 atoms (cells of a row are consecutive)
+    const int first = a0 - ((a0 - ab) & 16), last = min(first + 32, ae) - 1;
+    int cfirst = 0, clast = 0;
+    for (int c = 0; c < p.nc[0]; ++c) {
+      if (sm.cell_start[rowc + c] <= first) cfirst = c;
+      if (sm.cell_start[rowc + c] <= last) clast = c;
+    }
+    const int x0 = max(cfirst - 1, 0), x1 = min(clast + 1, p.nc[0] - 1);
+    const int half = lane >> 4;
+    const bool mine = a0 + (lane & 15) < ae;
+    const int i = mine ? a0 + (lane & 15) : a0;
+    const float4 q = sm.pos[i];
+    float3 lo = make_float3(q.x, q.y, q.z), up = lo;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+      lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+      lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+      up.x = fmaxf(up.x, __shfl_xor_sync(0xffffffffu, up.x, o));
+      up.y = fmaxf(up.y, __shfl_xor_sync(0xffffffffu, up.y, o));
+      up.z = fmaxf(up.z, __shfl_xor_sync(0xffffffffu, up.z, o));
+    }
+    int cnt = 0, queued = 0;
+    // entry e of atom i: row t = e / (4 tpa) of its list, lane g = e % tpa, slot k of
+    // the lane's 4-entry unit = (e / tpa) % 4, so at each slot the atom's tpa lanes read
+    // tpa consecutive entries (consecutive candidates in cell order: mostly distinct banks)
+    uint16_t *nl16 = reinterpret_cast<uint16_t *>(nl);
+    auto put = [&](int e, uint32_t j) {
+      const int t = e >> (ltpa + 2), g = e & (tpa - 1), k = (e >> ltpa) & 3;
+      nl16[((((size_t)t * n + i) << ltpa) + g) * 4 + k] = (uint16_t)j;
+    };
+    // exact test and entries of the first kn <= 32 queued candidates
+    auto settle = [&](int kn) {
+      const uint32_t own = lane < kn ? queue[lane] : 0xffffu;
+      const int kh = min(16, max(0, kn - 16 * half));
+      uint32_t hits = 0;
 #pragma unroll 4
-          for (int t = 0; t < kn; ++t) {
-            const float4 o = sm.pos[k0 + t];
-            const float dx = o.x - q.x, dy = o.y - q.y, dz = o.z - q.z;
-            const bool h = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < rl2;
-            hits |= (uint32_t)h << t;
-          }
-          if (k0 <= i && i < k0 + kn) hits &= ~(1u << (i - k0));  // not the atom itself
-          if (!mine) hits = 0;
-          while (hits) {
-            const int t = __ffs(hits) - 1;
-            hits &= hits - 1;
-            push((uint32_t)(k0 + t));
-          }
+      for (int t = 0; t < kh; ++t) {
+        const float4 o = sm.pos[queue[16 * half + t]];
+        const float dx = o.x - q.x, dy = o.y - q.y, dz = o.z - q.z;
+        const bool h = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < rl2;
+        hits |= (uint32_t)h << t;
+      }
+      // not the atom itself
+      for (uint32_t self = __ballot_sync(0xffffffffu, own - (uint32_t)a0 < 16u); self; self &= self - 1) {
+        const int t = __ffs(self) - 1;
+        const uint32_t k = __shfl_sync(0xffffffffu, own, t);
+        if (k == (uint32_t)i && (t >> 4) == half) hits &= ~(1u << (t & 15));
+      }
+      if (!mine) hits = 0;
+      const int found = __popc(hits), other = __shfl_xor_sync(0xffffffffu, found, 16);
+      int e = cnt + (half ? other : 0);
+      cnt += found + other;
+      for (; hits; hits &= hits - 1, ++e)
+        if (e < nb_cap) put(e, queue[16 * half + __ffs(hits) - 1]);
+    };
+    auto scan_range = [&](int kb, int ke) {
+      for (int k0 = kb; k0 < ke; k0 += 32) {
+        bool near = false;
+        if (k0 + lane < ke) {
+          const float4 o = sm.pos[k0 + lane];
+          const float ex = fmaxf(fmaxf(lo.x - o.x, o.x - up.x), 0.f), ey = fmaxf(fmaxf(lo.y - o.y, o.y - up.y), 0.f),
+                      ez = fmaxf(fmaxf(lo.z - o.z, o.z - up.z), 0.f);
+          near = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) < rl2;
         }
-      };
-      for (int z = z0; z <= z1; ++z)
-        for (int y = y0; y <= y1; ++y) {
-          const int row = (z * p.nc[1] + y) * p.nc[0];
-          scan_range(sm.cell_start[row + x0], sm.cell_start[row + x1 + 1]);
-          scan_range(n + sm.ghost_start[row + x0], n + sm.ghost_start[row + x1 + 1]);
+        const uint32_t m = __ballot_sync(0xffffffffu, near);
+        if (near) queue[queued + __popc(m & ((1u << lane) - 1))] = (uint16_t)(k0 + lane);
+        queued += __popc(m);
+        __syncwarp();
+        if (queued >= 32) {
+          settle(32);
+          queued -= 32;
+          const uint16_t moved = queue[32 + lane];
+          __syncwarp();
+          queue[lane] = moved;  // at most 31 of them are queued
+          __syncwarp();
         }
-      if (mine) {
-        const int total_cnt = cnt;
+      }
+    };
+    for (int z = z0; z <= z1; ++z)
+      for (int y = y0; y <= y1; ++y) {
+        const int row = (z * p.nc[1] + y) * p.nc[0];
+        scan_range(sm.cell_start[row + x0], sm.cell_start[row + x1 + 1]);
+        scan_range(n + sm.ghost_start[row + x0], n + sm.ghost_start[row + x1 + 1]);
+      }
+    settle(queued);
+    __syncwarp();
+    if (mine) {
+      const int total_cnt = cnt;
+      if (half == 0) {
         // pad the last row with the sentinel item (whole rows of at most nb_cap entries stay
         // below n * md_units_per_atom units, which rounds nb_cap / 4 up to 16 units)
         if (cnt <= nb_cap)
           for (; cnt & (4 * tpa - 1); ++cnt) put(cnt, sent);
         sm.nbr_count[i] = (uint16_t)min(total_cnt, nb_cap);
-        my_max = max(my_max, total_cnt);
       }
+      my_max = max(my_max, total_cnt);
     }
   }
   if (my_max > nb_cap) atomicMax(&sm.flag, my_max);
