@@ -64,6 +64,10 @@ enum {
 const char *kups_version(void);
 const char *kups_error_string(int32_t code);
 
+/* The state a call expects its status word in (code KUPS_OK, nothing required, first_bad -1), and
+ * n_counts counters after it set to zero, in one launch. */
+int32_t kups_status_init(kups_status *status, int64_t *counts, int32_t n_counts, void *stream);
+
 /* ------------------------------------------------------------------------
  * Neighbour list — replaces CellListNeighborList.__call__ and
  * DenseNearestNeighborList.__call__ (src/kups/core/neighborlist.py:985-1077,

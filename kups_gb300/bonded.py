@@ -181,9 +181,9 @@ def evaluate(terms, positions, system, species, tril):
     spc = torch.as_tensor(species, device=dev).to(torch.int32).contiguous()
     tr = torch.as_tensor(tril, dtype=torch.float64, device=dev).contiguous()
     S = tr.shape[0]
-    energy = torch.zeros(S, dtype=torch.float64, device=dev)
+    per_system = torch.zeros(7 * S, dtype=torch.float64, device=dev)
+    energy, grad_tril = per_system[:S], per_system[S:].view(S, 6)
     grad = torch.zeros_like(pos)
-    grad_tril = torch.zeros((S, 6), dtype=torch.float64, device=dev)
     status = new_status()
     for t in terms:
         t.add_to(pos, sysi, spc, tr, energy, grad, grad_tril, status)

@@ -317,7 +317,7 @@ class FusedLennardJonesMD:
         # objects are the ones it was built from (the usual loop feeds each output back in)
         packed = pack(state, reuse=self._last)
         self._last = packed
-        self.run_packed(packed, self.steps_per_call, key_to_seed(key), state.step)
+        self._run(packed, self.steps_per_call, key_to_seed(key), state.step, state=state)
         out = unpack(packed, state, INTEGRATORS[self.integrator])
         return replace(out, step=state.step + self.steps_per_call)
 
@@ -465,10 +465,9 @@ class FusedLennardJonesMD:
              virial: bool = True, trace_virial=None) -> _lib.MdArgs:
         s = packed.n_systems
         if packed.energy is None:
-            packed.energy = torch.zeros(s, device="cuda", dtype=torch.float64)
-            packed.kinetic = torch.zeros(s, device="cuda", dtype=torch.float64)
-            packed.virial = torch.zeros((s, 6), device="cuda", dtype=torch.float64)
-            packed.pressure = torch.zeros(s, device="cuda", dtype=torch.float64)
+            out = torch.zeros(9 * s, device="cuda", dtype=torch.float64)
+            packed.energy, packed.kinetic, packed.pressure = out[:s], out[s:2 * s], out[2 * s:3 * s]
+            packed.virial = out[3 * s:].view(s, 6)
         a = _lib.MdArgs()
         a.pos, a.mom, a.force = packed.pos4.data_ptr(), packed.mom4.data_ptr(), packed.frc4.data_ptr()
         a.sys_offset, a.order, a.tril = packed.sys_offset.data_ptr(), packed.order.data_ptr(), packed.tril32.data_ptr()
@@ -531,7 +530,13 @@ class FusedLennardJonesMD:
     def run_packed(self, packed: PackedMD, n_steps: int, seed: int = 0, step0: int = 0, trace: bool = False,
                    max_tries: int = 6):
         """Run and check the status; on a capacity overflow restore and retry."""
-        backup = packed.clone_dynamic()
+        return self._run(packed, n_steps, seed, step0, trace, max_tries)
+
+    def _run(self, packed: PackedMD, n_steps: int, seed: int, step0: int, trace: bool = False, max_tries: int = 6,
+             state: MDState | None = None):
+        """``run_packed``; with ``state``, ``packed`` is what ``pack`` made of it, and a retry packs it
+        again instead of taking a copy that every call would make."""
+        backup = packed.clone_dynamic() if state is None else None
         valid0 = packed.forces_valid
         for _ in range(max_tries):
             tpe = tke = None
@@ -543,6 +548,9 @@ class FusedLennardJonesMD:
             if status.code == _lib.KUPS_OK:
                 return (tpe, tke) if trace else None
             if status.code == _lib.KUPS_ERR_CAPACITY and status.detail == _lib.KUPS_CAP_NEIGHBORS:
+                if state is not None:
+                    again = pack(state, reuse=packed)
+                    backup = (again.pos4, again.mom4, again.frc4, again.cell)
                 packed.restore_dynamic(backup)
                 packed.forces_valid = valid0
                 self.neighbor_capacity = int(math.ceil(status.required * 1.25 / 16.0) * 16)

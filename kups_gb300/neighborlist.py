@@ -101,19 +101,18 @@ class CellListNeighborList:
         cap = max(1, self.avg_edges * n)
         edges = torch.empty((cap, 2), device="cuda", dtype=torch.int32)
         shifts = torch.empty((cap, 3), device="cuda", dtype=torch.int32)
-        n_edges = torch.zeros(1, device="cuda", dtype=torch.int64)
         ws_bytes = lib.kups_neighborlist_workspace_bytes(n, s)
         ws = torch.empty(ws_bytes, device="cuda", dtype=torch.uint8)
-        status = new_status()
+        status, n_edges = new_status_and_counts(1)
         rc = lib.kups_neighborlist_build(
             pos.data_ptr(), system.data_ptr(), incl.data_ptr(), excl.data_ptr(), n, n_incl, tril.data_ptr(),
             cut.data_ptr(), s, edges.data_ptr(), shifts.data_ptr(), cap, n_edges.data_ptr(), ws.data_ptr(),
             ws_bytes, status.data_ptr(), _stream(),
         )
         _lib.check(rc, "kups_neighborlist_build")
-        st = read_status(status)
+        st, (n,) = read_status_and_counts(status, n_edges)
         _lib.raise_status(st)
-        return Edges(edges, shifts.view(cap, 1, 3), int(n_edges.item()))
+        return Edges(edges, shifts.view(cap, 1, 3), n)
 
     def _call_rh(self, lh: NeighborListPoints, rh: NeighborListPoints, systems, cutoffs, rh_index_remap) -> Edges:
         """Edges (i in lh, j in rh) (kups_neighborlist_build_rh); with ``rh_index_remap`` the
@@ -141,18 +140,18 @@ class CellListNeighborList:
         cap = max(1, self.avg_edges * max(n_rh, 1) * (2 if remap is not None else 1))
         edges = torch.empty((cap, 2), device="cuda", dtype=torch.int32)
         shifts = torch.empty((cap, 3), device="cuda", dtype=torch.int32)
-        n_edges = torch.zeros(1, device="cuda", dtype=torch.int64)
         ws_bytes = lib.kups_neighborlist_rh_workspace_bytes(n_lh, n_rh, s)
         ws = torch.empty(ws_bytes, device="cuda", dtype=torch.uint8)
-        status = new_status()
+        status, n_edges = new_status_and_counts(1)
         rc = lib.kups_neighborlist_build_rh(
             lp.data_ptr(), lsys.data_ptr(), lincl.data_ptr(), lexcl.data_ptr(), n_lh, rp.data_ptr(), rsys.data_ptr(),
             rincl.data_ptr(), rexcl.data_ptr(), n_rh, remap.data_ptr() if remap is not None else None, n_incl,
             tril.data_ptr(), cut.data_ptr(), s, edges.data_ptr(), shifts.data_ptr(), cap, n_edges.data_ptr(),
             ws.data_ptr(), ws_bytes, status.data_ptr(), _stream())
         _lib.check(rc, "kups_neighborlist_build_rh")
-        _lib.raise_status(read_status(status))
-        return Edges(edges, shifts.view(cap, 1, 3), int(n_edges.item()))
+        st, (n,) = read_status_and_counts(status, n_edges)
+        _lib.raise_status(st)
+        return Edges(edges, shifts.view(cap, 1, 3), n)
 
     def fix(self, err: _lib.CapacityError, n_particles: int) -> "CellListNeighborList":
         per = err.required / max(1, n_particles)
@@ -241,20 +240,34 @@ def neighborlist_changes(neighborlist: CellListNeighborList, lh: NeighborListPoi
     return NeighborListChangesResult(*out)
 
 
+def _status_of(words: list) -> _lib.Status:
+    raw, required, first_bad = words[:3]
+    return _lib.Status(raw & 0xFFFFFFFF, (raw >> 32) & 0xFFFFFFFF, required, first_bad)
+
+
 def read_status(status: torch.Tensor) -> _lib.Status:
-    """Copy a device status word (int64[4]: code|detail, required, first_bad) to the host."""
-    h = status.cpu()
-    raw = int(h[0])
-    code = raw & 0xFFFFFFFF
-    detail = (raw >> 32) & 0xFFFFFFFF
-    return _lib.Status(code, detail, int(h[1]), int(h[2]))
+    """Copy a device status word (int64[3]: code|detail, required, first_bad) to the host."""
+    return _status_of(status.tolist())
 
 
 def new_status(device="cuda") -> torch.Tensor:
-    """Zeroed status word (kups_status is 24 bytes: i32, i32, i64, i64)."""
-    st = torch.zeros(3, device=device, dtype=torch.int64)
-    st[2:].fill_(-1)  # a device fill, safe inside CUDA-graph capture
-    return st
+    """A status word (kups_status is 24 bytes: i32, i32, i64, i64) with no error in it."""
+    return new_status_and_counts(0, device)[0]
+
+
+def new_status_and_counts(n: int, device="cuda") -> tuple[torch.Tensor, torch.Tensor]:
+    """A status word and n int64 counters at zero behind it (one allocation, one launch; capturable)."""
+    words = torch.empty(3 + n, device=device, dtype=torch.int64)
+    status, counts = words[:3], words[3:]
+    rc = _lib.load().kups_status_init(status.data_ptr(), counts.data_ptr() if n else None, n, _stream())
+    _lib.check(rc, "kups_status_init")
+    return status, counts
+
+
+def read_status_and_counts(status: torch.Tensor, counts: torch.Tensor) -> tuple[_lib.Status, list]:
+    """Both of ``new_status_and_counts`` in one copy to the host."""
+    words = status.as_strided((3 + counts.shape[0],), (1,)).tolist()
+    return _status_of(words), words[3:]
 
 
 def estimate_avg_edges(n_particles: int, volume: float, cutoff: float, multiplier: float = 1.0) -> int:
