@@ -541,6 +541,18 @@ int32_t kups_md_kick(double *momenta, const double *grad, const int32_t *system,
 int32_t kups_md_drift(double *positions, const double *momenta, const double *masses,
                       const int32_t *system, const double *dt, const double *tril, double scale,
                       int64_t n_particles, void *stream);
+/* a kick of kick_scale and a drift of drift_scale in one pass */
+int32_t kups_md_kick_drift(double *momenta, const double *grad, double *positions,
+                           const double *masses, const int32_t *system, const double *dt,
+                           const double *tril, double kick_scale, double drift_scale,
+                           int64_t n_particles, void *stream);
+/* grad = grad_a + grad_b [n, 3] and energy = energy_a + energy_b + energy_c [n_systems], then a
+ * kick by grad */
+int32_t kups_md_sum_kick(double *momenta, double *grad, const double *grad_a, const double *grad_b,
+                         const int32_t *system, const double *dt, double scale,
+                         int64_t n_particles, double *energy, const double *energy_a,
+                         const double *energy_b, const double *energy_c, int32_t n_systems,
+                         void *stream);
 int32_t kups_md_thermostat(double *momenta, const double *masses, const int32_t *system,
                            const double *dt, const double *kT, const double *friction,
                            uint64_t seed, uint64_t step, int64_t n_particles, void *stream);

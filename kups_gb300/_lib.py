@@ -123,6 +123,8 @@ SIGNATURES = {
     "kups_ewald_self": (_I32, [_P, _P, _I32, _P, C.c_double, _P, _P]),
     "kups_md_kick": (_I32, [_P, _P, _P, _P, C.c_double, _I64, _P]),
     "kups_md_drift": (_I32, [_P, _P, _P, _P, _P, _P, C.c_double, _I64, _P]),
+    "kups_md_kick_drift": (_I32, [_P, _P, _P, _P, _P, _P, _P, C.c_double, C.c_double, _I64, _P]),
+    "kups_md_sum_kick": (_I32, [_P, _P, _P, _P, _P, _P, C.c_double, _I64, _P, _P, _P, _P, _I32, _P]),
     "kups_md_thermostat": (_I32, [_P, _P, _P, _P, _P, _P, C.c_uint64, C.c_uint64, _I64, _P]),
     "kups_md_thermostat_counted": (_I32, [_P, _P, _P, _P, _P, _P, C.c_uint64, _P, _I64, _P]),
     "kups_virial_stress_workspace_bytes": (C.c_size_t, [_I32, _I32]),

@@ -32,11 +32,15 @@ namespace {
 
 constexpr int kMaxM = 16;            // |n_a| <= 16
 constexpr int kTab = 2 * kMaxM + 1;  // table entries per axis
+constexpr int kRow = 3 * kTab + 1;  // an atom's tables: 8 banks on from the last atom's, no conflicts of 4 atoms x 4 k
 constexpr int kAtomsPerChunk = 32;
 constexpr int kKPerBlock = 128;
+constexpr int kKPerThread = 2;  // of the structure factor
+constexpr int kForceTile = 4 * kKPerBlock;  // k staged at a time by the force kernel
+constexpr int kSetupThreads = 512;
 
 struct Coef {
-  double ps_c, ps_s, ck, pad;  // P S_c, P S_s, cell-gradient coefficient
+  double p, ck, pad[2];  // P(k), its cell-gradient coefficient per K |S|^2
 };
 
 struct RecipSys {
@@ -60,28 +64,41 @@ __device__ inline void kvec(const double *inv, const int n[3], double k[3]) {
   k[2] = tp * (inv[3] * n[0] + inv[4] * n[1] + inv[5] * n[2]);
 }
 
-// One block per system: cell, inverse, volume, and the largest |n_a| over the
-// system's k vectors (block reduction).
-__global__ void recip_setup_kernel(const double *tril, const int32_t *kn, int32_t s, int32_t nk,
-                                   RecipSys *sys, kups_status *status) {
+// One block per system: cell, inverse and volume (by the last warp), the largest |n_a| over the
+// system's k vectors, and zeros for what the later kernels add to: S(k), energy, cell gradient.
+__global__ void __launch_bounds__(kSetupThreads) recip_setup_kernel(const double *tril, const int32_t *kn, int32_t nk,
+                                                                    RecipSys *sys, double *sk, double *energy,
+                                                                    double *dtril, kups_status *status) {
   __shared__ int mx[3];
   const int i = blockIdx.x;
   if (threadIdx.x < 3) mx[threadIdx.x] = 0;
   __syncthreads();
   int m[3] = {0, 0, 0};
-  for (int k = threadIdx.x; k < nk; k += blockDim.x)
+#pragma unroll 4
+  for (int k = threadIdx.x; k < nk; k += kSetupThreads)
+#pragma unroll
     for (int a = 0; a < 3; ++a) m[a] = max(m[a], abs(kn[((int64_t)i * nk + k) * 3 + a]));
-  for (int a = 0; a < 3; ++a) atomicMax(&mx[a], m[a]);
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  RecipSys r;
-  const Tril64 L = load_tril64(tril + 6 * (int64_t)i);
-  const Tril64 inv = inverse_tril64(L);
-  for (int k = 0; k < 6; ++k) {
-    r.L[k] = L.t[k];
-    r.inv[k] = inv.t[k];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int v = __reduce_max_sync(0xffffffffu, m[c]);
+    if ((threadIdx.x & 31) == 0) atomicMax(&mx[c], v);
   }
-  r.volume = fabs(L.t[0] * L.t[2] * L.t[5]);
+  if (sk != nullptr)
+    for (int e = threadIdx.x; e < 2 * nk; e += kSetupThreads) sk[(int64_t)i * nk * 2 + e] = 0.0;
+  if (threadIdx.x == 0) energy[i] = 0.0;
+  if (threadIdx.x < 6 && dtril != nullptr) dtril[6 * (int64_t)i + threadIdx.x] = 0.0;
+  RecipSys r;
+  if (threadIdx.x == kSetupThreads - 1) {
+    const Tril64 L = load_tril64(tril + 6 * (int64_t)i);
+    const Tril64 inv = inverse_tril64(L);
+    for (int k = 0; k < 6; ++k) {
+      r.L[k] = L.t[k];
+      r.inv[k] = inv.t[k];
+    }
+    r.volume = fabs(L.t[0] * L.t[2] * L.t[5]);
+  }
+  __syncthreads();
+  if (threadIdx.x != kSetupThreads - 1) return;
   for (int a = 0; a < 3; ++a) {
     int v = mx[a];
     if (v > kMaxM) {
@@ -93,141 +110,152 @@ __global__ void recip_setup_kernel(const double *tril, const int32_t *kn, int32_
   sys[i] = r;
 }
 
-// Per-atom tables e^{2 pi i m f_a}, m in [-M, M], from sincospi of the
-// fundamental and complex products (error grows ~linearly in |m| <= 16).
-__device__ inline void fill_tables(float2 *tab, const double f[3]) {
-  for (int a = 0; a < 3; ++a) {
+// Per-atom tables e^{2 pi i m f_a}, m in [-M_a, M_a], from sincospi of the fundamental and complex
+// products (error grows ~linearly in |m| <= 16): thread t < 96 of a block fills axis t / 32 of atom
+// c0 + t % 32 (three short chains side by side instead of one of 48 products per atom).
+__device__ inline void fill_tables(float2 (*tab)[kRow], const double *pos, int64_t c0, int na, const RecipSys &P) {
+  static_assert(kAtomsPerChunk == 32, "one warp per axis");
+  const int t = threadIdx.x & 31;
+  if (t >= na) return;
+  for (int a = threadIdx.x >> 5; a < 3; a += (int)blockDim.x >> 5) {
+    const double *r = pos + 3 * (c0 + t), *inv = P.inv;
+    const double f = a == 0 ? (r[0] * inv[0] + r[1] * inv[1]) + r[2] * inv[3]
+                     : a == 1 ? r[1] * inv[2] + r[2] * inv[4]
+                              : r[2] * inv[5];
     float s1, c1;
     // reduce f to [-0.5, 0.5) in float64 first so the float32 argument is small
-    const double fr = f[a] - rint(f[a]);
+    const double fr = f - rint(f);
     sincospif((float)(2.0 * fr), &s1, &c1);
-    float2 *t = tab + a * kTab + kMaxM;
-    t[0] = make_float2(1.f, 0.f);
+    float2 *row = tab[t] + a * kTab + kMaxM;
+    row[0] = make_float2(1.f, 0.f);
     float cr = 1.f, ci = 0.f;
-    for (int m = 1; m <= kMaxM; ++m) {
-      const float nr = cr * c1 - ci * s1;
-      const float ni = cr * s1 + ci * c1;
+    const int m_max = P.m[a];
+    for (int m = 1; m <= m_max; ++m) {
+      const float nr = fmaf(cr, c1, -__fmul_rn(ci, s1));
+      const float ni = fmaf(cr, s1, __fmul_rn(ci, c1));
       cr = nr;
       ci = ni;
-      t[m] = make_float2(cr, ci);
-      t[-m] = make_float2(cr, -ci);
+      row[m] = make_float2(cr, ci);
+      row[-m] = make_float2(cr, -ci);
     }
   }
 }
 
-__device__ inline float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// Row of component n in an axis' table (the setup refuses |n| > kMaxM: any row of the table then)
+__device__ inline int table_row(int n) { return min(max(n, -kMaxM), kMaxM) + kMaxM; }
+
+// Complex products of the tables' entries.  Which product of each sum is rounded is written out: the
+// phases of S(k) and of the forces are the same to the bit, whatever surrounds them.
+__device__ inline float2 phase_xy(float2 x, float2 y) {
+  return make_float2(fmaf(x.x, y.x, -__fmul_rn(x.y, y.y)), fmaf(x.y, y.x, __fmul_rn(x.x, y.y)));
+}
+__device__ inline float2 phase_xyz(float2 a, float2 z) {
+  return make_float2(fmaf(a.x, z.x, -__fmul_rn(a.y, z.y)), fmaf(a.x, z.y, __fmul_rn(a.y, z.x)));
 }
 
-// S(k): grid (k tiles, atom chunks, systems).  Each block stages the tables of
-// 32 atoms in shared memory; each thread owns one k and accumulates the
-// chunk in float32, then adds it to S in float64.
-__global__ void structure_factor_kernel(const double *pos, const double *q, const int32_t *sys_offset,
-                                        const int32_t *kn, int32_t nk, const RecipSys *sysp,
-                                        double *sk, double *grad) {
-  __shared__ float2 tab[kAtomsPerChunk][3 * kTab];
+// P(k) and the coefficient of K |S(k)|^2 in the cell gradient, 0 for k = 0.
+__device__ inline Coef prefactor(const RecipSys &P, const int *nv, double a) {
+  const double tp = 6.283185307179586476925286766559;
+  const int n3[3] = {nv[0], nv[1], nv[2]};
+  double kv[3];
+  kvec(P.inv, n3, kv);
+  const double k2 = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
+  Coef c{0.0, 0.0, {0.0, 0.0}};
+  if (k2 > 0.0) {
+    c.p = (2.0 - (n3[0] == 0 ? 1.0 : 0.0)) * tp / P.volume * exp(-k2 / (4.0 * a * a)) / k2;
+    c.ck = c.p * (-1.0 / (2.0 * a * a) - 2.0 / k2);
+  }
+  return c;
+}
+
+// S(k): grid (k tiles, atom chunks, systems).  Each block stages the tables of 32 atoms
+// in shared memory; each thread owns two k and accumulates the chunk in float32, then adds it to S in
+// float64; the chunks' additions to the same addresses bound it.  The warp that has no table to fill forms
+// prefactors P(k) meanwhile: their float64 exponentials and divisions were 10 us of a launch of their own.
+// 2800 k, 4000 atoms: 16.6 us with one k per thread and a thread per atom's tables, now 15.7 (17.0 with one
+// k per thread, 17.7 with four).
+__global__ void __launch_bounds__(kKPerBlock) structure_factor_kernel(const double *pos, const double *q,
+                                                                      const int32_t *sys_offset, const int32_t *kn,
+                                                                      int32_t nk, const RecipSys *sysp,
+                                                                      const double *alpha, Coef *coef, double *sk,
+                                                                      double *grad) {
+  __shared__ float2 tab[kAtomsPerChunk][kRow];
   __shared__ float qs[kAtomsPerChunk];
   const int s = blockIdx.z;
+  const RecipSys &P = sysp[s];
+  const int kb = blockIdx.x * kKPerBlock * kKPerThread + threadIdx.x;
   const int a0 = sys_offset[s], a1 = sys_offset[s + 1];
   const int c0 = a0 + blockIdx.y * kAtomsPerChunk;
   if (c0 >= a1) return;
   const int na = min(kAtomsPerChunk, a1 - c0);
-  const RecipSys &P = sysp[s];
-  for (int t = threadIdx.x; t < na; t += blockDim.x) {
-    const double r[3] = {pos[3 * (c0 + t)], pos[3 * (c0 + t) + 1], pos[3 * (c0 + t) + 2]};
-    double f[3];
-    frac64(P.inv, r, f);
-    fill_tables(tab[t], f);
-    qs[t] = (float)q[c0 + t];
-    // the force kernel adds its k-range partials into grad: zero this chunk's rows first
-    if (blockIdx.x == 0 && grad != nullptr)
-      for (int a = 0; a < 3; ++a) grad[3 * (int64_t)(c0 + t) + a] = 0.0;
-  }
+  fill_tables(tab, pos, c0, na, P);
+  if (threadIdx.x >= 96)  // the warp without a table: the prefactors of 32 k of the tile for some chunks
+    for (int j = blockIdx.y; j < kKPerBlock * kKPerThread / 32; j += (a1 - a0 + kAtomsPerChunk - 1) / kAtomsPerChunk) {
+      const int64_t k = (int64_t)blockIdx.x * kKPerBlock * kKPerThread + 32 * j + (threadIdx.x - 96);
+      if (k < nk) coef[(int64_t)s * nk + k] = prefactor(P, kn + ((int64_t)s * nk + k) * 3, alpha[s]);
+    }
+  if (threadIdx.x < na) qs[threadIdx.x] = (float)q[c0 + threadIdx.x];
+  // the force kernel adds its k-range partials into grad: zero this chunk's rows first
+  if (blockIdx.x == 0 && grad != nullptr && threadIdx.x < 3 * na) grad[3 * (int64_t)c0 + threadIdx.x] = 0.0;
   __syncthreads();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nk) return;
-  const int *nv = kn + ((int64_t)s * nk + k) * 3;
-  const int nx = nv[0] + kMaxM, ny = nv[1] + kMaxM, nz = nv[2] + kMaxM;
-  float sc = 0.f, ss = 0.f;
-  for (int t = 0; t < na; ++t) {
-    const float2 e = cmul(cmul(tab[t][nx], tab[t][kTab + ny]), tab[t][2 * kTab + nz]);
-    sc = fmaf(qs[t], e.x, sc);
-    ss = fmaf(qs[t], e.y, ss);
+  int row[kKPerThread][3];
+  float sc[kKPerThread], ss[kKPerThread];
+#pragma unroll
+  for (int j = 0; j < kKPerThread; ++j) {
+    const int *nv = kn + ((int64_t)s * nk + min(kb + j * kKPerBlock, nk - 1)) * 3;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) row[j][a] = a * kTab + table_row(nv[a]);
+    sc[j] = ss[j] = 0.f;
   }
-  atomicAdd(&sk[((int64_t)s * nk + k) * 2], (double)sc);
-  atomicAdd(&sk[((int64_t)s * nk + k) * 2 + 1], (double)ss);
+  for (int t = 0; t < na; ++t)
+#pragma unroll
+    for (int j = 0; j < kKPerThread; ++j) {
+      const float2 e = phase_xyz(phase_xy(tab[t][row[j][0]], tab[t][row[j][1]]), tab[t][row[j][2]]);
+      sc[j] = fmaf(qs[t], e.x, sc[j]);
+      ss[j] = fmaf(qs[t], e.y, ss[j]);
+    }
+#pragma unroll
+  for (int j = 0; j < kKPerThread; ++j) {
+    const int64_t k = kb + j * kKPerBlock;
+    if (k >= nk) break;
+    atomicAdd(&sk[((int64_t)s * nk + k) * 2], (double)sc[j]);
+    atomicAdd(&sk[((int64_t)s * nk + k) * 2 + 1], (double)ss[j]);
+  }
 }
 
-// Per system: energy and the per-k coefficients; one block per system.
-//   coef[k] = (P S_c, P S_s, c_k)  with c_k for the cell gradient.
-__global__ void recip_energy_kernel(const int32_t *kn, int32_t nk, const double *alpha,
-                                    const RecipSys *sysp, const double *sk, double ke,
-                                    Coef *coef, double *energy, double *dtril) {
-  __shared__ double red[40];
+// K sum_k P(k) |S(k)|^2 of given structure factors, one warp per block: the float64 exponentials and
+// divisions of 32 k each spread over many SMs.
+__global__ void recip_energy_kernel(const int32_t *kn, int32_t nk, const double *alpha, const RecipSys *sysp,
+                                    const double *sk, double ke, double *energy) {
   const int s = blockIdx.y;
-  const RecipSys &P = sysp[s];
-  const double a = alpha[s];
-  const double tp = 6.283185307179586476925286766559;
-  double e = 0.0, w[6] = {0, 0, 0, 0, 0, 0};
-  // L^-T k: (L^-T)_{ab} = inv_{ba}
-  const double *iv = P.inv;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nk; k += gridDim.x * blockDim.x) {
-    const int *nv = kn + ((int64_t)s * nk + k) * 3;
-    const int n3[3] = {nv[0], nv[1], nv[2]};
-    double kv[3];
-    kvec(iv, n3, kv);
-    const double k2 = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
-    double p = 0.0, ck = 0.0;
+  const int64_t k = blockIdx.x * 32 + threadIdx.x;
+  double e = 0.0;
+  if (k < nk) {
     const double sc = sk[((int64_t)s * nk + k) * 2], ss = sk[((int64_t)s * nk + k) * 2 + 1];
-    const double s2 = sc * sc + ss * ss;
-    if (k2 > 0.0) {
-      p = (2.0 - (n3[0] == 0 ? 1.0 : 0.0)) * tp / P.volume * exp(-k2 / (4.0 * a * a)) / k2;
-      ck = ke * s2 * p * (-1.0 / (2.0 * a * a) - 2.0 / k2);
-    }
-    e += ke * p * s2;
-    coef[(int64_t)s * nk + k] = Coef{p * sc, p * ss, ck, 0.0};
-    // u = L^-T k
-    const double u0 = iv[0] * kv[0] + iv[1] * kv[1] + iv[3] * kv[2];
-    const double u1 = iv[2] * kv[1] + iv[4] * kv[2];
-    const double u2 = iv[5] * kv[2];
-    w[0] += ck * u0 * kv[0];
-    w[1] += ck * u1 * kv[0];
-    w[2] += ck * u1 * kv[1];
-    w[3] += ck * u2 * kv[0];
-    w[4] += ck * u2 * kv[1];
-    w[5] += ck * u2 * kv[2];
+    e = ke * prefactor(sysp[s], kn + ((int64_t)s * nk + k) * 3, alpha[s]).p * (sc * sc + ss * ss);
   }
-  const double et = block_sum(e, red);
-  __syncthreads();
-  double wt[6];
-  for (int c = 0; c < 6; ++c) {
-    wt[c] = block_sum(w[c], red);
-    __syncthreads();
-  }
-  // blocks of k vectors add their shares (energy and dtril zeroed by the launcher)
-  if (threadIdx.x == 0) {
-    atomicAdd(&energy[s], et);
-    if (dtril) {
-      const int diag[6] = {1, 0, 1, 0, 0, 1};
-      const int dk[6] = {0, -1, 2, -1, -1, 5};
-      for (int c = 0; c < 6; ++c) {
-        double v = -wt[c];
-        if (diag[c]) v -= et / P.L[dk[c]];
-        atomicAdd(&dtril[6 * (int64_t)s + c], v);  // the sum_i f F part is added by the force kernel
-      }
-    }
-  }
+  e = warp_sum(e);
+  if (threadIdx.x == 0) atomicAdd(&energy[s], e);  // zeroed by the setup
 }
 
-// dE/dr_i for every atom of every system (thread per atom; k coefficients
-// staged through shared memory), plus the sum_i f_ia F_ib part of dE/dL.
-__global__ void recip_force_kernel(const double *pos, const double *q, const int32_t *sys_offset,
-                                   const int32_t *kn, int32_t nk, const RecipSys *sysp,
-                                   const Coef *coef, double ke, double *grad, double *dtril,
-                                   int kblocks_per_split) {
-  __shared__ float2 tab[kAtomsPerChunk][3 * kTab];
-  __shared__ float4 kc[kKPerBlock];  // (P S_c, P S_s, -, -) as float
-  __shared__ int4 kni[kKPerBlock];
+// dE/dr_i for every atom of every system (four threads per atom; k coefficients staged through shared
+// memory), plus the sum_i f_ia F_ib part of dE/dL.  The blocks of the first atom chunk also add the
+// energy of their k and its part of the cell gradient, from the S(k) they stage.
+// Bound by shared memory and latency: with 32 bytes per k and a phase from three tables each time, 14
+// wavefronts for 32 terms; a k is 12 bytes and the x y phase is kept while n_z runs: 6.
+// 4000 atoms and 2800 k: 25.5 us and 10.5 for the launch that formed coefficients and energy, now 25.7
+// with both.  (Two atoms per thread take 5, but leave 1.6 warps per
+// scheduler: 28 us.)
+constexpr int kForceThreads = kAtomsPerChunk * 4;
+
+__global__ void __launch_bounds__(kForceThreads) recip_force_kernel(
+    const double *pos, const double *q, const int32_t *sys_offset, const int32_t *kn, int32_t nk, const RecipSys *sysp,
+    const Coef *coef, const double *sk, double ke, double *energy, double *grad, double *dtril,
+    int kblocks_per_split) {
+  __shared__ float2 tab[kAtomsPerChunk][kRow];
+  __shared__ float2 kc[kForceTile];    // P S_c, P S_s
+  __shared__ uint32_t kz[kForceTile];  // rows of the x, y and z tables from their starts, a byte each
+  __shared__ float gsum[kAtomsPerChunk][3];
   __shared__ double red[40];
   const int s = blockIdx.y;
   const int a0 = sys_offset[s], a1 = sys_offset[s + 1];
@@ -235,61 +263,86 @@ __global__ void recip_force_kernel(const double *pos, const double *q, const int
   if (c0 >= a1) return;
   const int na = min(kAtomsPerChunk, a1 - c0);
   const RecipSys &P = sysp[s];
-  const int t = threadIdx.x;  // blockDim.x == kAtomsPerChunk * 4: 4 lanes per atom split k
-  const int atom = t >> 2, sub = t & 3;
-  double f[3] = {0, 0, 0};
-  if (t < na) {
-    const double r[3] = {pos[3 * (c0 + t)], pos[3 * (c0 + t) + 1], pos[3 * (c0 + t) + 2]};
-    frac64(P.inv, r, f);
-    fill_tables(tab[t], f);
-  }
-  __syncthreads();
+  const int t = threadIdx.x, sub = t & 3, atom = t >> 2;  // every fourth k of an atom
+  fill_tables(tab, pos, c0, na, P);
   // gradient in fractional components: dE/df_a = sum_k 2 K q P 2 pi n_a (Ss c - Sc s)
-  float g0 = 0.f, g1 = 0.f, g2 = 0.f;
+  float g[3] = {0.f, 0.f, 0.f};
+  const float2 *row = tab[atom];
+  double e = 0.0, fw[6] = {0, 0, 0, 0, 0, 0};
   // this block's share of the k vectors (blockIdx.z); partials are added into grad
   const int kbeg = blockIdx.z * kblocks_per_split * kKPerBlock;
   const int kfin = min(nk, kbeg + kblocks_per_split * kKPerBlock);
-  for (int kb = kbeg; kb < kfin; kb += kKPerBlock) {
+  for (int kb = kbeg; kb < kfin; kb += kForceTile) {
     __syncthreads();
-    for (int j = threadIdx.x; j < kKPerBlock; j += blockDim.x) {
-      if (kb + j < nk) {
-        const Coef cc = coef[(int64_t)s * nk + kb + j];
-        kc[j] = make_float4((float)cc.ps_c, (float)cc.ps_s, 0.f, 0.f);
-        const int *nv = kn + ((int64_t)s * nk + kb + j) * 3;
-        kni[j] = make_int4(nv[0], nv[1], nv[2], 0);
-      } else {
-        kc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        kni[j] = make_int4(0, 0, 0, 0);
+    const int kend = min(kForceTile, kfin - kb);
+#pragma unroll 4
+    for (int j = threadIdx.x; j < kend; j += kForceThreads) {
+      {
+        const int64_t k = (int64_t)s * nk + kb + j;
+        const int n3[3] = {kn[3 * k], kn[3 * k + 1], kn[3 * k + 2]};
+        const double p = coef[k].p, sc = sk[2 * k], ss = sk[2 * k + 1];
+        kc[j] = make_float2((float)(p * sc), (float)(p * ss));
+        kz[j] = (uint32_t)(table_row(n3[0]) | table_row(n3[1]) << 8 | table_row(n3[2]) << 16);
+        if (blockIdx.x == 0) {
+          const double s2 = sc * sc + ss * ss, ek = ke * p * s2;
+          e += ek;
+          if (dtril != nullptr) {
+            const double *iv = P.inv;
+            const double ck = ke * s2 * coef[k].ck;
+            double kv[3];
+            kvec(iv, n3, kv);
+            // u = L^-T k: (L^-T)_ab = inv_ba
+            const double u0 = iv[0] * kv[0] + iv[1] * kv[1] + iv[3] * kv[2];
+            const double u1 = iv[2] * kv[1] + iv[4] * kv[2];
+            const double u2 = iv[5] * kv[2];
+            fw[0] -= ck * u0 * kv[0] + ek * iv[0];
+            fw[1] -= ck * u1 * kv[0];
+            fw[2] -= ck * u1 * kv[1] + ek * iv[2];
+            fw[3] -= ck * u2 * kv[0];
+            fw[4] -= ck * u2 * kv[1];
+            fw[5] -= ck * u2 * kv[2] + ek * iv[5];
+          }
+        }
       }
     }
     __syncthreads();
-    if (atom < na) {
-      const int kend = min(kKPerBlock, kfin - kb);
-      for (int j = sub; j < kend; j += 4) {
-        const int4 n3 = kni[j];
-        const float2 e = cmul(cmul(tab[atom][n3.x + kMaxM], tab[atom][kTab + n3.y + kMaxM]),
-                              tab[atom][2 * kTab + n3.z + kMaxM]);
-        const float4 c = kc[j];
-        const float w = c.y * e.x - c.x * e.y;  // P (S_s cos - S_c sin)
-        g0 = fmaf(w, (float)n3.x, g0);
-        g1 = fmaf(w, (float)n3.y, g1);
-        g2 = fmaf(w, (float)n3.z, g2);
-      }
+    uint32_t last = 0xffffffffu;
+    float2 xy = make_float2(1.f, 0.f);
+#pragma unroll 4
+    for (int j = sub; j < kend; j += 4) {
+      const uint32_t z = kz[j];
+      const float2 c = kc[j];
+      if ((z ^ last) & 0xffffu) xy = phase_xy(row[z & 0xffu], row[kTab + (z >> 8 & 0xffu)]);  // n_z runs fastest
+      last = z;
+      // the bytes as float32: 2^23 + byte by its bits, less 2^23 + kMaxM
+      const float nx = __uint_as_float(0x4b000000u | (z & 0xffu)) - (8388608.f + kMaxM),
+                  ny = __uint_as_float(0x4b000000u | (z >> 8 & 0xffu)) - (8388608.f + kMaxM),
+                  nz = __uint_as_float(0x4b000000u | z >> 16) - (8388608.f + kMaxM);
+      const float2 ph = phase_xyz(xy, row[2 * kTab + (z >> 16)]);
+      const float w = fmaf(c.y, ph.x, -__fmul_rn(c.x, ph.y));  // P (S_s cos - S_c sin)
+      g[0] = fmaf(w, nx, g[0]);
+      g[1] = fmaf(w, ny, g[1]);
+      g[2] = fmaf(w, nz, g[2]);
     }
+  }
+  if (blockIdx.x == 0) {
+    const double et = block_sum(e, red);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(&energy[s], et);
   }
   // reduce the 4 lanes of an atom
-  for (int o = 1; o < 4; o <<= 1) {
-    g0 += __shfl_xor_sync(0xffffffffu, g0, o);
-    g1 += __shfl_xor_sync(0xffffffffu, g1, o);
-    g2 += __shfl_xor_sync(0xffffffffu, g2, o);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    for (int o = 1; o < 4; o <<= 1) g[a] += __shfl_xor_sync(0xffffffffu, g[a], o);
+    if (sub == 0) gsum[atom][a] = g[a];
   }
-  double fw[6] = {0, 0, 0, 0, 0, 0};
-  if (atom < na && sub == 0) {
-    const int i = c0 + atom;
+  __syncthreads();
+  if (t < na) {  // float64, by one warp: a quarter of every warp took four times as long
+    const int i = c0 + t;
     const double tp = 6.283185307179586476925286766559;
     const double scale = 2.0 * ke * q[i] * tp;
     // dE/df -> dE/dr: r = f L  =>  f = r L^-1, dE/dr_b = sum_a dE/df_a (L^-1)_{ba}
-    const double df[3] = {scale * g0, scale * g1, scale * g2};
+    const double df[3] = {scale * gsum[t][0], scale * gsum[t][1], scale * gsum[t][2]};
     const double *iv = P.inv;
     const double gr[3] = {df[0] * iv[0], df[0] * iv[1] + df[1] * iv[2],
                           df[0] * iv[3] + df[1] * iv[4] + df[2] * iv[5]};
@@ -302,26 +355,26 @@ __global__ void recip_force_kernel(const double *pos, const double *q, const int
       grad[3 * (int64_t)i + 1] = gr[1];
       grad[3 * (int64_t)i + 2] = gr[2];
     }
-    // fractional coordinates of atom i (recomputed: the table owner is lane `atom`)
-    const double r[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-    double fi[3];
-    frac64(P.inv, r, fi);
-    // sum_i f_ia F_ib, F = -dE/dr
-    fw[0] = -fi[0] * gr[0];
-    fw[1] = -fi[1] * gr[0];
-    fw[2] = -fi[1] * gr[1];
-    fw[3] = -fi[2] * gr[0];
-    fw[4] = -fi[2] * gr[1];
-    fw[5] = -fi[2] * gr[2];
+    if (dtril != nullptr) {
+      const double r[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+      double fi[3];
+      frac64(P.inv, r, fi);
+      // sum_i f_ia F_ib, F = -dE/dr
+      fw[0] -= fi[0] * gr[0];
+      fw[1] -= fi[1] * gr[0];
+      fw[2] -= fi[1] * gr[1];
+      fw[3] -= fi[2] * gr[0];
+      fw[4] -= fi[2] * gr[1];
+      fw[5] -= fi[2] * gr[2];
+    }
   }
-  if (dtril) {
+  if (dtril != nullptr && (blockIdx.x == 0 || t < 32)) {  // other blocks: the first warp has all of it
     for (int c = 0; c < 6; ++c) {
-      const double v = block_sum(fw[c], red);
-      __syncthreads();
+      const double v = blockIdx.x == 0 ? block_sum(fw[c], red) : warp_sum(fw[c]);
+      if (blockIdx.x == 0) __syncthreads();
       if (threadIdx.x == 0) atomicAdd(&dtril[6 * (int64_t)s + c], v);
     }
   }
-  (void)f;
 }
 
 __global__ void self_energy_kernel(const double *q, const int32_t *sys_offset, const double *alpha,
@@ -443,6 +496,7 @@ int32_t launch_pair_edges(const double *positions, const int32_t *system, const 
 // time (a broadcast from L1).  The difference is formed in float64, the minimum image
 // and pair terms in float32, the 32 partial forces are summed in a fixed order through
 // shared memory and the energy is float64.
+constexpr int kRealBatch = 128;  // pairs whose forces a warp keeps before their atoms add them up
 constexpr int kRealAtoms = 16, kRealWarps = 16, kRealStreams = 2 * kRealWarps;
 
 __global__ void __launch_bounds__(32 * kRealWarps) real_allpairs_kernel(
@@ -558,91 +612,170 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_allpairs_kernel(
 //  * a pack kernel stores each coordinate as a float pair hi = fl(x), lo = fl(x - hi);
 //    a difference (hj - hi) + (lj - li) then carries float32 relative error in d
 //    itself (the rounding of hj - hi is relative to the result), with no float64;
-//  * the force kernel tests 32 partners per pass into a per-lane hit mask and then
-//    evaluates only the hits (loop count = the warp's largest hit count, not 32).
+//  * the force kernel tests 32 partners per pass into a per-lane hit mask, in float32
+//    fractional coordinates and the cell's metric, two partners per instruction (17
+//    instructions each, 34 for the difference of the hi / lo pairs); where a partner is
+//    closer to the cutoff than the rounding of either test, the pass is tested again by
+//    the pairs themselves, so the hits are exactly theirs;
+//  * the hits of a warp are queued and evaluated one per lane; their forces go through
+//    shared memory to the lane of their atom, which adds them up in order (shared-memory
+//    atomics to the same few addresses were more than half of the instructions).
+// 4000 ions, cutoff 12 in a 40 cube: 77 us, now 48, bound by issue at 1.6 blocks per SM.
 // Pair terms, the minimum image and the fixed-order reduction are those of the
 // all-pairs kernel.
 // Packed arrays are indexed by system * max_atoms + local index (inside the workspace
 // for any sys_offset); a system above max_atoms is refused.
-__global__ void real_pack_kernel(const double *pos, const double *q, const int32_t *species, const int32_t *sys_offset,
-                                 int terms, int max_atoms, float4 *hi, float4 *lo, kups_status *status) {
-  const int s = blockIdx.y;
-  const int a0 = sys_offset[s], n = sys_offset[s + 1] - a0;
-  if (n > max_atoms) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) status_error(status, KUPS_ERR_INVALID, s);
-    return;
-  }
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int64_t g = a0 + k, p = (int64_t)s * max_atoms + k;
-    float h[3], l[3];
-    for (int a = 0; a < 3; ++a) {
-      const double x = pos[3 * g + a];
-      h[a] = (float)x;
-      l[a] = (float)(x - (double)h[a]);
+// What the force kernel needs of a system, formed once per call in float64 (a few hundred float64
+// operations of one thread: 250 blocks forming them for themselves started 3 us late each).
+struct RealSys {
+  float L[6], I[6];             // cell and inverse
+  float g00, g01, g02, g11, g12, g22;  // |f L|^2 of fractional f, the mixed terms doubled
+  float rc2_lj, rc2_ew, rc2, alpha, ke;
+  float margin;                 // |r2 - rc2| below which the fractional test does not decide
+  int refused;
+};
+
+// Workspace of the packed path: hi, lo and fractional coordinates of every atom (one read past the end
+// of the last by a pass of 32 partners), and the systems' constants.
+struct RealWork {
+  float4 *hi, *lo, *frac;
+  RealSys *sys;
+  size_t bytes;
+};
+
+inline RealWork real_work(char *base, int32_t n_systems, int32_t max_atoms) {
+  auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+  const size_t rows = align((size_t)n_systems * (size_t)max_atoms * sizeof(float4));
+  RealWork w;
+  w.hi = (float4 *)base;
+  w.lo = (float4 *)(base + rows);
+  w.frac = (float4 *)(base + 2 * rows);
+  w.sys = (RealSys *)(base + 3 * rows + 32 * sizeof(float4));
+  w.bytes = 3 * rows + 32 * sizeof(float4) + align(sizeof(RealSys) * (size_t)n_systems);
+  return w;
+}
+
+// By threads 0 (inverse) and 32 (widths) of a block: two chains of float64 divisions side by side.
+__device__ inline void set_real_system(RealSys &r, const Tril64 &L64, double rlj, double rew, double alpha, double ke) {
+  const double rmax = fmax(rlj, rew), *t = L64.t;
+  if (threadIdx.x == 0) {
+    const Tril64 I64 = inverse_tril64(L64);
+    for (int k = 0; k < 6; ++k) {
+      r.L[k] = (float)t[k];
+      r.I[k] = (float)I64.t[k];
     }
-    hi[p] = make_float4(h[0], h[1], h[2], (float)q[g]);
-    lo[p] = make_float4(l[0], l[1], l[2], __int_as_float((terms & 1) ? species[g] : 0));
+    r.rc2_lj = (float)(rlj * rlj);
+    r.rc2_ew = (float)(rew * rew);
+    r.rc2 = (float)(rmax * rmax);
+    r.alpha = (float)alpha;
+    r.ke = (float)ke;
+  } else if (threadIdx.x == 32) {
+    double w[3];
+    perpendicular_widths64(L64, w);
+    const double wmin = fmin(w[0], fmin(w[1], w[2]));
+    const double g00 = t[0] * t[0], g11 = t[1] * t[1] + t[2] * t[2], g22 = t[3] * t[3] + t[4] * t[4] + t[5] * t[5];
+    const double g01 = 2.0 * t[0] * t[1], g02 = 2.0 * t[0] * t[3], g12 = 2.0 * (t[1] * t[3] + t[2] * t[4]);
+    r.refused = wmin < 2.0 * rmax;
+    r.g00 = (float)g00;
+    r.g01 = (float)g01;
+    r.g02 = (float)g02;
+    r.g11 = (float)g11;
+    r.g12 = (float)g12;
+    r.g22 = (float)g22;
+    // Both tests work on |f_a| <= 1/2 with errors below 4e-7 in f and 2^-21 of the terms' sizes in r^2,
+    // together under 5e-6 of S = sum |g| / 4; twice that decides.  Where a cell is so narrow that a
+    // partner at f = 1/2 could be within the cutoff, the two may take different images of it: never then.
+    const double size = 0.25 * (g00 + fabs(g01) + fabs(g02) + g11 + fabs(g12) + g22);
+    r.margin = wmin < 2.0 * rmax * (1.0 + 1e-4) ? INFINITY : (float)(1e-5 * size);
   }
 }
 
+// 1 / x to about 1e-14: a float32 reciprocal and one Newton step (float64 divisions are slow here).
+__device__ inline double reciprocal64(double x) {
+  const double y = (double)(1.0f / (float)x);
+  return y * fma(-x, y, 2.0);
+}
+
+__global__ void __launch_bounds__(256) real_pack_kernel(const double *pos, const double *q, const int32_t *species,
+                                                        const int32_t *sys_offset, const double *tril,
+                                                        const double *rc_lj, const double *alpha, const double *rc_ew,
+                                                        double ke, int terms, int max_atoms, RealWork w,
+                                                        double *energy, kups_status *status) {
+  const int s = blockIdx.y;
+  const int a0 = sys_offset[s], n = sys_offset[s + 1] - a0;
+  const Tril64 L = load_tril64(tril + 6 * (int64_t)s);
+  if (blockIdx.x == gridDim.x - 1) {  // the block after the last atom
+    __shared__ RealSys made;
+    set_real_system(made, L, (terms & 1) ? rc_lj[s] : 0.0, (terms & 2) ? rc_ew[s] : 0.0, (terms & 2) ? alpha[s] : 0.0,
+                    ke);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    w.sys[s] = made;
+    if (!(terms & 8)) energy[s] = 0.0;
+    if (n > max_atoms) status_error(status, KUPS_ERR_INVALID, s);
+    else if (n > 0 && made.refused) status_error(status, KUPS_ERR_UNSUPPORTED, s);
+    return;
+  }
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n > max_atoms || k >= n) return;
+  const int64_t g = a0 + k, p = (int64_t)s * max_atoms + k;
+  float h[3], l[3];
+  double x[3], f[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    x[a] = pos[3 * g + a];
+    h[a] = (float)x[a];
+    l[a] = (float)(x[a] - (double)h[a]);
+  }
+  // fractional coordinates to 1e-14 or so, then in [-1/2, 1/2]: f L = x solved from the last component
+  f[2] = x[2] * reciprocal64(L.t[5]);
+  f[1] = (x[1] - f[2] * L.t[4]) * reciprocal64(L.t[2]);
+  f[0] = (x[0] - f[1] * L.t[1] - f[2] * L.t[3]) * reciprocal64(L.t[0]);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) f[a] -= rint(f[a]);
+  w.hi[p] = make_float4(h[0], h[1], h[2], (float)q[g]);
+  w.lo[p] = make_float4(l[0], l[1], l[2], __int_as_float((terms & 1) ? species[g] : 0));
+  w.frac[p] = make_float4((float)f[0], (float)f[1], (float)f[2], 0.f);
+}
+
 __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
-    const int32_t *sys_offset, const double *tril, const double *lj_sigma, const double *lj_eps, int nsp,
-    const double *rc_lj, const double *alpha, const double *rc_ew, double ke, int terms, int max_atoms,
-    const float4 *hi, const float4 *lo, double *energy, double *grad, kups_status *status) {
+    const int32_t *sys_offset, const double *lj_sigma, const double *lj_eps, int nsp, int terms, int max_atoms,
+    RealWork w, double *energy, double *grad) {
   // blockIdx.z of gridDim.z takes an equal share of every atom's partners; with more than one
   // share the blocks add their partial forces (terms & 8 is then required)
   __shared__ float2 ljt[64];
   __shared__ float part[kRealStreams][kRealAtoms][3];
   __shared__ double red[40];
-  __shared__ uint16_t queue[kRealWarps][32 * 32];  // per warp: hits of one pass (half << 9 | slot << 5 | t)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  // per warp: the forces of kRealBatch hits; the hits of one pass (half << 9 | slot << 5 | t)
+  float4 *force = reinterpret_cast<float4 *>(smem_raw) + kRealBatch * (threadIdx.x >> 5);
+  uint16_t *wq = reinterpret_cast<uint16_t *>(smem_raw + sizeof(float4) * kRealBatch * kRealWarps) +
+                 32 * 32 * (threadIdx.x >> 5);
   const int s = blockIdx.y;
   const int a0 = sys_offset[s], n = sys_offset[s + 1] - a0;
   if ((int)blockIdx.x * kRealAtoms >= n || n > max_atoms) return;  // uniform over the block
   const int64_t pb = (int64_t)s * max_atoms;  // this system's rows of the packed arrays
-  // cell, inverse and widths once per block (float64 is scarce on this part)
-  __shared__ float cellf[12];
-  __shared__ int refused;
-  if (threadIdx.x == 0) {
-    const Tril64 L64 = load_tril64(tril + 6 * (int64_t)s);
-    const Tril64 I64 = inverse_tril64(L64);
-    double wd[3];
-    perpendicular_widths64(L64, wd);
-    const double rmax = fmax((terms & 1) ? rc_lj[s] : 0.0, (terms & 2) ? rc_ew[s] : 0.0);
-    refused = fmin(wd[0], fmin(wd[1], wd[2])) < 2.0 * rmax;
-    if (refused) status_error(status, KUPS_ERR_UNSUPPORTED, s);
-    for (int k = 0; k < 6; ++k) {
-      cellf[k] = (float)L64.t[k];
-      cellf[6 + k] = (float)I64.t[k];
-    }
-  }
-  __syncthreads();
-  if (refused) return;
-  float L[6], I[6];
-  for (int k = 0; k < 6; ++k) {
-    L[k] = cellf[k];
-    I[k] = cellf[6 + k];
-  }
-  const double rlj = (terms & 1) ? rc_lj[s] : 0.0, rew = (terms & 2) ? rc_ew[s] : 0.0;
-  const double rmax = fmax(rlj, rew);
-  const float kef = (float)ke;
+  const float4 *hi = w.hi + pb, *lo = w.lo + pb, *frac = w.frac + pb;
+  const RealSys S = w.sys[s];
+  if (S.refused) return;
+  const float *L = S.L, *I = S.I;
   if ((terms & 1) && nsp * nsp <= 64)
     for (int k = threadIdx.x; k < nsp * nsp; k += blockDim.x) {
       const double sg = lj_sigma[k];
       ljt[k] = make_float2((float)(sg * sg), (float)(4.0 * lj_eps[k]));
     }
   __syncthreads();
-  const float rc2_lj = (float)(rlj * rlj), rc2_ew = (float)(rew * rew), rc2 = (float)(rmax * rmax);
-  const float al = (terms & 2) ? (float)alpha[s] : 0.f;
-  const float two_al_rsqrtpi = 2.0f * al * 0.56418958354775628695f;
+  const float two_al_rsqrtpi = 2.0f * S.alpha * 0.56418958354775628695f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int slot = lane & (kRealAtoms - 1), stream_id = warp * 2 + (lane >> 4);
   const int il = blockIdx.x * kRealAtoms + slot;
   const bool act = il < n;
   const int64_t gi = a0 + (act ? il : 0);
-  const float4 hi_i = hi[pb + (act ? il : 0)], lo_i = lo[pb + (act ? il : 0)];
-  // minimum-image difference x_j - x_i from the hi / lo pairs
-  auto diff = [&](int64_t gj, float &dx, float &dy, float &dz, float &r2) {
-    const float4 hj = hi[gj], lj = lo[gj];
+  const int own = act ? il : 0;
+  const float4 frac_i = frac[own];
+  // minimum-image difference of rows gj and ii from the hi / lo pairs
+  auto diff = [&](const float4 &hi_i, const float4 &lo_i, const float4 &hj, const float4 &lj, float &dx, float &dy,
+                  float &dz, float &r2) {
     const float d0 = (hj.x - hi_i.x) + (lj.x - lo_i.x), d1 = (hj.y - hi_i.y) + (lj.y - lo_i.y),
                 d2 = (hj.z - hi_i.z) + (lj.z - lo_i.z);
     float f0 = (d0 * I[0] + d1 * I[1]) + d2 * I[3], f1 = d1 * I[2] + d2 * I[4], f2 = d2 * I[5];
@@ -654,29 +787,53 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
     dz = f2 * L[5];
     r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
   };
-  for (int k = threadIdx.x; k < kRealStreams * kRealAtoms * 3; k += blockDim.x) (&part[0][0][0])[k] = 0.f;
-  __syncthreads();
-  float ef = 0.f;
+  // |f L|^2 of the fractional differences to two partners, each to its nearest image
+  auto both = [](float x) { return make_float2(x, x); };
+  auto nearest = [&](float2 d) {
+    const float2 up = __fadd2_rn(d, both(12582912.f));  // 1.5 * 2^23: the sum is a whole number
+    const float2 n2 = __fadd2_rn(up, both(-12582912.f));
+    return __ffma2_rn(n2, both(-1.f), d);
+  };
+  auto near2 = [&](const float4 &p0, const float4 &p1) {
+    const float2 f0 = nearest(make_float2(p0.x - frac_i.x, p1.x - frac_i.x));
+    const float2 f1 = nearest(make_float2(p0.y - frac_i.y, p1.y - frac_i.y));
+    const float2 f2 = nearest(make_float2(p0.z - frac_i.z, p1.z - frac_i.z));
+    const float2 a = __ffma2_rn(both(S.g02), f2, __ffma2_rn(both(S.g01), f1, __fmul2_rn(both(S.g00), f0)));
+    const float2 b = __ffma2_rn(both(S.g12), f2, __fmul2_rn(both(S.g11), f1));
+    return __ffma2_rn(f0, a, __ffma2_rn(f1, b, __fmul2_rn(f2, __fmul2_rn(both(S.g22), f2))));
+  };
+  float ef = 0.f, fx = 0.f, fy = 0.f, fz = 0.f;  // energy of the pairs this lane evaluates; force of its atom
   const int n_streams = kRealStreams * (int)gridDim.z;
   const int per = (n + n_streams - 1) / n_streams;
   const int sbase = (int)blockIdx.z * kRealStreams;
   const int j0 = (sbase + stream_id) * per, j1 = min(n, j0 + per);
   // chunk starts of the warp's two streams
   const int j0h[2] = {(sbase + warp * 2) * per, (sbase + warp * 2 + 1) * per};
-  uint16_t *wq = queue[warp];
   const int passes = (per + 31) / 32;  // the same for both half-warps of a warp
   for (int pass = 0; pass < passes; ++pass) {
     const int c0 = j0 + pass * 32;
     const int cn = max(0, min(32, j1 - c0));
+    const float4 *fj = frac + min(c0, n);  // reads up to 32 rows, some past the stream's end
     uint32_t hits = 0;
+    float closest = INFINITY;  // to the cutoff, of any partner
 #pragma unroll 4
-    for (int t = 0; t < 32; ++t) {
-      if (t < cn) {  // four independent partner loads in flight
+    for (int t = 0; t < 32; t += 2) {
+      const float2 d = __fadd2_rn(near2(fj[t], fj[t + 1]), both(-S.rc2));  // signs: within the cutoff
+      hits = __funnelshift_l(__float_as_uint(d.x), hits, 1);
+      hits = __funnelshift_l(__float_as_uint(d.y), hits, 1);
+      closest = fminf(closest, fminf(fabsf(d.x), fabsf(d.y)));
+    }
+    hits = __brev(hits);
+    if (__any_sync(0xffffffffu, closest <= S.margin)) {  // the rounding of the hi / lo test decides
+      hits = 0;
+#pragma unroll 4
+      for (int t = 0; t < cn; ++t) {
         float dx, dy, dz, r2;
-        diff(pb + c0 + t, dx, dy, dz, r2);
-        hits |= (uint32_t)(r2 < rc2) << t;
+        diff(hi[own], lo[own], hi[c0 + t], lo[c0 + t], dx, dy, dz, r2);
+        hits |= (uint32_t)(r2 < S.rc2) << t;
       }
     }
+    if (cn < 32) hits &= (1u << cn) - 1;
     if (cn > 0 && c0 <= il && il < c0 + cn) hits &= ~(1u << (il - c0));  // not the atom itself
     if (!act) hits = 0;
     // append this lane's hits to the warp's queue (exclusive prefix of the counts)
@@ -686,8 +843,8 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
       const int y = __shfl_up_sync(0xffffffffu, off, o);
       if (lane >= o) off += y;
     }
-    const int total = __shfl_sync(0xffffffffu, off, 31);
-    off -= cnt;
+    const int total = __shfl_sync(0xffffffffu, off, 31), end = off, begin = off - cnt;
+    off = begin;
     const uint16_t tag = (uint16_t)(((lane >> 4) << 9) | (slot << 5));
     while (hits) {
       const int t = __ffs(hits) - 1;
@@ -695,42 +852,48 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
       wq[off++] = tag | (uint16_t)t;
     }
     __syncwarp();
-    // every lane takes queued pairs until the queue is empty
-    for (int e = lane; e < total; e += 32) {
-      const int code = wq[e];
-      const int h = code >> 9, sl = (code >> 5) & 15, t = code & 31;
-      const int64_t ii = pb + blockIdx.x * kRealAtoms + sl;
-      const int64_t gj = pb + j0h[h] + pass * 32 + t;
-      const float4 hi_a = hi[ii], lo_a = lo[ii], hj = hi[gj], lj = lo[gj];
-      const float d0 = (hj.x - hi_a.x) + (lj.x - lo_a.x), d1 = (hj.y - hi_a.y) + (lj.y - lo_a.y),
-                  d2 = (hj.z - hi_a.z) + (lj.z - lo_a.z);
-      float f0 = (d0 * I[0] + d1 * I[1]) + d2 * I[3], f1 = d1 * I[2] + d2 * I[4], f2 = d2 * I[5];
-      f0 -= rintf(f0);
-      f1 -= rintf(f1);
-      f2 -= rintf(f2);
-      const float dx = (f0 * L[0] + f1 * L[1]) + f2 * L[3], dy = f1 * L[2] + f2 * L[4], dz = f2 * L[5];
-      const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-      float dedr2 = 0.f;
-      const float ir = rsqrtf(r2);  // a few ulp; one MUFU op instead of IEEE sqrt and divisions
-      if ((terms & 1) && r2 < rc2_lj) {
-        const float2 c = ljt[__float_as_int(lo_a.w) * nsp + __float_as_int(lj.w)];
-        const float inv = ir * ir, s2 = c.x * inv, c6 = s2 * s2 * s2;
-        ef += c.y * (c6 * c6 - c6);
-        dedr2 += -0.5f * c.y * c6 * (12.f * c6 - 6.f) * inv;
+    // the lanes evaluate queued pairs; then each adds up its own atom's, in order
+    for (int eb = 0; eb < total; eb += kRealBatch) {
+      const int stop = min(total, eb + kRealBatch);
+#pragma unroll 2
+      for (int e = eb + lane; e < stop; e += 32) {
+        const int code = wq[e];
+        const int h = code >> 9, sl = (code >> 5) & 15, t = code & 31;
+        const int ii = blockIdx.x * kRealAtoms + sl, jj = j0h[h] + pass * 32 + t;
+        const float4 hi_a = hi[ii], lo_a = lo[ii], hj = hi[jj], lj = lo[jj];
+        float dx, dy, dz, r2;
+        diff(hi_a, lo_a, hj, lj, dx, dy, dz, r2);
+        float dedr2 = 0.f;
+        const float ir = rsqrtf(r2);  // a few ulp; one MUFU op instead of IEEE sqrt and divisions
+        if ((terms & 1) && r2 < S.rc2_lj) {
+          const float2 c = ljt[__float_as_int(lo_a.w) * nsp + __float_as_int(lj.w)];
+          const float inv = ir * ir, s2 = c.x * inv, c6 = s2 * s2 * s2;
+          ef += c.y * (c6 * c6 - c6);
+          dedr2 += -0.5f * c.y * c6 * (12.f * c6 - 6.f) * inv;
+        }
+        if ((terms & 2) && r2 < S.rc2_ew) {
+          const float r = r2 * ir, qq = (hi_a.w * S.ke) * hj.w, al = S.alpha;
+          const float er = erfc_cheb(al * r);
+          ef += qq * er * ir;
+          dedr2 += 0.5f * ir * qq * (-er * ir * ir - two_al_rsqrtpi * __expf(-al * al * r2) * ir);
+        }
+        const float m = -2.f * dedr2;
+        force[e - eb] = make_float4(__fmul_rn(m, dx), __fmul_rn(m, dy), __fmul_rn(m, dz), 0.f);
       }
-      if ((terms & 2) && r2 < rc2_ew) {
-        const float r = r2 * ir, qq = (hi_a.w * kef) * hj.w;
-        const float er = erfc_cheb(al * r);
-        ef += qq * er * ir;
-        dedr2 += 0.5f * ir * qq * (-er * ir * ir - two_al_rsqrtpi * __expf(-al * al * r2) * ir);
+      __syncwarp();
+      const int last = min(end, stop) - eb;
+      for (int j = max(begin, eb) - eb; j < last; ++j) {
+        const float4 v = force[j];
+        fx += v.x;
+        fy += v.y;
+        fz += v.z;
       }
-      float *pp = part[warp * 2 + h][sl];
-      atomicAdd(pp, -2.f * dedr2 * dx);
-      atomicAdd(pp + 1, -2.f * dedr2 * dy);
-      atomicAdd(pp + 2, -2.f * dedr2 * dz);
+      __syncwarp();
     }
-    __syncwarp();
   }
+  part[stream_id][slot][0] = fx;
+  part[stream_id][slot][1] = fy;
+  part[stream_id][slot][2] = fz;
   __syncthreads();
   if (threadIdx.x < kRealAtoms && act) {
     float gx = 0.f, gy = 0.f, gz = 0.f;
@@ -773,19 +936,15 @@ int32_t recip_launch(char *base, const double *positions, const double *charges,
                      double *grad_tril, double *structure_factor, kups_status *status, cudaStream_t stream) {
   RecipSys *sysp = (RecipSys *)base;
   Coef *coef = (Coef *)(base + align256(sizeof(RecipSys) * (size_t)n_systems));
-  recip_setup_kernel<<<n_systems, 256, 0, stream>>>(tril, kvec_n, n_systems, n_kvecs, sysp, status);
-  KUPS_CUDA_TRY(cudaMemsetAsync(structure_factor, 0, sizeof(double) * 2 * (size_t)n_systems * n_kvecs, stream));
+  recip_setup_kernel<<<n_systems, kSetupThreads, 0, stream>>>(tril, kvec_n, n_kvecs, sysp, structure_factor, energy,
+                                                              grad_tril, status);
   const int chunks = (max_atoms_per_system + kAtomsPerChunk - 1) / kAtomsPerChunk;
   if (n_kvecs > 0 && chunks > 0) {
-    dim3 g((n_kvecs + kKPerBlock - 1) / kKPerBlock, chunks, n_systems);
-    structure_factor_kernel<<<g, kKPerBlock, 0, stream>>>(positions, charges, sys_offset, kvec_n,
-                                                          n_kvecs, sysp, structure_factor, grad);
+    const int tile = kKPerBlock * kKPerThread;
+    dim3 g((n_kvecs + tile - 1) / tile, chunks, n_systems);
+    structure_factor_kernel<<<g, kKPerBlock, 0, stream>>>(positions, charges, sys_offset, kvec_n, n_kvecs, sysp, alpha,
+                                                          coef, structure_factor, grad);
   }
-  KUPS_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * (size_t)n_systems, stream));
-  if (grad_tril) KUPS_CUDA_TRY(cudaMemsetAsync(grad_tril, 0, sizeof(double) * 6 * (size_t)n_systems, stream));
-  // one warp per block: the per-k float64 exp and divisions spread over many SMs
-  recip_energy_kernel<<<dim3((unsigned)std::max(1, (n_kvecs + 31) / 32), n_systems), 32, 0, stream>>>(
-      kvec_n, n_kvecs, alpha, sysp, structure_factor, coulomb_k, coef, energy, grad_tril);
   if (chunks > 0 && n_kvecs > 0) {
     // enough k splits that the launch holds about 16 warps per SM
     const int kblocks = (n_kvecs + kKPerBlock - 1) / kKPerBlock;
@@ -793,14 +952,14 @@ int32_t recip_launch(char *base, const double *positions, const double *charges,
     const int splits = std::min(kblocks, want);
     const int per = (kblocks + splits - 1) / splits;
     dim3 g(chunks, n_systems, (kblocks + per - 1) / per);
-    recip_force_kernel<<<g, kAtomsPerChunk * 4, 0, stream>>>(positions, charges, sys_offset, kvec_n,
-                                                             n_kvecs, sysp, coef, coulomb_k, grad,
-                                                             grad_tril, per);
+    recip_force_kernel<<<g, kForceThreads, 0, stream>>>(positions, charges, sys_offset, kvec_n,
+                                                             n_kvecs, sysp, coef, structure_factor, coulomb_k, energy,
+                                                             grad, grad_tril, per);
   } else if (chunks > 0) {
     dim3 g(chunks, n_systems, 1);
-    recip_force_kernel<<<g, kAtomsPerChunk * 4, 0, stream>>>(positions, charges, sys_offset, kvec_n,
-                                                             n_kvecs, sysp, coef, coulomb_k, grad,
-                                                             grad_tril, 0);
+    recip_force_kernel<<<g, kForceThreads, 0, stream>>>(positions, charges, sys_offset, kvec_n,
+                                                             n_kvecs, sysp, coef, structure_factor, coulomb_k, energy,
+                                                             grad, grad_tril, 0);
   }
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
@@ -843,11 +1002,10 @@ extern "C" int32_t kups_ewald_recip_energy(const double *tril, const int32_t *kv
   if (n_systems == 0) return KUPS_OK;
   char *base = (char *)(((uintptr_t)workspace + 255) & ~uintptr_t(255));
   RecipSys *sysp = (RecipSys *)base;
-  Coef *coef = (Coef *)(base + align256(sizeof(RecipSys) * (size_t)n_systems));
-  recip_setup_kernel<<<n_systems, 256, 0, stream>>>(tril, kvec_n, n_systems, n_kvecs, sysp, status);
-  KUPS_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * (size_t)n_systems, stream));
+  recip_setup_kernel<<<n_systems, kSetupThreads, 0, stream>>>(tril, kvec_n, n_kvecs, sysp, nullptr, energy, nullptr,
+                                                              status);
   recip_energy_kernel<<<dim3((unsigned)std::max(1, (n_kvecs + 31) / 32), n_systems), 32, 0, stream>>>(
-      kvec_n, n_kvecs, alpha, sysp, structure_factor, coulomb_k, coef, energy, nullptr);
+      kvec_n, n_kvecs, alpha, sysp, structure_factor, coulomb_k, energy);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 
@@ -975,8 +1133,7 @@ extern "C" int32_t kups_lj_ewald_real_forces(const double *positions, const doub
 
 extern "C" size_t kups_lj_ewald_real_forces_workspace_bytes(int32_t n_systems, int32_t max_atoms_per_system) {
   if (n_systems <= 0 || max_atoms_per_system <= 0) return 256;
-  const size_t cap = (size_t)n_systems * (size_t)max_atoms_per_system;
-  return 2 * align256(cap * sizeof(float4)) + 256;
+  return real_work(nullptr, n_systems, max_atoms_per_system).bytes + 256;
 }
 
 extern "C" int32_t kups_lj_ewald_real_forces_packed(const double *positions, const double *charges,
@@ -995,27 +1152,28 @@ extern "C" int32_t kups_lj_ewald_real_forces_packed(const double *positions, con
   if ((terms & 1) && (n_species < 1 || n_species > 8 || lj_sigma == nullptr || lj_epsilon == nullptr))
     return KUPS_ERR_INVALID;
   if (n_systems == 0) return KUPS_OK;
-  if (!(terms & 8)) KUPS_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * (size_t)n_systems, stream));
-  if (max_atoms_per_system == 0) return KUPS_OK;
+  if (max_atoms_per_system == 0) {
+    if (!(terms & 8)) KUPS_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * (size_t)n_systems, stream));
+    return KUPS_OK;
+  }
   if (workspace == nullptr ||
       workspace_bytes < kups_lj_ewald_real_forces_workspace_bytes(n_systems, max_atoms_per_system))
     return KUPS_ERR_INVALID;
-  const size_t cap = (size_t)n_systems * (size_t)max_atoms_per_system;
   char *base = reinterpret_cast<char *>(((uintptr_t)workspace + 255) & ~uintptr_t(255));
-  float4 *hi = reinterpret_cast<float4 *>(base);
-  float4 *lo = reinterpret_cast<float4 *>(base + align256(cap * sizeof(float4)));
-  dim3 gp((max_atoms_per_system + 255) / 256, n_systems);
-  real_pack_kernel<<<gp, 256, 0, stream>>>(positions, charges, species, sys_offset, terms, max_atoms_per_system, hi,
-                                           lo, status);
+  const RealWork w = real_work(base, n_systems, max_atoms_per_system);
+  dim3 gp((max_atoms_per_system + 255) / 256 + 1, n_systems);
+  real_pack_kernel<<<gp, 256, 0, stream>>>(positions, charges, species, sys_offset, tril, lj_cutoff, alpha,
+                                           ewald_cutoff, coulomb_k, terms, max_atoms_per_system, w, energy, status);
   // partner shares: the caller's choice (a launch-shape tuner's), else one.  Shares add their
   // partial forces, so they need terms & 8 (the caller's gradient is the base).  One share
   // measured fastest on the 4000-ion melt (250 blocks on 152 SMs: 0.152 ms per force
   // evaluation against 0.164 / 0.166 / 0.171 for 2 / 3 / 4 shares).
   const int splits = (terms & 8) && splits_req > 0 ? splits_req : 1;
   dim3 g((max_atoms_per_system + kRealAtoms - 1) / kRealAtoms, n_systems, splits);
-  real_packed_kernel<<<g, 32 * kRealWarps, 0, stream>>>(sys_offset, tril, lj_sigma, lj_epsilon, n_species, lj_cutoff,
-                                                        alpha, ewald_cutoff, coulomb_k, terms, max_atoms_per_system,
-                                                        hi, lo, energy, grad, status);
+  const size_t smem = kRealWarps * (kRealBatch * sizeof(float4) + 32 * 32 * sizeof(uint16_t));
+  KUPS_CUDA_TRY(cudaFuncSetAttribute(real_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  real_packed_kernel<<<g, 32 * kRealWarps, smem, stream>>>(sys_offset, lj_sigma, lj_epsilon, n_species, terms,
+                                                        max_atoms_per_system, w, energy, grad);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 

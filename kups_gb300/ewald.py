@@ -442,27 +442,36 @@ class LJEwaldMD:
         # partner shares per 16-atom block of the all-pairs real space (0: the library default of
         # one; autotune.autotune_lj_ewald picks one per workload)
         self.real_splits = 0
+        self._side = None  # the stream of the all-pairs real space
         self.graph = None
 
-    def _forces(self):
+    def _force_terms(self):
+        """Energies and gradients of real space (``e_pair``, ``g_pair``) and of reciprocal space (``e_rec``,
+        ``g_rec``); without a list the two run side by side, real space on a stream of its own."""
         lib = _lib.load()
         pos = self.p.positions
+        terms = TERM_EWALD_REAL | (TERM_LJ if self.lj else 0)
         if self.allpairs:
-            terms = TERM_EWALD_REAL | (TERM_LJ if self.lj else 0)
             nsp = int(self.sig.shape[0]) if self.lj else 1
-            # reciprocal space writes energy and grad; real space adds onto them
-            ewald_recip(pos, self.q, self.off, self.max_atoms, self.tril, self.kn, self.alpha, grad_tril=False,
-                        ws=self.rws, out=(self.energy, self.grad, self.t_rec, self.sk), status=self.status)
-            rc = lib.kups_lj_ewald_real_forces_packed(
-                pos.data_ptr(), self.q.data_ptr(), self.species.data_ptr(), self.off.data_ptr(), self.s,
-                self.max_atoms, self.tril.data_ptr(), self.sig.data_ptr() if self.lj else None,
-                self.eps.data_ptr() if self.lj else None, nsp, self.rc_lj.data_ptr() if self.lj else None,
-                self.alpha.data_ptr(), self.rc_ew.data_ptr(), TO_STANDARD_UNITS,
-                terms | TERM_ACCUMULATE | (self.real_splits << 8),
-                self.energy.data_ptr(), self.grad.data_ptr(), self.real_ws.data_ptr(), self.real_ws.numel(),
-                self.status.data_ptr(), _stream())
-            _lib.check(rc, "kups_lj_ewald_real_forces_packed")
-            self.energy.add_(self.e_self)
+            here = torch.cuda.current_stream()
+            if self._side is None:
+                self._side = torch.cuda.Stream()
+            self._side.wait_stream(here)
+            with torch.cuda.stream(self._side):
+                if self.real_splits:  # several shares per atom add onto what is there
+                    self.e_pair.zero_()
+                    self.g_pair.zero_()
+                    terms |= TERM_ACCUMULATE | (self.real_splits << 8)
+                rc = lib.kups_lj_ewald_real_forces_packed(
+                    pos.data_ptr(), self.q.data_ptr(), self.species.data_ptr(), self.off.data_ptr(), self.s,
+                    self.max_atoms, self.tril.data_ptr(), self.sig.data_ptr() if self.lj else None,
+                    self.eps.data_ptr() if self.lj else None, nsp, self.rc_lj.data_ptr() if self.lj else None,
+                    self.alpha.data_ptr(), self.rc_ew.data_ptr(), TO_STANDARD_UNITS, terms, self.e_pair.data_ptr(),
+                    self.g_pair.data_ptr(), self.real_ws.data_ptr(), self.real_ws.numel(), self.status.data_ptr(),
+                    _stream())
+                _lib.check(rc, "kups_lj_ewald_real_forces_packed")
+            self._recip()
+            here.wait_stream(self._side)
             return
         rc = lib.kups_neighborlist_build(pos.data_ptr(), self.system.data_ptr(), self.incl.data_ptr(),
                                          self.excl.data_ptr(), self.n, self.s, self.tril.data_ptr(),
@@ -470,12 +479,18 @@ class LJEwaldMD:
                                          self.cap, self.n_edges.data_ptr(), self.nl_ws.data_ptr(), self.nl_ws.numel(),
                                          self.status.data_ptr(), _stream())
         _lib.check(rc, "kups_neighborlist_build")
-        terms = TERM_EWALD_REAL | (TERM_LJ if self.lj else 0)
         pair_edges(pos, self.system, self.species, self.q, self.tril, self.edges, self.shifts, self.cap, terms,
                    self.sig, self.eps, self.rc_lj, self.alpha, self.rc_ew, grad_tril=False,
                    out=(self.e_pair, self.g_pair, self.t_pair), status=self.status, paired=True)
-        ewald_recip(pos, self.q, self.off, self.max_atoms, self.tril, self.kn, self.alpha, grad_tril=False,
-                    ws=self.rws, out=(self.e_rec, self.g_rec, self.t_rec, self.sk), status=self.status)
+        self._recip()
+
+    def _recip(self):
+        ewald_recip(self.p.positions, self.q, self.off, self.max_atoms, self.tril, self.kn, self.alpha,
+                    grad_tril=False, ws=self.rws, out=(self.e_rec, self.g_rec, self.t_rec, self.sk),
+                    status=self.status)
+
+    def _forces(self):
+        self._force_terms()
         torch.add(self.g_pair, self.g_rec, out=self.grad)
         torch.add(self.e_pair, self.e_rec, out=self.energy)
         self.energy.add_(self.e_self)
@@ -484,22 +499,21 @@ class LJEwaldMD:
         lib = _lib.load()
         st = _stream()
         p = self.p
-        lib.kups_md_kick(p_mom := self.mom.data_ptr(), self.grad.data_ptr(), self.system.data_ptr(),
-                         self.dt.data_ptr(), 0.5, self.n, st)
+        half = 0.5 if self.integrator == "baoab" else 1.0
+        lib.kups_md_kick_drift(p_mom := self.mom.data_ptr(), self.grad.data_ptr(), p.positions.data_ptr(),
+                               self.masses.data_ptr(), self.system.data_ptr(), self.dt.data_ptr(),
+                               self.tril.data_ptr(), 0.5, half, self.n, st)
         if self.integrator == "baoab":
-            lib.kups_md_drift(p.positions.data_ptr(), p_mom, self.masses.data_ptr(), self.system.data_ptr(),
-                              self.dt.data_ptr(), self.tril.data_ptr(), 0.5, self.n, st)
             lib.kups_md_thermostat_counted(p_mom, self.masses.data_ptr(), self.system.data_ptr(),
                                            self.dt.data_ptr(), self.kT.data_ptr(), self.friction.data_ptr(),
                                            self.seed, self.counter.data_ptr(), self.n, st)
             self.counter.add_(1)
             lib.kups_md_drift(p.positions.data_ptr(), p_mom, self.masses.data_ptr(), self.system.data_ptr(),
                               self.dt.data_ptr(), self.tril.data_ptr(), 0.5, self.n, st)
-        else:
-            lib.kups_md_drift(p.positions.data_ptr(), p_mom, self.masses.data_ptr(), self.system.data_ptr(),
-                              self.dt.data_ptr(), self.tril.data_ptr(), 1.0, self.n, st)
-        self._forces()
-        lib.kups_md_kick(p_mom, self.grad.data_ptr(), self.system.data_ptr(), self.dt.data_ptr(), 0.5, self.n, st)
+        self._force_terms()
+        lib.kups_md_sum_kick(p_mom, self.grad.data_ptr(), self.g_pair.data_ptr(), self.g_rec.data_ptr(),
+                             self.system.data_ptr(), self.dt.data_ptr(), 0.5, self.n, self.energy.data_ptr(),
+                             self.e_pair.data_ptr(), self.e_rec.data_ptr(), self.e_self.data_ptr(), self.s, st)
 
     def start(self, momenta):
         self.mom = _f64(momenta).clone()
