@@ -23,11 +23,14 @@
 //    shifts are baked into the ghost copies), the exact r^2 < rc^2 test of
 //    lennard_jones_edge_energy, float32 arithmetic; per-system energies,
 //    kinetic energies and virials are reduced in float64;
+//  * where systems are few, a cluster of up to eight CTAs steps one of them, each
+//    with all positions and a share of the atoms (see team_rank below);
 //  * positions are re-wrapped into fractional [-0.5, 0.5) at every list
 //    build and on exit (the reference wraps every step with
 //    MinimumImageConventionFlow, integrators.py:104-141; wrapping between
 //    builds only changes the representation, never a distance).
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 
@@ -42,6 +45,8 @@ constexpr int kMaxSpecies = 8;
 constexpr int kShiftSide = 5;  // image offsets in [-2, 2]^3
 constexpr int kShiftCount = kShiftSide * kShiftSide * kShiftSide;
 constexpr int kThreads = 1024;
+constexpr int kTeamAtoms = 384, kPairAtoms = 768;  // atoms per system from which teams of 4 or 8, and of 2, gain
+constexpr int kMaxTeam = 8;  // CTAs per system: the portable cluster size
 constexpr int kScratchPerCta = 3 * kMaxAtoms > 2 * kMaxGhosts ? 3 * kMaxAtoms : 2 * kMaxGhosts;  // float4s
 
 // Per-system record kept in the workspace between calls: with it a call resumes a
@@ -153,7 +158,94 @@ struct Smem {
   float mu;     // barostat scale of this step
   float red_f[12 * 32];  // per-warp partials of block_sums
   double red_d[12];
+  int said[2 * kMaxTeam];  // a word from every CTA of the team: atoms that moved far, and its longest list
 };
+
+// A system is stepped by a team of C CTAs (a cluster; C = 1: one CTA).  Every CTA of the team holds all
+// positions, image copies and lists' lengths and builds the same cell order; thread t of the CTA of rank
+// r works only for its rank's warps (kThreads / 32 / C of them) on what thread t of a single CTA would
+// do, so that every sum has the terms and the order it has there, bit for bit.  An atom's momentum, force
+// and travelled distance are kept by the CTA of the thread that integrates it, atoms t and t + kThreads.
+template <int C>
+__device__ inline int team_rank() {
+  if constexpr (C == 1) return 0;
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+
+template <int C>
+__device__ inline bool team_mine(int rank) {  // whether this warp works for this rank
+  return C == 1 || (int)(threadIdx.x >> 5) / (kThreads / 32 / C) == rank;
+}
+
+template <int C>
+__device__ inline int team_owner(int atom) {  // rank that keeps the atom
+  return C == 1 ? 0 : (atom & (kThreads - 1)) / (kThreads / C);
+}
+
+// Every thread of the team; writes before it, to shared memory of any CTA and to global memory, are
+// seen after it.
+template <int C>
+__device__ inline void team_sync() {
+  if constexpr (C == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
+}
+
+// The address of this CTA's shared variable in the CTA of rank r.
+__device__ inline uint32_t team_address(const void *mine, int r) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"((uint32_t)r));
+  return a;
+}
+
+__device__ inline void team_store(const float4 *mine, int r, const float4 &v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(team_address(mine, r)), "f"(v.x), "f"(v.y),
+               "f"(v.z), "f"(v.w)
+               : "memory");
+}
+__device__ inline void team_store(const float *mine, int r, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(team_address(mine, r)), "f"(v) : "memory");
+}
+__device__ inline void team_store(const int *mine, int r, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(team_address(mine, r)), "r"(v) : "memory");
+}
+__device__ inline void team_store(const uint16_t *mine, int r, uint16_t v) {
+  asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(team_address(mine, r)), "h"(v) : "memory");
+}
+
+// v into the variable `mine` of every CTA of the team
+template <int C, typename T>
+__device__ inline void team_share(T *mine, const T &v) {
+  if constexpr (C == 1) {
+    *mine = v;
+  } else {
+#pragma unroll
+    for (int r = 0; r < C; ++r) team_store(mine, r, v);
+  }
+}
+
+// The largest of the CTAs' values of v (the same in all threads of a CTA), in every thread.  Between two
+// uses of the same words lies another team_sync.
+template <int C>
+__device__ inline int team_max(int *said, int v) {
+  if constexpr (C == 1) {
+    return v;
+  } else {
+    if ((int)threadIdx.x < C) team_store(said + team_rank<C>(), threadIdx.x, v);
+    team_sync<C>();
+    int m = said[0];
+#pragma unroll
+    for (int r = 1; r < C; ++r) m = max(m, said[r]);
+    return m;
+  }
+}
 
 
 // Explicit fused multiply-adds: every inlined copy rounds the same way (the compiler would
@@ -316,6 +408,18 @@ __device__ void sort_by_cell(Smem &sm, int count, int ncell, int *start) {
   __syncthreads();
 }
 
+// Index of a kept atom among its CTA's, and their number.
+template <int C>
+__device__ inline int team_slot(int atom, int rank) {
+  return atom / kThreads * (kThreads / C) + (atom & (kThreads - 1)) - rank * (kThreads / C);
+}
+template <int C>
+__device__ inline int team_kept(int n, int rank) {
+  int k = 0;
+  for (int b = rank * (kThreads / C); b < n; b += kThreads) k += min(n - b, kThreads / C);
+  return k;
+}
+
 // Wrap and cell-sort the atoms, build the cell-sorted ghost copies and the
 // Verlet list.  Returns false (and records the requirement) if a capacity is
 // exceeded.  `scratch` is this CTA's slice of global workspace (permutation
@@ -325,12 +429,22 @@ __device__ void sort_by_cell(Smem &sm, int count, int ncell, int *start) {
 // the atoms of a warp, read consecutive units.  Entry e of atom i is slot (e / tpa) % 4
 // of unit (e / (4 tpa)) * tpa + e % tpa: at each slot the atom's lanes hold consecutive
 // entries.  The last row of 4 tpa entries is padded with the far-away sentinel item.
+template <int C>
 __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tpa, uint2 *nl,
                                      int nb_cap, kups_status *status, int sys_index,
                                      unsigned long long *prof, float4 *scratch) {
   const int tid = threadIdx.x, nt = blockDim.x;
   long long tp = clock64();
   const int ncell = p.nc[0] * p.nc[1] * p.nc[2];
+  const int rank = team_rank<C>();
+  if (C > 1) {  // the new order has other keepers: every CTA gets every atom's momentum and force
+    if (team_mine<C>(rank))
+      for (int i = tid; i < n; i += nt) {
+        team_share<C>(&sm.mom[i], sm.mom[i]);
+        team_share<C>(&sm.frc[i], sm.frc[i]);
+      }
+    team_sync<C>();
+  }
   // 1. wrap atoms into [-0.5, 0.5), reset travelled distance, sort atoms by cell
   for (int i = tid; i < n; i += nt) {
     float4 q = sm.pos[i];
@@ -421,7 +535,7 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
   }
   __syncthreads();
   prof_add(prof, 7, tp);
-  // 3. Verlet list.  Work unit: a chunk of up to 16 consecutive (cell-sorted)
+  // 3. Verlet list.  Work unit: a chunk of up to A = 16 consecutive (cell-sorted)
   //    atoms of one x-row of cells, two lanes per atom (a system's atoms fill
   //    only the central rows of the extended grid, so whole rows as units left
   //    warps idle); sm.bin_b[r] holds the exclusive prefix of the rows' chunk
@@ -431,11 +545,14 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
   //    at a time, one per lane, against the chunk's bounding box: their squared
   //    distance to it, rounded as the test's, is never above that to an atom in
   //    it.  The third that is left is queued in order (sm.bin_a, 64 per warp)
-  //    and tested 32 at a time, lane h of an atom taking 16 of them (a
+  //    and tested 32 at a time, each of an atom's lanes its share of them (a
   //    shared-memory broadcast); the hits are appended in candidate order
   //    (deterministic), each lane its own, four entries per 8-byte unit.
   //    864 atoms with 75 neighbours: one lane per atom on all candidates was
-  //    bound by issue, 190 us on its SM; now 117.
+  //    bound by issue, 190 us on its SM; now 117.  A team's CTAs take chunks of 4
+  //    atoms, eight lanes each: there are no more than 8 chunks of 16 for each
+  //    CTA, and one is 40 us of a warp's latency.
+  constexpr int A = C == 1 ? 16 : 4;
   const int lane = threadIdx.x & 31;
   const int ltpa = __ffs(tpa) - 1;
   const uint32_t sent = (uint32_t)n_items;
@@ -446,7 +563,7 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
     int carry = 0;
     for (int r0 = 0; r0 < n_rows; r0 += nt) {
       const int r = r0 + tid;
-      const int v = r < n_rows ? (sm.cell_start[(r + 1) * p.nc[0]] - sm.cell_start[r * p.nc[0]] + 15) >> 4 : 0;
+      const int v = r < n_rows ? (sm.cell_start[(r + 1) * p.nc[0]] - sm.cell_start[r * p.nc[0]] + A - 1) / A : 0;
       int tot;
       const int ex = block_exclusive_scan<int>(v, sm.iscan, &tot);
       __syncthreads();
@@ -460,7 +577,7 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
   int my_max = 0;
   while (true) {
     int unit = 0;
-    if (lane == 0) unit = atomicAdd(&sm.work, 1);
+    if (lane == 0) unit = atomicAdd(&sm.work, 1) * C + rank;
     unit = __shfl_sync(0xffffffffu, unit, 0);
     if (unit >= n_chunks) break;
     int row = 0, hi = n_rows - 1;  // the last row with rowp[row] <= unit (empty rows share it)
@@ -474,22 +591,22 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
     const int z0 = max(cz - 1, 0), z1 = min(cz + 1, p.nc[2] - 1);
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, p.nc[1] - 1);
     const float rl2 = p.rl2;
-    const int a0 = ab + (unit - rowp[row]) * 16;
+    const int a0 = ab + (unit - rowp[row]) * A;
     // x-range of the cells of the chunk's 32 atoms (cells of a row are consecutive)
-    const int first = a0 - ((a0 - ab) & 16), last = min(first + 32, ae) - 1;
+    const int first = a0 - ((a0 - ab) & 31), last = min(first + 32, ae) - 1;
     int cfirst = 0, clast = 0;
     for (int c = 0; c < p.nc[0]; ++c) {
       if (sm.cell_start[rowc + c] <= first) cfirst = c;
       if (sm.cell_start[rowc + c] <= last) clast = c;
     }
     const int x0 = max(cfirst - 1, 0), x1 = min(clast + 1, p.nc[0] - 1);
-    const int half = lane >> 4;
-    const bool mine = a0 + (lane & 15) < ae;
-    const int i = mine ? a0 + (lane & 15) : a0;
+    const int part = lane / A;  // of an atom's lanes: takes candidates A part .. of a batch
+    const bool mine = a0 + lane % A < ae;
+    const int i = mine ? a0 + lane % A : a0;
     const float4 q = sm.pos[i];
     float3 lo = make_float3(q.x, q.y, q.z), up = lo;
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
+    for (int o = A / 2; o > 0; o >>= 1) {
       lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
       lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
       lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
@@ -509,27 +626,32 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
     // exact test and entries of the first kn <= 32 queued candidates
     auto settle = [&](int kn) {
       const uint32_t own = lane < kn ? queue[lane] : 0xffffu;
-      const int kh = min(16, max(0, kn - 16 * half));
+      const int kh = min(A, max(0, kn - A * part));
       uint32_t hits = 0;
 #pragma unroll 4
       for (int t = 0; t < kh; ++t) {
-        const float4 o = sm.pos[queue[16 * half + t]];
+        const float4 o = sm.pos[queue[A * part + t]];
         const float dx = o.x - q.x, dy = o.y - q.y, dz = o.z - q.z;
         const bool h = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < rl2;
         hits |= (uint32_t)h << t;
       }
       // not the atom itself
-      for (uint32_t self = __ballot_sync(0xffffffffu, own - (uint32_t)a0 < 16u); self; self &= self - 1) {
+      for (uint32_t self = __ballot_sync(0xffffffffu, own - (uint32_t)a0 < (uint32_t)A); self; self &= self - 1) {
         const int t = __ffs(self) - 1;
         const uint32_t k = __shfl_sync(0xffffffffu, own, t);
-        if (k == (uint32_t)i && (t >> 4) == half) hits &= ~(1u << (t & 15));
+        if (k == (uint32_t)i && t / A == part) hits &= ~(1u << (t % A));
       }
       if (!mine) hits = 0;
-      const int found = __popc(hits), other = __shfl_xor_sync(0xffffffffu, found, 16);
-      int e = cnt + (half ? other : 0);
-      cnt += found + other;
+      const int found = __popc(hits);
+      int e = cnt;
+#pragma unroll
+      for (int q = 0; q < 32 / A; ++q) {
+        const int other = __shfl_sync(0xffffffffu, found, q * A + lane % A);
+        if (q < part) e += other;
+        cnt += other;
+      }
       for (; hits; hits &= hits - 1, ++e)
-        if (e < nb_cap) put(e, queue[16 * half + __ffs(hits) - 1]);
+        if (e < nb_cap) put(e, queue[A * part + __ffs(hits) - 1]);
     };
     auto scan_range = [&](int kb, int ke) {
       for (int k0 = kb; k0 < ke; k0 += 32) {
@@ -564,12 +686,12 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
     __syncwarp();
     if (mine) {
       const int total_cnt = cnt;
-      if (half == 0) {
+      if (part == 0) {
         // pad the last row with the sentinel item (whole rows of at most nb_cap entries stay
         // below n * md_units_per_atom units, which rounds nb_cap / 4 up to 16 units)
         if (cnt <= nb_cap)
           for (; cnt & (4 * tpa - 1); ++cnt) put(cnt, sent);
-        sm.nbr_count[i] = (uint16_t)min(total_cnt, nb_cap);
+        team_share<C>(&sm.nbr_count[i], (uint16_t)min(total_cnt, nb_cap));
       }
       my_max = max(my_max, total_cnt);
     }
@@ -577,7 +699,9 @@ __device__ __noinline__ bool rebuild(Smem &sm, const SysParams &p, int n, int tp
   if (my_max > nb_cap) atomicMax(&sm.flag, my_max);
   __syncthreads();
   prof_add(prof, 9, tp);
-  const int need = sm.flag;
+  if (C > 1) __threadfence();  // the lists, before and after: other SMs read them through their L1
+  const int need = team_max<C>(sm.said + kMaxTeam, sm.flag);
+  if (C > 1) __threadfence();
   if (need > nb_cap) {
     if (tid == 0) status_capacity(status, KUPS_CAP_NEIGHBORS, need, sys_index);
     return false;
@@ -682,7 +806,9 @@ __device__ __forceinline__ void lj_pair2(const Smem &sm, const float4 &xi, int t
 // order instead, so that each thread's virial partial sums (and hence the block's sum) are the
 // same on every run.  Each lane loads a 4-entry list unit (8 bytes) per iteration, fetched
 // one iteration ahead, and evaluates its entries two at a time.
-template <bool ENERGY, bool VIRIAL, bool SINGLE>
+// A team's CTAs each take the groups of the atoms they keep; with VIRIAL each takes its warps' groups of
+// the single CTA's order and hands the results to the keepers.
+template <int C, bool ENERGY, bool VIRIAL, bool SINGLE>
 __device__ __forceinline__ void compute_forces(Smem &sm, int n, int nsp, int tpa, const uint2 *nl,
                                                float rc2, float sig2, float a4, float wv[6]) {
   const int lane = threadIdx.x & 31;
@@ -694,13 +820,20 @@ __device__ __forceinline__ void compute_forces(Smem &sm, int n, int nsp, int tpa
   pc.a12n = make_float2(-12.0f * a4, -12.0f * a4);
   pc.a6 = make_float2(6.0f * a4, 6.0f * a4);
   pc.a = make_float2(a4, a4);
-  const int n_warps = blockDim.x >> 5;
-  int next = threadIdx.x >> 5;  // static schedule (VIRIAL)
+  const int n_warps = blockDim.x >> 5, rank = team_rank<C>();
+  int next = threadIdx.x >> 5;  // static schedule (VIRIAL, teams)
+  if (C > 1 && VIRIAL && !team_mine<C>(rank)) return;
   while (true) {
     int wb = 0;
     if (VIRIAL) {
       wb = next * per_warp;
       next += n_warps;
+    } else if (C > 1) {
+      const int groups = kThreads / C / per_warp;  // of the first kThreads atoms, then of the others
+      wb = (next / groups) * kThreads + (rank * groups + next % groups) * per_warp;
+      if (next / groups * kThreads >= n) break;
+      next += n_warps;
+      if (wb >= n) continue;
     } else {
       if (lane == 0) wb = atomicAdd(&sm.work, per_warp);
       wb = __shfl_sync(0xffffffffu, wb, 0);
@@ -737,17 +870,27 @@ __device__ __forceinline__ void compute_forces(Smem &sm, int n, int nsp, int tpa
       fy += __shfl_xor_sync(0xffffffffu, fy, o);
       fz += __shfl_xor_sync(0xffffffffu, fz, o);
     }
+    const int keeper = VIRIAL ? team_owner<C>(i) : rank;
     if (active && lane_g == 0) {
-      float4 f = sm.frc[i];
-      f.x = fx;
-      f.y = fy;
-      f.z = fz;
-      sm.frc[i] = f;
+      if (keeper == rank) {
+        float4 f = sm.frc[i];
+        f.x = fx;
+        f.y = fy;
+        f.z = fz;
+        sm.frc[i] = f;
+      } else {
+        team_store(&sm.frc[i].x, keeper, fx);
+        team_store(&sm.frc[i].y, keeper, fy);
+        team_store(&sm.frc[i].z, keeper, fz);
+      }
     }
     if (ENERGY) {  // the atom's pair energy / 2, lanes summed in a fixed order
       float e = acc.e.x + acc.e.y;
       for (int o = tpa >> 1; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-      if (active && lane_g == 0) atom_energy(sm)[i] = 0.5f * e;
+      if (active && lane_g == 0) {
+        if (keeper == rank) atom_energy(sm)[i] = 0.5f * e;
+        else team_store(&atom_energy(sm)[i], keeper, 0.5f * e);
+      }
     }
     if (VIRIAL) {
 #pragma unroll
@@ -756,13 +899,13 @@ __device__ __forceinline__ void compute_forces(Smem &sm, int n, int nsp, int tpa
   }
 }
 
-template <bool ENERGY, bool VIRIAL>
+template <int C, bool ENERGY, bool VIRIAL>
 __device__ __forceinline__ void forces_dispatch(Smem &sm, int n, int nsp, int tpa, const uint2 *nl,
                                                 float rc2, float sig2, float a4, float wv[6]) {
   if (nsp == 1)
-    compute_forces<ENERGY, VIRIAL, true>(sm, n, nsp, tpa, nl, rc2, sig2, a4, wv);
+    compute_forces<C, ENERGY, VIRIAL, true>(sm, n, nsp, tpa, nl, rc2, sig2, a4, wv);
   else
-    compute_forces<ENERGY, VIRIAL, false>(sm, n, nsp, tpa, nl, rc2, sig2, a4, wv);
+    compute_forces<C, ENERGY, VIRIAL, false>(sm, n, nsp, tpa, nl, rc2, sig2, a4, wv);
 }
 
 static_assert(sizeof(Smem) <= 227 * 1024, "fused MD shared memory above the per-CTA limit");
@@ -776,8 +919,9 @@ constexpr uint64_t kChiSeed = 0xbb67ae8584caa73bull;
 // Block-wide sums of N floats, returned to every thread in float64: each warp
 // adds in float, then warp k adds the warp partials of value k in float64 (FP64
 // issue is scarce on this part, so only 32 x N double additions are made, the N
-// sums side by side).  Contains two __syncthreads().
-template <int N>
+// sums side by side).  Contains two barriers of the team, whose CTAs each contribute their warps'
+// partials to every CTA's 32.
+template <int C, int N>
 __device__ inline void block_sums(const float (&v)[N], Smem &sm, double (&out)[N]) {
   static_assert(N <= 12, "block_sums scratch holds 12 values");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -787,15 +931,15 @@ __device__ inline void block_sums(const float (&v)[N], Smem &sm, double (&out)[N
     float x = v[k];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) sm.red_f[k * 32 + wid] = x;
+    if (lane == 0 && team_mine<C>(team_rank<C>())) team_share<C>(&sm.red_f[k * 32 + wid], x);
   }
-  __syncthreads();
+  team_sync<C>();
   // warp k adds the warp partials of value k in float64 (the N sums run side by side)
   for (int k = wid; k < N; k += nw) {
     const double x = warp_sum(lane < nw ? (double)sm.red_f[k * 32 + lane] : 0.0);
     if (lane == 0) sm.red_d[k] = x;
   }
-  __syncthreads();
+  team_sync<C>();
 #pragma unroll
   for (int k = 0; k < N; ++k) out[k] = sm.red_d[k];
 }
@@ -803,12 +947,14 @@ __device__ inline void block_sums(const float (&v)[N], Smem &sm, double (&out)[N
 // Sum of the per-atom energies of the last ENERGY force evaluation (thread k takes atoms
 // k, k + blockDim.x, ...: a fixed order, so the result does not depend on which warp took
 // which atom in the force phase), returned to every thread.
+template <int C>
 __device__ inline double atom_energy_sum(Smem &sm, int n) {
   float e = 0.f;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) e += atom_energy(sm)[i];
+  if (team_mine<C>(team_rank<C>()))
+    for (int i = threadIdx.x; i < n; i += blockDim.x) e += atom_energy(sm)[i];
   const float v[1] = {e};
   double r[1];
-  block_sums<1>(v, sm, r);
+  block_sums<C>(v, sm, r);
   return r[0];
 }
 
@@ -957,14 +1103,16 @@ __device__ __noinline__ bool try_resume(Smem &sm, const SysParams &p, const kups
 }
 
 // Record of system s for the next call (all threads call).
+template <int C>
 __device__ void save_record(const Smem &sm, const kups_md_args &a, const MdWork &w, int s, int a0, int n, int tpa,
                             bool valid) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int i = tid; i < n; i += nt) {
+  const int tid = threadIdx.x, nt = blockDim.x, rank = team_rank<C>();
+  for (int i = tid; i < n && team_mine<C>(rank); i += nt) {
     w.apos[a0 + i] = sm.pos[i];
     w.ameta[a0 + i] = (uint32_t)sm.gid[i] | ((uint32_t)sm.nbr_count[i] << 16);
     w.atrav[a0 + i] = sm.frc[i].w;
   }
+  if (rank != 0) return;
   const int ng = sm.n_ghosts;
   for (int k = tid; k < ng; k += nt) w.gmeta[(size_t)s * kMaxGhosts + k] = sm.ghost_meta[k];
   if (tid == 0) {
@@ -1011,7 +1159,7 @@ __device__ inline void set_inverse64(SysParams &p) {
 __device__ double virial_from_sums(const SysParams &p, const double r[12], double *out) {
   // only thread 0 forms the cell inverse (float64 divisions: a handful of FP64 operations per
   // thread of a 1024-thread block would cost the whole block tens of microseconds per call)
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && out != nullptr) {
     double W[3][3];
     W[0][0] = r[0];
     W[1][0] = W[0][1] = r[1];
@@ -1029,7 +1177,7 @@ __device__ double virial_from_sums(const SysParams &p, const double r[12], doubl
   return r[0] + r[2] + r[5];
 }
 
-template <int INTEGRATOR>
+template <int INTEGRATOR, int C>
 __global__ void __launch_bounds__(kThreads, 1)
 md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1039,16 +1187,20 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
   float4 *gmom = reinterpret_cast<float4 *>(a.mom);
   float4 *gfrc = reinterpret_cast<float4 *>(a.force);
   float4 *scratch = w.scratch + (size_t)blockIdx.x * kScratchPerCta;
-  unsigned long long *prof = reinterpret_cast<unsigned long long *>(a.profile);
+  const int rank = team_rank<C>();
+  const bool lead = rank == 0, mine = team_mine<C>(rank);
+  unsigned long long *prof = lead ? reinterpret_cast<unsigned long long *>(a.profile) : nullptr;
   const int nsp = a.n_species;
   for (int k = tid; k < nsp * nsp; k += nt)
     sm.lj[k] = make_float2(a.lj_table[2 * k], a.lj_table[2 * k + 1]);
   const float sig2_0 = a.lj_table[0], a4_0 = a.lj_table[1];
 
+  int turn = (int)blockIdx.x / C - (int)gridDim.x / C;  // teams: systems dealt out in order
   while (true) {
-    if (tid == 0) sm.next_sys = atomicAdd(queue, 1);
+    if (C > 1) team_sync<C>();  // the last system's shared memory is read
+    if (C == 1 && tid == 0) sm.next_sys = atomicAdd(queue, 1);
     __syncthreads();
-    const int q = sm.next_sys;
+    const int q = C == 1 ? sm.next_sys : (turn += (int)gridDim.x / C);
     __syncthreads();
     if (q >= a.n_systems) break;
     const int s = a.order[q];
@@ -1111,7 +1263,8 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
     bool ok = true;
     const bool resumed = INTEGRATOR != 3 && a.reuse_lists != 0 &&
                          try_resume(sm, p, a, w, s, a0, n, tpa, gpos, gmom, gfrc);
-    if (tid == 0) w.rec[s].valid = 0;  // set again when this call has written the record
+    if (C > 1) team_sync<C>();  // every CTA has read the record
+    if (lead && tid == 0) w.rec[s].valid = 0;  // set again when this call has written the record
     if (!resumed) {
       int bad_species = 0;
       for (int i = tid; i < n; i += nt) {
@@ -1127,11 +1280,11 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
         if (tid == 0) status_error(status, KUPS_ERR_INVALID, s);
         continue;
       }
-      ok = rebuild(sm, p, n, tpa, nl, a.neighbor_capacity, status, s, prof, scratch);
+      ok = rebuild<C>(sm, p, n, tpa, nl, a.neighbor_capacity, status, s, prof, scratch);
       if (tid == 0) sm.work = 0;
       __syncthreads();
       if (!ok) continue;
-      if (tid == 0 && a.rebuilds != nullptr) a.rebuilds[s] += 1;
+      if (lead && tid == 0 && a.rebuilds != nullptr) a.rebuilds[s] += 1;
     }
     prof_add(prof, 0, t0);
     // hot scalars in registers
@@ -1147,24 +1300,28 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
     bool energy_valid = false;  // atom_energy holds the current forces' energies
     if (!a.forces_valid) {
       if (a.n_steps == 0 && a.virial != nullptr)
-        forces_dispatch<true, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+        forces_dispatch<C, true, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
       else
-        forces_dispatch<true, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
-      __syncthreads();
+        forces_dispatch<C, true, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+      team_sync<C>();
       energy_valid = true;
     }
     if (INTEGRATOR >= 2 && a.n_steps > 0) {
       float ke = 0.f;
-      for (int i = tid; i < n; i += nt) {
+      for (int i = tid; i < n && mine; i += nt) {
         const float4 m = sm.mom[i];
         ke += 0.5f * fmaf(m.z, m.z, fmaf(m.y, m.y, m.x * m.x)) / m.w;
       }
       const float kv[1] = {ke};
       double kt[1];
-      block_sums<1>(kv, sm, kt);
+      block_sums<C>(kv, sm, kt);
       csvr_alpha(sm, kt[0], a.seed, a.system_base + s, a.step0);
     }
     const bool trace_v = INTEGRATOR != 3 && a.trace_virial != nullptr;
+    // teams: the next step's normals of the kept atoms, drawn by the last warps while the first
+    // evaluate forces (in the scratch of the list builds, which end before)
+    float *noise = reinterpret_cast<float *>(sm.bin_b);
+    static_assert(sizeof(Smem::bin_b) >= 3 * kMaxAtoms / 2 * sizeof(float), "the kept atoms' normals fit the scratch");
     for (int step = 0; step < a.n_steps && ok; ++step) {
       const bool last = step == a.n_steps - 1;
       const bool want_e = last || a.trace_pe != nullptr || a.trace_ke != nullptr || trace_v;
@@ -1172,7 +1329,7 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
       const float alpha = INTEGRATOR >= 2 ? sm.alpha : 1.0f;
       if (tid == 0) sm.work = 0;
       int moved_far = 0;
-      for (int i = tid; i < n; i += nt) {
+      for (int i = tid; i < n && mine; i += nt) {
         float4 x = sm.pos[i], m = sm.mom[i], f = sm.frc[i];
         const float inv_m = 1.0f / m.w;
         if (INTEGRATOR >= 2) {
@@ -1195,7 +1352,11 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
           dy = m.y * sc;
           dz = m.z * sc;
           float eta[4];
-          normal4(a.seed, (uint64_t)(a.atom_base + a0 + sm.gid[i]), a.step0 + (uint64_t)step, eta);
+          if (C > 1 && step > 0) {
+            for (int c = 0; c < 3; ++c) eta[c] = noise[3 * team_slot<C>(i, rank) + c];
+          } else {
+            normal4(a.seed, (uint64_t)(a.atom_base + a0 + sm.gid[i]), a.step0 + (uint64_t)step, eta);
+          }
           const float amp = c2 * sqrtf(m.w);
           m.x = fmaf(c1, m.x, amp * eta[0]);
           m.y = fmaf(c1, m.y, amp * eta[1]);
@@ -1213,15 +1374,15 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
         else
           f.w += len;
         moved_far |= f.w > thr;
-        sm.pos[i] = x;
+        team_share<C>(&sm.pos[i], x);
         sm.mom[i] = m;
         sm.frc[i] = f;
       }
-      const int need = __syncthreads_or(moved_far);
+      const int need = team_max<C>(sm.said, __syncthreads_or(moved_far));
       prof_add(prof, 1, t0);
       if (need) {
-        if (tid == 0 && a.rebuilds != nullptr) a.rebuilds[s] += 1;
-        ok = rebuild(sm, p, n, tpa, nl, a.neighbor_capacity, status, s, prof, scratch);
+        if (lead && tid == 0 && a.rebuilds != nullptr) a.rebuilds[s] += 1;
+        ok = rebuild<C>(sm, p, n, tpa, nl, a.neighbor_capacity, status, s, prof, scratch);
         if (!ok) break;
         mcum = 1.0;
         thr = half_skin;
@@ -1238,25 +1399,32 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
         // the barostat needs the pair virial at every step
 #pragma unroll
         for (int k = 0; k < 6; ++k) wv[k] = 0.f;
-        forces_dispatch<false, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+        forces_dispatch<C, false, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
       } else if ((last && a.virial != nullptr) || trace_v) {
         if (trace_v) {
 #pragma unroll
           for (int k = 0; k < 6; ++k) wv[k] = 0.f;
         }
-        forces_dispatch<true, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+        forces_dispatch<C, true, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
       } else if (want_e) {
-        forces_dispatch<true, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+        forces_dispatch<C, true, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
       } else {
-        forces_dispatch<false, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+        forces_dispatch<C, false, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
       }
-      __syncthreads();
+      if (C > 1 && INTEGRATOR == 1 && !last)
+        for (int l = kThreads - 1 - tid, kept = team_kept<C>(n, rank); l < kept; l += kThreads) {
+          const int i = l / (kThreads / C) * kThreads + rank * (kThreads / C) + l % (kThreads / C);
+          float eta[4];
+          normal4(a.seed, (uint64_t)(a.atom_base + a0 + sm.gid[i]), a.step0 + (uint64_t)step + 1, eta);
+          for (int c = 0; c < 3; ++c) noise[3 * l + c] = eta[c];
+        }
+      team_sync<C>();  // forces are with their keepers, and no one reads the positions any more
       prof_add(prof, 3, t0);
       // ---- B (and kinetic energy when recorded or needed by the thermostat)
       const bool need_ke = want_e || INTEGRATOR >= 2;
       float ke = 0.f;
       float fwt[6] = {0, 0, 0, 0, 0, 0};  // sum_i f_i,a F_i,b (per-step virial record)
-      for (int i = tid; i < n; i += nt) {
+      for (int i = tid; i < n && mine; i += nt) {
         float4 m = sm.mom[i];
         const float4 f = sm.frc[i];
         m.x = fmaf(f.x, hdt, m.x);
@@ -1274,21 +1442,21 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
       if (INTEGRATOR != 3 && trace_v) {
         const float v[12] = {wv[0], wv[1], wv[2], wv[3], wv[4], wv[5], fwt[0], fwt[1], fwt[2], fwt[3], fwt[4], fwt[5]};
         double r[12];
-        block_sums<12>(v, sm, r);
-        virial_from_sums(p, r, a.trace_virial + ((int64_t)step * a.n_systems + s) * 6);
+        block_sums<C>(v, sm, r);
+        virial_from_sums(p, r, lead ? a.trace_virial + ((int64_t)step * a.n_systems + s) * 6 : nullptr);
       }
       double ke_tot = 0.0;
       double w6[6];
       if (INTEGRATOR == 3) {
         const float v[7] = {ke, wv[0], wv[1], wv[2], wv[3], wv[4], wv[5]};
         double r[7];
-        block_sums<7>(v, sm, r);
+        block_sums<C>(v, sm, r);
         ke_tot = r[0];
         for (int k = 0; k < 6; ++k) w6[k] = r[k + 1];
       } else if (need_ke) {
         const float v[1] = {ke};
         double r[1];
-        block_sums<1>(v, sm, r);
+        block_sums<C>(v, sm, r);
         ke_tot = r[0];
       }
       prof_add(prof, 4, t0);
@@ -1334,11 +1502,11 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
           x.y = __fmul_rn(x.y, mu);
           x.z = __fmul_rn(x.z, mu);
           sm.pos[i] = x;
-          far |= sm.frc[i].w > thr;
+          far |= mine && sm.frc[i].w > thr;
         }
-        if (__syncthreads_or(far)) {
-          if (tid == 0 && a.rebuilds != nullptr) a.rebuilds[s] += 1;
-          ok = rebuild(sm, p, n, tpa, nl, a.neighbor_capacity, status, s, prof, scratch);
+        if (team_max<C>(sm.said, __syncthreads_or(far))) {
+          if (lead && tid == 0 && a.rebuilds != nullptr) a.rebuilds[s] += 1;
+          ok = rebuild<C>(sm, p, n, tpa, nl, a.neighbor_capacity, status, s, prof, scratch);
           if (!ok) break;
           mcum = 1.0;
           thr = half_skin;
@@ -1354,18 +1522,18 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
         if (last && a.virial != nullptr) {
 #pragma unroll
           for (int k = 0; k < 6; ++k) wv[k] = 0.f;
-          forces_dispatch<true, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+          forces_dispatch<C, true, true>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
         } else if (want_e) {
-          forces_dispatch<true, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+          forces_dispatch<C, true, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
         } else {
-          forces_dispatch<false, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
+          forces_dispatch<C, false, false>(sm, n, nsp, tpa, nl, rc2, sig2_0, a4_0, wv);
         }
-        __syncthreads();
+        team_sync<C>();
         prof_add(prof, 3, t0);
       }
       if (want_e) {
-        const double pe_tot = atom_energy_sum(sm, n);
-        if (tid == 0) {
+        const double pe_tot = atom_energy_sum<C>(sm, n);
+        if (lead && tid == 0) {
           if (a.trace_pe) a.trace_pe[(int64_t)step * a.n_systems + s] = pe_tot;
           if (a.trace_ke) a.trace_ke[(int64_t)step * a.n_systems + s] = ke_tot;
           if (last) {
@@ -1381,13 +1549,13 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
       }
     }
     if (!ok) continue;
-    if (a.n_steps == 0) {
+    if (C == 1 && a.n_steps == 0) {  // teams take no call without steps
       float ke = 0.f;
       for (int i = tid; i < n; i += nt) {
         const float4 m = sm.mom[i];
         ke += 0.5f * fmaf(m.z, m.z, fmaf(m.y, m.y, m.x * m.x)) / m.w;
       }
-      const double pe_tot = energy_valid ? atom_energy_sum(sm, n) : 0.0;
+      const double pe_tot = energy_valid ? atom_energy_sum<C>(sm, n) : 0.0;
       const double ke_tot = block_sum((double)ke, sm.red + 36);
       if (tid == 0) {
         a.energy[s] = pe_tot;
@@ -1397,7 +1565,7 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
     // ---- write back (wrapped positions), virial dE/dtril
     float fw[6] = {0, 0, 0, 0, 0, 0};  // sum_i f_i,a F_i,b for (a, b) in tril order
     __syncthreads();
-    for (int i = tid; i < n; i += nt) {
+    for (int i = tid; i < n && mine; i += nt) {
       float4 x = sm.pos[i];
       float f[3];
       wrap_position(p, x, f);
@@ -1412,18 +1580,18 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
     if (a.virial != nullptr) {
       const float v[12] = {wv[0], wv[1], wv[2], wv[3], wv[4], wv[5], fw[0], fw[1], fw[2], fw[3], fw[4], fw[5]};
       double r[12];
-      block_sums<12>(v, sm, r);
-      const double trw = virial_from_sums(p, r, a.virial + 6 * (int64_t)s);
-      if (tid == 0 && a.pressure != nullptr) {
+      block_sums<C>(v, sm, r);
+      const double trw = virial_from_sums(p, r, lead ? a.virial + 6 * (int64_t)s : nullptr);
+      if (lead && tid == 0 && a.pressure != nullptr) {
         // sum_i dU/dr_i (x) r_i + h^T dU/dh = sum over pairs of d (x) dU/dd = W for a pair
         // potential: P = (2 K - Tr W) / 3V
         const double vol = fabs(p.Ld[0] * p.Ld[2] * p.Ld[5]);
         a.pressure[s] = (2.0 * a.kinetic[s] - trw) / (3.0 * vol);
       }
     }
-    if (INTEGRATOR == 3 && tid == 0)
+    if (INTEGRATOR == 3 && lead && tid == 0)
       for (int k = 0; k < 6; ++k) a.cell[6 * (int64_t)s + k] = p.Ld[k];
-    save_record(sm, a, w, s, a0, n, tpa, INTEGRATOR != 3);
+    save_record<C>(sm, a, w, s, a0, n, tpa, INTEGRATOR != 3);
     prof_add(prof, 5, t0);
     __syncthreads();
   }
@@ -1434,14 +1602,76 @@ md_lj_kernel(kups_md_args a, MdWork w, int *queue, kups_status *status) {
 
 using namespace kups;
 
-template <int INTEGRATOR>
-static cudaError_t launch_md(const kups_md_args &a, int ctas, int threads, size_t smem, const MdWork &w,
-                             int *queue, kups_status *status, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(md_lj_kernel<INTEGRATOR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+template <int INTEGRATOR, int C>
+static cudaLaunchConfig_t md_config(int ctas, int threads, size_t smem, cudaStream_t stream,
+                                    cudaLaunchAttribute *attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = C;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  return cfg;
+}
+
+// How many teams of C the current device holds at once (asked once per device).
+template <int INTEGRATOR, int C>
+static int md_teams() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if ((n = known[dev].load(std::memory_order_relaxed)) == 0) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = md_config<INTEGRATOR, C>(C, kThreads, sizeof(Smem), nullptr, &attr);
+    if (cudaFuncSetAttribute(md_lj_kernel<INTEGRATOR, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(Smem)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, md_lj_kernel<INTEGRATOR, C>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      n = 0;
+    }
+    n = n > 0 ? n : -1;
+    known[dev].store(n, std::memory_order_relaxed);
+  }
+  return n > 0 ? n : 0;
+}
+
+template <int INTEGRATOR, int C>
+static cudaError_t launch_team(const kups_md_args &a, int ctas, int threads, const MdWork &w, int *queue,
+                               kups_status *status, cudaStream_t stream) {
+  const cudaError_t e = cudaFuncSetAttribute(md_lj_kernel<INTEGRATOR, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(Smem));
   if (e != cudaSuccess) return e;
-  md_lj_kernel<INTEGRATOR><<<ctas, threads, smem, stream>>>(a, w, queue, status);
-  return cudaSuccess;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = md_config<INTEGRATOR, C>(ctas, threads, sizeof(Smem), stream, &attr);
+  return cudaLaunchKernelEx(&cfg, md_lj_kernel<INTEGRATOR, C>, a, w, queue, status);
+}
+
+template <int INTEGRATOR>
+static cudaError_t launch_md(const kups_md_args &a, int ctas, int threads, const MdWork &w, int *queue,
+                             kups_status *status, cudaStream_t stream) {
+  // Few systems leave the chip idle with a CTA each: the largest teams that all run at once.  A step's
+  // two barriers of the team cost 1.5 us.  20 steps in us, one CTA / a team (BAOAB, cutoff 2.2 sigma,
+  // reduced density 0.8):
+  //   atoms   1 system (8)   16 systems (8)   32 systems (4)   64 systems (2)
+  //     256     186 / 187      232 / 243        232 / 241        233 / 259
+  //     384     230 / 193      243 / 235        293 / 256        292 / 314
+  //     768     301 / 214      404 / 288        412 / 287        409 / 359
+  //    2000     584 / 254      790 / 406        790 / 408        797 / 585
+  // A caller's own grid or block size, and calls without steps, keep one CTA per system.
+  auto atoms = [&](int64_t per) { return a.n_atoms >= per * a.n_systems; };
+  if (a.n_ctas <= 0 && threads == kThreads && a.n_steps > 0 && atoms(kTeamAtoms)) {
+    if (a.n_systems <= md_teams<INTEGRATOR, 8>())
+      return launch_team<INTEGRATOR, 8>(a, 8 * a.n_systems, threads, w, queue, status, stream);
+    if (a.n_systems <= md_teams<INTEGRATOR, 4>())
+      return launch_team<INTEGRATOR, 4>(a, 4 * a.n_systems, threads, w, queue, status, stream);
+    if (a.n_systems <= md_teams<INTEGRATOR, 2>() && atoms(kPairAtoms))
+      return launch_team<INTEGRATOR, 2>(a, 2 * a.n_systems, threads, w, queue, status, stream);
+  }
+  return launch_team<INTEGRATOR, 1>(a, ctas, threads, w, queue, status, stream);
 }
 
 extern "C" int32_t kups_lj_md_max_atoms(void) { return kMaxAtoms; }
@@ -1490,12 +1720,11 @@ extern "C" int32_t kups_lj_md_run(const kups_md_args *a, void *workspace, size_t
   w.gmeta = reinterpret_cast<uint32_t *>(base + l.gmeta);
   w.lists = reinterpret_cast<uint2 *>(base + l.lists);
   KUPS_CUDA_TRY(cudaMemsetAsync(queue, 0, sizeof(int), stream));
-  const size_t smem = sizeof(Smem);
   switch (a->integrator) {
-    case 0: KUPS_CUDA_TRY(launch_md<0>(args, ctas, threads, smem, w, queue, status, stream)); break;
-    case 1: KUPS_CUDA_TRY(launch_md<1>(args, ctas, threads, smem, w, queue, status, stream)); break;
-    case 2: KUPS_CUDA_TRY(launch_md<2>(args, ctas, threads, smem, w, queue, status, stream)); break;
-    default: KUPS_CUDA_TRY(launch_md<3>(args, ctas, threads, smem, w, queue, status, stream)); break;
+    case 0: KUPS_CUDA_TRY(launch_md<0>(args, ctas, threads, w, queue, status, stream)); break;
+    case 1: KUPS_CUDA_TRY(launch_md<1>(args, ctas, threads, w, queue, status, stream)); break;
+    case 2: KUPS_CUDA_TRY(launch_md<2>(args, ctas, threads, w, queue, status, stream)); break;
+    default: KUPS_CUDA_TRY(launch_md<3>(args, ctas, threads, w, queue, status, stream)); break;
   }
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
