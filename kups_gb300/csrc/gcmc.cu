@@ -179,6 +179,33 @@ __device__ inline float pair_u(float r2, int ti, int tj, float qq, const float2 
   return e;
 }
 
+// Whether the box of fractional centre c and half extents h may hold a point whose difference to f, taken
+// to the nearest image along each axis, has a squared Cartesian length below r2.  Each Cartesian
+// component is bounded over the box (the lower-triangular cell's z by f_2 alone, y by f_1 and f_2, x by
+// all); an axis along which the box reaches past half a cell counts with both images.  The bound along
+// the cell's faces alone kept 174 of 250 groups of a hexagonal host, 86 of which hold a pair; this keeps 132.
+__device__ inline bool box_within(const float4 &f, const float4 &c, const float4 &h, const float L[6], float r2) {
+  float d[3] = {f.x - c.x, f.y - c.y, f.z - c.z};
+  const float e[3] = {h.x, h.y, h.z};
+  int other[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    d[a] -= rintf(d[a]);
+    other[a] = fabsf(d[a]) + e[a] > 0.4999f;
+  }
+  const float hx = e[0] * fabsf(L[0]) + e[1] * fabsf(L[1]) + e[2] * fabsf(L[3]);
+  const float hy = e[1] * fabsf(L[2]) + e[2] * fabsf(L[4]), hz = e[2] * fabsf(L[5]);
+  for (int k = 0; k < 8; ++k) {
+    if (((k & 1) && !other[0]) || ((k & 2) && !other[1]) || ((k & 4) && !other[2])) continue;
+    const float d0 = (k & 1) ? d[0] - copysignf(1.f, d[0]) : d[0], d1 = (k & 2) ? d[1] - copysignf(1.f, d[1]) : d[1],
+                d2 = (k & 4) ? d[2] - copysignf(1.f, d[2]) : d[2];
+    const float x = fmaxf(fabsf(d0 * L[0] + d1 * L[1] + d2 * L[3]) - hx, 0.f);
+    const float y = fmaxf(fabsf(d1 * L[2] + d2 * L[4]) - hy, 0.f), z = fmaxf(fabsf(d2 * L[5]) - hz, 0.f);
+    if (x * x + y * y + z * z < r2) return true;
+  }
+  return false;
+}
+
 // Sum over the reference's image set of the pair (a at fa, j at fj) for one
 // term configuration; `excl` drops the minimum image (same molecule).
 __device__ inline float pair_images(const float L[6], const float fa[3], const float fj[3], int ti,
@@ -299,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 896 / kThreads) gcmc_kernel(kups_gcm
   // [(sigma/rc)^9 / 3 - (sigma/rc)^3] / V, masked):
   //   E_tail(N) = sum_ab coef_ab c_a c_b, c = fw + N motif  =>  E_tail(N) - E_tail(0) = b N + c N^2
   __shared__ struct {
-    double energy, tail_b, tail_c, self_excl;
+    double energy, tail_b, tail_c, self_excl, inv_kT, lnfv;
     int n_mol;
     float width[4], width_max[4];
     uint32_t hist[4][4];
@@ -340,17 +367,19 @@ __global__ void __launch_bounds__(kThreads, 896 / kThreads) gcmc_kernel(kups_gcm
     ss.tail_c = tcq;
   }
   __syncthreads();
-  // image configurations of the two terms (neighborlist.py:461-466)
-  ImgCfg li, ei;
-  float wdt[3];  // perpendicular widths
-  {
+  // image configurations of the two terms (neighborlist.py:461-466), the cell's perpendicular widths and
+  // the acceptance's constants: by one thread, as every thread of 7 CTAs on the float64 units of an SM
+  // took 90 us of a launch
+  __shared__ ImgCfg img[2];
+  __shared__ float widths[3];
+  if (tid == 0) {
     const Tril64 L = load_tril64(a.tril + 6 * (int64_t)s);
     double w[3];
     perpendicular_widths64(L, w);
-    for (int d = 0; d < 3; ++d) wdt[d] = (float)w[d];
+    for (int d = 0; d < 3; ++d) widths[d] = (float)w[d];
     const double rcs[2] = {a.rc_lj[s], a.rc_ew[s]};
     for (int t = 0; t < 2; ++t) {
-      ImgCfg &c = t == 0 ? li : ei;
+      ImgCfg &c = img[t];
       int prod = 1;
       for (int d = 0; d < 3; ++d) {
         int n = (int)ceil(2.0 * rcs[t] / w[d]);
@@ -358,7 +387,7 @@ __global__ void __launch_bounds__(kThreads, 896 / kThreads) gcmc_kernel(kups_gcm
         if (n % 2 == 0) n += 1;
         if (n > kMaxImg) {
           n = kMaxImg;
-          if (tid == 0) status_error(status, KUPS_ERR_UNSUPPORTED, s);
+          status_error(status, KUPS_ERR_UNSUPPORTED, s);
         }
         c.n[d] = n;
         prod *= n;
@@ -366,17 +395,18 @@ __global__ void __launch_bounds__(kThreads, 896 / kThreads) gcmc_kernel(kups_gcm
       c.image_mode = prod > 1;
       c.rc2 = (float)(rcs[t] * rcs[t]);
     }
+    ss.inv_kT = 1.0 / a.kT[s];
+    ss.lnfv = a.log_activity[s] + log(fabs(L.t[0] * L.t[2] * L.t[5]));  // ln(f V / kT), once per launch
   }
+  __syncthreads();
+  const ImgCfg li = img[0], ei = img[1];
+  const float wdt[3] = {widths[0], widths[1], widths[2]};
   const bool min_image = !li.image_mode && !ei.image_mode;
   const float rc2_any = fmaxf(li.rc2, ei.rc2), rc_any = sqrtf(rc2_any);
   const float4 *grp = reinterpret_cast<const float4 *>(a.fw_group);
   const int lane = tid & 31;
   const float alpha = (float)a.alpha[s];
   const float ke = (float)a.coulomb_k;
-  const double kT = a.kT[s];
-  const double volume = fabs(a.tril[6 * (int64_t)s] * a.tril[6 * (int64_t)s + 2] * a.tril[6 * (int64_t)s + 5]);
-  const double inv_kT = 1.0 / kT;
-  const double lnfv = a.log_activity[s] + log(volume);  // ln(f V / kT), once per launch
   const int fw0 = a.fw_start[s], fwn = a.fw_count[s];
   float4 *gpos = reinterpret_cast<float4 *>(a.guest_pos) + (int64_t)s * a.max_mol * apm;
   const float4 *motif = reinterpret_cast<const float4 *>(a.motif_pos);
@@ -620,7 +650,7 @@ __global__ void __launch_bounds__(kThreads, 896 / kThreads) gcmc_kernel(kups_gcm
             dz = fabsf(dz - rintf(dz));
             const float sep = fmaxf(fmaxf(fmaxf(dx - h.x, 0.f) * wdt[0], fmaxf(dy - h.y, 0.f) * wdt[1]),
                                     fmaxf(dz - h.z, 0.f) * wdt[2]);
-            if (sep < rc_any) mk |= 1u << m;
+            if (sep < rc_any && box_within(fa, c, h, Lf, 1.0001f * rc2_any)) mk |= 1u << m;
           }
           gm[slot] = mk;
           const unsigned old_bits = (1u << apm) - 1u;
@@ -862,10 +892,10 @@ __global__ void __launch_bounds__(kThreads, 896 / kThreads) gcmc_kernel(kups_gcm
         const double dn = (double)(n_new - n_old), dn2 = (double)n_new * n_new - (double)n_old * n_old;
         de += ss.tail_b * dn + ss.tail_c * dn2;
       }
-      double logp = -de * inv_kT + sh.ln_ratio;
+      double logp = -de * ss.inv_kT + sh.ln_ratio;
       if (n_new != n_old) {
         // ln n_old! - ln n_new! for n_new = n_old +- 1 is -ln n_new (insert) or +ln n_old (delete)
-        logp += (n_new - n_old) * lnfv + (n_new > n_old ? -log((double)n_new) : log((double)n_old));
+        logp += (n_new - n_old) * ss.lnfv + (n_new > n_old ? -log((double)n_new) : log((double)n_old));
       }
       const U4 r4 = rng4(a.seed, 1 + (uint64_t)s, 8 * ctr + 4);
       const double u = ((double)(r4.w >> 8) + 1.0) * (1.0 / 16777216.0);  // (0, 1]
