@@ -24,6 +24,8 @@
 // the centred n_x x n_y x n_z grid is tried (no minimum image on axes with
 // n_a == 1), and intramolecular pairs are excluded on the minimum image only.
 // Pair arithmetic float32, energy differences and the log acceptance float64.
+#include <type_traits>
+
 #include "common.cuh"
 #include "proposal.cuh"
 
@@ -854,18 +856,37 @@ __global__ void __launch_bounds__(kThreads, 896 / kThreads) gcmc_kernel(kups_gcm
     // phase tables; the commit forms it again on acceptance instead of storing it every step
     auto delta_sk = [&](float2 pkk, float &dc, float &ds) {
       const uint32_t packed = __float_as_uint(pkk.y);
-      const int n0 = packed & 0xffu, n1 = (packed >> 8) & 0xffu, n2 = (packed >> 16) & 0xffu;
+      const float2 *ta = ph + (packed & 0xffu), *tb = ph + kTab + ((packed >> 8) & 0xffu),
+                   *tc = ph + 2 * kTab + ((packed >> 16) & 0xffu);
       dc = 0.f;
       ds = 0.f;
-      for (int m = 0; m < nm; ++m) {
-        if (!mon[m]) continue;
-        const float2 *t = ph + m * 3 * kTab;
-        const float2 a = t[n0], b = t[kTab + n1], c = t[2 * kTab + n2];
+      auto atom = [&](int m, float w) {
+        const float2 a = ta[m * 3 * kTab], b = tb[m * 3 * kTab], c = tc[m * 3 * kTab];
         const float abr = a.x * b.x - a.y * b.y, abi = a.x * b.y + a.y * b.x;
         const float cs = abr * c.x - abi * c.y, sn = abr * c.y + abi * c.x;
-        const float w = m < apm ? -mq[m] : mq[m];
         dc += w * cs;
         ds += w * sn;
+      };
+      // small molecules unrolled: the tables at fixed offsets, no index arithmetic per atom
+      auto atoms = [&](auto count) {
+        constexpr int n = decltype(count)::value;
+        if (has_old) {
+#pragma unroll
+          for (int m = 0; m < n; ++m) atom(m, -mq[m]);
+        }
+        if (has_new) {
+#pragma unroll
+          for (int m = 0; m < n; ++m) atom(n + m, mq[n + m]);
+        }
+      };
+      switch (apm) {
+        case 1: atoms(std::integral_constant<int, 1>()); break;
+        case 2: atoms(std::integral_constant<int, 2>()); break;
+        case 3: atoms(std::integral_constant<int, 3>()); break;
+        case 4: atoms(std::integral_constant<int, 4>()); break;
+        default:
+          for (int m = 0; m < nm; ++m)
+            if (m < apm ? has_old : has_new) atom(m, m < apm ? -mq[m] : mq[m]);
       }
     };
     for (int k = tid; k < nk; k += kThreads) {
