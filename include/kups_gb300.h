@@ -68,6 +68,11 @@ const char *kups_error_string(int32_t code);
  * n_counts counters after it set to zero, in one launch. */
 int32_t kups_status_init(kups_status *status, int64_t *counts, int32_t n_counts, void *stream);
 
+/* Atoms per system as offsets [n_systems + 1] (the atoms grouped by system), and in stats: the most
+ * atoms of a system, the number of indices outside [0, n_systems) (which count nowhere), a scratch word. */
+int32_t kups_system_offsets(const int32_t *system, int64_t n_particles, int32_t n_systems,
+                            int32_t *offsets, int32_t stats[3], void *stream);
+
 /* ------------------------------------------------------------------------
  * Neighbour list — replaces CellListNeighborList.__call__ and
  * DenseNearestNeighborList.__call__ (src/kups/core/neighborlist.py:985-1077,

@@ -95,6 +95,7 @@ SIGNATURES = {
     "kups_version": (C.c_char_p, []),
     "kups_error_string": (C.c_char_p, [_I32]),
     "kups_status_init": (_I32, [_P, _P, _I32, _P]),
+    "kups_system_offsets": (_I32, [_P, _I64, _I32, _P, _P, _P]),
     "kups_neighborlist_workspace_bytes": (_SZ, [_I64, _I32]),
     "kups_neighborlist_build": (_I32, [_P, _P, _P, _P, _I64, _I32, _P, _P, _I32, _P, _P, _I64, _P, _P, _SZ, _P, _P]),
     "kups_neighborlist_rh_workspace_bytes": (_SZ, [_I64, _I64, _I32]),

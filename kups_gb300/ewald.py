@@ -138,10 +138,16 @@ class EwaldParameters:
 
 # ----------------------------------------------------------------------------- kernels
 def _offsets(system: torch.Tensor, s: int) -> tuple[torch.Tensor, int]:
-    counts = torch.bincount(system.long(), minlength=s)
-    off = torch.zeros(s + 1, dtype=torch.int32, device="cuda")
-    off[1:] = torch.cumsum(counts, 0).to(torch.int32)
-    return off, int(counts.max()) if s > 0 else 0
+    """Offsets [S + 1] of the systems' atoms and the most atoms of a system (one launch, one read)."""
+    words = torch.empty(s + 4, dtype=torch.int32, device="cuda")
+    off, stats = words[:s + 1], words[s + 1:]
+    rc = _lib.load().kups_system_offsets(system.data_ptr(), system.shape[0], s, off.data_ptr(), stats.data_ptr(),
+                                         _stream())
+    _lib.check(rc, "kups_system_offsets")
+    most, outside, _ = stats.tolist()
+    if outside:
+        raise RuntimeError(f"{outside} system indices outside [0, {s})")
+    return off, most
 
 
 class RecipWorkspace:
@@ -273,6 +279,7 @@ class LJEwaldPotential:
         self.neighborlist = neighborlist or CellListNeighborList(avg_edges=512)
         self.exclusion_edges = exclusion_edges  # (edges [E,2], shifts [E,3]) intramolecular pairs
         self.ws = RecipWorkspace()
+        self._side = None  # the stream of reciprocal space
 
     def __call__(self, particles: EwaldParticles, tril, patch=None, cache: LJEwaldCache | None = None) -> PotentialOut:
         tril = _f64(tril)
@@ -288,16 +295,31 @@ class LJEwaldPotential:
             terms |= TERM_LJ
         if patch is not None:
             return self._patched(particles, tril, patch, cache, terms, sig, eps, rc_lj, alpha, rc_ew, rc_nl)
+        off, mx = _offsets(_i32(particles.system), s)
         pts = NeighborListPoints(particles.positions, particles.system, None, particles.exclusion)
         e, self.neighborlist = self.neighborlist.call_and_fix(pts, None, tril, rc_nl)
-        en, g, gt = pair_edges(particles.positions, particles.system, particles.species, particles.charges, tril,
-                               e.indices, e.shifts.view(-1, 3), e.n_edges, terms, sig, eps, rc_lj, alpha, rc_ew,
-                               paired=lists_pairs(self.neighborlist))
-        off, mx = _offsets(_i32(particles.system), s)
-        self._last_recip = ewald_recip(particles.positions, particles.charges, off, mx, tril,
-                                       self.ewald.reciprocal_lattice_shifts, alpha, ws=self.ws)
+        # reciprocal space beside the edges (float64 units against the others), on a stream of its own;
+        # its outputs and scratch belong to this stream, which waits for it before anything reads them
+        kn = _i32(self.ewald.reciprocal_lattice_shifts)
+        n, f64 = _f64(particles.positions).shape[0], dict(dtype=torch.float64, device="cuda")
+        out = (torch.empty(s, **f64), torch.empty((n, 3), **f64), torch.empty((s, 6), **f64),
+               torch.empty((s, kn.shape[1], 2), **f64))
+        self.ws.get(_lib.load().kups_ewald_recip_workspace_bytes(s, kn.shape[1]))
+        pos, q, status = _f64(particles.positions), _f64(particles.charges), new_status()
+        here = torch.cuda.current_stream()
+        if self._side is None or self._side.device != here.device:
+            self._side = torch.cuda.Stream()
+        self._side.wait_stream(here)
+        with torch.cuda.stream(self._side):
+            self._last_recip = ewald_recip(pos, q, off, mx, tril, kn, alpha, ws=self.ws, out=out, status=status)
+        try:
+            en, g, gt = pair_edges(particles.positions, particles.system, particles.species, particles.charges, tril,
+                                   e.indices, e.shifts.view(-1, 3), e.n_edges, terms, sig, eps, rc_lj, alpha, rc_ew,
+                                   paired=lists_pairs(self.neighborlist))
+            es = ewald_self(q, off, alpha, s)
+        finally:
+            here.wait_stream(self._side)
         el, gl, gtl, _, _ = self._last_recip
-        es = ewald_self(particles.charges, off, alpha, s)
         energy, grad, gtril = en + el + es, g + gl, gt + gtl
         if self.exclusion_edges is not None:
             xe, xs = self.exclusion_edges
