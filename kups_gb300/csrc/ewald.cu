@@ -24,6 +24,8 @@
 #include <algorithm>
 #include <mutex>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "pair_runs.cuh"
 
@@ -620,7 +622,7 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_allpairs_kernel(
 //  * the hits of a warp are queued and evaluated one per lane; their forces go through
 //    shared memory to the lane of their atom, which adds them up in order (shared-memory
 //    atomics to the same few addresses were more than half of the instructions).
-// 4000 ions, cutoff 12 in a 40 cube: 77 us, now 48, bound by issue at 1.6 blocks per SM.
+// 4000 ions, cutoff 12 in a 40 cube: 77 us, now 43, bound by issue and the latency of 26 warps per SM.
 // Pair terms, the minimum image and the fixed-order reduction are those of the
 // all-pairs kernel.
 // Packed arrays are indexed by system * max_atoms + local index (inside the workspace
@@ -738,22 +740,27 @@ __global__ void __launch_bounds__(256) real_pack_kernel(const double *pos, const
   w.frac[p] = make_float4((float)f[0], (float)f[1], (float)f[2], 0.f);
 }
 
-__global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
+// A block's 16 warps are a cluster of four CTAs, whose forces the first adds up through distributed
+// shared memory: 4000 ions are 250 blocks, one or two per SM, or 1000 CTAs, six or seven (48 us and 43).
+constexpr int kRealCtas = 4, kCtaWarps = kRealWarps / kRealCtas;
+
+__global__ void __cluster_dims__(kRealCtas, 1, 1) __launch_bounds__(32 * kCtaWarps) real_packed_kernel(
     const int32_t *sys_offset, const double *lj_sigma, const double *lj_eps, int nsp, int terms, int max_atoms,
     RealWork w, double *energy, double *grad) {
   // blockIdx.z of gridDim.z takes an equal share of every atom's partners; with more than one
   // share the blocks add their partial forces (terms & 8 is then required)
   __shared__ float2 ljt[64];
-  __shared__ float part[kRealStreams][kRealAtoms][3];
+  __shared__ float part[2 * kCtaWarps][kRealAtoms][3];  // this CTA's streams
   __shared__ double red[40];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // per warp: the forces of kRealBatch hits; the hits of one pass (half << 9 | slot << 5 | t)
   float4 *force = reinterpret_cast<float4 *>(smem_raw) + kRealBatch * (threadIdx.x >> 5);
-  uint16_t *wq = reinterpret_cast<uint16_t *>(smem_raw + sizeof(float4) * kRealBatch * kRealWarps) +
+  uint16_t *wq = reinterpret_cast<uint16_t *>(smem_raw + sizeof(float4) * kRealBatch * kCtaWarps) +
                  32 * 32 * (threadIdx.x >> 5);
   const int s = blockIdx.y;
   const int a0 = sys_offset[s], n = sys_offset[s + 1] - a0;
-  if ((int)blockIdx.x * kRealAtoms >= n || n > max_atoms) return;  // uniform over the block
+  const int rank = (int)blockIdx.x % kRealCtas, block = (int)blockIdx.x / kRealCtas;
+  if (block * kRealAtoms >= n || n > max_atoms) return;  // uniform over the cluster
   const int64_t pb = (int64_t)s * max_atoms;  // this system's rows of the packed arrays
   const float4 *hi = w.hi + pb, *lo = w.lo + pb, *frac = w.frac + pb;
   const RealSys S = w.sys[s];
@@ -766,9 +773,9 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
     }
   __syncthreads();
   const float two_al_rsqrtpi = 2.0f * S.alpha * 0.56418958354775628695f;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = rank * kCtaWarps + (threadIdx.x >> 5);
   const int slot = lane & (kRealAtoms - 1), stream_id = warp * 2 + (lane >> 4);
-  const int il = blockIdx.x * kRealAtoms + slot;
+  const int il = block * kRealAtoms + slot;
   const bool act = il < n;
   const int64_t gi = a0 + (act ? il : 0);
   const int own = act ? il : 0;
@@ -859,7 +866,7 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
       for (int e = eb + lane; e < stop; e += 32) {
         const int code = wq[e];
         const int h = code >> 9, sl = (code >> 5) & 15, t = code & 31;
-        const int ii = blockIdx.x * kRealAtoms + sl, jj = j0h[h] + pass * 32 + t;
+        const int ii = block * kRealAtoms + sl, jj = j0h[h] + pass * 32 + t;
         const float4 hi_a = hi[ii], lo_a = lo[ii], hj = hi[jj], lj = lo[jj];
         float dx, dy, dz, r2;
         diff(hi_a, lo_a, hj, lj, dx, dy, dz, r2);
@@ -875,7 +882,9 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
           const float r = r2 * ir, qq = (hi_a.w * S.ke) * hj.w, al = S.alpha;
           const float er = erfc_cheb(al * r);
           ef += qq * er * ir;
-          dedr2 += 0.5f * ir * qq * (-er * ir * ir - two_al_rsqrtpi * __expf(-al * al * r2) * ir);
+          const float t = two_al_rsqrtpi * __expf(-al * al * r2);
+          // which product is rounded written out: the same bits whatever surrounds it
+          dedr2 = fmaf(0.5f * ir * qq, fmaf(-t, ir, __fmul_rn(-er * ir, ir)), dedr2);
         }
         const float m = -2.f * dedr2;
         force[e - eb] = make_float4(__fmul_rn(m, dx), __fmul_rn(m, dy), __fmul_rn(m, dz), 0.f);
@@ -891,16 +900,22 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
       __syncwarp();
     }
   }
-  part[stream_id][slot][0] = fx;
-  part[stream_id][slot][1] = fy;
-  part[stream_id][slot][2] = fz;
-  __syncthreads();
-  if (threadIdx.x < kRealAtoms && act) {
+  const int mine = stream_id - rank * 2 * kCtaWarps;
+  part[mine][slot][0] = fx;
+  part[mine][slot][1] = fy;
+  part[mine][slot][2] = fz;
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  if (rank == 0 && threadIdx.x < kRealAtoms && act) {
     float gx = 0.f, gy = 0.f, gz = 0.f;
-    for (int k = 0; k < kRealStreams; ++k) {
-      gx += part[k][slot][0];
-      gy += part[k][slot][1];
-      gz += part[k][slot][2];
+    for (int r = 0; r < kRealCtas; ++r) {
+      const float *p = cluster.map_shared_rank(&part[0][slot][0], r);
+#pragma unroll
+      for (int k = 0; k < 2 * kCtaWarps; ++k, p += 3 * kRealAtoms) {
+        gx += p[0];
+        gy += p[1];
+        gz += p[2];
+      }
     }
     if (gridDim.z > 1) {  // several blocks share atom gi
       atomicAdd(&grad[3 * gi], (double)gx);
@@ -918,6 +933,7 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_packed_kernel(
   }
   const double esum = block_sum(0.5 * (double)ef, red);
   if (threadIdx.x == 0) atomicAdd(&energy[s], esum);
+  cluster.sync();  // the first CTA has read the others' forces
 }
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -930,12 +946,23 @@ inline size_t recip_scratch_bytes(int32_t n_systems, int32_t n_kvecs) {
          align256(sizeof(Coef) * (size_t)n_systems * (size_t)n_kvecs);
 }
 
+// Kernels run on an SM at the same time only under one division of its memory into shared memory and
+// cache: real and reciprocal space, side by side in a molecular-dynamics step, ask for the same (65 % of
+// it shared).  A step of 4000 ions: 86.0 us with the driver's choices, 81.4 with 65, 83.4 with 80.
+template <typename F>
+inline cudaError_t same_carveout(F *kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 65);
+}
+
 int32_t recip_launch(char *base, const double *positions, const double *charges, const int32_t *sys_offset,
                      int32_t n_systems, int32_t max_atoms_per_system, const double *tril, const int32_t *kvec_n,
                      int32_t n_kvecs, const double *alpha, double coulomb_k, double *energy, double *grad,
                      double *grad_tril, double *structure_factor, kups_status *status, cudaStream_t stream) {
   RecipSys *sysp = (RecipSys *)base;
   Coef *coef = (Coef *)(base + align256(sizeof(RecipSys) * (size_t)n_systems));
+  KUPS_CUDA_TRY(same_carveout(recip_setup_kernel));
+  KUPS_CUDA_TRY(same_carveout(structure_factor_kernel));
+  KUPS_CUDA_TRY(same_carveout(recip_force_kernel));
   recip_setup_kernel<<<n_systems, kSetupThreads, 0, stream>>>(tril, kvec_n, n_kvecs, sysp, structure_factor, energy,
                                                               grad_tril, status);
   const int chunks = (max_atoms_per_system + kAtomsPerChunk - 1) / kAtomsPerChunk;
@@ -1162,6 +1189,7 @@ extern "C" int32_t kups_lj_ewald_real_forces_packed(const double *positions, con
   char *base = reinterpret_cast<char *>(((uintptr_t)workspace + 255) & ~uintptr_t(255));
   const RealWork w = real_work(base, n_systems, max_atoms_per_system);
   dim3 gp((max_atoms_per_system + 255) / 256 + 1, n_systems);
+  KUPS_CUDA_TRY(same_carveout(real_pack_kernel));
   real_pack_kernel<<<gp, 256, 0, stream>>>(positions, charges, species, sys_offset, tril, lj_cutoff, alpha,
                                            ewald_cutoff, coulomb_k, terms, max_atoms_per_system, w, energy, status);
   // partner shares: the caller's choice (a launch-shape tuner's), else one.  Shares add their
@@ -1169,10 +1197,11 @@ extern "C" int32_t kups_lj_ewald_real_forces_packed(const double *positions, con
   // measured fastest on the 4000-ion melt (250 blocks on 152 SMs: 0.152 ms per force
   // evaluation against 0.164 / 0.166 / 0.171 for 2 / 3 / 4 shares).
   const int splits = (terms & 8) && splits_req > 0 ? splits_req : 1;
-  dim3 g((max_atoms_per_system + kRealAtoms - 1) / kRealAtoms, n_systems, splits);
-  const size_t smem = kRealWarps * (kRealBatch * sizeof(float4) + 32 * 32 * sizeof(uint16_t));
+  dim3 g(kRealCtas * ((max_atoms_per_system + kRealAtoms - 1) / kRealAtoms), n_systems, splits);
+  const size_t smem = kCtaWarps * (kRealBatch * sizeof(float4) + 32 * 32 * sizeof(uint16_t));
   KUPS_CUDA_TRY(cudaFuncSetAttribute(real_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  real_packed_kernel<<<g, 32 * kRealWarps, smem, stream>>>(sys_offset, lj_sigma, lj_epsilon, n_species, terms,
+  KUPS_CUDA_TRY(same_carveout(real_packed_kernel));
+  real_packed_kernel<<<g, 32 * kCtaWarps, smem, stream>>>(sys_offset, lj_sigma, lj_epsilon, n_species, terms,
                                                         max_atoms_per_system, w, energy, grad);
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }

@@ -464,12 +464,13 @@ class LJEwaldMD:
         # partner shares per 16-atom block of the all-pairs real space (0: the library default of
         # one; autotune.autotune_lj_ewald picks one per workload)
         self.real_splits = 0
-        self._side = None  # the stream of the all-pairs real space
+        self._side = None  # the stream of reciprocal space beside the all-pairs real space
         self.graph = None
 
     def _force_terms(self):
         """Energies and gradients of real space (``e_pair``, ``g_pair``) and of reciprocal space (``e_rec``,
-        ``g_rec``); without a list the two run side by side, real space on a stream of its own."""
+        ``g_rec``); without a list the two run side by side, reciprocal space, whose kernels are the
+        shorter ones, on a stream of its own and of higher priority."""
         lib = _lib.load()
         pos = self.p.positions
         terms = TERM_EWALD_REAL | (TERM_LJ if self.lj else 0)
@@ -477,23 +478,23 @@ class LJEwaldMD:
             nsp = int(self.sig.shape[0]) if self.lj else 1
             here = torch.cuda.current_stream()
             if self._side is None:
-                self._side = torch.cuda.Stream()
+                self._side = torch.cuda.Stream(priority=-1)
             self._side.wait_stream(here)
             with torch.cuda.stream(self._side):
-                if self.real_splits:  # several shares per atom add onto what is there
-                    self.e_pair.zero_()
-                    self.g_pair.zero_()
-                    terms |= TERM_ACCUMULATE | (self.real_splits << 8)
-                rc = lib.kups_lj_ewald_real_forces_packed(
-                    pos.data_ptr(), self.q.data_ptr(), self.species.data_ptr(), self.off.data_ptr(), self.s,
-                    self.max_atoms, self.tril.data_ptr(), self.sig.data_ptr() if self.lj else None,
-                    self.eps.data_ptr() if self.lj else None, nsp, self.rc_lj.data_ptr() if self.lj else None,
-                    self.alpha.data_ptr(), self.rc_ew.data_ptr(), TO_STANDARD_UNITS, terms, self.e_pair.data_ptr(),
-                    self.g_pair.data_ptr(), self.real_ws.data_ptr(), self.real_ws.numel(), self.status.data_ptr(),
-                    _stream())
-                _lib.check(rc, "kups_lj_ewald_real_forces_packed")
-            self._recip()
+                self._recip()
+            if self.real_splits:  # several shares per atom add onto what is there
+                self.e_pair.zero_()
+                self.g_pair.zero_()
+                terms |= TERM_ACCUMULATE | (self.real_splits << 8)
+            rc = lib.kups_lj_ewald_real_forces_packed(
+                pos.data_ptr(), self.q.data_ptr(), self.species.data_ptr(), self.off.data_ptr(), self.s,
+                self.max_atoms, self.tril.data_ptr(), self.sig.data_ptr() if self.lj else None,
+                self.eps.data_ptr() if self.lj else None, nsp, self.rc_lj.data_ptr() if self.lj else None,
+                self.alpha.data_ptr(), self.rc_ew.data_ptr(), TO_STANDARD_UNITS, terms, self.e_pair.data_ptr(),
+                self.g_pair.data_ptr(), self.real_ws.data_ptr(), self.real_ws.numel(), self.status.data_ptr(),
+                _stream())
             here.wait_stream(self._side)
+            _lib.check(rc, "kups_lj_ewald_real_forces_packed")
             return
         rc = lib.kups_neighborlist_build(pos.data_ptr(), self.system.data_ptr(), self.incl.data_ptr(),
                                          self.excl.data_ptr(), self.n, self.s, self.tril.data_ptr(),
