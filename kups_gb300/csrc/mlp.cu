@@ -1060,20 +1060,21 @@ __global__ void proposal_density_kernel(const float *node, const double *cdf, in
 // Fused forward pass (inference: kups_mlp_fwd and the grid refresh).  A persistent CTA works on two
 // tiles of 128 points at a time, each with its own A operand in shared memory and its own 256-column
 // accumulator in tensor memory, by three kinds of warps that meet only at mbarriers:
-//   * eight epilogue warps per tile: features of the tile's points (coordinates reduced to
-//     [-0.5, 0.5) once in float64 and split into float pairs, the 32 phases as float pairs,
-//     phase_sincos) written as the first layer's A operand (bfloat16, no-swizzle K-major core
-//     matrices); after each layer tcgen05.ld, bias, softplus, and the next layer's A operand, or
+//   * sixteen epilogue warps, all on one tile and then on the other: features of the tile's points
+//     (coordinates reduced to [-0.5, 0.5) once in float64 and split into float pairs, the 32 phases as
+//     float pairs, phase_sincos) written as the first layer's A operand (bfloat16, no-swizzle K-major
+//     core matrices); after each layer tcgen05.ld, bias, softplus, and the next layer's A operand, or
 //     after the last the head (w4 . h3 + b4);
 //   * one warp loading the weights by TMA, 64 columns of W (256 rows, 128-byte swizzle, 32 KB) at a
 //     time, through a ring of two stages, in the order the MMAs take them;
 //   * one warp issuing tcgen05.mma (128 x 256 x 16, BF16 in, FP32 accumulate): the layers of the two
 //     tiles in turn, so that one tile's MMAs run under the other tile's epilogue.
-// What bounds it is the epilogue's issue slots (about ten instructions per activation, two of them on
-// the SFU, which is a third busy) with the hand-overs between layers: 52 % issue, tensor pipe 24 %.
-// 3e5 points: 158 us (162 without the next 16 columns on their way during the epilogue's work); 292 us
-// with one tile of 256 points whose MMAs and epilogue took turns, block barriers at every weight
-// chunk and 16-byte copies by all threads.
+// What bounds it is the epilogue's issue slots and SFU operations (about ten instructions per
+// activation, two of them on the SFU) with the hand-overs between layers: 54 % issue, tensor pipe 25 %.
+// 3e5 points: 152 us (158 with eight epilogue warps for each tile, which idle together while its MMAs
+// run; 162 without the next 16 columns on their way during the epilogue's work); 292 us with one tile of
+// 256 points whose MMAs and epilogue took turns, block barriers at every weight chunk and 16-byte
+// copies by all threads.
 // Every mbarrier wait is bounded; the one that runs out raises a flag that ends the others, the
 // kernel records KUPS_ERR_UNSUPPORTED, waits (bounded) for its copies and MMAs, frees its tensor
 // memory and returns.
@@ -1150,7 +1151,7 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kFwdOffBar);
   uint64_t *full = bars, *freed = bars + 2;        // [2] weight stage landed / its MMAs done
   uint64_t *ready = bars + 4, *acc = bars + 6;     // [2] tile's A operand written / accumulator complete
-  uint64_t *meet = bars + 8;                       // [2] the epilogue threads of a tile meet
+  uint64_t *meet = bars + 8;                       // the epilogue threads meet
   uint64_t *drained = bars + 10;                   // every MMA done (after a stop)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 11);
   volatile int *stop = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -1172,10 +1173,10 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
     for (int k = 0; k < 2; ++k) {
       mbar_init(smem_u32(&full[k]), 1);
       mbar_init(smem_u32(&freed[k]), 1);
-      mbar_init(smem_u32(&ready[k]), 32 * kFwdEpiWarps / 2);
+      mbar_init(smem_u32(&ready[k]), 32 * kFwdEpiWarps);
       mbar_init(smem_u32(&acc[k]), 1);
-      mbar_init(smem_u32(&meet[k]), 32 * kFwdEpiWarps / 2);
     }
+    mbar_init(smem_u32(meet), 32 * kFwdEpiWarps);
     mbar_init(smem_u32(drained), 1);
     *stop = 0;
   }
@@ -1192,15 +1193,13 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
   };
   const int64_t count[2] = {tiles_of(0), tiles_of(1)};  // count[0] >= count[1]
   if (warp < kFwdEpiWarps) {
-    const int h = warp >> 3, ht = tid & 255;                     // tile slot, thread inside it
-    const int quarter = warp & 3, colh = (warp >> 2) & 1;        // TMEM lanes 32 quarter .., columns 128 colh ..
-    const int row = quarter * 32 + lane;
-    __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smem + kFwdOffA + h * kFwdA);
-    float *part = reinterpret_cast<float *>(smem + kFwdOffPart) + h * 4 * kFwdTile;
-    float *fr = reinterpret_cast<float *>(smem + kFwdOffFr) + h * 6 * kFwdTile;
+    const int quarter = warp & 3, cq = warp >> 2, row = quarter * 32 + lane, cb = cq * 64;  // TMEM lanes, columns
+    const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+    __nv_bfloat16 *const sA0 = reinterpret_cast<__nv_bfloat16 *>(smem + kFwdOffA);
+    float *part = reinterpret_cast<float *>(smem + kFwdOffPart), *fr = reinterpret_cast<float *>(smem + kFwdOffFr);
     const float *w4 = spar + 3 * kHid;
     bool ok = true;
-    uint32_t parity = 0u, met = 0u;  // of the slot's next accumulator and next meeting
+    uint32_t parity[2] = {0u, 0u}, met = 0u;  // of the slots' next accumulators and of the next meeting
     // waits end alike for a whole warp (tcgen05.ld is a warp's operation)
     auto wait = [&](uint64_t *bar, uint32_t &phase) {
       const bool done = __all_sync(0xffffffffu, mbar_wait_or_stop(smem_u32(bar), phase, stop));
@@ -1208,13 +1207,21 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
       return done;
     };
     auto meeting = [&]() {
-      mbar_arrive(smem_u32(&meet[h]));
-      return wait(&meet[h], met);
+      mbar_arrive(smem_u32(meet));
+      return wait(meet, met);
     };
-    for (int64_t t = 0; t < count[h] && ok; ++t) {
-      const int64_t row0 = (blockIdx.x + (int64_t)gridDim.x * (2 * t + h)) * kFwdTile;
-      if (ht < kFwdTile) {  // coordinates reduced to [-0.5, 0.5) in float64, kept as float pairs
-        const int64_t pt = row0 + ht;
+    // slot h's A operand is visible to the tensor cores and its accumulator read: its next layer may start
+    auto start_layer = [&](int h) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(smem_u32(&ready[h]));
+    };
+    for (int64_t t = 0; t < count[0]; ++t) {
+      const int slots = t < count[1] ? 2 : 1;
+      auto first_row = [&](int h) { return (blockIdx.x + (int64_t)gridDim.x * (2 * t + h)) * kFwdTile; };
+      if (tid < slots * kFwdTile) {  // coordinates reduced to [-0.5, 0.5) in float64, kept as float pairs
+        const int h = tid / kFwdTile, ht = tid % kFwdTile;
+        const int64_t pt = first_row(h) + ht;
         double f[3] = {0.0, 0.0, 0.0};
         if (pt < n) {
           if (x != nullptr) {
@@ -1229,86 +1236,89 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
         for (int a = 0; a < 3; ++a) {
           const double red = f[a] - rint(f[a]);
           const float hi = (float)red;
-          fr[a * kFwdTile + ht] = hi;
-          fr[(3 + a) * kFwdTile + ht] = (float)(red - (double)hi);
+          fr[(6 * h + a) * kFwdTile + ht] = hi;
+          fr[(6 * h + 3 + a) * kFwdTile + ht] = (float)(red - (double)hi);
         }
       }
       ok = meeting();
       if (!ok) break;
-      {
-        const int r = ht & (kFwdTile - 1);
-        const bool in = row0 + r < n;
-        const float fh[3] = {fr[r], fr[kFwdTile + r], fr[2 * kFwdTile + r]};
-        const float fl[3] = {fr[3 * kFwdTile + r], fr[4 * kFwdTile + r], fr[5 * kFwdTile + r]};
-        for (int j = ht / kFwdTile; j < kFreq; j += 2) {
+      for (int h = 0; h < slots; ++h) {  // 8 of the 32 phases of a row
+        const float *c = fr + 6 * h * kFwdTile + row;
+        const bool in = first_row(h) + row < n;
+        const float fh[3] = {c[0], c[kFwdTile], c[2 * kFwdTile]};
+        const float fl[3] = {c[3 * kFwdTile], c[4 * kFwdTile], c[5 * kFwdTile]};
+        __nv_bfloat16 *sA = sA0 + h * (kFwdA / 2);
+#pragma unroll 2
+        for (int j = 8 * cq; j < 8 * cq + 8; ++j) {
           float sn = 0.f, cs = 0.f;
           if (in) phase_sincos(sfreq + 3 * j, fh, fl, sn, cs);
-          *reinterpret_cast<__nv_bfloat162 *>(sA + fwd_core(r, 2 * j, kIn)) = __floats2bfloat162_rn(sn, cs);
+          *reinterpret_cast<__nv_bfloat162 *>(sA + fwd_core(row, 2 * j, kIn)) = __floats2bfloat162_rn(sn, cs);
         }
+        start_layer(h);
       }
-      for (int layer = 0; layer < 3; ++layer) {
-        // the A operand is visible to the tensor cores and the accumulator read: the layer may start
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(smem_u32(&ready[h]));
-        ok = wait(&acc[h], parity);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float *bias = spar + layer * kHid;
-        float head = 0.f;
-        // 16 columns at a time, the next 16 on their way from tensor memory meanwhile
-        uint32_t next[16];
-        const uint32_t t0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * kHid + colh * 128);
-        tmem_load16(t0, next);
+      for (int layer = 0; layer < 3 && ok; ++layer)
+        for (int h = 0; h < slots; ++h) {
+          ok = wait(&acc[h], parity[h]);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const float *bias = spar + layer * kHid;
+          __nv_bfloat16 *sA = sA0 + h * (kFwdA / 2);
+          float head = 0.f;
+          // 16 columns at a time, the next 16 on their way from tensor memory meanwhile
+          uint32_t next[16];
+          const uint32_t t0 = lanes + (uint32_t)(h * kHid + cb);
+          tmem_load16(t0, next);
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          const int c0 = colh * 128 + 16 * s;
-          uint32_t r[16];
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int s = 0; s < 4; ++s) {
+            const int c0 = cb + 16 * s;
+            uint32_t r[16];
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int i = 0; i < 16; ++i) r[i] = next[i];
-          if (s < 7) tmem_load16(t0 + 16 * (s + 1), next);
-          const float4 *b4 = reinterpret_cast<const float4 *>(bias + c0);
-          float v[16];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 b = b4[q];
-            v[4 * q] = softplus_fast(__uint_as_float(r[4 * q]) + b.x);
-            v[4 * q + 1] = softplus_fast(__uint_as_float(r[4 * q + 1]) + b.y);
-            v[4 * q + 2] = softplus_fast(__uint_as_float(r[4 * q + 2]) + b.z);
-            v[4 * q + 3] = softplus_fast(__uint_as_float(r[4 * q + 3]) + b.w);
-          }
-          if (layer < 2) {
-            // next layer's A operand: 2 core-matrix rows of 8 bfloat16 (16 bytes each)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              __nv_bfloat162 hv[4];
-#pragma unroll
-              for (int u = 0; u < 4; ++u) hv[u] = __floats2bfloat162_rn(v[q * 8 + 2 * u], v[q * 8 + 2 * u + 1]);
-              *reinterpret_cast<uint4 *>(sA + fwd_core(row, c0 + q * 8, kHid)) = *reinterpret_cast<uint4 *>(hv);
-            }
-          } else {
-            const float4 *h4 = reinterpret_cast<const float4 *>(w4 + c0);
+            for (int i = 0; i < 16; ++i) r[i] = next[i];
+            if (s < 3) tmem_load16(t0 + 16 * (s + 1), next);
+            const float4 *b4 = reinterpret_cast<const float4 *>(bias + c0);
+            float v[16];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const float4 w = h4[q];
-              head = fmaf(v[4 * q], w.x, head);
-              head = fmaf(v[4 * q + 1], w.y, head);
-              head = fmaf(v[4 * q + 2], w.z, head);
-              head = fmaf(v[4 * q + 3], w.w, head);
+              const float4 b = b4[q];
+              v[4 * q] = softplus_fast(__uint_as_float(r[4 * q]) + b.x);
+              v[4 * q + 1] = softplus_fast(__uint_as_float(r[4 * q + 1]) + b.y);
+              v[4 * q + 2] = softplus_fast(__uint_as_float(r[4 * q + 2]) + b.z);
+              v[4 * q + 3] = softplus_fast(__uint_as_float(r[4 * q + 3]) + b.w);
             }
-            if ((s & 3) == 3) {  // sums of 64 columns
-              part[(c0 >> 6) * kFwdTile + row] = head;
-              head = 0.f;
+            if (layer < 2) {
+              // next layer's A operand: 2 core-matrix rows of 8 bfloat16 (16 bytes each)
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                __nv_bfloat162 hv[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) hv[u] = __floats2bfloat162_rn(v[q * 8 + 2 * u], v[q * 8 + 2 * u + 1]);
+                *reinterpret_cast<uint4 *>(sA + fwd_core(row, c0 + q * 8, kHid)) = *reinterpret_cast<uint4 *>(hv);
+              }
+            } else {
+              const float4 *h4 = reinterpret_cast<const float4 *>(w4 + c0);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const float4 w = h4[q];
+                head = fmaf(v[4 * q], w.x, head);
+                head = fmaf(v[4 * q + 1], w.y, head);
+                head = fmaf(v[4 * q + 2], w.z, head);
+                head = fmaf(v[4 * q + 3], w.w, head);
+              }
             }
           }
+          if (layer < 2) start_layer(h);
+          else part[(4 * h + cq) * kFwdTile + row] = head;  // of 64 columns
         }
-      }
       if (!ok) break;
       ok = meeting();
-      if (ok && ht < kFwdTile && row0 + ht < n)
-        g_out[row0 + ht] = ((part[ht] + part[kFwdTile + ht]) + (part[2 * kFwdTile + ht] + part[3 * kFwdTile + ht])) +
-                           sb4[0];
+      if (!ok) break;
+      if (tid < slots * kFwdTile) {
+        const int h = tid / kFwdTile, ht = tid % kFwdTile;
+        const float *g = part + 4 * h * kFwdTile + ht;
+        if (first_row(h) + ht < n)
+          g_out[first_row(h) + ht] = ((g[0] + g[kFwdTile]) + (g[2 * kFwdTile] + g[3 * kFwdTile])) + sb4[0];
+      }
     }
   } else if (warp == kFwdEpiWarps) {
     if (lane == 0) {  // weights, in the order of the MMAs
@@ -1404,7 +1414,8 @@ inline unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 // the kernel's only other traffic, 2.7 KB per point.  A second kernel forms all three weight
 // gradients dz^T h from those rows (points along K, both operands MN-major), so no transposed copy is
 // written.  Sixteen launches with float32 activations, transposed copies and column sums in memory
-// took 172 us of device time for 16384 points and 199 us with their enqueueing; three with Adam now take 70 us, enqueueing included (46 + 18 + 4).
+// took 172 us of device time for 16384 points and 199 us with their enqueueing; three with Adam now take
+// 70 us, enqueueing included (46 + 18 + 4).
 constexpr int kTrainStages = 4, kTrainEpi = 512, kTrainThreads = kTrainEpi + 64;
 // shared memory: weight stages | A operand | head partials [4][128] | coordinates [6][128] | biases
 // b1 b2 b3 and head weights w4 [4][256] | column sums of dz1, dz2, dz3 and of dL/dg h3 [4][256] |
