@@ -523,7 +523,33 @@ struct PairSearch {
   const int4 *label;
 };
 
-// The query of particle i and its candidate runs, by a whole warp; null if it has no edges.  `tmp`:
+// Whether the box of fractional offsets of centre c and half extents h may hold one whose nearest image
+// has a squared length below r2: each Cartesian component is bounded over the box (z by the third offset
+// alone, y by two, x by all three), an axis along which the box reaches past half a cell counts with both
+// images.
+__device__ inline bool offsets_within(const float c[3], const float h[3], const float L[6], float r2) {
+  const float hx = h[0] * fabsf(L[0]) + h[1] * fabsf(L[1]) + h[2] * fabsf(L[3]);
+  const float hy = h[1] * fabsf(L[2]) + h[2] * fabsf(L[4]), hz = h[2] * fabsf(L[5]);
+  auto within = [&](float d0, float d1, float d2) {
+    const float x = fmaxf(fabsf(d0 * L[0] + d1 * L[1] + d2 * L[3]) - hx, 0.f);
+    const float y = fmaxf(fabsf(d1 * L[2] + d2 * L[4]) - hy, 0.f), z = fmaxf(fabsf(d2 * L[5]) - hz, 0.f);
+    return x * x + y * y + z * z < r2;
+  };
+  if (within(c[0], c[1], c[2])) return true;
+  int other = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) other |= (fabsf(c[a]) + h[a] > 0.4999f) << a;
+  for (int k = 1; k < 8; ++k)
+    if ((k & ~other) == 0 && within((k & 1) ? c[0] - copysignf(1.f, c[0]) : c[0],
+                                    (k & 2) ? c[1] - copysignf(1.f, c[1]) : c[1],
+                                    (k & 4) ? c[2] - copysignf(1.f, c[2]) : c[2]))
+      return true;
+  return false;
+}
+
+// The query of particle i and its candidate runs, by a whole warp; null if it has no edges.  Cells that
+// the cutoff does not reach from where the particle lies in its own are left out (a third to a half of
+// the candidates where an axis has four cells or more; the margin of 1e-4 covers the float32 offsets).  `tmp`:
 // 32 rows of shared memory of the warp's own.
 __device__ const SysNL *pair_query(const PairSearch &a, int64_t i, PairQuery &q, CandRuns &rg, uint2 *tmp) {
   const int lane = threadIdx.x & 31;
@@ -556,8 +582,21 @@ __device__ const SysNL *pair_query(const PairSearch &a, int64_t i, PairQuery &q,
     int x, y, z;
     if (axis(cx, nx, lane % 3, x) & axis(cy, ny, (lane / 3) % 3, y) & axis(cz, nz, lane / 9, z)) {
       const int c = (int)p.cell_base + (z * ny + y) * nx + x;
-      first = a.cell_start[c];
-      len = a.cell_start[c + 1] - first;
+      float centre[3], half[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int m = k == 0 ? nx : k == 1 ? ny : nz, at = k == 0 ? cx : k == 1 ? cy : cz;
+        const int t = (k == 0 ? lane % 3 : k == 1 ? (lane / 3) % 3 : lane / 9) - 1;
+        const float w = k == 0 ? q.wi.x : k == 1 ? q.wi.y : q.wi.z;
+        float u = (w - floorf(w)) * (float)m - (float)at;  // place in the own cell, of m cells around
+        u -= (float)m * rintf(u / (float)m);
+        centre[k] = m > 2 ? (u - (float)t - 0.5f) / (float)m : 0.f;
+        half[k] = m > 2 ? 0.5f / (float)m : 1.f;
+      }
+      if (offsets_within(centre, half, q.L, 1.0001f * q.hi2)) {
+        first = a.cell_start[c];
+        len = a.cell_start[c + 1] - first;
+      }
     }
   }
   int sum = len;
@@ -586,7 +625,7 @@ __device__ const SysNL *pair_query(const PairSearch &a, int64_t i, PairQuery &q,
 // that more blocks fit an SM (4000 ions with 450 edges each: 85 against 124 us).  A particle whose edges do not fit its
 // `room` rows, or with shifts beyond 10 bits, is searched again to write them.  Bounded by issue:
 // about 40 instructions per 32 candidates, and 80 per 32 edges.  264 k particles in 256 systems
-// (about 500 candidates each): 0.73 ms (0.89 ms with the wait, 1.29 ms also with labels and shifts
+// (about 500 candidates each, 350 in cells within reach): 0.70 ms (0.73 ms with all 27 cells, 0.89 ms with the wait, 1.29 ms also with labels and shifts
 // taken up candidate by candidate); the float64 test per candidate (30 operations at 2 per clock per
 // SM, one thread per particle, a counting and a writing pass) took 19.3 ms.
 __global__ void __launch_bounds__(32 * kPairWarps, 4) pairs_kernel(PairSearch a, int room, bool defer, int64_t n_groups,
