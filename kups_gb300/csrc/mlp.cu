@@ -849,6 +849,7 @@ __device__ inline void store_bf16(__nv_bfloat16 *pb, __nv_bfloat16 *pbt, int64_t
 
 __global__ void adam_kernel(float *p, __nv_bfloat16 *pb, __nv_bfloat16 *pbt, float *g, float *m, float *v, int64_t n,
                             float lr, float b1, float b2, float eps, float c1, float c2) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -1521,13 +1522,6 @@ mlp_train_kernel(const __grid_constant__ TrainMaps maps, const float *p, const i
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ready + 4);
   volatile int *stop = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int e = tid; e < 4 * kHid; e += kTrainThreads) {
-    const int which = e / kHid;
-    const int64_t off = which == 0 ? kOffB1 : which == 1 ? kOffB2 : which == 2 ? kOffB3 : kOffW4;
-    spar[e] = p[off + e % kHid];
-    sums[e] = 0.f;
-  }
-  for (int e = tid; e < 3 * kFreq; e += kTrainThreads) sfreq[e] = freq[e];
   if (warp == kTrainEpi / 32) {
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -1546,7 +1540,17 @@ mlp_train_kernel(const __grid_constant__ TrainMaps maps, const float *p, const i
     *stop = 0;
   }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("fence.proxy.async;" ::: "memory");
+  for (int e = tid; e < 4 * kHid; e += kTrainThreads) {
+    const int which = e / kHid;
+    const int64_t off = which == 0 ? kOffB1 : which == 1 ? kOffB2 : which == 2 ? kOffB3 : kOffW4;
+    spar[e] = p[off + e % kHid];
+    sums[e] = 0.f;
+  }
+  for (int e = tid; e < 3 * kFreq; e += kTrainThreads) sfreq[e] = freq[e];
   __syncthreads();
+  asm volatile("griddepcontrol.launch_dependents;");  // tensor memory is held: the next grid cannot take it away
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   const int64_t n_tiles = (n + kFwdTile - 1) / kFwdTile;
@@ -1843,7 +1847,11 @@ mlp_weight_grad_kernel(const __grid_constant__ GradMaps maps, int64_t n, int sha
     *ok_flag = 1;
   }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  // the rows are whole when the training kernel has ended; every thread waits, so this grid ends after it
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("fence.proxy.async;" ::: "memory");
   __syncthreads();
+  asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   if (tid == 0) {
@@ -1911,6 +1919,30 @@ mlp_weight_grad_kernel(const __grid_constant__ GradMaps maps, int64_t n, int sha
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128));
+}
+
+// Launches a kernel that may start while its predecessor on the stream still runs: it sets up (barriers,
+// tensor memory), and every one of its threads waits (griddepcontrol.wait) before it reads or writes
+// memory of others, so it also ends after all that came before.  A kernel lets its successor start only
+// once it holds its tensor memory, which the successor could otherwise take while waiting for it.
+// Training step of 16384 points: 63.7 us (69.8 with each kernel set up after the last had drained; 68.2
+// with the weight gradients alone started early).  A captured launch keeps its full dependency.
+template <typename... P, typename... A>
+int32_t launch_early(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  KUPS_CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &early;
+  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  KUPS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+  return KUPS_OK;
 }
 
 }  // namespace
@@ -1999,15 +2031,15 @@ extern "C" int32_t kups_mlp_bwd(const kups_mlp *net, const double *x, const floa
                                      (int)kWgSmem));
   const int64_t tiles = (n + kFwdTile - 1) / kFwdTile, chunks = (n + 63) / 64;
   const TrainRows rows{w.feat, w.h1b, w.h2b, w.dz1, w.dz2, w.dz3, w.h1};
-  mlp_train_kernel<<<(unsigned)std::min<int64_t>(tiles, device_sm_count()), kTrainThreads, kTrainSmem, st>>>(
-      tm, net->param, net->freq, x, label, n, rows, net->grad, loss, status);
+  const int32_t rc = launch_early(mlp_train_kernel, (int)std::min<int64_t>(tiles, device_sm_count()), kTrainThreads,
+                                  kTrainSmem, st, tm, net->param, net->freq, x, label, n, rows, net->grad, loss, status);
+  if (rc != KUPS_OK) return rc;
   // shares of the points: 8 x 16 + 2 x 10 CTAs for a batch that gives each at least two chunks of 64
   const int shares = (int)std::min<int64_t>(16, std::max<int64_t>(1, chunks / 2));
   const int shares1 = (int)std::min<int64_t>(10, std::max<int64_t>(1, chunks / 2));
   const int aligned = ((uintptr_t)net->grad & 15) == 0;
-  mlp_weight_grad_kernel<<<8 * shares + 2 * shares1, kWgThreads, kWgSmem, st>>>(gm, n, shares, shares1, net->grad,
-                                                                                aligned, status);
-  return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
+  return launch_early(mlp_weight_grad_kernel, 8 * shares + 2 * shares1, kWgThreads, kWgSmem, st, gm, n, shares, shares1,
+                      net->grad, aligned, status);
 }
 
 extern "C" int32_t kups_mlp_adam(const kups_mlp *net, int64_t t, float lr, float beta1, float beta2, float eps,
@@ -2015,10 +2047,9 @@ extern "C" int32_t kups_mlp_adam(const kups_mlp *net, int64_t t, float lr, float
   if (net == nullptr || t < 1) return KUPS_ERR_INVALID;
   const float c1 = (float)(1.0 / (1.0 - pow((double)beta1, (double)t)));
   const float c2 = (float)(1.0 / (1.0 - pow((double)beta2, (double)t)));
-  adam_kernel<<<blocks(kParams, 256), 256, 0, (cudaStream_t)stream>>>(
-      net->param, (__nv_bfloat16 *)net->param_bf16, (__nv_bfloat16 *)net->param_bf16_t, net->grad, net->adam_m,
-      net->adam_v, kParams, lr, beta1, beta2, eps, c1, c2);
-  return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
+  return launch_early(adam_kernel, (int)blocks(kParams, 256), 256, 0, (cudaStream_t)stream, net->param,
+                      (__nv_bfloat16 *)net->param_bf16, (__nv_bfloat16 *)net->param_bf16_t, net->grad, net->adam_m,
+                      net->adam_v, kParams, lr, beta1, beta2, eps, c1, c2);
 }
 
 extern "C" int32_t kups_mlp_grid_norm(const kups_mlp *net, int32_t grid, float temper, float floor_frac,
