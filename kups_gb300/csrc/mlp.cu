@@ -1416,7 +1416,7 @@ inline unsigned blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 // gradients dz^T h from those rows (points along K, both operands MN-major), so no transposed copy is
 // written.  Sixteen launches with float32 activations, transposed copies and column sums in memory
 // took 172 us of device time for 16384 points and 199 us with their enqueueing; three with Adam now take
-// 70 us, enqueueing included (46 + 18 + 4).
+// 64 us, enqueueing included (46 + 18 + 4, overlapping at their ends; 70 us one after the other).
 constexpr int kTrainStages = 4, kTrainEpi = 512, kTrainThreads = kTrainEpi + 64;
 // shared memory: weight stages | A operand | head partials [4][128] | coordinates [6][128] | biases
 // b1 b2 b3 and head weights w4 [4][256] | column sums of dz1, dz2, dz3 and of dL/dg h3 [4][256] |
