@@ -549,7 +549,7 @@ __device__ inline bool offsets_within(const float c[3], const float h[3], const 
 
 // The query of particle i and its candidate runs, by a whole warp; null if it has no edges.  Cells that
 // the cutoff does not reach from where the particle lies in its own are left out (a third to a half of
-// the candidates where an axis has four cells or more; the margin of 1e-4 covers the float32 offsets).  `tmp`:
+// the candidates where an axis has four cells or more; hi2's margin and 1e-4 cover the float32 offsets).  `tmp`:
 // 32 rows of shared memory of the warp's own.
 __device__ const SysNL *pair_query(const PairSearch &a, int64_t i, PairQuery &q, CandRuns &rg, uint2 *tmp) {
   const int lane = threadIdx.x & 31;
@@ -622,12 +622,13 @@ __device__ const SysNL *pair_query(const PairSearch &a, int64_t i, PairQuery &q,
 // place with coalesced stores.  With `defer`, blocks take the next eight particles before they resolve
 // the prefix of the last eight, so no warp waits for a slower predecessor (with a wait after every
 // search a third of the warps' time went into it); a list of few groups takes one buffer instead, so
-// that more blocks fit an SM (4000 ions with 450 edges each: 85 against 124 us).  A particle whose edges do not fit its
-// `room` rows, or with shifts beyond 10 bits, is searched again to write them.  Bounded by issue:
-// about 40 instructions per 32 candidates, and 80 per 32 edges.  264 k particles in 256 systems
-// (about 500 candidates each, 350 in cells within reach): 0.70 ms (0.73 ms with all 27 cells, 0.89 ms with the wait, 1.29 ms also with labels and shifts
-// taken up candidate by candidate); the float64 test per candidate (30 operations at 2 per clock per
-// SM, one thread per particle, a counting and a writing pass) took 19.3 ms.
+// that more blocks fit an SM (4000 ions with 450 edges each: 85 against 124 us).  A particle whose edges
+// do not fit its `room` rows, or with shifts beyond 10 bits, is searched again to write them.  Bounded
+// by issue: about 40 instructions per 32 candidates, and 80 per 32 edges.  264 k particles in 256
+// systems (about 500 candidates each, 350 in cells within reach): 0.70 ms (0.73 ms with all 27 cells,
+// 0.89 ms with the wait, 1.29 ms also with labels and shifts taken up candidate by candidate); the
+// float64 test per candidate (30 operations at 2 per clock per SM, one thread per particle, a counting
+// and a writing pass) took 19.3 ms.
 __global__ void __launch_bounds__(32 * kPairWarps, 4) pairs_kernel(PairSearch a, int room, bool defer, int64_t n_groups,
                                                                    unsigned *ticket, unsigned long long *state,
                                                                    int64_t *n_edges, int32_t *edges, int32_t *shifts,
