@@ -153,8 +153,10 @@ def autotune_lj_ewald(sim, calls: int = 30, candidates=LJ_EWALD_SPLITS) -> Tuned
     """Partner shares per 16-atom block of the all-pairs LJ + Ewald real space
     (``kups_lj_ewald_real_forces_packed``, terms bits 8-11; 0 is the library default, one share)
     for an ``ewald.LJEwaldMD`` whose real space runs without a list.
-    Each candidate is timed over `calls` force evaluations at the current positions (a force
-    evaluation does not advance the state), after one untimed call; the fastest is set on `sim`
+    Each candidate is timed over `calls` replays of a captured force evaluation at the current
+    positions (a force evaluation does not advance the state), as steps are replayed: enqueued one by
+    one, an evaluation of 4000 ions takes the host 110 us with any number of shares, replayed 83 us
+    with one and 95 with four, so eager timings chose by noise.  The fastest is set on `sim`
     (before its step is captured as a CUDA graph) and cached per workload signature (systems,
     largest system, cutoffs).  The returned table lists (shares, 0, ms per force evaluation)."""
     if not sim.allpairs:
@@ -173,10 +175,15 @@ def autotune_lj_ewald(sim, calls: int = 30, candidates=LJ_EWALD_SPLITS) -> Tuned
         for sp in candidates:
             sim.real_splits = sp
             sim._forces()
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                sim._forces()
+            graph.replay()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
             for _ in range(calls):
-                sim._forces()
+                graph.replay()
             e1.record()
             torch.cuda.synchronize()
             ok = read_status(sim.status).code == _lib.KUPS_OK

@@ -1195,8 +1195,8 @@ extern "C" int32_t kups_lj_ewald_real_forces_packed(const double *positions, con
                                            ewald_cutoff, coulomb_k, terms, max_atoms_per_system, w, energy, status);
   // partner shares: the caller's choice (a launch-shape tuner's), else one.  Shares add their
   // partial forces, so they need terms & 8 (the caller's gradient is the base).  One share
-  // measured fastest on the 4000-ion melt (250 blocks on 152 SMs: 0.152 ms per force
-  // evaluation against 0.164 / 0.166 / 0.171 for 2 / 3 / 4 shares).
+  // measured fastest on the 4000-ion melt (250 clusters of four CTAs on 152 SMs: 0.083 ms per
+  // replayed force evaluation against 0.086 / 0.097 / 0.095 for 2 / 3 / 4 shares).
   const int splits = (terms & 8) && splits_req > 0 ? splits_req : 1;
   dim3 g(kRealCtas * ((max_atoms_per_system + kRealAtoms - 1) / kRealAtoms), n_systems, splits);
   const size_t smem = kCtaWarps * (kRealBatch * sizeof(float4) + 32 * 32 * sizeof(uint16_t));

@@ -482,7 +482,7 @@ class LJEwaldMD:
             self._side.wait_stream(here)
             with torch.cuda.stream(self._side):
                 self._recip()
-            if self.real_splits:  # several shares per atom add onto what is there
+            if self.real_splits > 1:  # several shares per atom add onto what is there
                 self.e_pair.zero_()
                 self.g_pair.zero_()
                 terms |= TERM_ACCUMULATE | (self.real_splits << 8)
