@@ -24,6 +24,7 @@ struct SysNL {
   double rc2;
   float Lf[6];
   float lo2, hi2;  // float32 squared distance below lo2: surely inside the cutoff, at or above hi2: outside
+  int tie;         // a pair within the cutoff may lie half a cell apart, with another image far away
   int nc[3];
   int nimg[3];
   int image_mode;  // prod(nimg) > 1: explicit image offsets, all system pairs are candidates
@@ -116,7 +117,7 @@ constexpr int kSetupSystems = 32;
 __global__ void __launch_bounds__(4 * kSetupSystems) setup_systems_kernel(const double *tril, const double *cutoffs,
                                                                          int32_t s, SysNL *sys, unsigned *ticket,
                                                                          kups_status *status) {
-  __shared__ int nimg[3][kSetupSystems], ncell[3][kSetupSystems];
+  __shared__ int nimg[3][kSetupSystems], ncell[3][kSetupSystems], narrow[3][kSetupSystems];
   __shared__ int64_t scratch[32];
   __shared__ unsigned done;
   const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(4 * kSetupSystems) setup_systems_kernel(const 
       }
       nimg[role][lane] = n;
       ncell[role][lane] = c;
+      narrow[role][lane] = finite && w < 2.0 * fabs(rc) * (1.0 + 1e-4);
     } else {
       const Tril64 inv = inverse_tril64(L);
       SysNL &p = sys[k];
@@ -174,6 +176,8 @@ __global__ void __launch_bounds__(4 * kSetupSystems) setup_systems_kernel(const 
     // 2^-24 (plus its own rounding), the products with L and their sum by a few 2^-24 of the terms;
     // 2^-19 sum|L| bounds the error of the distance with a factor of several to spare, and 2^-16 of
     // the squared cutoff the rounding of its square.  Between lo2 and hi2 the float64 test decides.
+    // Two particles half a cell apart may round to the other image of the two, which in a skewed cell is
+    // far away: where the cutoff reaches half a cell width, such candidates are kept whatever their distance.
     const double rc2 = rc * rc;
     double sum = 0.0;
     for (int a = 0; a < 6; ++a) {
@@ -186,6 +190,7 @@ __global__ void __launch_bounds__(4 * kSetupSystems) setup_systems_kernel(const 
     p.rc2 = rc2;
     p.hi2 = finite ? (float)(rc2 + margin) : (float)rc2;
     p.lo2 = finite ? (float)(rc2 - margin) : -1.0f;
+    p.tie = (p.Lf[1] != 0.f || p.Lf[3] != 0.f || p.Lf[4] != 0.f) && (narrow[0][lane] | narrow[1][lane] | narrow[2][lane]);
     for (int a = 0; a < 3; ++a) {
       p.nimg[a] = n[a];
       p.nc[a] = nc[a];
@@ -354,9 +359,14 @@ __device__ inline float image_distance(const float4 &wi, const float4 &c, const 
   return fmaf(Z, Z, fmaf(Y, Y, X * X));
 }
 
+// Whether an offset lies within 2^-18 of half a cell, where float32 may take the other image.
+__device__ inline bool beside_half(const float d[3]) {
+  return fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fabsf(d[2])) > 0.5f - 1.0f / 262144.0f;
+}
+
 // What a search makes of particle i (the same in every lane of its warp).
 struct PairQuery {
-  int i, inc, exi;
+  int i, inc, exi, tie;
   float4 wi;
   float L[6], lo2, hi2;
 };
@@ -370,21 +380,20 @@ __device__ __noinline__ bool exact_pair(const SysNL &p, const double *frac, int 
 
 // Whether record k is an edge of the particle at its minimum image, with its shift.  The float32
 // distance settles nearly every candidate; within the margin of the cutoff, within 2^-18 of half a
-// cell (the rounding of the image) and for images beyond 10 bits the float64 test decides, so the
-// edge set is that of the float64 test alone.
+// cell (the rounding of the image; with `tie` at any distance, see the setup) and for images beyond 10
+// bits the float64 test decides, so the edge set is that of the float64 test alone.
 __device__ inline bool settle_pair(const SysNL &p, const PairQuery &q, const float4 *cand, const int4 *label,
                                    const double *frac, int k, int &j, int sh[3]) {
-  constexpr float kHalf = 0.5f - 1.0f / 262144.0f;
   const float4 c = cand[k];
   float d[3], r[3];
   const float d2 = image_distance(q.wi, c, q.L, d, r);
-  if (!(d2 < q.hi2)) return false;
+  if (!(d2 < q.hi2) && !(q.tie && beside_half(d))) return false;
   const int4 lb = label[k];
   if (lb.x != q.inc) return false;
   j = __float_as_int(c.w);
   const int wn = __float_as_int(q.wi.w);
   const bool same_ex = lb.y == q.exi;
-  if (!(d2 < q.lo2) || fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fabsf(d[2])) > kHalf || ((wn | lb.z) & kWideImage)) {
+  if (!(d2 < q.lo2) || beside_half(d) || ((wn | lb.z) & kWideImage)) {
     const int o[3] = {0, 0, 0};
     return exact_pair(p, frac, q.i, j, o, false, same_ex, sh);
   }
@@ -411,12 +420,12 @@ __device__ int search_staged(const SysNL &p, const PairQuery &q, const CandRuns 
 #pragma unroll 2
   for (int base = 0; base < rg.total; base += 32) {
     const int k = cand_record(rg, base, a);
-    float d2 = INFINITY;
+    bool in = false;
     if (base + lane < rg.total) {
       float d[3], r[3];
-      d2 = image_distance(q.wi, cand[k], q.L, d, r);
+      in = image_distance(q.wi, cand[k], q.L, d, r) < q.hi2;
+      if (q.tie) in |= beside_half(d);
     }
-    const bool in = d2 < q.hi2;
     const unsigned m = __ballot_sync(0xffffffffu, in);
     const int at = near + __popc(m & below);
     if (in && at < room) stage[at].x = (unsigned)k;
@@ -564,6 +573,7 @@ __device__ const SysNL *pair_query(const PairSearch &a, int64_t i, PairQuery &q,
   q.wi = a.wrapped[i];
   q.lo2 = p.lo2;
   q.hi2 = p.hi2;
+  q.tie = p.tie;
 #pragma unroll
   for (int k = 0; k < 6; ++k) q.L[k] = p.Lf[k];
   int first = 0, len = 0;
