@@ -193,7 +193,8 @@ int32_t kups_lj_edges(const double *positions, const int32_t *system,
                       int32_t pair_fp32, kups_status *status, void *stream);
 /* kups_lj_edges_paired: the same sums for a list that holds every edge (i, j, s) together with its
  * reverse (j, i, -s), as kups_neighborlist_build writes it: one of the two is evaluated for both.
- * Results differ from kups_lj_edges by the rounding of the float64 sums.  Padding rows as there. */
+ * Results differ from kups_lj_edges by the rounding of the float64 sums, also for tables that are not
+ * symmetric.  Padding rows as there. */
 int32_t kups_lj_edges_paired(const double *positions, const int32_t *system,
                              const int32_t *species, int64_t n_particles,
                              const double *tril, const double *cutoffs, int32_t n_systems,

@@ -1,0 +1,46 @@
+"""The paired edge kernels with species tables that are not symmetric: an edge and its reverse then carry
+different terms, and the one that is evaluated stands for both.  Reference and tolerances as for the
+symmetric tables."""
+
+import numpy as np
+import pytest
+
+import test_gpu_pair_lists as lists
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [5, 90])
+@pytest.mark.parametrize("sig, eps", [([[2.0, 2.3], [2.1, 2.6]], [[0.01, 0.02], [0.02, 0.03]]),
+                                      ([[2.0, 2.3], [2.3, 2.6]], [[0.01, 0.02], [0.0, 0.03]])])
+@pytest.mark.parametrize("paired", [False, True])
+def test_tables_that_are_not_symmetric(monkeypatch, n, sig, eps, paired):
+    monkeypatch.setattr(lists, "SIG", np.array(sig))
+    monkeypatch.setattr(lists, "EPS", np.array(eps))
+    pos, system, species, q, e, s = lists.system_of(n, n)
+    for terms in (1, 3):
+        lists.close(lists.pair(pos, system, species, q, e, s, terms, paired),
+                    lists.reference(pos, system, species, q, e, s, terms))
+    want = lists.reference(pos, system, species, q, e, s, 1)
+    lists.close(lists.lj(pos, system, species, e, s, False, paired), want)
+    lists.close(lists.lj(pos, system, species, e, s, True, paired), want, 2e-5)  # float32 pairs
+
+
+def test_potential_with_a_table_that_is_not_symmetric():
+    from kups_gb300 import potential
+    from kups_gb300.neighborlist import CellListNeighborList
+
+    class Own(CellListNeighborList):
+        """A neighbour list of the caller's: nothing is known of its edges."""
+
+    pos, system, species, _, _, _ = lists.system_of(90, 4)
+    t = lists.t
+    prm = potential.LennardJonesParameters(("A", "B"), t([[2.0, 2.3], [2.1, 2.6]]), t([[0.01, 0.02], [0.015, 0.03]]),
+                                           t(lists.RC))
+    st = potential.LJState(potential.LJParticles(t(pos), t(species, lists.torch.int32), t(system, lists.torch.int32)),
+                           t(lists.CELLS), prm)
+    results = []
+    for neighbors in (CellListNeighborList(64), Own(64)):
+        out = potential.LennardJonesPotential(neighbors, pair_fp32=False)(st)
+        results.append([x.cpu().numpy() for x in (out.total_energies, out.gradients.positions, out.gradients.unitcell)])
+    lists.close(*results, 1e-10)
