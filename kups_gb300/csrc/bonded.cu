@@ -137,8 +137,8 @@ __device__ inline double root64(double x, double &inv) {
 }
 
 // Tests of float64 values by their bits: a float64 comparison, minimum or conversion takes the
-// float64 pipe like an addition.
-__device__ inline bool positive64(double x) { return __double_as_longlong(x) > 0; }
+// float64 pipe like an addition.  A NaN of either sign is not zero.
+__device__ inline bool nonzero64(double x) { return (__double_as_longlong(x) << 1) != 0; }
 __device__ inline int exponent64(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }  // biased by 1023
 __device__ inline double clamp_unit(double c) {  // c to [-1, 1] (a NaN to an end)
   const int hi = __double2hiint(c);
@@ -257,7 +257,7 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
     cross3(b1, b2, m);
     cross3(b2, b3, n);
     const R mm = dot3(m, m), nn = dot3(n, n), l2 = dot3(b2, b2);
-    const bool bent = positive64((double)mm) && positive64((double)nn) && positive64((double)l2);
+    const bool bent = nonzero64((double)mm) && nonzero64((double)nn) && nonzero64((double)l2);
     double ilb = 0.0;
     const R lb = bent ? (R)root64((double)l2, ilb) : R(0.0);
     R y = R(0.0), x = R(0.0);
@@ -391,8 +391,8 @@ __device__ R edge_energy_grad(const R (*v)[3], const R *p, R (*g)[3]) {
     cross3(v[1], v[2], n);
     const R nn = dot3(n, n), aa = dot3(v[0], v[0]), an = dot3(v[0], n);
     double iln = 1.0, ila = 1.0;
-    const R ln = positive64((double)nn) ? (R)root64((double)nn, iln) : R(0.0);
-    const R la = positive64((double)aa) ? (R)root64((double)aa, ila) : R(0.0);
+    const R ln = nonzero64((double)nn) ? (R)root64((double)nn, iln) : R(0.0);
+    const R la = nonzero64((double)aa) ? (R)root64((double)aa, ila) : R(0.0);
     const R inv_la = (R)inverse_regularised((double)la, ila), inv_ln = (R)inverse_regularised((double)ln, iln);
     const double s_raw = (double)(an * inv_ln * inv_la), s = clamp_unit(s_raw);
     const double w2 = fma(-s, s, 1.0), icw = rsqrt(exponent64(w2) < 1023 - 100 ? 1e-30 : w2), cw = w2 * icw;
