@@ -281,6 +281,9 @@ class LJEwaldPotential:
         self.ws = RecipWorkspace()
         self._side = None  # the stream of reciprocal space
 
+    def __getstate__(self):  # a copy makes its own stream
+        return {**self.__dict__, "_side": None}
+
     def __call__(self, particles: EwaldParticles, tril, patch=None, cache: LJEwaldCache | None = None) -> PotentialOut:
         tril = _f64(tril)
         s = tril.shape[0]
@@ -466,6 +469,9 @@ class LJEwaldMD:
         self.real_splits = 0
         self._side = None  # the stream of reciprocal space beside the all-pairs real space
         self.graph = None
+
+    def __getstate__(self):  # a copy makes its own stream
+        return {**self.__dict__, "_side": None}
 
     def _force_terms(self):
         """Energies and gradients of real space (``e_pair``, ``g_pair``) and of reciprocal space (``e_rec``,
