@@ -313,14 +313,14 @@ class LJEwaldPotential:
         if self._side is None or self._side.device != here.device:
             self._side = torch.cuda.Stream()
         self._side.wait_stream(here)
-        with torch.cuda.stream(self._side):
-            self._last_recip = ewald_recip(pos, q, off, mx, tril, kn, alpha, ws=self.ws, out=out, status=status)
         try:
+            with torch.cuda.stream(self._side):
+                self._last_recip = ewald_recip(pos, q, off, mx, tril, kn, alpha, ws=self.ws, out=out, status=status)
             en, g, gt = pair_edges(particles.positions, particles.system, particles.species, particles.charges, tril,
                                    e.indices, e.shifts.view(-1, 3), e.n_edges, terms, sig, eps, rc_lj, alpha, rc_ew,
                                    paired=lists_pairs(self.neighborlist))
             es = ewald_self(q, off, alpha, s)
-        finally:
+        finally:  # also before an exception gives this stream's memory back
             here.wait_stream(self._side)
         el, gl, gtl, _, _ = self._last_recip
         energy, grad, gtril = en + el + es, g + gl, gt + gtl
@@ -486,20 +486,22 @@ class LJEwaldMD:
             if self._side is None:
                 self._side = torch.cuda.Stream(priority=-1)
             self._side.wait_stream(here)
-            with torch.cuda.stream(self._side):
-                self._recip()
-            if self.real_splits > 1:  # several shares per atom add onto what is there
-                self.e_pair.zero_()
-                self.g_pair.zero_()
-                terms |= TERM_ACCUMULATE | (self.real_splits << 8)
-            rc = lib.kups_lj_ewald_real_forces_packed(
-                pos.data_ptr(), self.q.data_ptr(), self.species.data_ptr(), self.off.data_ptr(), self.s,
-                self.max_atoms, self.tril.data_ptr(), self.sig.data_ptr() if self.lj else None,
-                self.eps.data_ptr() if self.lj else None, nsp, self.rc_lj.data_ptr() if self.lj else None,
-                self.alpha.data_ptr(), self.rc_ew.data_ptr(), TO_STANDARD_UNITS, terms, self.e_pair.data_ptr(),
-                self.g_pair.data_ptr(), self.real_ws.data_ptr(), self.real_ws.numel(), self.status.data_ptr(),
-                _stream())
-            here.wait_stream(self._side)
+            try:
+                with torch.cuda.stream(self._side):
+                    self._recip()
+                if self.real_splits > 1:  # several shares per atom add onto what is there
+                    self.e_pair.zero_()
+                    self.g_pair.zero_()
+                    terms |= TERM_ACCUMULATE | (self.real_splits << 8)
+                rc = lib.kups_lj_ewald_real_forces_packed(
+                    pos.data_ptr(), self.q.data_ptr(), self.species.data_ptr(), self.off.data_ptr(), self.s,
+                    self.max_atoms, self.tril.data_ptr(), self.sig.data_ptr() if self.lj else None,
+                    self.eps.data_ptr() if self.lj else None, nsp, self.rc_lj.data_ptr() if self.lj else None,
+                    self.alpha.data_ptr(), self.rc_ew.data_ptr(), TO_STANDARD_UNITS, terms, self.e_pair.data_ptr(),
+                    self.g_pair.data_ptr(), self.real_ws.data_ptr(), self.real_ws.numel(), self.status.data_ptr(),
+                    _stream())
+            finally:  # also before an exception gives this stream's memory back
+                here.wait_stream(self._side)
             _lib.check(rc, "kups_lj_ewald_real_forces_packed")
             return
         rc = lib.kups_neighborlist_build(pos.data_ptr(), self.system.data_ptr(), self.incl.data_ptr(),

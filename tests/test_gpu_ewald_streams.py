@@ -1,4 +1,5 @@
-"""The second stream of the LJ + Ewald classes: objects that have made one are copied and pickled as before."""
+"""The second stream of the LJ + Ewald classes: objects that have made one are copied and pickled as before,
+and a call that fails on the host leaves no work of that stream unordered with the caller's."""
 
 import copy
 import pickle
@@ -42,3 +43,34 @@ def test_objects_with_a_second_stream_are_copied(copied):
         s.run(3)
         s.check()
     assert torch.allclose(sim.energy, twin.energy, rtol=1e-9, atol=0)
+
+
+@pytest.mark.parametrize("what", ["potential", "simulation"])
+def test_a_failing_call_waits_for_the_second_stream(monkeypatch, what):
+    """The launch on the second stream raises after it has enqueued work; what the caller's stream does next
+    comes after that work."""
+    from kups_gb300 import ewald
+
+    parts, tril, prm, lj, masses, momenta = salt()
+    mark = torch.zeros(1, device="cuda")
+
+    def late(*args, **kwargs):
+        torch.cuda._sleep(100_000_000)  # about 50 ms
+        mark.fill_(1)
+        raise RuntimeError("a launch refused")
+
+    if what == "potential":
+        pot = ewald.LJEwaldPotential(prm, *lj)
+        call = lambda: pot(parts, tril)
+        call()
+    else:
+        sim = ewald.LJEwaldMD(parts, masses, tril, prm, 0.01, *lj)
+        sim.start(momenta)
+        assert sim.allpairs
+        call = sim._forces
+    torch.cuda.synchronize()
+    monkeypatch.setattr(ewald, "ewald_recip", late)
+    with pytest.raises(RuntimeError, match="a launch refused"):
+        call()
+    seen = mark.clone()
+    assert float(seen) == 1.0
