@@ -368,6 +368,10 @@ int32_t kups_ewald_recip(const double *positions, const double *charges,
                          double coulomb_k, double *energy, double *grad, double *grad_tril,
                          double *structure_factor, void *workspace, size_t workspace_bytes,
                          kups_status *status, void *stream);
+/* The number of components above that limit, added to *outside: for callers that read a word of theirs
+ * before they launch the rest. */
+int32_t kups_ewald_kvecs_outside(const int32_t *kvec_n, int32_t n_systems, int32_t n_kvecs,
+                                 int32_t *outside, void *stream);
 /* kups_ewald_recip_energy: E = K sum_k P(k) |S(k)|^2 per system from given
  * structure factors (float64 [S, n_kvecs, 2]), the long-range energy of a
  * cached S(k) (EwaldCache / EwaldLongRangeComposer, src/kups/potential/

@@ -116,6 +116,7 @@ SIGNATURES = {
     "kups_md_unpack": (_I32, [_P, _P, _P, _P, _I64, _P, _P, _P, _P]),
     "kups_ewald_recip_workspace_bytes": (_SZ, [_I32, _I32]),
     "kups_ewald_recip": (_I32, [_P, _P, _P, _I32, _I32, _P, _P, _I32, _P, C.c_double, _P, _P, _P, _P, _P, _SZ, _P, _P]),
+    "kups_ewald_kvecs_outside": (_I32, [_P, _I32, _I32, _P, _P]),
     "kups_ewald_recip_energy": (_I32, [_P, _P, _I32, _P, _I32, C.c_double, _P, _P, _P, _SZ, _P, _P]),
     "kups_ewald_recip_static": (_I32, [_P, _P, _P, _I32, _I32, _P, _P, _I32, _P, C.c_double, _P, _P, _P, _P, _P, _P]),
     "kups_lj_ewald_real_forces": (_I32, [_P, _P, _P, _P, _I32, _I32, _P, _P, _P, _I32, _P, _P, _P, C.c_double, _I32, _P, _P, _P, _P]),

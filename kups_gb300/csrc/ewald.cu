@@ -112,6 +112,14 @@ __global__ void __launch_bounds__(kSetupThreads) recip_setup_kernel(const double
   sys[i] = r;
 }
 
+// The setup's test of |n_a| alone, for callers that need its answer before they use what the rest returns.
+__global__ void __launch_bounds__(256) kvec_limit_kernel(const int32_t *kn, int64_t count, int32_t *outside) {
+  int beyond = 0;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < count; e += (int64_t)gridDim.x * 256)
+    beyond += kn[e] > kMaxM || kn[e] < -kMaxM;
+  if (beyond != 0) atomicAdd(outside, beyond);
+}
+
 // Per-atom tables e^{2 pi i m f_a}, m in [-M_a, M_a], from sincospi of the fundamental and complex
 // products (error grows ~linearly in |m| <= 16): thread t < 96 of a block fills axis t / 32 of atom
 // c0 + t % 32 (three short chains side by side instead of one of 48 products per atom).
@@ -1029,6 +1037,16 @@ extern "C" int32_t kups_ewald_recip(const double *positions, const double *charg
   return recip_launch(base, positions, charges, sys_offset, n_systems, max_atoms_per_system, tril, kvec_n,
                       n_kvecs, alpha, coulomb_k, energy, grad, grad_tril, structure_factor, status,
                       (cudaStream_t)stream_);
+}
+
+extern "C" int32_t kups_ewald_kvecs_outside(const int32_t *kvec_n, int32_t n_systems, int32_t n_kvecs,
+                                            int32_t *outside, void *stream) {
+  if (n_systems < 0 || n_kvecs < 0 || outside == nullptr) return KUPS_ERR_INVALID;
+  const int64_t count = 3 * (int64_t)n_systems * n_kvecs;
+  if (count == 0) return KUPS_OK;
+  const unsigned blocks = (unsigned)std::min<int64_t>((count + 255) / 256, 4 * (int64_t)device_sm_count());
+  kvec_limit_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(kvec_n, count, outside);
+  return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 
 // Reciprocal energy from given structure factors (the energy step of the launch

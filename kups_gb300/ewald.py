@@ -137,16 +137,24 @@ class EwaldParameters:
 
 
 # ----------------------------------------------------------------------------- kernels
-def _offsets(system: torch.Tensor, s: int) -> tuple[torch.Tensor, int]:
-    """Offsets [S + 1] of the systems' atoms and the most atoms of a system (one launch, one read)."""
+def _offsets(system: torch.Tensor, s: int, kvec_n: torch.Tensor | None = None) -> tuple[torch.Tensor, int]:
+    """Offsets [S + 1] of the systems' atoms and the most atoms of a system (one launch, one read); with
+    ``kvec_n`` the same read tells of k vectors beyond the kernels' tables, and they are refused."""
     words = torch.empty(s + 4, dtype=torch.int32, device="cuda")
     off, stats = words[:s + 1], words[s + 1:]
-    rc = _lib.load().kups_system_offsets(system.data_ptr(), system.shape[0], s, off.data_ptr(), stats.data_ptr(),
-                                         _stream())
+    lib, st = _lib.load(), _stream()
+    rc = lib.kups_system_offsets(system.data_ptr(), system.shape[0], s, off.data_ptr(), stats.data_ptr(), st)
     _lib.check(rc, "kups_system_offsets")
+    if kvec_n is not None:  # counted where indices outside are
+        rc = lib.kups_ewald_kvecs_outside(kvec_n.data_ptr(), kvec_n.shape[0], kvec_n.shape[1], stats.data_ptr() + 4, st)
+        _lib.check(rc, "kups_ewald_kvecs_outside")
     most, outside, _ = stats.tolist()
     if outside:
-        raise RuntimeError(f"{outside} system indices outside [0, {s})")
+        bad = int(((system < 0) | (system >= s)).sum())
+        if bad:
+            raise RuntimeError(f"{bad} system indices outside [0, {s})")
+        first = int((kvec_n.abs() > 16).flatten(1).any(1).nonzero()[0])
+        _lib.raise_status(_lib.Status(_lib.KUPS_ERR_UNSUPPORTED, 0, 0, first))
     return off, most
 
 
@@ -298,12 +306,12 @@ class LJEwaldPotential:
             terms |= TERM_LJ
         if patch is not None:
             return self._patched(particles, tril, patch, cache, terms, sig, eps, rc_lj, alpha, rc_ew, rc_nl)
-        off, mx = _offsets(_i32(particles.system), s)
+        kn = _i32(self.ewald.reciprocal_lattice_shifts)
+        off, mx = _offsets(_i32(particles.system), s, kn)
         pts = NeighborListPoints(particles.positions, particles.system, None, particles.exclusion)
         e, self.neighborlist = self.neighborlist.call_and_fix(pts, None, tril, rc_nl)
         # reciprocal space beside the edges (float64 units against the others), on a stream of its own;
         # its outputs and scratch belong to this stream, which waits for it before anything reads them
-        kn = _i32(self.ewald.reciprocal_lattice_shifts)
         n, f64 = _f64(particles.positions).shape[0], dict(dtype=torch.float64, device="cuda")
         out = (torch.empty(s, **f64), torch.empty((n, 3), **f64), torch.empty((s, 6), **f64),
                torch.empty((s, kn.shape[1], 2), **f64))
@@ -362,11 +370,10 @@ class LJEwaldPotential:
         order = torch.argsort(both_sys, stable=True)
         pos_m = torch.cat([old[idx], new[idx]])[order].contiguous()
         q_m = torch.cat([-q, q])[order].contiguous()
-        off_m, mx = _offsets(both_sys[order], s)
-        _, _, _, dsk, _ = ewald_recip(pos_m, q_m, off_m, mx, tril, self.ewald.reciprocal_lattice_shifts, alpha,
-                                      grad_tril=False, ws=self.ws)
+        kn = _i32(self.ewald.reciprocal_lattice_shifts)
+        off_m, mx = _offsets(both_sys[order], s, kn)
+        _, _, _, dsk, _ = ewald_recip(pos_m, q_m, off_m, mx, tril, kn, alpha, grad_tril=False, ws=self.ws)
         sk_new = cache.structure_factor + dsk
-        kn = self.ewald.reciprocal_lattice_shifts
         de = de + ewald_recip_energy(tril, kn, alpha, sk_new, ws=self.ws) - ewald_recip_energy(
             tril, kn, alpha, cache.structure_factor, ws=self.ws)
         e_new = cache.total_energies + de
