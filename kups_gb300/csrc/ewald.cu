@@ -405,9 +405,7 @@ __global__ void self_energy_kernel(const double *q, const int32_t *sys_offset, c
 //   VACUUM (exclusion correction, subtracted) K q_i q_j / r, no cutoff
 // Each term is summed / 2 per system (directed edges), gradients as in
 // kups_lj_edges.  Float64 distance; pair arithmetic in float64, one reciprocal square
-// root per pair in place of the divisions by r, r^2 and r^3.  With PAIRED one edge stands for both
-// directions: in LJ tables that are not symmetric these differ, and their mean is taken.
-template <bool PAIRED>
+// root per pair in place of the divisions by r, r^2 and r^3.
 struct EwaldPairEval {
   const int32_t *species;
   const double *q, *lj_sigma, *lj_eps, *rc_lj, *alpha, *rc_ew;
@@ -415,7 +413,6 @@ struct EwaldPairEval {
   double ke;
   int ti, key;
   double sig2, eps4, rc2_lj, al, rcew, rc2_ew, qi;
-  bool both;  // the two directions differ
 
   __device__ void load_system(int s) {
     if (terms & 1) rc2_lj = rc_lj[s] * rc_lj[s];
@@ -439,20 +436,10 @@ struct EwaldPairEval {
         key = k;
         sig2 = lj_sigma[k] * lj_sigma[k];
         eps4 = 4.0 * lj_eps[k];
-        if (PAIRED) {
-          const int back = species[j] * nsp + ti;
-          both = lj_sigma[back] != lj_sigma[k] || lj_eps[back] != lj_eps[k];
-        }
       }
       const double s2 = sig2 * inv, c6 = s2 * s2 * s2;
       en += eps4 * (c6 * c6 - c6);
       dedr2 -= 3.0 * eps4 * c6 * (2.0 * c6 - 1.0) * inv;
-      if (PAIRED && both) {
-        const int back = species[j] * nsp + ti;
-        const double t2 = lj_sigma[back] * lj_sigma[back] * inv, b6 = t2 * t2 * t2, eps4_back = 4.0 * lj_eps[back];
-        en = 0.5 * (en + eps4_back * (b6 * b6 - b6));
-        dedr2 = 0.5 * (dedr2 - 3.0 * eps4_back * b6 * (2.0 * b6 - 1.0) * inv);
-      }
     }
     if (terms & 6) {
       const double qq = qi * q[j] * ir;  // K q_i q_j / r
@@ -470,12 +457,13 @@ struct EwaldPairEval {
   }
 };
 
-// 4000 ions, 1.8 M directed edges, LJ + Ewald: 0.36 ms with PAIRED, 0.69 ms without; a thread per
+// 4000 ions, 1.8 M directed edges, LJ + Ewald: 0.38 ms with PAIRED, 0.70 ms without; a thread per
 // edge with thirteen atomics (seven of them on one system's sums) took 12.3 ms.
 template <bool PAIRED>
-__global__ void __launch_bounds__(32 * kRunWarps) pair_edges_kernel(PairList p, EwaldPairEval<PAIRED> ev) {
+__global__ void __launch_bounds__(32 * kRunWarps) pair_edges_kernel(PairList p, EwaldPairEval ev) {
   ev.key = -1;
-  run_pairs<PAIRED>(p, ev);
+  const bool symmetric = PAIRED && ((ev.terms & 1) == 0 || tables_symmetric(ev.lj_sigma, ev.lj_eps, ev.nsp));
+  run_pairs<PAIRED>(p, ev, symmetric);
 }
 
 template <bool PAIRED>
@@ -495,7 +483,7 @@ int32_t launch_pair_edges(const double *positions, const int32_t *system, const 
   if (n_edges == 0) return KUPS_OK;
   const int64_t per = run_edges_per_warp(n_edges);
   const PairList p{positions, system, n, tril, n_systems, edges, shifts, n_edges, energy, grad, grad_tril, per};
-  EwaldPairEval<PAIRED> ev{};
+  EwaldPairEval ev{};
   ev.species = species;
   ev.q = charges;
   ev.lj_sigma = lj_sigma;
@@ -1162,7 +1150,9 @@ extern "C" int32_t kups_pair_edges_paired(const double *positions, const int32_t
                                    double *energy, double *grad, double *grad_tril,
                                    kups_status *status, void *stream) {
   (void)status;
-  return launch_pair_edges<true>(positions, system, species, charges, n, tril, n_systems, lj_sigma, lj_epsilon,
+  const bool one_of_two = (terms & 1) == 0 || n_species <= kTableSpecies;
+  const auto launch = one_of_two ? launch_pair_edges<true> : launch_pair_edges<false>;
+  return launch(positions, system, species, charges, n, tril, n_systems, lj_sigma, lj_epsilon,
                                   n_species, lj_cutoff, alpha, ewald_cutoff, coulomb_k, terms, edges, shifts, n_edges,
                                   energy, grad, grad_tril, (cudaStream_t)stream);
 }

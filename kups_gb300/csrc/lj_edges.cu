@@ -15,18 +15,9 @@
 namespace kups {
 namespace {
 
-template <typename R>
-__device__ inline void lj_terms(R inv, R sig, R eps, R &e, R &d) {
-  const R s2 = sig * sig * inv;
-  const R c6 = s2 * s2 * s2;
-  e = R(4) * eps * (c6 * c6 - c6);
-  d = R(-12) * eps * c6 * (R(2) * c6 - R(1)) * inv;
-}
-
 // LJ terms of a run of edges sharing their first particle; the species pair's constants are kept
-// while the second particle's species does not change.  With PAIRED one edge stands for both
-// directions: in tables that are not symmetric these differ, and their mean is taken.
-template <typename R, bool PAIRED>
+// while the second particle's species does not change.
+template <typename R>
 struct LjEval {
   const int32_t *species;
   const double *sigma, *epsilon, *cutoffs;
@@ -34,7 +25,6 @@ struct LjEval {
   kups_status *status;
   int ti, key;
   R rc2, sig, eps;
-  bool both;  // the two directions differ
 
   __device__ void load_system(int s) {
     const double rc = cutoffs[s];
@@ -47,23 +37,15 @@ struct LjEval {
       key = k;
       sig = (R)sigma[k];
       eps = (R)epsilon[k];
-      if (PAIRED) {
-        const int back = species[j] * nsp + ti;
-        both = (R)sigma[back] != sig || (R)epsilon[back] != eps;
-      }
     }
     const R r2 = (R)r2d;
     R e = R(0), d = R(0);
     if (r2 < rc2) {
       const R inv = R(1) / r2;
-      lj_terms(inv, sig, eps, e, d);
-      if (PAIRED && both) {
-        const int back = species[j] * nsp + ti;
-        R e2, d2;
-        lj_terms(inv, (R)sigma[back], (R)epsilon[back], e2, d2);
-        e = R(0.5) * (e + e2);
-        d = R(0.5) * (d + d2);
-      }
+      const R s2 = sig * sig * inv;
+      const R c6 = s2 * s2 * s2;
+      e = R(4) * eps * (c6 * c6 - c6);
+      d = R(-12) * eps * c6 * (R(2) * c6 - R(1)) * inv;
     }
     if (!isfinite(e) || !isfinite(d)) status_error(status, KUPS_ERR_NONFINITE, edge);
     en = (double)e;
@@ -71,12 +53,13 @@ struct LjEval {
   }
 };
 
-// 264 k particles in 256 systems, 14 M directed edges, float32 pairs: 0.52 ms with PAIRED, 0.9 ms
-// without (0.61 and 1.0 ms with shifted and other edges mixed); one thread per edge with six atomics and seven float64 warp sums took 2.47 ms.
+// 264 k particles in 256 systems, 14 M directed edges, float32 pairs: 0.53 ms with PAIRED, 0.82 ms
+// without (0.61 and 1.0 ms with shifted and other edges mixed); one thread per edge with six atomics and
+// seven float64 warp sums took 2.47 ms.
 template <typename R, bool PAIRED>
-__global__ void __launch_bounds__(32 * kRunWarps) lj_edges_kernel(PairList p, LjEval<R, PAIRED> ev) {
+__global__ void __launch_bounds__(32 * kRunWarps) lj_edges_kernel(PairList p, LjEval<R> ev) {
   ev.key = -1;
-  run_pairs<PAIRED>(p, ev);
+  run_pairs<PAIRED>(p, ev, PAIRED && tables_symmetric(ev.sigma, ev.epsilon, ev.nsp));
 }
 
 template <bool PAIRED>
@@ -96,10 +79,10 @@ int32_t launch_lj_edges(const double *positions, const int32_t *system, const in
   const PairList p{positions, system, n, tril, s, edges, shifts, n_edges, energy, grad, grad_tril, per};
   const unsigned grid = run_blocks(n_edges, per);
   if (pair_fp32) {
-    const LjEval<float, PAIRED> ev{species, sigma, epsilon, cutoffs, nsp, status, 0, -1};
+    const LjEval<float> ev{species, sigma, epsilon, cutoffs, nsp, status, 0, -1, 0.f, 0.f, 0.f};
     lj_edges_kernel<float, PAIRED><<<grid, 32 * kRunWarps, 0, stream>>>(p, ev);
   } else {
-    const LjEval<double, PAIRED> ev{species, sigma, epsilon, cutoffs, nsp, status, 0, -1};
+    const LjEval<double> ev{species, sigma, epsilon, cutoffs, nsp, status, 0, -1, 0.0, 0.0, 0.0};
     lj_edges_kernel<double, PAIRED><<<grid, 32 * kRunWarps, 0, stream>>>(p, ev);
   }
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
@@ -128,7 +111,8 @@ extern "C" int32_t kups_lj_edges_paired(const double *positions, const int32_t *
                                         const int32_t *shifts, int64_t n_edges, double *energy,
                                         double *grad, double *grad_tril, int32_t pair_fp32,
                                         kups_status *status, void *stream) {
-  return launch_lj_edges<true>(positions, system, species, n, tril, cutoffs, s, sigma, epsilon, nsp, edges, shifts,
+  const auto launch = nsp <= kTableSpecies ? launch_lj_edges<true> : launch_lj_edges<false>;
+  return launch(positions, system, species, n, tril, cutoffs, s, sigma, epsilon, nsp, edges, shifts,
                                n_edges, energy, grad, grad_tril, pair_fp32, status, (cudaStream_t)stream);
 }
 

@@ -9,7 +9,9 @@
 //    per component per run (a shuffle tree over the warp costs five float64 additions per edge and
 //    component, an atomic per edge as much traffic again as the second particle's);
 //  * with PAIRED the list is known to hold every edge together with its reverse (what the neighbour
-//    list writes): only one of the two is evaluated, with twice its weight;
+//    list writes): only one of the two is evaluated, with twice its weight, unless the species tables
+//    are not symmetric and the two differ.  Every block looks through the tables first, which leaves
+//    the loop over pairs as it is (a test of the species pair in there made pair_edges 10 % slower);
 //  * edges with and without an image shift are collected apart, so that the shift's three float64
 //    additions and the six of dE/dtril are spent on shifted edges only, with every lane at work
 //    (mixed, 40 float64 instructions were issued per 32 pairs of which 17 lanes' worth did work);
@@ -71,9 +73,25 @@ struct Const {
   static constexpr bool value = B;
 };
 
+// Species up to which a block looks through the tables; with more, every edge is evaluated.  14 M edges,
+// float32 pairs: 528 us with one species, 548 with 32, against 824 edge by edge (at 32 the look takes 4 us
+// of a kernel's start).
+constexpr int kTableSpecies = 32;
+
+// Whether two tables [n, n] are symmetric, by a whole block.
+__device__ inline bool tables_symmetric(const double *a, const double *b, int n) {
+  bool same = true;
+  for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
+    const int i = k / n, j = k - i * n;
+    if (i < j) same = same && a[k] == a[j * n + i] && b[k] == b[j * n + i];
+  }
+  return __syncthreads_and(same);
+}
+
 // Eval: load_system(s), load_first(i), and eval(e, j, r2, en, dedr2): energy and dE/d(r^2) of edge e.
+// symmetric (PAIRED): whether an edge and its reverse carry the same terms.
 template <bool PAIRED, typename Eval>
-__device__ void run_pairs(const PairList &p, Eval &ev) {
+__device__ void run_pairs(const PairList &p, Eval &ev, bool symmetric) {
   // edges to evaluate: [0] without a shift, [1] shifted; qe: the edge's number from the warp's first
   // (a report names it)
   __shared__ int q_i[kRunWarps][2][kRunQueue], q_j[kRunWarps][2][kRunQueue], q_e[kRunWarps][2][kRunQueue];
@@ -87,7 +105,8 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
   double en_sum = 0.0, dl[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, gi[3] = {0.0, 0.0, 0.0}, xi[3] = {0.0, 0.0, 0.0};
   Tril64 L;
   bool any_dl = false;
-  constexpr double kShare = PAIRED ? 1.0 : 0.5;  // of an edge's energy
+  const bool single = PAIRED && symmetric;  // one edge of each pair
+  const double share = single ? 1.0 : 0.5;  // of an edge's energy
   auto flush_first = [&]() {
     if (fi >= 0)
       for (int a = 0; a < 3; ++a) atomicAdd(&p.grad[3 * (int64_t)fi + a], gi[a]);
@@ -95,7 +114,7 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
   };
   auto flush_system = [&]() {  // this lane's sums of the system it leaves
     if (sys >= 0) {
-      atomicAdd(&p.energy[sys], kShare * en_sum);
+      atomicAdd(&p.energy[sys], share * en_sum);
       if (any_dl && p.grad_tril)
         for (int a = 0; a < 6; ++a) atomicAdd(&p.grad_tril[6 * (int64_t)sys + a], dl[a]);
     }
@@ -141,7 +160,7 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
       double en, dedr2;
       ev.eval(e0 + qe[k], j, r2, en, dedr2);
       // a directed edge carries half of its pair: g / 2 = dE/d(r^2) d
-      const double f = PAIRED ? 2.0 * dedr2 : dedr2;
+      const double f = PAIRED ? 2.0 * share * dedr2 : dedr2;
       const double h[3] = {f * d[0], f * d[1], f * d[2]};
       en_sum += en;
       for (int a = 0; a < 3; ++a) {
@@ -194,7 +213,7 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
       }
       bool take = i >= 0 && i < p.n && j >= 0 && j < p.n;
       int s0 = 0, s1 = 0, s2 = 0;
-      if (take && PAIRED) take = j >= i;
+      if (take && single) take = j >= i;
       if (take) {
         s0 = p.shifts[3 * e];
         s1 = p.shifts[3 * e + 1];
@@ -202,7 +221,7 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
         const int si = p.system[i];
         take = si >= 0 && si < p.s;
         // a particle and its own images: the shift that is lexicographically positive
-        if (PAIRED && i == j) take = take && (s0 > 0 || (s0 == 0 && (s1 > 0 || (s1 == 0 && s2 > 0))));
+        if (single && i == j) take = take && (s0 > 0 || (s0 == 0 && (s1 > 0 || (s1 == 0 && s2 > 0))));
       }
       const int kind = (s0 | s1 | s2) != 0;
       const unsigned m1 = __ballot_sync(0xffffffffu, take && kind == 1);
@@ -233,7 +252,7 @@ __device__ void run_pairs(const PairList &p, Eval &ev) {
   if (__all_sync(0xffffffffu, sys == top || sys < 0)) {
     if (top >= 0) {
       en_sum = warp_sum(en_sum);
-      if (lane == 0) atomicAdd(&p.energy[top], kShare * en_sum);
+      if (lane == 0) atomicAdd(&p.energy[top], share * en_sum);
       if (__any_sync(0xffffffffu, any_dl) && p.grad_tril)
         for (int a = 0; a < 6; ++a) {
           const double v = warp_sum(dl[a]);

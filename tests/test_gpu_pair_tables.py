@@ -44,3 +44,20 @@ def test_potential_with_a_table_that_is_not_symmetric():
         out = potential.LennardJonesPotential(neighbors, pair_fp32=False)(st)
         results.append([x.cpu().numpy() for x in (out.total_energies, out.gradients.positions, out.gradients.unitcell)])
     lists.close(*results, 1e-10)
+
+
+@pytest.mark.parametrize("species", [8, 32, 33])  # the largest tables that are looked through, and beyond
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_large_tables(monkeypatch, species, symmetric):
+    rng = np.random.default_rng(species)
+    sig, eps = rng.uniform(1.8, 2.6, (2, species, species)) * np.array([[[1.0]], [[0.01]]])
+    if symmetric:
+        sig, eps = (sig + sig.T) / 2, (eps + eps.T) / 2
+    monkeypatch.setattr(lists, "SIG", sig)
+    monkeypatch.setattr(lists, "EPS", eps)
+    pos, system, _, q, e, s = lists.system_of(90, species)
+    kinds = rng.integers(0, species, len(pos))
+    for terms in (1, 3):
+        lists.close(lists.pair(pos, system, kinds, q, e, s, terms, True),
+                    lists.reference(pos, system, kinds, q, e, s, terms))
+    lists.close(lists.lj(pos, system, kinds, e, s, False, True), lists.reference(pos, system, kinds, q, e, s, 1))
