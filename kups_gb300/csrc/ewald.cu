@@ -419,7 +419,7 @@ struct EwaldPairEval {
     if (terms & 2) {
       al = alpha[s];
       rcew = rc_ew[s];
-      rc2_ew = rcew * rcew;
+      rc2_ew = rcew * fabs(rcew);  // no pair is within a negative cutoff
     }
   }
   __device__ void load_first(int i) {

@@ -1,6 +1,5 @@
 """The paired edge kernels with species tables that are not symmetric: an edge and its reverse then carry
-different terms, and the one that is evaluated stands for both.  Reference and tolerances as for the
-symmetric tables."""
+different terms.  And cutoffs that no pair is within.  Reference and tolerances as for the pair lists' test."""
 
 import numpy as np
 import pytest
@@ -61,3 +60,13 @@ def test_large_tables(monkeypatch, species, symmetric):
         lists.close(lists.pair(pos, system, kinds, q, e, s, terms, True),
                     lists.reference(pos, system, kinds, q, e, s, terms))
     lists.close(lists.lj(pos, system, kinds, e, s, False, True), lists.reference(pos, system, kinds, q, e, s, 1))
+
+
+@pytest.mark.parametrize("paired", [False, True])
+@pytest.mark.parametrize("cutoff", [0.0, -4.0])
+def test_no_pair_is_within_a_cutoff_of_nothing(monkeypatch, paired, cutoff):
+    """One system's real-space electrostatics switched off by its cutoff: r < cutoff holds for no pair."""
+    monkeypatch.setattr(lists, "RCE", np.array([5.0, cutoff, 5.2]))
+    pos, system, species, q, e, s = lists.system_of(90, 7)
+    lists.close(lists.pair(pos, system, species, q, e, s, 3, paired),
+                lists.reference(pos, system, species, q, e, s, 3))
