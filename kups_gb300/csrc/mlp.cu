@@ -1386,10 +1386,15 @@ mlp_forward_kernel(const __grid_constant__ CUtensorMap w1, const __grid_constant
   }
 }
 
-int32_t fused_forward(const kups_mlp *net, const double *x, int64_t n, int grid, float *g, kups_status *status,
-                      cudaStream_t st) {
+// copy: room for the weights, taken where theirs do not start on a 16-byte boundary (TMA reads from those)
+int32_t fused_forward(const kups_mlp *net, const double *x, int64_t n, int grid, float *g, __nv_bfloat16 *copy,
+                      kups_status *status, cudaStream_t st) {
   if (n <= 0) return KUPS_OK;
   const __nv_bfloat16 *pb = (const __nv_bfloat16 *)net->param_bf16;
+  if (((uintptr_t)pb & 15) != 0) {
+    KUPS_CUDA_TRY(cudaMemcpyAsync(copy, pb, 2 * kParams, cudaMemcpyDeviceToDevice, st));
+    pb = copy;
+  }
   CUtensorMap w1, w2, w3;
   if (!operand_map(&w1, pb + kOffW1, kHid, kIn, kIn, kHid) || !operand_map(&w2, pb + kOffW2, kHid, kHid, kHid, kHid) ||
       !operand_map(&w3, pb + kOffW3, kHid, kHid, kHid, kHid))
@@ -1991,8 +1996,8 @@ extern "C" int32_t kups_mlp_fwd(const kups_mlp *net, const double *x, int64_t n,
                                 size_t workspace_bytes, kups_status *status, void *stream) {
   if (net == nullptr || n < 0 || (n > 0 && (x == nullptr || g == nullptr))) return KUPS_ERR_INVALID;
   if (workspace_bytes < kups_mlp_workspace_bytes(n)) return KUPS_ERR_INVALID;
-  (void)workspace;
-  return fused_forward(net, x, n, 0, g, status, (cudaStream_t)stream);
+  const MlpWork w = carve(workspace, std::min<int64_t>(n, kChunk));
+  return fused_forward(net, x, n, 0, g, w.weights, status, (cudaStream_t)stream);
 }
 
 extern "C" int32_t kups_mlp_nce_batch(const double *data, int64_t n_data, int32_t batch, uint64_t seed,
@@ -2063,7 +2068,7 @@ extern "C" int32_t kups_mlp_grid_norm(const kups_mlp *net, int32_t grid, float t
   if (workspace_bytes < kups_mlp_workspace_bytes(n)) return KUPS_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
   const MlpWork w = carve(workspace, std::min<int64_t>(n, kChunk));
-  const int32_t rc = fused_forward(net, nullptr, n, grid, node, status, st);
+  const int32_t rc = fused_forward(net, nullptr, n, grid, node, w.weights, status, st);
   if (rc) return rc;
   double *partial = w.partial;
   const int n_norm = (int)std::min<int64_t>(kNormBlocks, (n + kNormThreads - 1) / kNormThreads);
