@@ -799,7 +799,7 @@ int32_t kups_gemm_bf16(const void *a, int32_t a_bf16, int64_t sa_row, int64_t sa
 #define KUPS_MLP_PARAMS 148481
 typedef struct kups_mlp {
   float *param;        /* [KUPS_MLP_PARAMS] float32 master copy */
-  void *param_bf16;    /* [KUPS_MLP_PARAMS] bfloat16 copy the GEMMs read */
+  void *param_bf16;    /* [KUPS_MLP_PARAMS] bfloat16 copy that the matrix products read */
   float *grad;         /* [KUPS_MLP_PARAMS] accumulated by kups_mlp_bwd, zeroed by kups_mlp_adam */
   float *adam_m;       /* [KUPS_MLP_PARAMS] */
   float *adam_v;       /* [KUPS_MLP_PARAMS] */
@@ -807,8 +807,8 @@ typedef struct kups_mlp {
   void *param_bf16_t;  /* [2, 256, 256] bfloat16 W2^T, W3^T (kept by init / Adam) */
 } kups_mlp;
 
-/* workspace for kups_mlp_fwd / kups_mlp_bwd / kups_mlp_grid_norm over n points
- * (forward passes run in chunks of at most 65536 points) */
+/* workspace for kups_mlp_fwd / kups_mlp_bwd / kups_mlp_grid_norm over n points (that of 65536 points
+ * for more: backward passes take no more, forward passes keep nothing per point) */
 size_t kups_mlp_workspace_bytes(int64_t n_points);
 /* weights uniform with variance 1 / fan_in from Philox(seed), biases, moments, gradient zero */
 int32_t kups_mlp_init(const kups_mlp *net, uint64_t seed, void *stream);

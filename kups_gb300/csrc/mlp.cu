@@ -469,12 +469,11 @@ int32_t launch_gemm(const GemmArgs &g, kups_status *status, cudaStream_t stream)
 }
 
 // ---------------------------------------------------------------------------
-// TMA-fed variant for bfloat16 operands with K contiguous (every GEMM of the network's
-// training step): one thread issues cp.async.bulk.tensor loads of 64-wide K chunks (128-byte
-// rows, 128-byte swizzle) into a ring of STAGES stages, each completing on its mbarrier, and
-// the MMAs of a chunk as soon as it has landed; the ring holds the whole K extent of the
-// network's GEMMs (K <= 256), so every load of a tile is in flight at once.  A stage is
-// refilled only after the commit of the MMAs that read it.  The other threads wait at the
+// TMA-fed variant for bfloat16 operands with K contiguous: one thread issues
+// cp.async.bulk.tensor loads of 64-wide K chunks (128-byte rows, 128-byte swizzle) into a
+// ring of STAGES stages, each completing on its mbarrier, and the MMAs of a chunk as soon as
+// it has landed; the ring holds a K of up to 256 whole, so every load of such a tile is in
+// flight at once.  A stage is refilled only after the commit of the MMAs that read it.  The other threads wait at the
 // block barrier, then all run the register epilogue.  Every wait is bounded; on time-out the
 // thread waits (bounded) for the loads and MMAs it issued, records KUPS_ERR_UNSUPPORTED, and
 // the tile frees its tensor memory without writing C.
@@ -621,7 +620,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // Tensor map of a bfloat16 [rows, k] operand with row stride sr elements (K contiguous), boxes
 // of 64 x box_rows, 128-byte swizzle; out-of-range elements read as zero.  The last maps made
-// are kept (a training step passes the same workspace operands every step), so encoding runs
+// are kept (a training step passes the same weights and rows every step), so encoding runs
 // once per distinct operand; the cache is per host thread.
 bool operand_map(CUtensorMap *m, const void *p, int64_t rows, int64_t k, int64_t sr, int box_rows) {
   struct Entry {
@@ -686,9 +685,6 @@ int32_t launch_gemm_tma(const GemmArgs &g, kups_status *status, cudaStream_t str
   return cudaGetLastError() == cudaSuccess ? KUPS_OK : KUPS_ERR_CUDA;
 }
 
-// Tile width: 128 (64 for N <= 64), narrowed to 64 while the grid would leave SMs idle
-// (fewer than two CTAs per SM of 148).  128-wide tiles (64 KB of pipeline buffers, three
-// CTAs per SM) beat 256-wide ones (two CTAs per SM) on the network's K <= 256 GEMMs.
 // Whether the register epilogue of gemm_tcgen05_kernel applies: float32 C (and the optional
 // bias, gate and bfloat16 copy) row-major with unit column stride and 16-byte aligned rows,
 // N a multiple of 32, no beta term.
@@ -712,19 +708,20 @@ int32_t dispatch_gemm(const GemmArgs &g0, kups_status *status, cudaStream_t st) 
   if (tma_operands(g)) {  // one tile column per 256 of N; the tile ring holds K <= 256 whole
     // tiles as wide as N (up to 256, one CTA per SM) with a four-stage ring: measured against
     // 128 x 128 and 128 x 64 tiles with two stages (three and four CTAs per SM) and with four
-    // stages, it was the fastest on the network's training step (0.194 against 0.196-0.214 ms)
+    // stages, it was the fastest on a network step by separate products, 16384 x 256 x 256 and their
+    // gradients (0.194 against 0.196-0.214 ms)
     bool launched = false;
     const int32_t rc = g.n <= 64    ? launch_gemm_tma<64, 4, 1>(g, status, st, launched)
                        : g.n <= 128 ? launch_gemm_tma<128, 4, 1>(g, status, st, launched)
                                     : launch_gemm_tma<256, 4, 1>(g, status, st, launched);
     if (launched || rc != KUPS_OK) return rc;
   }
+  // Tile width: 128 (64 for N <= 64), narrowed to 64 while the grid would leave SMs idle (fewer than
+  // two CTAs per SM of 148).
   const int64_t rows = ((int64_t)g.m + kBM - 1) / kBM * g.split_k;
   int bn = g.n <= 64 ? 64 : 128;
   while (bn > 64 && rows * ((g.n + bn - 1) / bn) < 2 * 148) bn >>= 1;
-  if (bn == 64) return launch_gemm<64>(g, status, st);
-  if (bn == 128) return launch_gemm<128>(g, status, st);
-  return launch_gemm<256>(g, status, st);
+  return bn == 64 ? launch_gemm<64>(g, status, st) : launch_gemm<128>(g, status, st);
 }
 
 // ============================================================================
@@ -732,10 +729,10 @@ int32_t dispatch_gemm(const GemmArgs &g0, kups_status *status, cudaStream_t st) 
 //
 // Fixed architecture: 64 Fourier features of the fractional position f,
 // (sin, cos)(2 pi m_j . f) for 32 integer vectors m_j, three softplus layers of
-// width 256 (tensor-core GEMMs, bfloat16 operands, float32 accumulation) and
+// width 256 (tensor-core products, bfloat16 operands, float32 accumulation) and
 // a linear output g(f).  Parameters are one flat float32 array at the kOff*
-// offsets plus a bfloat16 copy that the matrix products read.  Training minimises the noise-contrastive
-// loss with equal halves of data and uniform points,
+// offsets plus a bfloat16 copy that the matrix products read.  Training minimises
+// the noise-contrastive loss with equal halves of data and uniform points,
 //   L = (1/n) [sum_data softplus(-g) + sum_uniform softplus(g)],
 // whose minimiser is g(f) = ln p_data(f) for f uniform on the unit cube.
 constexpr int kFreq = 32, kIn = 2 * kFreq, kHid = 256;
@@ -743,7 +740,7 @@ constexpr int64_t kOffW1 = 0, kOffB1 = kOffW1 + kHid * kIn, kOffW2 = kOffB1 + kH
                   kOffW3 = kOffB2 + kHid, kOffB3 = kOffW3 + kHid * kHid, kOffW4 = kOffB3 + kHid,
                   kOffB4 = kOffW4 + kHid, kParams = kOffB4 + 1;
 static_assert(kParams == KUPS_MLP_PARAMS, "parameter layout");
-constexpr int64_t kChunk = 65536;  // points per forward pass over the workspace
+constexpr int64_t kChunk = 65536;  // points of the largest training batch, and that a workspace is sized for
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -836,7 +833,7 @@ __global__ void nce_batch_kernel(const double *data, int64_t n_data, int64_t bat
 // Adam (Kingma & Ba 2015) with bias corrections c1 = 1 / (1 - beta1^t),
 // c2 = 1 / (1 - beta2^t); refreshes the bfloat16 copy and zeroes the gradient.
 // bfloat16 copies of a parameter: the flat copy, and for W2 / W3 the transposed copy
-// (W^T[in][out]) that the backward GEMMs read as a K-contiguous operand.
+// (W^T[in][out]) that the training kernel multiplies the next layer's gradients by.
 __device__ inline void store_bf16(__nv_bfloat16 *pb, __nv_bfloat16 *pbt, int64_t i, float v) {
   const __nv_bfloat16 b = __float2bfloat16(v);
   pb[i] = b;

@@ -56,12 +56,13 @@ inline cudaError_t exclusive_scan(T *data, int64_t n, T *block_sums, T *total, c
 }
 
 // ---------------------------------------------------------------- single-pass prefix
-// Chained prefix over blocks that take their numbers from a ticket (a block's predecessors have
-// therefore started before it): state[b] holds a 2-bit flag above a 62-bit value, 0 = nothing yet,
-// 1 = the block's own sum, 2 = the sum of blocks 0..b, 3 = a predecessor's wait ran out.  The words
-// must be zero before the launch.  A block first publishes its own sum, then (at once or after other
-// work) one full warp of it asks for the sum of blocks 0..b-1, which every lane returns.  The wait for a predecessor is bounded: when it runs out the block publishes flag 3,
-// so no later block waits on it, and ok comes back false.
+// Chained prefix over blocks (the single-pass scan with decoupled look-back of Merrill and Garland,
+// 2016) that take their numbers from a ticket, so that a block's predecessors have started before it:
+// state[b] holds a 2-bit flag above a 62-bit value, 0 = nothing yet, 1 = the block's own sum, 2 = the
+// sum of blocks 0..b, 3 = a predecessor's wait ran out.  The words must be zero before the launch.  A
+// block first publishes its own sum, then (at once or after other work) one full warp of it asks for
+// the sum of blocks 0..b-1, which every lane returns.  The wait for a predecessor is bounded: when it
+// runs out the block publishes flag 3, so no later block waits on it, and ok comes back false.
 constexpr int kPrefixPolls = 1 << 22;
 
 __device__ inline unsigned long long prefix_load(const unsigned long long *p) {

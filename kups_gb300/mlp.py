@@ -8,7 +8,7 @@ src/kups/core/propagator.py:330-334).
 Network: 64 Fourier features of the fractional position f (sin / cos of
 2 pi m . f for 32 fixed integer vectors m) -> 3 hidden layers of width 256
 (softplus) -> 1 output g(f), BF16 weights and activations, FP32
-accumulation (``kups_gemm_bf16``).  The density is exp(g) evaluated on the
+accumulation (``kups_mlp_fwd``, ``kups_mlp_bwd``).  The density is exp(g) evaluated on the
 nodes of a periodic 64^3 grid and interpolated trilinearly; its exact
 normaliser is the node mean, and sampling is exact (cell by its mass, then
 a corner by its weight, then per-axis linear densities), so the proposal
