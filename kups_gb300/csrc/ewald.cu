@@ -752,6 +752,10 @@ __global__ void __launch_bounds__(256) real_pack_kernel(const double *pos, const
 
 // A block's 16 warps are a cluster of four CTAs, whose forces the first adds up through distributed
 // shared memory: 4000 ions are 250 blocks, one or two per SM, or 1000 CTAs, six or seven (48 us and 43).
+// Ten steps in us with 1 / 2 / 4 / 8 CTAs: 216 ions 316 / 316 / 316 / 315, 1000 ions 354 / 337 / 336 / 339,
+// 2000 ions 455 / 421 / 410 / 421, 4000 ions 890 / 865 / 811 / 887, 8000 ions 2178 / 2083 / 2121 / 2528, 32
+// systems of 216 ions 500 / 479 / 486 / 573, 16 of 1000 ions 1343 / 1283 / 1312 / 1551: two are 2 % better
+// where 16-atom blocks fill the chip by themselves, four up to 12 % where they do not.
 constexpr int kRealCtas = 4, kCtaWarps = kRealWarps / kRealCtas;
 
 __global__ void __cluster_dims__(kRealCtas, 1, 1) __launch_bounds__(32 * kCtaWarps) real_packed_kernel(
@@ -958,7 +962,9 @@ inline size_t recip_scratch_bytes(int32_t n_systems, int32_t n_kvecs) {
 
 // Kernels run on an SM at the same time only under one division of its memory into shared memory and
 // cache: real and reciprocal space, side by side in a molecular-dynamics step, ask for the same (65 % of
-// it shared).  A step of 4000 ions: 86.0 us with the driver's choices, 81.4 with 65, 83.4 with 80.
+// it shared).  A step of 4000 ions: 86.0 us with the driver's choices, 81.4 with 65, 83.4 with 80.  Ten steps
+// with the driver's choice / 65 %: 216 ions 315 / 316 us, 512 ions 304 / 295, 2000 ions 436 / 410, 8000 ions
+// 2290 / 2121, 32 systems of 216 ions 511 / 486.
 template <typename F>
 inline cudaError_t same_carveout(F *kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 65);
