@@ -655,8 +655,8 @@ def run_observables(a, reps=20):
     return {"workload": f"{S} systems x {n_mol} three-atom molecules ({n} atoms), all outputs", "ms_per_call": ms,
             "atoms_per_s": n / (ms / 1e3),
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
-                         "peak_source": kind, "note": "float64 throughout; molecular centres take three extra "
-                                                      "passes (anchor, minimum-image sums, centre)"}}
+                         "peak_source": kind, "note": "float64 throughout; a thread forms the centre of a whole "
+                                                      "molecule, group passes only where one is not a single run"}}
 
 
 def run_mliap(a, reps=10):

@@ -588,7 +588,7 @@ class LennardJonesMD64:
     src/kups/md/integrators.py:273-318, 405-455) with its derivative computation as the reference's MD
     application runs it (application/md/simulation.py:74-119): the neighbour list rebuilt at every step
     (``kups_neighborlist_build``, exact float64 membership), LJ energy and gradients over the edges in
-    float64 (``kups_lj_edges``), and the float64 integrator blocks (``kups_md_kick`` / ``kups_md_drift``
+    float64 (``kups_lj_edges_paired``), and the float64 integrator blocks (``kups_md_kick`` / ``kups_md_drift``
     with the wrap / ``kups_md_thermostat``).  Every launch is stream-ordered with no host
     synchronisation; velocity-Verlet steps replay from one captured CUDA graph.  This is the float64
     counterpart of ``FusedLennardJonesMD`` (float32 pair arithmetic), for small systems that must
