@@ -178,7 +178,7 @@ int32_t kups_edge_gradients(const double *dE_dd, const int32_t *system, int64_t 
  * PositionAndUnitCell (src/kups/potential/common/energy.py:264-355).
  *
  *   species    i32 [n_particles]  index into the n_species x n_species tables
- *   sigma, epsilon f64 [n_species * n_species] (row-major, symmetric)
+ *   sigma, epsilon f64 [n_species * n_species] (row-major: [species of i, species of j])
  *   energy     f64 [n_systems]        out: sum_edges E_e / 2
  *   grad       f64 [n_particles, 3]   out: dE/dx (zeroed by the call)
  *   grad_tril  f64 [n_systems, 6]     out: dE/dtril at fixed Cartesian x
